@@ -972,7 +972,7 @@ def run_fxc(args):
                    "host-buffer call, copies included"},
         "e2e": {"value": round(ms, 4), "unit": "ms", "h2d_bytes_per_step": FXC_TRIALS * n * n * 8,
                 "d2h_bytes_per_step": FXC_TRIALS * n * n * 8},
-        "gpu_launches": 3 * FXC_TRIALS if prec == "mixed" else 1 + FXC_TRIALS,
+        "gpu_launches": 3 * FXC_TRIALS,
         "clocks": clk,
         "fp64_plain_ms": round(statistics.mean(t64), 4),
         "speedup_vs_fp64_plain": round(statistics.mean(t64) / ms, 3),

@@ -23,6 +23,7 @@ CUDA_UNITS = {
     "capi.cu": [],
     "vxc_fp64.cu": [],
     "vxc_mixed.cu": [],
+    "vxc_f64tc.cu": [],
     "grid_build.cu": ["-fmad=false"],
     "noalloc.cu": [],
     "mlp.cu": [],

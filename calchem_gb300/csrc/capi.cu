@@ -27,6 +27,16 @@ namespace {
 
 constexpr int kPlanes = 5;
 
+// AO cache of one form (EvalArgs::ao_cache): 0 = decide at the form's next evaluation, 1 = off
+// (disabled, over the cap or no memory), 2 = allocated
+struct AoCache {
+  int state = 0;
+  unsigned char* d = nullptr;
+  long long* d_off = nullptr;
+  int* d_ok = nullptr;
+  size_t bytes = 0;
+};
+
 struct Entry {
   int n_pts = 0, n_ao = 0, n_shells = 0, n_batches = 0, max_m = 0;
   int n_prims = 0, n_comps = 0;
@@ -86,13 +96,13 @@ struct Entry {
   double* d_fxc_m = nullptr;        // trial matrices / results of host-buffer contractions
   double* d_fxc_v = nullptr;
   int fxc_cap = 0;                  // trial matrices d_fxc_m and d_fxc_v hold
-  // AO cache of the tensor-core form (EvalArgs::ao_cache): 0 = decide at the next tensor-core
-  // evaluation, 1 = off (disabled, over the cap or no memory), 2 = allocated
-  int ao_cache_state = 0;
-  unsigned char* d_ao_cache = nullptr;
-  long long* d_ao_cache_off = nullptr;
-  int* d_ao_cache_ok = nullptr;
-  size_t ao_cache_bytes = 0;
+  // FP64 form on the tensor cores: scratch per CTA (0 CTAs: the budget or the batches' size leaves the
+  // SIMT form, launch_fp64)
+  unsigned char* d_f64_slab = nullptr;
+  size_t f64_slab_stride = 0;
+  int f64_ctas = 0;
+  AoCache ao_cache;   // of the tensor-core form (vxc_mixed.cu)
+  AoCache f64_cache;  // of the FP64 form (vxc_f64tc.cu)
   // per-atom share sums (calchem_xc_set_point_atoms): planned point indices grouped by host atom
   int n_share_atoms = 0;
   int* d_atom_pts = nullptr;
@@ -106,8 +116,8 @@ struct Entry {
     void* ptrs[] = {d_shells, d_prims, d_comps, d_prim_f, d_comp_f, d_shell_cf, d_pts,  d_batches, d_cand,  d_cand_loc, d_bao,   d_order,
                     d_P,      d_Pb,    d_V,     d_Vb,   d_rg,      d_red,   d_res,      d_counter, d_slab,
                     d_mixed_ws, d_mixed_slab, d_mol_n, d_mol_off, d_mol_ao_off, d_mol_boff, d_pt_out,
-                    d_fxc, d_fxc_m, d_fxc_v, d_ao_cache, d_ao_cache_off, d_ao_cache_ok, d_atom_pts, d_atom_off,
-                    d_atom_out};
+                    d_fxc, d_fxc_m, d_fxc_v, ao_cache.d, ao_cache.d_off, ao_cache.d_ok, f64_cache.d, f64_cache.d_off,
+                    f64_cache.d_ok, d_f64_slab, d_atom_pts, d_atom_off, d_atom_out};
     for (void* p : ptrs)
       if (p) cudaFree(p);
     if (graph) cudaGraphExecDestroy(graph);
@@ -244,6 +254,20 @@ size_t workspace_bytes(const Entry& e) {
   return t;
 }
 
+// CTAs of the FP64 form on the tensor cores (two per SM) that fit the grid's budget beside `total` bytes.
+// The SIMT form (one CTA per SM, the scratch already counted) is kept instead where a batch has more AOs
+// than the kernel holds or where so few CTAs fit that it would be no slower: one CTA of this form works
+// ~5 times as fast as one of the SIMT form (C8H18, m ~ 150), and a factor 4 is asked for.
+void plan_f64tc(Entry& e, size_t& total, size_t mem_limit) {
+  e.f64_ctas = 0;
+  if (e.max_m > f64tc_max_m() || total > mem_limit) return;
+  e.f64_slab_stride = f64tc_slab_bytes(e.max_m);
+  const int n = (int)std::min<size_t>(std::min(e.n_batches, 2 * g_sm_count), (mem_limit - total) / e.f64_slab_stride);
+  if (n < 1 || 4 * n < e.n_ctas) return;
+  e.f64_ctas = n;
+  total += e.f64_slab_stride * n;
+}
+
 // Allocates the evaluation workspace on first use.  Uploads through calchem_xc_upload_points and
 // groups defer it, so that grids uploaded only to be grouped hold no workspace.
 int ensure_ws(Entry& e) {
@@ -271,6 +295,11 @@ int ensure_ws(Entry& e) {
     e.h_stage = nullptr;
     e.stream = nullptr;
     return -4;
+  }
+  if (e.f64_ctas > 0 && cudaMalloc(&e.d_f64_slab, e.f64_slab_stride * e.f64_ctas) != cudaSuccess) {
+    cudaGetLastError();  // no room for the FP64 form's own scratch: the SIMT form runs
+    e.d_f64_slab = nullptr;
+    e.f64_ctas = 0;
   }
   e.ws = true;
   return 0;
@@ -318,7 +347,6 @@ int upload_impl(const AoShellGpu* h_shells, int n_shells, const AoPrimGpu* h_pri
   e->n_shells = n_shells;
   e->n_batches = nb;
   e->max_m = hp.max_m;
-  e->bytes = total;
   e->mem_limit = mem_limit;
   e->sum_m2n = hp.sum_m2n;
   e->sum_m2 = hp.sum_m2;
@@ -326,6 +354,8 @@ int upload_impl(const AoShellGpu* h_shells, int n_shells, const AoPrimGpu* h_pri
   e->slab_stride = slab_stride;
   e->mixed_ctas = mixed_ctas;
   e->mixed_slab_stride = mixed_stride;
+  plan_f64tc(*e, total, mem_limit);
+  e->bytes = total;
   e->n_prims = n_prims;
   e->n_comps = n_comps;
   e->n_cand = hp.cand.size();
@@ -442,24 +472,24 @@ size_t ao_cache_cap() {
   return (size_t)32 << 30;
 }
 
-void ao_cache_free(Entry& e) {
-  if (e.d_ao_cache) cudaFree(e.d_ao_cache);
-  if (e.d_ao_cache_off) cudaFree(e.d_ao_cache_off);
-  if (e.d_ao_cache_ok) cudaFree(e.d_ao_cache_ok);
-  e.d_ao_cache = nullptr;
-  e.d_ao_cache_off = nullptr;
-  e.d_ao_cache_ok = nullptr;
-  e.ao_cache_bytes = 0;
+void ao_cache_free(AoCache& c) {
+  if (c.d) cudaFree(c.d);
+  if (c.d_off) cudaFree(c.d_off);
+  if (c.d_ok) cudaFree(c.d_ok);
+  c = AoCache();
 }
 
-// Decides and allocates the AO cache on the first tensor-core evaluation (not inside a stream
+// Decides and allocates a form's AO cache on its first evaluation (not inside a stream
 // capture: callers that capture decide first).  The per-batch AO values and gradients depend only on
 // the grid and basis, so CalChem's engine computes them once per geometry and reuses them every
 // SCF iteration (vxc.rs:386-394, 600-716); here the cache also holds the packed GEMM1 operand and
-// the row exponents.  Off when the blocks exceed the cap or the free device memory (minus 1 GiB).
-void ao_cache_decide(Entry& e) {
-  if (e.ao_cache_state != 0) return;
-  e.ao_cache_state = 1;
+// the row exponents.  Off when the blocks exceed the cap or the free device memory (minus 1 GiB).  The
+// FP64 form's cache (`fp64`) also stays within a quarter of the free memory: its blocks are 56 B per AO and
+// point, and a program may hold many FP64 engines.
+void ao_cache_decide(Entry& e, bool fp64) {
+  AoCache& c = fp64 ? e.f64_cache : e.ao_cache;
+  if (c.state != 0) return;
+  c.state = 1;
   std::vector<BatchDesc> hb(e.n_batches);
   if (cudaMemcpy(hb.data(), e.d_batches, hb.size() * sizeof(BatchDesc), cudaMemcpyDeviceToHost) != cudaSuccess) {
     cudaGetLastError();
@@ -473,30 +503,44 @@ void ao_cache_decide(Entry& e) {
   // the cache's limit: the cap, the grid's budget and the free device memory less 1 GiB; batches (in
   // batch order) whose blocks fit within it get one (offset -1: evaluated every time)
   const size_t reserve = (size_t)1 << 30;
-  const size_t budget = e.mem_limit > e.bytes ? e.mem_limit - e.bytes : 0;  // within the grid's budget
-  const size_t limit = std::min({ao_cache_cap(), budget, free_b > reserve ? free_b - reserve : (size_t)0});
+  const size_t used = e.bytes + e.ao_cache.bytes + e.f64_cache.bytes;
+  const size_t budget = e.mem_limit > used ? e.mem_limit - used : 0;  // within the grid's budget
+  size_t limit = std::min({ao_cache_cap(), budget, free_b > reserve ? free_b - reserve : (size_t)0});
+  if (fp64) limit = std::min(limit, free_b / 4);
   std::vector<long long> off(e.n_batches, -1);
   size_t total = 0;
   for (int b = 0; b < e.n_batches; ++b) {
-    const size_t bb = ao_cache_block_bytes(hb[b].m);
+    const size_t bb = fp64 ? f64tc_cache_block_bytes(hb[b].m) : ao_cache_block_bytes(hb[b].m);
     if (total + bb > limit) continue;
     off[b] = (long long)total;
     total += bb;
   }
   if (total == 0) return;
-  const bool ok = cudaMalloc(&e.d_ao_cache, total) == cudaSuccess &&
-                  cudaMalloc(&e.d_ao_cache_off, off.size() * sizeof(long long)) == cudaSuccess &&
-                  cudaMalloc(&e.d_ao_cache_ok, (size_t)e.n_batches * sizeof(int)) == cudaSuccess &&
-                  cudaMemcpy(e.d_ao_cache_off, off.data(), off.size() * sizeof(long long), cudaMemcpyHostToDevice) ==
+  const bool ok = cudaMalloc(&c.d, total) == cudaSuccess &&
+                  cudaMalloc(&c.d_off, off.size() * sizeof(long long)) == cudaSuccess &&
+                  cudaMalloc(&c.d_ok, (size_t)e.n_batches * sizeof(int)) == cudaSuccess &&
+                  cudaMemcpy(c.d_off, off.data(), off.size() * sizeof(long long), cudaMemcpyHostToDevice) ==
                       cudaSuccess &&
-                  cudaMemset(e.d_ao_cache_ok, 0, (size_t)e.n_batches * sizeof(int)) == cudaSuccess;
+                  cudaMemset(c.d_ok, 0, (size_t)e.n_batches * sizeof(int)) == cudaSuccess;
   if (!ok) {
     cudaGetLastError();
-    ao_cache_free(e);
+    ao_cache_free(c);
+    c.state = 1;
     return;
   }
-  e.ao_cache_bytes = total;
-  e.ao_cache_state = 2;
+  c.bytes = total;
+  c.state = 2;
+}
+
+// A form's AO cache for a launch on st: decided now unless st is being captured.
+void use_ao_cache(Entry& e, bool fp64, cudaStream_t st, EvalArgs& A) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) ao_cache_decide(e, fp64);
+  const AoCache& c = fp64 ? e.f64_cache : e.ao_cache;
+  if (c.state != 2) return;
+  A.ao_cache = c.d;
+  A.ao_cache_off = c.d_off;
+  A.ao_cache_ok = c.d_ok;
 }
 
 // Tensor-core CTAs to launch for the grid's tile (never more than the workspace has slabs for).
@@ -504,11 +548,33 @@ int mixed_launch_ctas(const Entry& e) {
   return std::max(1, std::min(e.mixed_ctas, g_sm_count * mixed_ctas_per_sm(e.tile_n)));
 }
 
+// Fixed-point copies of the densities for the FP64 form: [alpha n^2][beta n^2] of 8 bytes, then the rows'
+// exponents [alpha n][beta n] (the layout of the tensor-core form's split densities).
+bool f64tc_prepare(Entry& e, const double* Pa, const double* Pb, cudaStream_t st, int* launches) {
+  const size_t nn = (size_t)e.nn_total;
+  unsigned long long* y = reinterpret_cast<unsigned long long*>(e.d_mixed_ws);
+  int* fx = reinterpret_cast<int*>(y + 2 * nn);
+  for (int s = 0; s < (Pb ? 2 : 1); ++s) {
+    if (launch_f64tc_prepare(s ? Pb : Pa, e.n_ao, e.d_mol_n, e.d_mol_off, e.d_mol_ao_off, e.n_mols, y + s * nn,
+                             fx + s * (size_t)e.n_ao, st) != cudaSuccess)
+      return false;
+    ++*launches;
+  }
+  return true;
+}
+
+void f64tc_args(Entry& e, cudaStream_t st, EvalArgs& A) {
+  A.Pa = reinterpret_cast<const double*>(e.d_mixed_ws);
+  A.slab = reinterpret_cast<double*>(e.d_f64_slab);
+  A.slab_stride = e.f64_slab_stride / sizeof(double);
+  use_ao_cache(e, true, st, A);
+}
+
 // shares_only (closed shell, with point_out): the per-point shares, Exc and Nelec without the Vxc
-// contraction; Va is not touched.
+// contraction; Va is not touched.  simt: the FP64 SIMT form (launch_fp64) in any case.
 int enqueue_eval(Entry& e, int mode, int xc, int precision, const double* Pa, const double* Pb, double* Va,
                  double* Vb, const double* wv, double* rho_out, double* result, cudaStream_t st,
-                 double* point_out = nullptr, bool shares_only = false) {
+                 double* point_out = nullptr, bool shares_only = false, bool simt = false) {
   const size_t nn = (size_t)e.nn_total;
   int launches = 0;
   if (mode != kModeRho && !shares_only) {
@@ -533,6 +599,7 @@ int enqueue_eval(Entry& e, int mode, int xc, int precision, const double* Pa, co
   const DevGrid G = dev_grid(e);
   cudaError_t err;
   const bool prof = e.profiling && e.ev0 && e.ev1;
+  const bool f64tc = precision == CALCHEM_XC_FP64 && e.f64_ctas > 0 && !simt;
   if (precision == CALCHEM_XC_MIXED) {
     // packed fixed-point densities: [alpha n^2][beta n^2] uint2, then row exponents [alpha n][beta n]
     uint2* pk = reinterpret_cast<uint2*>(e.d_mixed_ws);
@@ -550,16 +617,16 @@ int enqueue_eval(Entry& e, int mode, int xc, int precision, const double* Pa, co
     A.slab = e.d_mixed_slab;
     A.slab_stride = e.mixed_slab_stride;
     A.Pa = (const double*)e.d_mixed_ws;  // the tensor-core kernel reads the split copies
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) ao_cache_decide(e);
-    if (e.ao_cache_state == 2) {
-      A.ao_cache = e.d_ao_cache;
-      A.ao_cache_off = e.d_ao_cache_off;
-      A.ao_cache_ok = e.d_ao_cache_ok;
-    }
+    use_ao_cache(e, false, st, A);
     A.tile_n = e.tile_n;
     if (prof) cudaEventRecord(e.ev0, st);
     err = launch_mixed(G, A, mixed_launch_ctas(e), st);
+    if (prof) cudaEventRecord(e.ev1, st);
+  } else if (f64tc) {
+    if (mode != kModeAccum && !f64tc_prepare(e, Pa, mode == kModeUks ? Pb : nullptr, st, &launches)) return -5;
+    f64tc_args(e, st, A);
+    if (prof) cudaEventRecord(e.ev0, st);
+    err = launch_f64tc(G, A, e.f64_ctas, st);
     if (prof) cudaEventRecord(e.ev1, st);
   } else {
     A.slab = e.d_slab;
@@ -574,16 +641,18 @@ int enqueue_eval(Entry& e, int mode, int xc, int precision, const double* Pa, co
     if (launch_reduce(e.d_red, e.n_batches, e.d_mol_boff, e.n_mols, result, mode == kModeRks ? 2 : 3, st) !=
         cudaSuccess)
       return -5;
-    const int from_upper = precision == CALCHEM_XC_MIXED ? 1 : 0;
     ++launches;
-    if (!shares_only) {
-      if (launch_mirror(Va, e.max_n, e.d_mol_n, e.d_mol_off, e.n_mols, from_upper, st) != cudaSuccess) return -5;
+    auto complete = [&](double* V) {
       ++launches;
-    }
-    if (mode == kModeUks) {
-      if (launch_mirror(Vb, e.max_n, e.d_mol_n, e.d_mol_off, e.n_mols, from_upper, st) != cudaSuccess) return -5;
-      ++launches;
-    }
+      return f64tc ? launch_symmetrise(V, e.max_n, e.d_mol_n, e.d_mol_off, e.n_mols, 0, st)
+                   : launch_mirror(V, e.max_n, e.d_mol_n, e.d_mol_off, e.n_mols,
+                                   precision == CALCHEM_XC_MIXED ? 1 : 0, st);
+    };
+    if (!shares_only && complete(Va) != cudaSuccess) return -5;
+    if (mode == kModeUks && complete(Vb) != cudaSuccess) return -5;
+  } else if (mode == kModeAccum && f64tc) {
+    if (launch_symmetrise(Va, e.max_n, e.d_mol_n, e.d_mol_off, e.n_mols, 1, st) != cudaSuccess) return -5;
+    ++launches;
   }
   e.last_launches = launches;
   return 0;
@@ -595,6 +664,29 @@ int enqueue_fxc(Entry& e, int triplet, const double* d_m, int n_trials, double* 
   if (cudaMemsetAsync(d_v, 0, nn * n_trials * sizeof(double), st) != cudaSuccess ||
       cudaMemsetAsync(e.d_counter, 0, 4 * sizeof(int), st) != cudaSuccess)
     return -5;
+  if (e.f64_ctas > 0) {  // one launch per trial matrix; the AO cache, filled by the first, serves them all
+    int launches = 0;
+    for (int t = 0; t < n_trials; ++t) {
+      // the queue head only: the status word keeps an earlier trial's failure
+      if (t > 0 && cudaMemsetAsync(e.d_counter, 0, sizeof(int), st) != cudaSuccess) return -5;
+      EvalArgs A{};
+      A.mode = kModeFxc;
+      A.Va = d_v + t * nn;
+      A.fxc_coef = e.d_fxc;
+      A.triplet = triplet ? 1 : 0;
+      A.batch_red = e.d_red;
+      A.counter = e.d_counter;
+      A.max_m = e.max_m;
+      if (!f64tc_prepare(e, d_m + t * nn, nullptr, st, &launches)) return -5;
+      f64tc_args(e, st, A);
+      if (launch_f64tc(dev_grid(e), A, e.f64_ctas, st) != cudaSuccess ||
+          launch_symmetrise(A.Va, e.n_ao, nullptr, nullptr, 1, 0, st) != cudaSuccess)
+        return -5;
+      launches += 2;
+    }
+    e.last_launches = launches;
+    return 0;
+  }
   EvalArgs A{};
   A.mode = kModeFxc;
   A.xc = e.fxc_code;
@@ -621,8 +713,6 @@ int enqueue_fxc(Entry& e, int triplet, const double* d_m, int n_trials, double* 
 int enqueue_fxc_mixed(Entry& e, int triplet, const double* d_m, int n_trials, double* d_v, cudaStream_t st) {
   const size_t nn = (size_t)e.n_ao * e.n_ao;
   if (mixed_set_attributes() != cudaSuccess) return -5;
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) ao_cache_decide(e);
   uint2* pk = reinterpret_cast<uint2*>(e.d_mixed_ws);
   int* fx = reinterpret_cast<int*>(pk + 2 * nn);
   const DevGrid G = dev_grid(e);
@@ -645,17 +735,22 @@ int enqueue_fxc_mixed(Entry& e, int triplet, const double* d_m, int n_trials, do
     A.max_m = e.max_m;
     A.slab = e.d_mixed_slab;
     A.slab_stride = e.mixed_slab_stride;
-    if (e.ao_cache_state == 2) {
-      A.ao_cache = e.d_ao_cache;
-      A.ao_cache_off = e.d_ao_cache_off;
-      A.ao_cache_ok = e.d_ao_cache_ok;
-    }
+    use_ao_cache(e, false, st, A);
     A.tile_n = e.tile_n;
     if (launch_mixed(G, A, mixed_launch_ctas(e), st) != cudaSuccess) return -5;
     if (launch_mirror(v, e.n_ao, 1, st) != cudaSuccess) return -5;
   }
   e.last_launches = 3 * n_trials;
   return 0;
+}
+
+// Waits for the grid's stream; -7 when a device-side wait of the last evaluation gave up.
+int finish(Entry& e) {
+  int* h_status = reinterpret_cast<int*>(e.h_stage + 2 * (size_t)e.nn_total + 3 * (size_t)e.n_mols + 1);
+  if (cudaMemcpyAsync(h_status, e.d_counter + 2, sizeof(int), cudaMemcpyDeviceToHost, e.stream) != cudaSuccess ||
+      cudaStreamSynchronize(e.stream) != cudaSuccess)
+    return -5;
+  return *h_status != 0 ? -7 : 0;
 }
 
 bool valid_xc(int xc) { return xc >= 0 && xc <= 8; }
@@ -962,10 +1057,9 @@ int calchem_cuda_vxc_eval_rho(uint64_t grid_id, const double* h_p_mat, double* h
                         nullptr, e->stream);
   if (rc) return rc;
   if (cudaMemcpyAsync(h_rho_grad_out, e->d_rg, (size_t)n_pts * 4 * sizeof(double), cudaMemcpyDeviceToHost,
-                      e->stream) != cudaSuccess ||
-      cudaStreamSynchronize(e->stream) != cudaSuccess)
+                      e->stream) != cudaSuccess)
     return -5;
-  return 0;
+  return finish(*e);
 }
 
 int calchem_cuda_vxc_accum(uint64_t grid_id, const double* h_wv_in, double* h_vxc_out, int n_pts, int n_ao) {
@@ -982,9 +1076,9 @@ int calchem_cuda_vxc_accum(uint64_t grid_id, const double* h_wv_in, double* h_vx
   int rc = enqueue_eval(*e, kModeAccum, 0, CALCHEM_XC_FP64, nullptr, nullptr, e->d_V, nullptr, e->d_rg, nullptr,
                         nullptr, e->stream);
   if (rc) return rc;
-  if (cudaMemcpyAsync(e->h_stage, e->d_V, nn * sizeof(double), cudaMemcpyDeviceToHost, e->stream) != cudaSuccess ||
-      cudaStreamSynchronize(e->stream) != cudaSuccess)
+  if (cudaMemcpyAsync(e->h_stage, e->d_V, nn * sizeof(double), cudaMemcpyDeviceToHost, e->stream) != cudaSuccess)
     return -5;
+  if ((rc = finish(*e))) return rc;
   std::memcpy(h_vxc_out, e->h_stage, nn * sizeof(double));
   return 0;
 }
@@ -1217,13 +1311,13 @@ int calchem_xc_set_ao_cache(uint64_t grid_id, int enable, size_t* bytes_out) {
   Entry* e = find(grid_id);
   if (!e) return -2;
   if (enable < 0) {  // query only
-    if (bytes_out) *bytes_out = e->ao_cache_bytes;
+    if (bytes_out) *bytes_out = e->ao_cache.bytes;
     return 0;
   }
   if (bytes_out) *bytes_out = 0;
   const int want = enable ? 0 : 1;  // 0: allowed (decided at the next evaluation), 1: off
-  if (enable && e->ao_cache_state != 1) {  // already allowed
-    if (bytes_out) *bytes_out = e->ao_cache_bytes;
+  if (enable && e->ao_cache.state != 1 && e->f64_cache.state != 1) {  // already allowed
+    if (bytes_out) *bytes_out = e->ao_cache.bytes;
     return 0;
   }
   // evaluations in flight on any stream may still read the cache
@@ -1232,8 +1326,10 @@ int calchem_xc_set_ao_cache(uint64_t grid_id, int enable, size_t* bytes_out) {
     cudaGraphExecDestroy(e->graph);
     e->graph = nullptr;
   }
-  ao_cache_free(*e);
-  e->ao_cache_state = want;
+  for (AoCache* c : {&e->ao_cache, &e->f64_cache}) {
+    ao_cache_free(*c);
+    c->state = want;
+  }
   return 0;
 }
 
@@ -1555,13 +1651,16 @@ int calchem_xc_fxc_prepare(uint64_t grid_id, int xc_code, const double* h_d_tota
   std::memcpy(e->h_stage, h_d_total, nn * sizeof(double));
   if (cudaMemcpyAsync(e->d_P, e->h_stage, nn * sizeof(double), cudaMemcpyHostToDevice, e->stream) != cudaSuccess)
     return -5;
+  // The SIMT form's densities: once per ground state, so its speed matters little, while the kernel's finite
+  // differences turn another form's roundings of rho (1e-16) into 5e-12 of dV, and into 4e-9 where the
+  // tensor-core contraction rounds the coefficients to FP32.
   int rc = enqueue_eval(*e, kModeRho, 0, CALCHEM_XC_FP64, e->d_P, nullptr, nullptr, nullptr, nullptr, e->d_rg,
-                        nullptr, e->stream);
+                        nullptr, e->stream, nullptr, false, true);
   if (rc) return rc;
   if (launch_fxc_coef(e->d_rg, e->d_pts + 3 * (size_t)e->n_pts, e->n_pts, xc_code, e->d_fxc, e->stream) !=
-          cudaSuccess ||
-      cudaStreamSynchronize(e->stream) != cudaSuccess)
+      cudaSuccess)
     return -5;
+  if ((rc = finish(*e))) return rc;
   e->fxc_code = xc_code;
   return 0;
 }
@@ -1724,12 +1823,13 @@ int calchem_xc_group_create(const uint64_t* member_ids, int n_members, uint64_t 
                  (size_t)n_pts * 4 * sizeof(double) + (size_t)n_b * (sizeof(BatchDesc) + sizeof(int)) +
                  (size_t)n_cand * 2 * sizeof(int) + (size_t)n_bao * sizeof(int) + (size_t)n_members * 32;
   total += workspace_bytes(*g);
-  g->bytes = total;
   g->mem_limit = memory_limit_bytes;
   if (total > memory_limit_bytes) {
     delete g;
     return -3;
   }
+  plan_f64tc(*g, total, memory_limit_bytes);
+  g->bytes = total;
   auto fail = [&](int code) {
     cudaGetLastError();
     g->free_all();
@@ -1837,8 +1937,10 @@ int calchem_xc_graph_capture(uint64_t grid_id, int mode, int xc_code, int precis
   if (!e->has_w) return -1;
   if (int rc0 = ensure_ws(*e)) return rc0;
   // kernel attributes are set, and the AO cache decided, outside the capture
-  if (fp64_set_attributes() != cudaSuccess || mixed_set_attributes() != cudaSuccess) return -5;
-  if (precision == CALCHEM_XC_MIXED) ao_cache_decide(*e);
+  if (fp64_set_attributes() != cudaSuccess || mixed_set_attributes() != cudaSuccess ||
+      f64tc_set_attributes() != cudaSuccess)
+    return -5;
+  if (precision == CALCHEM_XC_MIXED || e->f64_ctas > 0) ao_cache_decide(*e, precision != CALCHEM_XC_MIXED);
   if (e->graph) {
     cudaGraphExecDestroy(e->graph);
     e->graph = nullptr;

@@ -21,6 +21,18 @@ cudaError_t launch_mirror(double* V, int n, int from_upper, cudaStream_t st);
 // Per-atom (Exc, tr(D Vxc)) shares: out[2 a ..] = sums of point_out over atom a's points.
 cudaError_t launch_atom_shares(const double* point_out, const int* atom_pts, const int* atom_off, int n_atoms,
                                double* out, cudaStream_t st);
+// FP64 form with its contractions on the tensor cores (vxc_f64tc.cu): A.Pa points at the fixed-point
+// densities of launch_f64tc_prepare (alpha, then beta, then the rows' exponents); V is accumulated as the
+// full square and completed by launch_symmetrise.
+int f64tc_max_m();
+size_t f64tc_slab_bytes(int max_m);
+size_t f64tc_cache_block_bytes(int m);
+cudaError_t f64tc_set_attributes();
+cudaError_t launch_f64tc(const DevGrid& G, const EvalArgs& A, int n_ctas, cudaStream_t st);
+cudaError_t launch_f64tc_prepare(const double* P, int n_total, const int* mol_n, const long long* mol_off,
+                                 const int* mol_ao_off, int n_mols, void* out, int* fexp, cudaStream_t st);
+cudaError_t launch_symmetrise(double* V, int max_n, const int* mol_n, const long long* mol_off, int n_mols,
+                              int lower_only, cudaStream_t st);
 // Tensor-core form (vxc_mixed.cu)
 int mixed_supported(int mode);
 size_t mixed_slab_doubles(int max_m);

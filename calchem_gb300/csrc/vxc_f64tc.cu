@@ -1,0 +1,680 @@
+// vxc_f64tc.cu -- the FP64 XC quadrature with its contractions on the tensor cores (tcgen05).
+//
+// Same phases, screening and FP64 arithmetic as vxc_fp64.cu; the two contractions of a batch of m AOs
+// and 128 points, T = P_sub Phi and W = Z Phi^T, run as exact integer-slice products (f64_slices.cuh)
+// instead of FP64 FMAs.  Each operand vector (an AO row of P, a point's or an AO's row of Phi, an AO's
+// row of Z) is cut into six 9-bit BF16 slices relative to its largest element; the 21 slice products
+// i + j <= 5 go into five FP32 accumulators in TMEM (levels 0-3 exact over 64 terms, levels 4 and 5
+// together), which are drained every 64 terms into 64-bit integers.  The products left out and the
+// operands' rounding are below 2^-54 of the row maxima's product per term, as the roundings of an FP64
+// FMA chain are; rho, the functional, Z and all sums stay in FP64.
+//
+// What bounds it: GB300 has 2 FP64 FMA lanes per SM and clock, so the SIMT form spends 4 m^2 FP64 FMAs a
+// point there; here the tensor cores take them and the FP64 pipe is left with ~m (4 for rho and
+// grad rho, 4 for Z, 2 for the conversion of T) FMAs a point and the functional.  Two CTAs of 256
+// threads share an SM (240 TMEM columns and ~103 KB of shared memory each), so that one CTA's FP64
+// phases run under the other's copies and MMAs.  N = 48 columns is what five accumulators leave of
+// 256 TMEM columns.
+//
+// Measured against the SIMT form (whole host calls, FP64): C8H18 B3LYP Fine 32.9 -> 2.73 ms, 24 waters
+// B3LYP Medium 30.9 -> 2.47 ms, C6H14 PBE open shell 7.34 -> 0.83 ms, one water 0.63 -> 0.16 ms; the
+// relative error of V against a plain FP64 evaluation is the same (2.6e-15 on C8H18, 2.7e-15 before).
+//
+// AO values, their packed slices and exponents depend on the grid and basis only: batches with a block
+// in the grid's AO cache compute them in the first launch that reaches them and read them afterwards,
+// as the tensor-core form of vxc_mixed.cu does.
+//
+// V is accumulated as the full square sum_b Z Phi^T (transposed, so that a warp's lanes add to
+// neighbouring elements) and symmetrised by a last kernel: half the MMAs of Z Phi^T + Phi Z^T on one
+// triangle.  Every mbarrier wait is bounded; one that expires sets the status word, waits (bounded) for
+// the CTA's own MMAs and copies, frees TMEM and returns.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "common.cuh"
+#include "f64_slices.cuh"
+#include "fp64_ao.cuh"
+#include "mixed_ops.cuh"
+#include "tc_ptx.cuh"
+#include "xc_device.cuh"
+
+namespace cxc {
+
+namespace {
+
+using mix::st_shared_v4;
+using mix::sw128;
+using namespace f64s;
+
+constexpr int kT = 256;                       // threads per CTA, two CTAs per SM
+constexpr int kN = 48;                        // AO columns per accumulator
+constexpr int kCols = kN / 2;                 // columns per thread (two thread groups of 128)
+constexpr int kLevels = 5;
+constexpr uint32_t kTmem = 256;
+constexpr int kTiles = kSlices / 2;           // 128-byte rows hold two slices of 32 K values
+constexpr int kABytes = kTiles * 128 * 128;   // one K block (32) of a 128-row operand
+constexpr int kBTile = kN * 128;
+constexpr int kBBytes = kTiles * kBTile;
+constexpr int kMaxM = 2048;
+constexpr uint32_t kSpin = 1u << 26;
+
+constexpr int kOffCoef = kABytes + kBBytes;         // double [8][128]
+constexpr int kOffAo = kOffCoef + 8 * 128 * 8;      // int [kMaxM]: global AO of each local row
+constexpr int kOffEz = kOffAo + kMaxM * 4;          // int [kMaxM]: biased exponents of the Z rows
+constexpr int kOffEp = kOffEz + kMaxM * 4;          // int [kMaxM]: of the Phi rows
+constexpr int kOffEg = kOffEp + kMaxM * 4;          // int [128]: of the points
+constexpr int kOffEf = kOffEg + 128 * 4;            // int [2][64]: of the chunk's density rows
+constexpr int kOffRed = kOffEf + 128 * 4;           // double [3][kT / 32]
+constexpr int kOffMisc = kOffRed + 3 * (kT / 32) * 8;
+constexpr int kSmem = kOffMisc + 64 + 1024;
+static_assert(2 * (kSmem + 1024) <= 233472, "two CTAs share one SM's shared memory");
+static_assert(kLevels * kN <= (int)kTmem, "the accumulators fit the CTA's TMEM columns");
+static_assert(8 * 128 * 8 <= kABytes, "the density sums live in the idle operand stage");
+constexpr int kENan = 1980;  // row exponents from here on (2^957 and above, infinities, NaN) give NaN
+
+__host__ __device__ constexpr size_t up(size_t x, size_t k) { return (x + k - 1) / k * k; }
+
+// A batch's block: FP64 planes [4][m_k][128], the GEMM1 operand (m_k / 32 K blocks of 48 KB), the Phi
+// image (four 32-point K blocks of three tiles [m_r][128 B]), the Phi rows' exponents, the points'.
+struct Block {
+  size_t plane, apack, img, ep, eg, bytes;
+  int m_r;
+  __host__ __device__ explicit Block(int m) {
+    const size_t m_k = up(m, 32);
+    m_r = (int)up(m, kN);
+    plane = m_k * 128;
+    apack = 4 * plane * 8;
+    img = apack + m_k / 32 * kABytes;
+    ep = img + (size_t)12 * m_r * 128;
+    eg = ep + up(4 * (size_t)m, 16);
+    bytes = up(eg + 512, 1024);
+  }
+};
+
+__host__ __device__ constexpr size_t z_bytes(int m) { return 12 * up(m, 128) * 128; }
+
+// Byte offset of slice s (even element pair words) for chunk c (8 K values) of row r in a K block's tiles.
+__device__ __forceinline__ uint32_t slice_off(int s, int r, int c) { return sw128(r, (s & 1) * 4 + c); }
+
+// Slices of 8 consecutive K values (Y[8]) stored as six 16-byte chunks: tile s >> 1 at base + (s >> 1) * tile.
+template <typename Store>
+__device__ __forceinline__ void store8(const unsigned long long (&Y)[8], int r, int c, Store&& store) {
+  uint32_t w[4][kSlices];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) slice_pairs(Y[2 * k], Y[2 * k + 1], w[k]);
+#pragma unroll
+  for (int s = 0; s < kSlices; ++s) store(s >> 1, slice_off(s, r, c), make_uint4(w[0][s], w[1][s], w[2][s], w[3][s]));
+}
+
+// The GEMM1 A operand: Phi[g][mu] for 128 points, K = AOs, relative to each point's exponent.
+__device__ void pack_points(unsigned char* __restrict__ apack, const double* __restrict__ phi, const int* s_eg, int m,
+                            int m_k) {
+  for (int e = threadIdx.x; e < m_k / 8 * 128; e += kT) {
+    const int g = e & 127, c8 = e >> 7;
+    const int E = s_eg[g];
+    unsigned long long Y[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int mu = 8 * c8 + k;
+      Y[k] = mu < m ? to_fixed(phi[(size_t)mu * 128 + g], E) : kBias;
+    }
+    unsigned char* t = apack + (size_t)(c8 >> 2) * kABytes;
+    store8(Y, g, c8 & 3, [&](int tile, uint32_t off, uint4 v) {
+      *reinterpret_cast<uint4*>(t + tile * 16384 + off) = v;
+    });
+  }
+}
+
+// One AO row over the batch's points into an image [4 K blocks][3 tiles][m_r rows][128 B], by one warp:
+// lane l holds points 4 l .. 4 l + 3.  Returns the row's exponent.
+__device__ __forceinline__ int pack_row(unsigned char* __restrict__ img, int m_r, int row, const double (&x)[4]) {
+  const int lane = threadIdx.x & 31;
+  uint32_t mx = 0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) mx = max(mx, (uint32_t)__double2hiint(x[k]) & 0x7FFFFFFFu);
+  mx = __reduce_max_sync(0xFFFFFFFFu, mx);
+  const int E = (int)(mx >> 20);
+  unsigned long long Y[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) Y[k] = to_fixed(x[k], E);
+  uint32_t w0[kSlices], w1[kSlices];
+  slice_pairs(Y[0], Y[1], w0);
+  slice_pairs(Y[2], Y[3], w1);
+  unsigned char* t = img + (size_t)(lane >> 3) * 3 * m_r * 128 + (lane & 1) * 8;
+#pragma unroll
+  for (int s = 0; s < kSlices; ++s)
+    *reinterpret_cast<uint2*>(t + (size_t)(s >> 1) * m_r * 128 + (size_t)(row & ~7) * 128 +
+                              slice_off(s, row & 7, (lane & 7) >> 1)) = make_uint2(w0[s], w1[s]);
+  return E;
+}
+
+__device__ __forceinline__ void load4(const double* p, double (&x)[4]) {
+  const double2 a = *reinterpret_cast<const double2*>(p), b = *reinterpret_cast<const double2*>(p + 2);
+  x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
+}
+
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr));
+}
+
+__global__ void __launch_bounds__(kT, 2) vxc_f64tc_kernel(DevGrid G, EvalArgs A) {
+  extern __shared__ unsigned char smem_raw[];
+  unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  unsigned char* stage = base;
+  double(*coef)[128] = reinterpret_cast<double(*)[128]>(base + kOffCoef);
+  double(*dens)[4][128] = reinterpret_cast<double(*)[4][128]>(base);  // [2], the stage idle
+  int* s_ao = reinterpret_cast<int*>(base + kOffAo);
+  int* s_ez = reinterpret_cast<int*>(base + kOffEz);
+  int* s_ep = reinterpret_cast<int*>(base + kOffEp);
+  int* s_eg = reinterpret_cast<int*>(base + kOffEg);
+  int* s_ef = reinterpret_cast<int*>(base + kOffEf);
+  double(*red)[kT / 32] = reinterpret_cast<double(*)[kT / 32]>(base + kOffRed);
+  uint64_t* mbar = reinterpret_cast<uint64_t*>(base + kOffMisc);      // MMA commits
+  uint64_t* tbar = reinterpret_cast<uint64_t*>(base + kOffMisc + 8);  // operand bulk copies
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(base + kOffMisc + 16);
+  int* s_batch = reinterpret_cast<int*>(base + kOffMisc + 20);
+
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int g = tid & 127, h = tid >> 7;
+  const bool uks = A.mode == kModeUks;
+
+  if (tid == 0) {
+    mbar_init(mbar, 1);
+    mbar_init(tbar, 1);
+    fence_mbar_init();
+  }
+  if (warp == 0) {
+    tmem_alloc(tmem_slot, kTmem);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+  const uint32_t tl = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(h * kCols);  // this thread's columns
+  const uint32_t sb = smem_addr(stage);
+  const uint32_t idesc = idesc_bf16_f32(128, kN);
+  uint32_t phase = 0, tphase = 0;
+  bool tma_busy = false, failed = false;
+
+  unsigned char* const slab = reinterpret_cast<unsigned char*>(A.slab + (size_t)blockIdx.x * A.slab_stride);
+  unsigned char* const zimg = slab;  // the Z image, then the block of a batch without a cache block
+  const unsigned long long* const Y0 = reinterpret_cast<const unsigned long long*>(A.Pa);
+  const int* const f0 = reinterpret_cast<const int*>(Y0 + 2 * G.nn_total);
+  const uint64_t pol_keep = l2_policy_evict_last();
+
+  auto wait_mma = [&]() -> bool {
+    const bool ok = mbar_wait_bounded(mbar, phase, kSpin);
+    phase ^= 1u;
+    tc_fence_after();
+    return __syncthreads_or(!ok) == 0;
+  };
+  auto wait_tma = [&]() -> bool {
+    const bool ok = mbar_wait_bounded(tbar, tphase, kSpin);
+    if (ok) {
+      tphase ^= 1u;
+      tma_busy = false;
+    }
+    return __syncthreads_or(!ok) == 0;
+  };
+  // one K block of 32: slice products i + j <= 5, level min(i + j, 4) into accumulator columns 48 level
+  auto mma_block = [&](bool first) {
+    tc_fence_after();
+    uint64_t a[kTiles], b[kTiles];
+#pragma unroll
+    for (int t = 0; t < kTiles; ++t) {
+      a[t] = sdesc_sw128(sb + t * 16384);
+      b[t] = sdesc_sw128(sb + kABytes + t * kBTile);
+    }
+#pragma unroll
+    for (int ks = 0; ks < 2; ++ks)
+#pragma unroll
+      for (int i = 0; i < kSlices; ++i)
+#pragma unroll
+        for (int j = 0; i + j < kSlices; ++j) {
+          const int lev = i + j < kLevels ? i + j : kLevels - 1;
+          // each level's first product (i = 0, levels 0..4) overwrites at the start of a K group
+          const uint32_t acc = (first && ks == 0 && i == 0 && j < kLevels) ? 0u : 1u;
+          mma_bf16_ss(tmem + lev * kN, a[i >> 1] + (i & 1) * 4 + ks * 2, b[j >> 1] + (j & 1) * 4 + ks * 2, idesc, acc);
+        }
+    mma_commit(mbar);
+  };
+  // the accumulators' K group into the thread's 64-bit sums
+  auto drain = [&](long long (&V)[kCols], int sh) {
+#pragma unroll
+    for (int c = 0; c < kCols; c += 8) {
+      uint32_t r[kLevels][8];
+#pragma unroll
+      for (int l = 0; l < kLevels; ++l) tmem_ld8(tl + l * kN + c, r[l]);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+      for (int l = 0; l < kLevels; ++l)  // the loads' results are read after the wait
+#pragma unroll
+        for (int k = 0; k < 8; ++k) asm volatile("" : "+r"(r[l][k]));
+#pragma unroll
+      for (int k = 0; k < 8; ++k)
+        V[c + k] += level_sum(__uint_as_float(r[0][k]), __uint_as_float(r[1][k]), __uint_as_float(r[2][k]),
+                              __uint_as_float(r[3][k]), __uint_as_float(r[4][k])) >> sh;
+    }
+    tc_fence_before();
+  };
+
+  while (!failed) {
+    if (tid == 0) *s_batch = atomicAdd(A.counter, 1);
+    __syncthreads();
+    const int q = *s_batch;
+    __syncthreads();
+    if (q >= G.n_batches) break;
+    const int b = G.order[q];
+    const BatchDesc bd = G.batches[b];
+    const int m = bd.m, m_k = (m + 31) / 32 * 32, nkb = m_k / 32;
+    const int n = mol_nao(G, bd.mol);
+    const long long moff = mol_mat(G, bd.mol);
+    const int roff = mol_row(G, bd.mol);
+    const Block L(m);
+    const int m_z = (m + 127) / 128 * 128;
+    for (int i = tid; i < m; i += kT) s_ao[i] = G.batch_ao[bd.ao_start + i];
+    long long off = -1;
+    if (A.ao_cache) off = A.ao_cache_off[b];
+    unsigned char* const blk = off >= 0 ? A.ao_cache + off : slab + z_bytes(A.max_m);
+    double* const phi = reinterpret_cast<double*>(blk);
+    // only this CTA writes the flag, at the end of the fill below
+    const bool cached = off >= 0 && *reinterpret_cast<volatile int*>(A.ao_cache_ok + b) != 0;
+    int* const blk_ep = reinterpret_cast<int*>(blk + L.ep);
+    int* const blk_eg = reinterpret_cast<int*>(blk + L.eg);
+    __syncthreads();
+    if (cached) {
+      if (h == 0) s_eg[g] = blk_eg[g];
+      for (int i = tid; i < m; i += kT) s_ep[i] = blk_ep[i];
+      __syncthreads();
+    } else {
+      const uint32_t vmax = eval_batch_aos<kT>(G, bd, phi, L.plane);
+      uint32_t* sc = reinterpret_cast<uint32_t*>(stage);
+      sc[tid] = vmax;
+      __syncthreads();
+      if (h == 0) {
+        const int E = (int)(max(sc[g], sc[128 + g]) >> 20);
+        s_eg[g] = E;
+        blk_eg[g] = E;
+      }
+      __syncthreads();
+      pack_points(blk + L.apack, phi, s_eg, m, m_k);
+      for (int row = warp; row < m; row += kT / 32) {
+        double x[4];
+        load4(phi + (size_t)row * 128 + 4 * lane, x);
+        const int E = pack_row(blk + L.img, L.m_r, row, x);
+        if (lane == 0) s_ep[row] = blk_ep[row] = E;
+      }
+      fence_proxy_async_global();  // the packed operands are read by bulk copies, the stage written by them
+      fence_proxy_async_smem();
+      __syncthreads();
+      if (off >= 0 && tid == 0) {
+        __threadfence();
+        A.ao_cache_ok[b] = 1;  // read by later launches only
+      }
+    }
+
+    const int sh = m > 1024 ? 1 : 0;
+    double rho[2] = {0, 0}, gx[2] = {0, 0}, gy[2] = {0, 0}, gz[2] = {0, 0};
+    for (int s = 0; s < (A.mode == kModeAccum ? 0 : uks ? 2 : 1) && !failed; ++s) {
+      const unsigned long long* Yp = Y0 + (s ? G.nn_total : 0) + moff;
+      const int* fp = f0 + (s ? G.n_total : 0) + roff;
+      double sr = 0, sx = 0, sy = 0, sz = 0;
+      for (int nc = 0; nc < m && !failed; nc += kN) {
+        // (double-buffered: slower threads may still read the previous chunk's)
+        int* const ef = s_ef + (nc / kN & 1) * 64;
+        if (tid < kN) ef[tid] = nc + tid < m ? fp[s_ao[nc + tid]] : 0;
+        long long V[kCols];
+#pragma unroll
+        for (int k = 0; k < kCols; ++k) V[k] = 0;
+        for (int kb = 0; kb < nkb; ++kb) {
+          if (tid == 0) {
+            mbar_arrive_expect_tx(tbar, kABytes);
+            bulk_g2s_hint(sb, blk + L.apack + (size_t)kb * kABytes, kABytes, tbar, pol_keep);
+            tma_busy = true;
+          }
+          // B operand: kN density rows x 32 K, gathered through the batch's AO list
+          if (tid < kN * 4) {
+            const int r = tid >> 2, c = tid & 3;
+            const int k0 = kb * 32 + c * 8;
+            unsigned long long Y[8];
+            const unsigned long long* row = Yp + (nc + r < m ? (size_t)s_ao[nc + r] * n : 0);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) Y[k] = (nc + r < m && k0 + k < m) ? __ldg(row + s_ao[k0 + k]) : kBias;
+            store8(Y, r, c, [&](int tile, uint32_t o, uint4 v) { st_shared_v4(sb + kABytes + tile * kBTile + o, v); });
+          }
+          fence_proxy_async_smem();
+          if (!wait_tma()) { failed = true; break; }
+          if (tid == 0) mma_block((kb & 1) == 0);
+          if (!wait_mma()) { failed = true; break; }
+          if ((kb & 1) || kb == nkb - 1) {
+            drain(V, sh);
+            __syncthreads();
+          }
+        }
+        if (failed) break;
+        // rho = sum phi T, grad rho = 2 sum grad phi T; T = V 2^(E_f + E_g - 2096 + sh), the point's part
+        // of the exponent applied to the sums
+#pragma unroll
+        for (int j = 0; j < kCols; ++j) {
+          const int i = nc + h * kCols + j;
+          if (i < m) {
+            const int E = ef[h * kCols + j];
+            double t = scaled(V[j], E - 1023 + sh);
+            if (E >= kENan) t = __longlong_as_double(0x7FF8000000000000ll);
+            const double* p = phi + (size_t)i * 128 + g;
+            sr = fma(p[0], t, sr);
+            sx = fma(p[L.plane], t, sx);
+            sy = fma(p[2 * L.plane], t, sy);
+            sz = fma(p[3 * L.plane], t, sz);
+          }
+        }
+      }
+      if (failed) break;
+      const int E = s_eg[g];
+      const double seg = E >= kENan ? __longlong_as_double(0x7FF8000000000000ll)
+                                    : (E > 51 ? __hiloint2double((E - 50) << 20, 0) : 0.0);
+      __syncthreads();
+      dens[h][0][g] = sr * seg;
+      dens[h][1][g] = sx * seg;
+      dens[h][2][g] = sy * seg;
+      dens[h][3][g] = sz * seg;
+      __syncthreads();
+      rho[s] = dens[0][0][g] + dens[1][0][g];
+      gx[s] = 2.0 * (dens[0][1][g] + dens[1][1][g]);
+      gy[s] = 2.0 * (dens[0][2][g] + dens[1][2][g]);
+      gz[s] = 2.0 * (dens[0][3][g] + dens[1][3][g]);
+      fence_proxy_async_smem();  // the stage is written by bulk copies next
+      __syncthreads();
+    }
+    if (failed) break;
+
+    // the functional, one thread per point; a closed shell's exchange and VWN terms in the threads
+    // h == 0, its other correlation terms in h == 1
+    const bool live = g < bd.n_pts;
+    const size_t pt = (size_t)bd.pt_start + g;
+    double e_loc = 0, na_loc = 0, nb_loc = 0;
+    if (A.mode == kModeRks) {
+      XcCs part{0.0, 0.0, 0.0};
+      const bool on = live && !(rho[0] < 1e-18);
+      const double gam = gx[0] * gx[0] + gy[0] * gy[0] + gz[0] * gz[0];
+      if (on) part = xc_eval_cs(A.xc, 0.5 * rho[0], 0.25 * gam, h ? 2 : 1);
+      if (h == 1) {
+        dens[1][0][g] = part.f;
+        dens[1][1][g] = part.vr;
+        dens[1][2][g] = part.vg;
+      }
+      __syncthreads();
+      if (h == 0) {
+        double c0 = 0, us = 0;
+        if (on) {
+          const double w = G.pw[pt];
+          const double vr = part.vr + dens[1][1][g];
+          e_loc = w * (part.f + dens[1][0][g]);
+          na_loc = w * rho[0];
+          us = w * (part.vg + dens[1][2][g]);
+          c0 = 0.5 * w * vr;
+          if (A.point_out) {
+            A.point_out[2 * pt] = e_loc;
+            A.point_out[2 * pt + 1] = w * vr * rho[0] + us * gam;
+          }
+        }
+        coef[0][g] = c0;
+        coef[1][g] = us * gx[0];
+        coef[2][g] = us * gy[0];
+        coef[3][g] = us * gz[0];
+      }
+    } else if (h == 0) {
+#pragma unroll
+      for (int k = 0; k < 8; ++k) coef[k][g] = 0.0;
+      if (A.mode == kModeAccum) {
+        if (live)
+#pragma unroll
+          for (int k = 0; k < 4; ++k) coef[k][g] = A.wv_in[4 * pt + k];
+      } else if (A.mode == kModeRho) {
+        if (live) {
+          A.rho_out[4 * pt] = rho[0];
+          A.rho_out[4 * pt + 1] = gx[0];
+          A.rho_out[4 * pt + 2] = gy[0];
+          A.rho_out[4 * pt + 3] = gz[0];
+        }
+      } else if (A.mode == kModeFxc) {
+        if (live) {  // the density is the trial matrix: rho = eta, (gx, gy, gz) = xi (fxc.rs:374-645)
+          const double* c = A.fxc_coef + 11 * pt;
+          const double* kc = c + (A.triplet ? 7 : 3);
+          const double w = G.pw[pt];
+          const double sigma = c[0] * gx[0] + c[1] * gy[0] + c[2] * gz[0];
+          const double dv = kc[0] * rho[0] + kc[1] * sigma;
+          const double gc = kc[1] * rho[0] + kc[2] * sigma;
+          coef[0][g] = 0.5 * w * dv;
+          coef[1][g] = w * (kc[3] * gx[0] + gc * c[0]);
+          coef[2][g] = w * (kc[3] * gy[0] + gc * c[1]);
+          coef[3][g] = w * (kc[3] * gz[0] + gc * c[2]);
+        }
+      } else {
+        const double ra = fmax(rho[0], 0.0), rb = fmax(rho[1], 0.0);
+        if (live && !(ra + rb < 1e-18)) {
+          const double w = G.pw[pt];
+          const double gaa = gx[0] * gx[0] + gy[0] * gy[0] + gz[0] * gz[0];
+          const double gab = gx[0] * gx[1] + gy[0] * gy[1] + gz[0] * gz[1];
+          const double gbb = gx[1] * gx[1] + gy[1] * gy[1] + gz[1] * gz[1];
+          const XcVal o = xc_eval(A.xc, ra, rb, gaa, gab, gbb);
+          e_loc = w * o.f;
+          na_loc = w * ra;
+          nb_loc = w * rb;
+          coef[0][g] = 0.5 * w * o.vra;
+          coef[1][g] = w * (2.0 * o.vgaa * gx[0] + o.vgab * gx[1]);
+          coef[2][g] = w * (2.0 * o.vgaa * gy[0] + o.vgab * gy[1]);
+          coef[3][g] = w * (2.0 * o.vgaa * gz[0] + o.vgab * gz[1]);
+          coef[4][g] = 0.5 * w * o.vrb;
+          coef[5][g] = w * (2.0 * o.vgbb * gx[1] + o.vgab * gx[0]);
+          coef[6][g] = w * (2.0 * o.vgbb * gy[1] + o.vgab * gy[0]);
+          coef[7][g] = w * (2.0 * o.vgbb * gz[1] + o.vgab * gz[0]);
+        }
+      }
+    }
+    if (A.mode == kModeRks || uks) {
+      double v[3] = {e_loc, na_loc, nb_loc};
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_down_sync(0xffffffffu, v[k], o);
+        if (lane == 0) red[k][warp] = v[k];
+      }
+    }
+    __syncthreads();
+    if ((A.mode == kModeRks || uks) && tid < 3) {
+      double t = 0;
+      for (int k = 0; k < kT / 32; ++k) t += red[tid][k];
+      A.batch_red[3 * (size_t)b + tid] = t;
+    }
+    if (A.mode == kModeRho || A.shares_only) continue;
+
+    for (int s = 0; s < (uks ? 2 : 1) && !failed; ++s) {
+      double* Vm = (s ? A.Vb : A.Va) + moff;
+      if (s) __syncthreads();  // the exponents of the first spin's rows have been read
+      {
+        // Z = (w v_rho / 2) Phi + (w u) . grad Phi, one warp per row, four points per lane
+        double c0[4], cx[4], cy[4], cz[4];
+        load4(&coef[4 * s][4 * lane], c0);
+        load4(&coef[4 * s + 1][4 * lane], cx);
+        load4(&coef[4 * s + 2][4 * lane], cy);
+        load4(&coef[4 * s + 3][4 * lane], cz);
+        for (int row = warp; row < m; row += kT / 32) {
+          const double* p = phi + (size_t)row * 128 + 4 * lane;
+          double x[4], y[4], z[4];
+          load4(p, x);
+          load4(p + L.plane, y);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) z[k] = fma(cx[k], y[k], c0[k] * x[k]);
+          load4(p + 2 * L.plane, x);
+          load4(p + 3 * L.plane, y);
+#pragma unroll
+          for (int k = 0; k < 4; ++k) z[k] = fma(cz[k], y[k], fma(cy[k], x[k], z[k]));
+          const int E = pack_row(zimg, m_z, row, z);
+          if (lane == 0) s_ez[row] = E;
+        }
+      }
+      fence_proxy_async_global();
+      fence_proxy_async_smem();
+      __syncthreads();
+      for (int I = 0; I < m && !failed; I += 128) {
+        for (int J = 0; J < m && !failed; J += kN) {
+          long long V[kCols];
+#pragma unroll
+          for (int k = 0; k < kCols; ++k) V[k] = 0;
+          for (int kb = 0; kb < 4; ++kb) {
+            if (tid == 0) {
+              mbar_arrive_expect_tx(tbar, kABytes + kBBytes);
+#pragma unroll
+              for (int t = 0; t < kTiles; ++t) {
+                bulk_g2s_hint(sb + t * 16384, zimg + ((size_t)(kb * 3 + t) * m_z + I) * 128, 16384, tbar, pol_keep);
+                bulk_g2s_hint(sb + kABytes + t * kBTile, blk + L.img + ((size_t)(kb * 3 + t) * L.m_r + J) * 128, kBTile,
+                              tbar, pol_keep);
+              }
+              tma_busy = true;
+            }
+            if (!wait_tma()) { failed = true; break; }
+            if (tid == 0) mma_block((kb & 1) == 0);
+            if (!wait_mma()) { failed = true; break; }
+            if (kb & 1) {
+              drain(V, 0);
+              __syncthreads();
+            }
+          }
+          if (failed) break;
+          // V[j][i] += W_ij = V 2^(E_z + E_p - 2096)
+          const int i = I + g;
+          if (i < m) {
+            const int ez = s_ez[i], ai = s_ao[i];
+#pragma unroll
+            for (int k = 0; k < kCols; ++k) {
+              const int j = J + h * kCols + k;
+              if (j < m) {
+                const int ep = s_ep[j], e = ez + ep - 2096;
+                const bool bad = ez >= kENan || ep >= kENan;
+                if (bad || (V[k] != 0 && e > -900))
+                  atomicAdd(&Vm[(size_t)s_ao[j] * n + ai], bad ? __longlong_as_double(0x7FF8000000000000ll) : scaled(V[k], e));
+              }
+            }
+          }
+        }
+      }
+    }
+  }
+
+  if (failed) {
+    if (tid == 0) atomicExch(A.counter + 2, 1);
+    mbar_wait_bounded(mbar, phase ^ 1u, kSpin);
+    if (tma_busy) mbar_wait_bounded(tbar, tphase, kSpin);
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  if (warp == 0) tmem_dealloc(tmem, kTmem);
+}
+
+// One CTA per packed density row: the row's exponent and the fixed-point Y of its elements.
+__global__ void __launch_bounds__(256) fixed_density_kernel(const double* __restrict__ D, int n_single,
+                                                           const int* __restrict__ mol_n,
+                                                           const long long* __restrict__ mol_off,
+                                                           const int* __restrict__ mol_ao_off, int n_mols,
+                                                           unsigned long long* __restrict__ out,
+                                                           int* __restrict__ fexp) {
+  __shared__ uint32_t red[8];
+  int mol = 0;
+  if (mol_ao_off) {  // the molecule whose row range holds this row
+    int lo = 0, hi = n_mols - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (mol_ao_off[mid] <= (int)blockIdx.x) lo = mid; else hi = mid - 1;
+    }
+    mol = lo;
+  }
+  const int n = mol_n ? mol_n[mol] : n_single;
+  const size_t o = (size_t)(mol_off ? mol_off[mol] : 0ll) +
+                   (size_t)((int)blockIdx.x - (mol_ao_off ? mol_ao_off[mol] : 0)) * n;
+  uint32_t mx = 0;
+  for (int j = threadIdx.x; j < n; j += 256) mx = max(mx, (uint32_t)__double2hiint(D[o + j]) & 0x7FFFFFFFu);
+  mx = __reduce_max_sync(0xFFFFFFFFu, mx);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < 8; ++k) mx = max(mx, red[k]);
+  const int E = max((int)(mx >> 20), 64);  // rows below 2^-959 count as zeros
+  if (threadIdx.x == 0) fexp[blockIdx.x] = E;
+  for (int j = threadIdx.x; j < n; j += 256) out[o + j] = to_fixed(D[o + j], E);
+}
+
+// V <- V + V^T of each molecule's block (blockIdx.y), 32 x 32 tile pairs; lower_only: the sums in the
+// lower triangle and zeros above it (the drop-in accumulation's result).
+__global__ void __launch_bounds__(256) symmetrise_kernel(double* __restrict__ V, int n_single,
+                                                        const int* __restrict__ mol_n,
+                                                        const long long* __restrict__ mol_off, int lower_only) {
+  __shared__ double ta[32][33], tb[32][33];
+  const int n = mol_n ? mol_n[blockIdx.y] : n_single;
+  double* Vm = V + (mol_off ? mol_off[blockIdx.y] : 0ll);
+  const int nt = (n + 31) / 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  for (int p = blockIdx.x; p < nt * (nt + 1) / 2; p += gridDim.x) {
+    int I = (int)((sqrtf(8.f * p + 1.f) - 1.f) * 0.5f);
+    while (I * (I + 1) / 2 > p) --I;
+    while ((I + 1) * (I + 2) / 2 <= p) ++I;
+    const int J = p - I * (I + 1) / 2;  // tile (I, J), J <= I
+    for (int r = ty; r < 32; r += 8) {
+      const int ai = 32 * I + r, aj = 32 * J + tx, bi = 32 * J + r, bj = 32 * I + tx;
+      ta[r][tx] = ai < n && aj < n ? Vm[(size_t)ai * n + aj] : 0.0;
+      tb[r][tx] = bi < n && bj < n ? Vm[(size_t)bi * n + bj] : 0.0;
+    }
+    __syncthreads();
+    for (int r = ty; r < 32; r += 8) {
+      const int ai = 32 * I + r, aj = 32 * J + tx, bi = 32 * J + r, bj = 32 * I + tx;
+      if (ai < n && aj < n) Vm[(size_t)ai * n + aj] = lower_only && aj > ai ? 0.0 : ta[r][tx] + tb[tx][r];
+      if (I != J && bi < n && bj < n) Vm[(size_t)bi * n + bj] = lower_only ? 0.0 : ta[tx][r] + tb[r][tx];
+    }
+    __syncthreads();
+  }
+}
+
+}  // namespace
+
+int f64tc_max_m() { return kMaxM; }
+
+size_t f64tc_slab_bytes(int max_m) { return z_bytes(max_m) + Block(max_m).bytes; }
+
+size_t f64tc_cache_block_bytes(int m) { return Block(m).bytes; }
+
+cudaError_t f64tc_set_attributes() {
+  static bool attr = false;
+  if (attr) return cudaSuccess;
+  const cudaError_t e = cudaFuncSetAttribute(vxc_f64tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+  if (e == cudaSuccess) attr = true;
+  return e;
+}
+
+cudaError_t launch_f64tc(const DevGrid& G, const EvalArgs& A, int n_ctas, cudaStream_t st) {
+  if (A.max_m > kMaxM) return cudaErrorInvalidValue;
+  const cudaError_t e = f64tc_set_attributes();
+  if (e != cudaSuccess) return e;
+  vxc_f64tc_kernel<<<n_ctas, kT, kSmem, st>>>(G, A);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_f64tc_prepare(const double* P, int n_total, const int* mol_n, const long long* mol_off,
+                                 const int* mol_ao_off, int n_mols, void* out, int* fexp, cudaStream_t st) {
+  fixed_density_kernel<<<n_total, 256, 0, st>>>(P, n_total, mol_n, mol_off, mol_ao_off, n_mols,
+                                                reinterpret_cast<unsigned long long*>(out), fexp);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_symmetrise(double* V, int max_n, const int* mol_n, const long long* mol_off, int n_mols,
+                              int lower_only, cudaStream_t st) {
+  const int nt = (max_n + 31) / 32;
+  const unsigned bx = (unsigned)std::min(nt * (nt + 1) / 2, 4096);
+  symmetrise_kernel<<<dim3(bx, (unsigned)n_mols), 256, 0, st>>>(V, max_n, mol_n, mol_off, lower_only);
+  return cudaGetLastError();
+}
+
+}  // namespace cxc

@@ -1,4 +1,9 @@
-// vxc_fp64.cu -- plain all-FP64 XC quadrature kernels (the drop-in form).
+// vxc_fp64.cu -- the FP64 XC quadrature on the SIMT FP64 pipe, and the small kernels both FP64 forms share.
+//
+// vxc_f64tc.cu does the same work with the contractions on the tensor cores, 8-12 times as fast.  This form
+// runs where that one cannot: batches of more than 2048 AOs, grids whose memory budget leaves no room for
+// its scratch, the allocation-free entry point (noalloc.cu), and the densities of the TD-DFT kernel's
+// finite differences (calchem_xc_fxc_prepare).
 //
 // One persistent CTA works through a device queue of 128-point batches, largest first.  For each
 // batch it
@@ -21,6 +26,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "fp64_ao.cuh"
 #include "xc_device.cuh"
 
 namespace cxc {
@@ -52,69 +58,6 @@ struct Fp64Smem {
 };
 
 __host__ size_t fp64_smem_bytes() { return sizeof(Fp64Smem); }
-
-__device__ __forceinline__ void pow_d1(double x, int l, double& p, double& d) {
-  if (l == 0) { p = 1.0; d = 0.0; }
-  else if (l == 1) { p = x; d = 1.0; }
-  else if (l == 2) { p = x * x; d = 2.0 * x; }
-  else { p = x * x * x; d = 3.0 * x * x; }
-}
-
-// (A) AO values and gradients of the batch into the slab planes 0..3.
-__device__ void eval_batch_aos(const DevGrid& G, const BatchDesc& bd, double* __restrict__ slab, int m_pad) {
-  const int tid = threadIdx.x;
-  const int g = tid & (kBlockPts - 1);
-  const bool live = g < bd.n_pts;
-  double x = 0, y = 0, z = 0;
-  if (live) {
-    x = G.px[bd.pt_start + g];
-    y = G.py[bd.pt_start + g];
-    z = G.pz[bd.pt_start + g];
-  }
-  const size_t plane = (size_t)m_pad * kBlockPts;
-  for (int ci = tid >> 7; ci < bd.n_cand; ci += kThreads / kBlockPts) {
-    const AoShellGpu sh = G.shells[G.cand_shells[bd.cand_start + ci]];
-    const int loc = G.cand_loc[bd.cand_start + ci];
-    double r0 = 0.0, r1 = 0.0, dx = 0, dy = 0, dz = 0;
-    bool on = false;
-    if (live) {
-      dx = x - sh.center[0];
-      dy = y - sh.center[1];
-      dz = z - sh.center[2];
-      const double r2 = dx * dx + dy * dy + dz * dz;
-      if (!(r2 > sh.r2_cutoff)) {
-        for (int p = 0; p < sh.n_prims; ++p) {
-          const AoPrimGpu pr = G.prims[sh.prim_start + p];
-          const double e = pr.weighted_norm * exp(-pr.exponent * r2);
-          r0 += e;
-          r1 -= 2.0 * pr.exponent * e;
-        }
-        on = !(fabs(r0) < 1e-18 && fabs(r1) < 1e-18);
-      }
-    }
-    for (int c = 0; c < sh.n_funcs; ++c) {
-      double v = 0, gx = 0, gy = 0, gz = 0;
-      if (on) {
-        const AoCompGpu cp = G.comps[sh.comp_start + c];
-        double px, dpx, py, dpy, pz, dpz;
-        pow_d1(dx, cp.lx, px, dpx);
-        pow_d1(dy, cp.ly, py, dpy);
-        pow_d1(dz, cp.lz, pz, dpz);
-        const double mm = px * py * pz;
-        v = cp.scale * mm * r0;
-        gx = cp.scale * (dpx * py * pz * r0 + mm * dx * r1);
-        gy = cp.scale * (px * dpy * pz * r0 + mm * dy * r1);
-        gz = cp.scale * (px * py * dpz * r0 + mm * dz * r1);
-        if (!(fabs(v) > 1e-16 || fabs(gx) > 1e-16 || fabs(gy) > 1e-16 || fabs(gz) > 1e-16)) v = gx = gy = gz = 0;
-      }
-      const size_t o = (size_t)(loc + c) * kBlockPts + g;
-      slab[o] = v;
-      slab[plane + o] = gx;
-      slab[2 * plane + o] = gy;
-      slab[3 * plane + o] = gz;
-    }
-  }
-}
 
 // (B) rho and grad rho (unscaled sum of grad Phi T) of density P for the batch; result in dens[0][..]
 // after the call (summed over both halves).
@@ -276,7 +219,7 @@ __global__ void __launch_bounds__(kThreads, 1) vxc_fp64_kernel(DevGrid G, EvalAr
     if (q >= G.n_batches) break;
     const int b = G.order[q];
     const BatchDesc bd = G.batches[b];
-    eval_batch_aos(G, bd, slab, m_pad);
+    eval_batch_aos<kThreads>(G, bd, slab, (size_t)m_pad * kBlockPts);
     __syncthreads();
     if (A.mode == kModeFxc) {
       // The batch's AOs serve every trial matrix: response density eta = sum M phi phi and its

@@ -506,7 +506,9 @@ __host__ __device__ __forceinline__ XcVal xc_eval(int code, double rho_a, double
 // rho^(-11/3) = rho^(-2/3) / rho^3), asinh(s) = log1p(s + s^2 / (1 + sqrt(1 + s^2))) reuses the
 // square root B88 needs anyway, exp(w) = expm1(w) + 1, and the constant factors are literals (their
 // values computed in double precision from the definitions beside them).  The results agree with
-// xc_eval(code, r, r, g, g, g) to rounding (~1e-15 relative).
+// xc_eval(code, r, r, g, g, g) to rounding (~1e-15 relative).  `parts` selects terms so that two thread
+// groups can share a point: bit 0 exchange and VWN (and the range-separated codes whole), bit 1 the LYP
+// and PBE correlation terms; the two parts add up to the whole.
 struct XcCs {
   double f;   // energy density
   double vr;  // dF/drho_a (= dF/drho_b)
@@ -529,8 +531,10 @@ constexpr VwnPara kVwn5Para{0.0310907, -0.10498, 3.72744, 12.9352,
 constexpr VwnPara kVwnRpaPara{0.0310907, -0.409286, 13.0720, 42.7198,
                               0.0448998886415768, 582.2731590427809, -0.14253052416798392, 545.8110641572265};
 
-__host__ __device__ __forceinline__ XcCs xc_eval_cs(int code, double r_in, double g_in) {
+__host__ __device__ __forceinline__ XcCs xc_eval_cs(int code, double r_in, double g_in, int parts = 3) {
+  const bool px = (parts & 1) != 0, pc = (parts & 2) != 0;
   if (code >= 6) {  // range-separated functionals: the spin form at rho_a = rho_b
+    if (!px) return XcCs{0.0, 0.0, 0.0};
     const XcVal v = xc_eval(code, r_in, r_in, g_in, g_in, g_in);
     return XcCs{v.f, v.vra, v.vgaa + 0.5 * v.vgab};
   }
@@ -541,7 +545,7 @@ __host__ __device__ __forceinline__ XcCs xc_eval_cs(int code, double r_in, doubl
   const double g = fmax(g_in, 0.0);
   const double c13 = cbrt(r);
   const double rho13 = kCsCbrt2 * c13;
-  const bool spin_on = !(r < kRhoFloor);  // the per-spin floor of the exchange terms
+  const bool spin_on = px && !(r < kRhoFloor);  // the per-spin floor of the exchange terms
   if (spin_on && (code == 0 || code == 1 || code == 3 || code == 4)) {  // Slater
     const double sc = (code == 3 || code == 4) ? 0.80 : 1.0;
     o.f += sc * (-2.0 * kCsCx * r * c13);
@@ -576,7 +580,7 @@ __host__ __device__ __forceinline__ XcCs xc_eval_cs(int code, double r_in, doubl
     o.vr += sc * ((4.0 / 3.0) * kCsCxu * rho13 * fx + exl * dfx * (-(8.0 / 3.0) * s2 / rho));
     o.vg += sc * (2.0 * (exl * dfx / den_s2));
   }
-  if (code == 0 || code == 3 || code == 4) {  // VWN5 / VWN_RPA, paramagnetic channel
+  if (px && (code == 0 || code == 3 || code == 4)) {  // VWN5 / VWN_RPA, paramagnetic channel
     const double sc = code == 0 ? 1.0 : 0.19;
     const VwnPara ch = code == 3 ? kVwnRpaPara : kVwn5Para;
     const double x = sqrt(kCsRsK / rho13);
@@ -588,7 +592,7 @@ __host__ __device__ __forceinline__ XcCs xc_eval_cs(int code, double r_in, doubl
     o.f += sc * (rho * ep);
     o.vr += sc * (ep - (1.0 / 3.0) * dp);
   }
-  if (code == 1 || code == 3 || code == 4) {  // LYP
+  if (pc && (code == 1 || code == 3 || code == 4)) {  // LYP
     const double sc = code == 1 ? 1.0 : 0.81;
     const double A = 0.04918, B = 0.132, C = 0.2533, D = 0.349;
     const double rm13 = 1.0 / rho13;
@@ -628,7 +632,7 @@ __host__ __device__ __forceinline__ XcCs xc_eval_cs(int code, double r_in, doubl
       o.vg += sc * (-ab * omega * (aaa + 0.5 * aab));
     }
   }
-  if (code == 2 || code == 5) {  // PBE correlation on the paramagnetic PW92 channel
+  if (pc && (code == 2 || code == 5)) {  // PBE correlation on the paramagnetic PW92 channel
     const double gt = 4.0 * g;
     const double rs = kCsRsK / rho13;
     const double drs = -rs / (3.0 * rho);

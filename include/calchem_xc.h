@@ -231,7 +231,9 @@ int calchem_xc_set_weights(uint64_t grid_id, const double* h_weights, int n_pts)
  * others evaluate their AOs every time (the reference caches all or nothing).  enable = 0 waits for the device,
  * frees the cache, disables it and drops a captured graph; enable = 1 allows it again (a no-op when
  * allowed, the default); -1 only reports its size in *bytes_out (0 when none).  Results are the
- * same with and without the cache. */
+ * same with and without the cache.  The FP64 form keeps a cache of its own under the same switch, cap and
+ * budget (FP64 planes and packed slices, 56 B per AO and point, within a quarter of the free device
+ * memory); its size is not part of *bytes_out. */
 int calchem_xc_set_ao_cache(uint64_t grid_id, int enable, size_t* bytes_out);
 
 /* Number of batches and the sum over batches of m_b^2 * n_b (m_b AOs, n_b points): the
