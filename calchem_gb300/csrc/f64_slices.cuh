@@ -68,10 +68,14 @@ __device__ __forceinline__ long long level_sum(float s0, float s1, float s2, flo
   return ((long long)i0 << 36) + ((long long)i1 << 27) + ((long long)i2 << 18) + ((long long)i3 << 9) + i4;
 }
 
-// V 2^e as a double (the exponent is added in the FP64 pattern; V = 0 stays 0; e within +-900)
-__device__ __forceinline__ double scaled(long long V, int e) {
+// V 2^e as a double, by adding e to the FP64 pattern's exponent (V = 0 stays 0; kScaleMin <= e), or NaN from
+// e = kScaleNan on (an operand vector of 2^957 and above, or with infinities or NaN).
+constexpr int kScaleMin = -1000;
+constexpr int kScaleNan = 957;
+__device__ __forceinline__ double scaled_or_nan(long long V, int e) {
   const double d = __ll2double_rn(V);
-  return V == 0 ? 0.0 : __hiloint2double(__double2hiint(d) + (e << 20), __double2loint(d));
+  const int hi = V == 0 ? 0 : __double2hiint(d) + (e << 20);
+  return __hiloint2double(e >= kScaleNan ? 0x7FF80000 : hi, __double2loint(d));
 }
 
 }  // namespace f64s

@@ -12,14 +12,20 @@
 // What bounds it: GB300 has 2 FP64 FMA lanes per SM and clock, so the SIMT form spends 4 m^2 FP64 FMAs a
 // point there; here the tensor cores take them and the FP64 pipe is left with ~m (4 for rho and
 // grad rho, 4 for Z, 2 for the conversion of T) FMAs a point and the functional.  Two CTAs of 256
-// threads share an SM (240 TMEM columns and ~103 KB of shared memory each), so that one CTA's FP64
+// threads share an SM (240 TMEM columns and ~109 KB of shared memory each), so that one CTA's FP64
 // phases run under the other's copies and MMAs.  N = 48 columns is what five accumulators leave of
 // 256 TMEM columns.
 //
-// Measured against the SIMT form (whole host calls, FP64): C8H18 B3LYP Fine 32.9 -> 2.73 ms, 24 waters
-// B3LYP Medium 30.9 -> 2.47 ms, C6H14 PBE open shell 7.34 -> 0.83 ms, one water 0.63 -> 0.16 ms; the
+// Measured against the SIMT form (whole host calls, FP64): C8H18 B3LYP Fine 32.9 -> 2.42 ms, 24 waters
+// B3LYP Medium 30.9 -> 2.20 ms, C6H14 PBE open shell 7.33 -> 0.79 ms, one water 0.63 -> 0.16 ms; the
 // relative error of V against a plain FP64 evaluation is the same (2.6e-15 on C8H18, 2.7e-15 before).
-//
+// On C8H18 a batch takes a CTA 280 us (210 alone on its SM): 36 % in MMA rounds, whose 128 x 32-byte A
+// reads bind them to shared memory (44 cycles per MMA of N = 48, 43 at N = 16), 46 % in rho, functional
+// and Z on the FP64 pipe, 10 % draining accumulators, 7 % in V's reductions.  What shortened it from 2.72
+// ms: A tiles reloaded one by one under the others' MMAs and B gathered under them (-4 %), MMAs issued
+// from uniform registers (-3 %), rho's loads and V's reductions free of branches (-5 %).  Measured without
+// effect: L2 prefetches of the operands and planes, the next Z row's loads in registers.
+
 // AO values, their packed slices and exponents depend on the grid and basis only: batches with a block
 // in the grid's AO cache compute them in the first launch that reaches them and read them afterwards,
 // as the tensor-core form of vxc_mixed.cu does.
@@ -59,19 +65,20 @@ constexpr int kBBytes = kTiles * kBTile;
 constexpr int kMaxM = 2048;
 constexpr uint32_t kSpin = 1u << 26;
 
-constexpr int kOffCoef = kABytes + kBBytes;         // double [8][128]
-constexpr int kOffAo = kOffCoef + 8 * 128 * 8;      // int [kMaxM]: global AO of each local row
-constexpr int kOffEz = kOffAo + kMaxM * 4;          // int [kMaxM]: biased exponents of the Z rows
-constexpr int kOffEp = kOffEz + kMaxM * 4;          // int [kMaxM]: of the Phi rows
-constexpr int kOffEg = kOffEp + kMaxM * 4;          // int [128]: of the points
+constexpr int kOffCoef = kABytes + 2 * kBBytes;     // double [8][128]; two B buffers before it
+constexpr int kOffAo = kOffCoef + 8 * 128 * 8;      // uint16 [kMaxM]: AO (within the molecule) of each local row
+constexpr int kOffEz = kOffAo + kMaxM * 2;          // uint16 [kMaxM]: biased exponents of the Z rows
+constexpr int kOffEp = kOffEz + kMaxM * 2;          // uint16 [kMaxM]: of the Phi rows
+constexpr int kOffEg = kOffEp + kMaxM * 2;          // int [128]: of the points
 constexpr int kOffEf = kOffEg + 128 * 4;            // int [2][64]: of the chunk's density rows
 constexpr int kOffRed = kOffEf + 128 * 4;           // double [3][kT / 32]
 constexpr int kOffMisc = kOffRed + 3 * (kT / 32) * 8;
-constexpr int kSmem = kOffMisc + 64 + 1024;
+constexpr int kSmem = kOffMisc + 96 + 1024;
 static_assert(2 * (kSmem + 1024) <= 233472, "two CTAs share one SM's shared memory");
 static_assert(kLevels * kN <= (int)kTmem, "the accumulators fit the CTA's TMEM columns");
 static_assert(8 * 128 * 8 <= kABytes, "the density sums live in the idle operand stage");
-constexpr int kENan = 1980;  // row exponents from here on (2^957 and above, infinities, NaN) give NaN
+constexpr int kENan = kScaleNan + 1023;  // biased exponents from here on give NaN
+constexpr int kENanMark = 4096;          // and are kept as this one where two of them are added up
 
 __host__ __device__ constexpr size_t up(size_t x, size_t k) { return (x + k - 1) / k * k; }
 
@@ -154,6 +161,13 @@ __device__ __forceinline__ void load4(const double* p, double (&x)[4]) {
   x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
 }
 
+// *p += v where `on` (a predicated reduction: no branch)
+__device__ __forceinline__ void red_add_if(double* p, double v, bool on) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q red.global.add.f64 [%0], %1;\n\t}" ::"l"(p), "d"(v),
+               "r"((int)on)
+               : "memory");
+}
+
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
@@ -166,24 +180,24 @@ __global__ void __launch_bounds__(kT, 2) vxc_f64tc_kernel(DevGrid G, EvalArgs A)
   unsigned char* stage = base;
   double(*coef)[128] = reinterpret_cast<double(*)[128]>(base + kOffCoef);
   double(*dens)[4][128] = reinterpret_cast<double(*)[4][128]>(base);  // [2], the stage idle
-  int* s_ao = reinterpret_cast<int*>(base + kOffAo);
-  int* s_ez = reinterpret_cast<int*>(base + kOffEz);
-  int* s_ep = reinterpret_cast<int*>(base + kOffEp);
+  uint16_t* s_ao = reinterpret_cast<uint16_t*>(base + kOffAo);
+  uint16_t* s_ez = reinterpret_cast<uint16_t*>(base + kOffEz);
+  uint16_t* s_ep = reinterpret_cast<uint16_t*>(base + kOffEp);
   int* s_eg = reinterpret_cast<int*>(base + kOffEg);
   int* s_ef = reinterpret_cast<int*>(base + kOffEf);
   double(*red)[kT / 32] = reinterpret_cast<double(*)[kT / 32]>(base + kOffRed);
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(base + kOffMisc);      // MMA commits
-  uint64_t* tbar = reinterpret_cast<uint64_t*>(base + kOffMisc + 8);  // operand bulk copies
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(base + kOffMisc + 16);
-  int* s_batch = reinterpret_cast<int*>(base + kOffMisc + 20);
+  uint64_t* full = reinterpret_cast<uint64_t*>(base + kOffMisc);            // [3] A tile t has arrived
+  uint64_t* empty = reinterpret_cast<uint64_t*>(base + kOffMisc + 24);      // [3] the MMAs reading A tile t are done
+  uint64_t* full_b = reinterpret_cast<uint64_t*>(base + kOffMisc + 48);     // [2] B buffer (GEMM2) has arrived
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(base + kOffMisc + 64);
+  int* s_batch = reinterpret_cast<int*>(base + kOffMisc + 68);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = tid & 127, h = tid >> 7;
   const bool uks = A.mode == kModeUks;
 
   if (tid == 0) {
-    mbar_init(mbar, 1);
-    mbar_init(tbar, 1);
+    for (int k = 0; k < 8; ++k) mbar_init(full + k, 1);  // full, empty, full_b
     fence_mbar_init();
   }
   if (warp == 0) {
@@ -193,12 +207,12 @@ __global__ void __launch_bounds__(kT, 2) vxc_f64tc_kernel(DevGrid G, EvalArgs A)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = warp_uniform(*tmem_slot);
   const uint32_t tl = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(h * kCols);  // this thread's columns
-  const uint32_t sb = smem_addr(stage);
+  const uint32_t sb = warp_uniform(smem_addr(stage));
+  const bool issuer = warp_uniform(warp) == 0 && elect_one();  // copies the operands and issues the MMAs
   const uint32_t idesc = idesc_bf16_f32(128, kN);
-  uint32_t phase = 0, tphase = 0;
-  bool tma_busy = false, failed = false;
+  bool failed = false;
 
   unsigned char* const slab = reinterpret_cast<unsigned char*>(A.slab + (size_t)blockIdx.x * A.slab_stride);
   unsigned char* const zimg = slab;  // the Z image, then the block of a batch without a cache block
@@ -206,41 +220,76 @@ __global__ void __launch_bounds__(kT, 2) vxc_f64tc_kernel(DevGrid G, EvalArgs A)
   const int* const f0 = reinterpret_cast<const int*>(Y0 + 2 * G.nn_total);
   const uint64_t pol_keep = l2_policy_evict_last();
 
-  auto wait_mma = [&]() -> bool {
-    const bool ok = mbar_wait_bounded(mbar, phase, kSpin);
-    phase ^= 1u;
-    tc_fence_after();
-    return __syncthreads_or(!ok) == 0;
+  // One thread copies the operands and issues the MMAs.  An A tile (two slices) is copied again as soon as
+  // the MMAs reading it are done, so that the next K block's tiles arrive under the MMAs of the others.
+  // The state is that thread's: phases of the barriers, tiles whose release has not been waited for, copies
+  // not waited for (bits 0-2 A tiles, 3-4 B buffers).
+  uint32_t ph_full = 0, ph_empty = 0, pend = 0, inflight = 0;
+  auto wait_full = [&](int k) -> bool {  // k: 0-2 A tiles, 3-4 B buffers
+    uint64_t* bar = k < 3 ? full + k : full_b + (k - 3);
+    if (!mbar_wait_bounded(bar, (ph_full >> k) & 1u, kSpin)) return false;
+    ph_full ^= 1u << k;
+    inflight &= ~(1u << k);
+    return true;
   };
-  auto wait_tma = [&]() -> bool {
-    const bool ok = mbar_wait_bounded(tbar, tphase, kSpin);
-    if (ok) {
-      tphase ^= 1u;
-      tma_busy = false;
-    }
-    return __syncthreads_or(!ok) == 0;
+  auto wait_empty = [&](int t) -> bool {
+    if (!(pend >> t & 1u)) return true;
+    if (!mbar_wait_bounded(empty + t, (ph_empty >> t) & 1u, kSpin)) return false;
+    ph_empty ^= 1u << t;
+    pend &= ~(1u << t);
+    return true;
   };
-  // one K block of 32: slice products i + j <= 5, level min(i + j, 4) into accumulator columns 48 level
-  auto mma_block = [&](bool first) {
-    tc_fence_after();
-    uint64_t a[kTiles], b[kTiles];
+  auto load_a = [&](const unsigned char* src, size_t tile_stride) -> bool {  // the three tiles of a K block
 #pragma unroll
     for (int t = 0; t < kTiles; ++t) {
-      a[t] = sdesc_sw128(sb + t * 16384);
-      b[t] = sdesc_sw128(sb + kABytes + t * kBTile);
+      if (!wait_empty(t)) return false;
+      mbar_arrive_expect_tx(full + t, 16384);
+      bulk_g2s_hint(sb + t * 16384, src + t * tile_stride, 16384, full + t, pol_keep);
+      inflight |= 1u << t;
     }
+    return true;
+  };
+  auto load_b = [&](int buf, const unsigned char* src, size_t tile_stride) {
+    mbar_arrive_expect_tx(full_b + buf, kBBytes);
 #pragma unroll
-    for (int ks = 0; ks < 2; ++ks)
+    for (int t = 0; t < kTiles; ++t)
+      bulk_g2s_hint(sb + kABytes + buf * kBBytes + t * kBTile, src + t * tile_stride, kBTile, full_b + buf, pol_keep);
+    inflight |= 8u << buf;
+  };
+  // One K block of 32 against B buffer buf: slice products i + j <= 5, level min(i + j, 4) into
+  // accumulator columns 48 level; then the next K block's A copies (next != nullptr).  Returns with the
+  // MMAs done.
+  auto mma_round = [&](bool first, int buf, const unsigned char* next, size_t tile_stride) -> bool {
+    tc_fence_after();
+    const uint64_t db = sdesc_sw128(sb + kABytes) + (uint32_t)buf * (kBBytes >> 4);
 #pragma unroll
-      for (int i = 0; i < kSlices; ++i)
+    for (int t = 0; t < kTiles; ++t) {
+      if (!wait_full(t)) return false;
+      const uint64_t a = sdesc_sw128(sb) + t * 1024;
 #pragma unroll
-        for (int j = 0; i + j < kSlices; ++j) {
-          const int lev = i + j < kLevels ? i + j : kLevels - 1;
-          // each level's first product (i = 0, levels 0..4) overwrites at the start of a K group
-          const uint32_t acc = (first && ks == 0 && i == 0 && j < kLevels) ? 0u : 1u;
-          mma_bf16_ss(tmem + lev * kN, a[i >> 1] + (i & 1) * 4 + ks * 2, b[j >> 1] + (j & 1) * 4 + ks * 2, idesc, acc);
-        }
-    mma_commit(mbar);
+      for (int ks = 0; ks < 2; ++ks)
+#pragma unroll
+        for (int i = 2 * t; i < 2 * t + 2; ++i)
+#pragma unroll
+          for (int j = 0; i + j < kSlices; ++j) {
+            const int lev = i + j < kLevels ? i + j : kLevels - 1;
+            // each level's first product (i = 0, levels 0..4) overwrites at the start of a K group
+            const uint32_t acc = (first && ks == 0 && i == 0 && j < kLevels) ? 0u : 1u;
+            mma_bf16_ss(tmem + lev * kN, a + (i & 1) * 4 + ks * 2,
+                        db + (j >> 1) * (kBTile >> 4) + (j & 1) * 4 + ks * 2, idesc, acc);
+          }
+      mma_commit(empty + t);
+      pend |= 1u << t;
+    }
+    if (next) {
+      if (!load_a(next, tile_stride)) return false;
+    } else {
+#pragma unroll
+      for (int t = 0; t < kTiles; ++t)
+        if (!wait_empty(t)) return false;
+    }
+    tc_fence_before();
+    return true;
   };
   // the accumulators' K group into the thread's 64-bit sums
   auto drain = [&](long long (&V)[kCols], int sh) {
@@ -288,7 +337,7 @@ __global__ void __launch_bounds__(kT, 2) vxc_f64tc_kernel(DevGrid G, EvalArgs A)
     __syncthreads();
     if (cached) {
       if (h == 0) s_eg[g] = blk_eg[g];
-      for (int i = tid; i < m; i += kT) s_ep[i] = blk_ep[i];
+      for (int i = tid; i < m; i += kT) s_ep[i] = (uint16_t)(blk_ep[i] >= kENan ? kENanMark : blk_ep[i]);
       __syncthreads();
     } else {
       const uint32_t vmax = eval_batch_aos<kT>(G, bd, phi, L.plane);
@@ -306,7 +355,10 @@ __global__ void __launch_bounds__(kT, 2) vxc_f64tc_kernel(DevGrid G, EvalArgs A)
         double x[4];
         load4(phi + (size_t)row * 128 + 4 * lane, x);
         const int E = pack_row(blk + L.img, L.m_r, row, x);
-        if (lane == 0) s_ep[row] = blk_ep[row] = E;
+        if (lane == 0) {
+          s_ep[row] = (uint16_t)(E >= kENan ? kENanMark : E);
+          blk_ep[row] = E;
+        }
       }
       fence_proxy_async_global();  // the packed operands are read by bulk copies, the stage written by them
       fence_proxy_async_smem();
@@ -323,6 +375,24 @@ __global__ void __launch_bounds__(kT, 2) vxc_f64tc_kernel(DevGrid G, EvalArgs A)
       const unsigned long long* Yp = Y0 + (s ? G.nn_total : 0) + moff;
       const int* fp = f0 + (s ? G.n_total : 0) + roff;
       double sr = 0, sx = 0, sy = 0, sz = 0;
+      // B operand: kN density rows x 32 K, gathered through the batch's AO list (warps 2-7, under the MMAs
+      // of the K block before)
+      auto gather = [&](int nc, int kb, int buf) {
+        const int r = (tid - 64) >> 2, c = tid & 3;
+        const int k0 = kb * 32 + c * 8;
+        unsigned long long Y[8];
+        const unsigned long long* row = Yp + (nc + r < m ? (size_t)s_ao[nc + r] * n : 0);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) Y[k] = (nc + r < m && k0 + k < m) ? __ldg(row + s_ao[k0 + k]) : kBias;
+        const uint32_t o = sb + kABytes + buf * kBBytes;
+        store8(Y, r, c, [&](int tile, uint32_t off, uint4 v) { st_shared_v4(o + tile * kBTile + off, v); });
+        fence_proxy_async_smem();
+      };
+      int buf = 0;
+      bool bad = false;
+      if (issuer) bad = !load_a(blk + L.apack, 16384);
+      if (tid >= 64) gather(0, 0, 0);
+      __syncthreads();
       for (int nc = 0; nc < m && !failed; nc += kN) {
         // (double-buffered: slower threads may still read the previous chunk's)
         int* const ef = s_ef + (nc / kN & 1) * 64;
@@ -330,27 +400,17 @@ __global__ void __launch_bounds__(kT, 2) vxc_f64tc_kernel(DevGrid G, EvalArgs A)
         long long V[kCols];
 #pragma unroll
         for (int k = 0; k < kCols; ++k) V[k] = 0;
-        for (int kb = 0; kb < nkb; ++kb) {
-          if (tid == 0) {
-            mbar_arrive_expect_tx(tbar, kABytes);
-            bulk_g2s_hint(sb, blk + L.apack + (size_t)kb * kABytes, kABytes, tbar, pol_keep);
-            tma_busy = true;
-          }
-          // B operand: kN density rows x 32 K, gathered through the batch's AO list
-          if (tid < kN * 4) {
-            const int r = tid >> 2, c = tid & 3;
-            const int k0 = kb * 32 + c * 8;
-            unsigned long long Y[8];
-            const unsigned long long* row = Yp + (nc + r < m ? (size_t)s_ao[nc + r] * n : 0);
-#pragma unroll
-            for (int k = 0; k < 8; ++k) Y[k] = (nc + r < m && k0 + k < m) ? __ldg(row + s_ao[k0 + k]) : kBias;
-            store8(Y, r, c, [&](int tile, uint32_t o, uint4 v) { st_shared_v4(sb + kABytes + tile * kBTile + o, v); });
-          }
-          fence_proxy_async_smem();
-          if (!wait_tma()) { failed = true; break; }
-          if (tid == 0) mma_block((kb & 1) == 0);
-          if (!wait_mma()) { failed = true; break; }
-          if ((kb & 1) || kb == nkb - 1) {
+        for (int kb = 0; kb < nkb; ++kb, buf ^= 1) {
+          const bool last_k = kb == nkb - 1;
+          const bool more = !last_k || nc + kN < m;
+          const int kb1 = last_k ? 0 : kb + 1;
+          if (issuer)
+            bad = bad || !mma_round((kb & 1) == 0, buf, more ? blk + L.apack + (size_t)kb1 * kABytes : nullptr, 16384);
+          else if (tid >= 64 && more)
+            gather(last_k ? nc + kN : nc, kb1, buf ^ 1);
+          if (__syncthreads_or(bad)) { failed = true; break; }
+          if ((kb & 1) || last_k) {
+            tc_fence_after();
             drain(V, sh);
             __syncthreads();
           }
@@ -358,18 +418,24 @@ __global__ void __launch_bounds__(kT, 2) vxc_f64tc_kernel(DevGrid G, EvalArgs A)
         if (failed) break;
         // rho = sum phi T, grad rho = 2 sum grad phi T; T = V 2^(E_f + E_g - 2096 + sh), the point's part
         // of the exponent applied to the sums
+        // (columns beyond m have V = 0 and read the last row: no branches between the loads of a group)
 #pragma unroll
-        for (int j = 0; j < kCols; ++j) {
-          const int i = nc + h * kCols + j;
-          if (i < m) {
-            const int E = ef[h * kCols + j];
-            double t = scaled(V[j], E - 1023 + sh);
-            if (E >= kENan) t = __longlong_as_double(0x7FF8000000000000ll);
-            const double* p = phi + (size_t)i * 128 + g;
-            sr = fma(p[0], t, sr);
-            sx = fma(p[L.plane], t, sx);
-            sy = fma(p[2 * L.plane], t, sy);
-            sz = fma(p[3 * L.plane], t, sz);
+        for (int j0 = 0; j0 < kCols; j0 += 4) {
+          if (nc + h * kCols + j0 >= m) break;
+          double p[4][4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const double* r = phi + (size_t)min(nc + h * kCols + j0 + j, m - 1) * 128 + g;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) p[j][k] = r[k * L.plane];
+          }
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const double t = scaled_or_nan(V[j0 + j], ef[h * kCols + j0 + j] - 1023 + sh);
+            sr = fma(p[j][0], t, sr);
+            sx = fma(p[j][1], t, sx);
+            sy = fma(p[j][2], t, sy);
+            sz = fma(p[j][3], t, sz);
           }
         }
       }
@@ -515,50 +581,55 @@ __global__ void __launch_bounds__(kT, 2) vxc_f64tc_kernel(DevGrid G, EvalArgs A)
 #pragma unroll
           for (int k = 0; k < 4; ++k) z[k] = fma(cz[k], y[k], fma(cy[k], x[k], z[k]));
           const int E = pack_row(zimg, m_z, row, z);
-          if (lane == 0) s_ez[row] = E;
+          if (lane == 0) s_ez[row] = (uint16_t)(E >= kENan ? kENanMark : E);
         }
       }
       fence_proxy_async_global();
       fence_proxy_async_smem();
       __syncthreads();
+      // operand addresses of K block kb of tile (I, J)
+      auto src_a = [&](int I, int kb) { return zimg + ((size_t)kb * 3 * m_z + I) * 128; };
+      auto src_b = [&](int J, int kb) { return blk + L.img + ((size_t)kb * 3 * L.m_r + J) * 128; };
+      const size_t st_a = (size_t)m_z * 128, st_b = (size_t)L.m_r * 128;
+      bool bad = false;
+      if (issuer) {
+        bad = !load_a(src_a(0, 0), st_a);
+        load_b(0, src_b(0, 0), st_b);
+      }
       for (int I = 0; I < m && !failed; I += 128) {
         for (int J = 0; J < m && !failed; J += kN) {
           long long V[kCols];
 #pragma unroll
           for (int k = 0; k < kCols; ++k) V[k] = 0;
-          for (int kb = 0; kb < 4; ++kb) {
-            if (tid == 0) {
-              mbar_arrive_expect_tx(tbar, kABytes + kBBytes);
-#pragma unroll
-              for (int t = 0; t < kTiles; ++t) {
-                bulk_g2s_hint(sb + t * 16384, zimg + ((size_t)(kb * 3 + t) * m_z + I) * 128, 16384, tbar, pol_keep);
-                bulk_g2s_hint(sb + kABytes + t * kBTile, blk + L.img + ((size_t)(kb * 3 + t) * L.m_r + J) * 128, kBTile,
-                              tbar, pol_keep);
+          const int J1 = J + kN < m ? J + kN : 0, I1 = J1 ? I : I + 128;  // the next tile
+          for (int kh = 0; kh < 2; ++kh) {
+            if (issuer)
+              for (int kb = 2 * kh; kb < 2 * kh + 2 && !bad; ++kb) {
+                const bool more = kb < 3 || I1 < m;
+                const unsigned char* next = nullptr;
+                if (more) {  // the other B buffer's MMAs (the K block before) are done
+                  next = kb < 3 ? src_a(I, kb + 1) : src_a(I1, 0);
+                  load_b((kb + 1) & 1, kb < 3 ? src_b(J, kb + 1) : src_b(J1, 0), st_b);
+                }
+                bad = !wait_full(3 + (kb & 1)) || !mma_round((kb & 1) == 0, kb & 1, next, st_a);
               }
-              tma_busy = true;
-            }
-            if (!wait_tma()) { failed = true; break; }
-            if (tid == 0) mma_block((kb & 1) == 0);
-            if (!wait_mma()) { failed = true; break; }
-            if (kb & 1) {
-              drain(V, 0);
-              __syncthreads();
-            }
+            if (__syncthreads_or(bad)) { failed = true; break; }
+            tc_fence_after();
+            drain(V, 0);
+            __syncthreads();
           }
           if (failed) break;
-          // V[j][i] += W_ij = V 2^(E_z + E_p - 2096)
+          // V[j][i] += W_ij = V 2^(E_z + E_p - 2096), without branches between the elements
           const int i = I + g;
           if (i < m) {
-            const int ez = s_ez[i], ai = s_ao[i];
+            const int ez = s_ez[i] - 2096;
+            double* const col = Vm + s_ao[i];
 #pragma unroll
             for (int k = 0; k < kCols; ++k) {
-              const int j = J + h * kCols + k;
-              if (j < m) {
-                const int ep = s_ep[j], e = ez + ep - 2096;
-                const bool bad = ez >= kENan || ep >= kENan;
-                if (bad || (V[k] != 0 && e > -900))
-                  atomicAdd(&Vm[(size_t)s_ao[j] * n + ai], bad ? __longlong_as_double(0x7FF8000000000000ll) : scaled(V[k], e));
-              }
+              if (k % 8 == 0 && J + h * kCols + k >= m) break;
+              const int j = min(J + h * kCols + k, m - 1);
+              const double w = scaled_or_nan(V[k], max(ez + (int)s_ep[j], kScaleMin));
+              red_add_if(col + (size_t)s_ao[j] * n, w, J + h * kCols + k < m && w != 0.0);
             }
           }
         }
@@ -568,8 +639,11 @@ __global__ void __launch_bounds__(kT, 2) vxc_f64tc_kernel(DevGrid G, EvalArgs A)
 
   if (failed) {
     if (tid == 0) atomicExch(A.counter + 2, 1);
-    mbar_wait_bounded(mbar, phase ^ 1u, kSpin);
-    if (tma_busy) mbar_wait_bounded(tbar, tphase, kSpin);
+    if (issuer) {
+      for (int k = 0; k < 5; ++k)
+        if (inflight >> k & 1u) wait_full(k);
+      for (int t = 0; t < kTiles; ++t) wait_empty(t);
+    }
   }
   tc_fence_before();
   __syncthreads();
