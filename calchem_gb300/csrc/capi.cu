@@ -84,7 +84,7 @@ struct Entry {
   double* d_mixed_slab = nullptr;
   int mixed_ctas = 0;               // tensor-core CTAs the workspace has slabs for
   int tile_n = 64;                  // tensor-core GEMM1 N chunk (calchem_xc_set_tile)
-  double* h_stage = nullptr;  // pinned: 2 n^2 + 4 doubles
+  double* h_stage = nullptr;  // pinned: the sums and the status word (3 n_mols + 8 doubles)
   cudaStream_t stream = nullptr;
   int last_launches = 0;
   bool profiling = false;
@@ -279,7 +279,7 @@ int ensure_ws(Entry& e) {
             dalloc(&e.d_slab, e.slab_stride * e.n_ctas) &&
             cudaMalloc(&e.d_mixed_ws, nn * sizeof(uint2) * 2 + (size_t)e.n_ao * 2 * sizeof(int)) == cudaSuccess &&
             dalloc(&e.d_mixed_slab, e.mixed_slab_stride * e.mixed_ctas) &&
-            cudaMallocHost((void**)&e.h_stage, (2 * nn + 3 * (size_t)e.n_mols + 8) * sizeof(double)) == cudaSuccess &&
+            cudaMallocHost((void**)&e.h_stage, (3 * (size_t)e.n_mols + 8) * sizeof(double)) == cudaSuccess &&
             cudaStreamCreateWithFlags(&e.stream, cudaStreamNonBlocking) == cudaSuccess;
   if (!ok) {
     cudaGetLastError();
@@ -295,11 +295,6 @@ int ensure_ws(Entry& e) {
     e.h_stage = nullptr;
     e.stream = nullptr;
     return -4;
-  }
-  if (e.f64_ctas > 0 && cudaMalloc(&e.d_f64_slab, e.f64_slab_stride * e.f64_ctas) != cudaSuccess) {
-    cudaGetLastError();  // no room for the FP64 form's own scratch: the SIMT form runs
-    e.d_f64_slab = nullptr;
-    e.f64_ctas = 0;
   }
   e.ws = true;
   return 0;
@@ -548,6 +543,21 @@ int mixed_launch_ctas(const Entry& e) {
   return std::max(1, std::min(e.mixed_ctas, g_sm_count * mixed_ctas_per_sm(e.tile_n)));
 }
 
+// Whether the FP64 form on the tensor cores runs for an evaluation on st: its scratch is allocated on first
+// use, but not inside a stream capture (calchem_xc_graph_capture asks before it begins), where the SIMT
+// form's scratch, there since the workspace was allocated, serves.
+bool f64tc_ready(Entry& e, cudaStream_t st) {
+  if (e.f64_ctas <= 0) return false;
+  if (e.d_f64_slab) return true;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return false;
+  if (cudaMalloc(&e.d_f64_slab, e.f64_slab_stride * e.f64_ctas) == cudaSuccess) return true;
+  cudaGetLastError();  // no room
+  e.d_f64_slab = nullptr;
+  e.f64_ctas = 0;
+  return false;
+}
+
 // Fixed-point copies of the densities for the FP64 form: [alpha n^2][beta n^2] of 8 bytes, then the rows'
 // exponents [alpha n][beta n] (the layout of the tensor-core form's split densities).
 bool f64tc_prepare(Entry& e, const double* Pa, const double* Pb, cudaStream_t st, int* launches) {
@@ -599,7 +609,7 @@ int enqueue_eval(Entry& e, int mode, int xc, int precision, const double* Pa, co
   const DevGrid G = dev_grid(e);
   cudaError_t err;
   const bool prof = e.profiling && e.ev0 && e.ev1;
-  const bool f64tc = precision == CALCHEM_XC_FP64 && e.f64_ctas > 0 && !simt;
+  const bool f64tc = precision == CALCHEM_XC_FP64 && !simt && f64tc_ready(e, st);
   if (precision == CALCHEM_XC_MIXED) {
     // packed fixed-point densities: [alpha n^2][beta n^2] uint2, then row exponents [alpha n][beta n]
     uint2* pk = reinterpret_cast<uint2*>(e.d_mixed_ws);
@@ -664,7 +674,7 @@ int enqueue_fxc(Entry& e, int triplet, const double* d_m, int n_trials, double* 
   if (cudaMemsetAsync(d_v, 0, nn * n_trials * sizeof(double), st) != cudaSuccess ||
       cudaMemsetAsync(e.d_counter, 0, 4 * sizeof(int), st) != cudaSuccess)
     return -5;
-  if (e.f64_ctas > 0) {  // one launch per trial matrix; the AO cache, filled by the first, serves them all
+  if (f64tc_ready(e, st)) {  // one launch per trial matrix; the AO cache, filled by the first, serves them all
     int launches = 0;
     for (int t = 0; t < n_trials; ++t) {
       // the queue head only: the status word keeps an earlier trial's failure
@@ -744,9 +754,26 @@ int enqueue_fxc_mixed(Entry& e, int triplet, const double* d_m, int n_trials, do
   return 0;
 }
 
+// Makes the pages of an output buffer resident (each one's first word written back to itself) while the GPU
+// works: the copies go straight between the caller's memory and the device, which this CPU and GPU share
+// page tables for, and a copy into pages never touched faults each of them on its way (10.7 MB: 65 us into
+// resident pages, 240-700 us into fresh ones; through a pinned staging buffer the host's own copies took
+// 0.4 ms in and 0.7 ms out).  The contents do not change, so an output may be the input itself.
+void touch_pages(double* p, size_t n) {
+  constexpr size_t kStep = 4096 / sizeof(double);
+  for (size_t i = 0; i < n; i += kStep) {
+    volatile double* x = p + i;
+    *x = *x;
+  }
+  if (n) {
+    volatile double* x = p + n - 1;
+    *x = *x;
+  }
+}
+
 // Waits for the grid's stream; -7 when a device-side wait of the last evaluation gave up.
 int finish(Entry& e) {
-  int* h_status = reinterpret_cast<int*>(e.h_stage + 2 * (size_t)e.nn_total + 3 * (size_t)e.n_mols + 1);
+  int* h_status = reinterpret_cast<int*>(e.h_stage + 3 * (size_t)e.n_mols + 1);
   if (cudaMemcpyAsync(h_status, e.d_counter + 2, sizeof(int), cudaMemcpyDeviceToHost, e.stream) != cudaSuccess ||
       cudaStreamSynchronize(e.stream) != cudaSuccess)
     return -5;
@@ -1050,8 +1077,7 @@ int calchem_cuda_vxc_eval_rho(uint64_t grid_id, const double* h_p_mat, double* h
   if (!e || e->n_mols != 1 || e->n_pts != n_pts || e->n_ao != n_ao) return -2;
   if (int rc0 = ensure_ws(*e)) return rc0;
   const size_t nn = (size_t)n_ao * n_ao;
-  std::memcpy(e->h_stage, h_p_mat, nn * sizeof(double));
-  if (cudaMemcpyAsync(e->d_P, e->h_stage, nn * sizeof(double), cudaMemcpyHostToDevice, e->stream) != cudaSuccess)
+  if (cudaMemcpyAsync(e->d_P, h_p_mat, nn * sizeof(double), cudaMemcpyHostToDevice, e->stream) != cudaSuccess)
     return -5;
   int rc = enqueue_eval(*e, kModeRho, 0, CALCHEM_XC_FP64, e->d_P, nullptr, nullptr, nullptr, nullptr, e->d_rg,
                         nullptr, e->stream);
@@ -1076,11 +1102,10 @@ int calchem_cuda_vxc_accum(uint64_t grid_id, const double* h_wv_in, double* h_vx
   int rc = enqueue_eval(*e, kModeAccum, 0, CALCHEM_XC_FP64, nullptr, nullptr, e->d_V, nullptr, e->d_rg, nullptr,
                         nullptr, e->stream);
   if (rc) return rc;
-  if (cudaMemcpyAsync(e->h_stage, e->d_V, nn * sizeof(double), cudaMemcpyDeviceToHost, e->stream) != cudaSuccess)
+  touch_pages(h_vxc_out, nn);
+  if (cudaMemcpyAsync(h_vxc_out, e->d_V, nn * sizeof(double), cudaMemcpyDeviceToHost, e->stream) != cudaSuccess)
     return -5;
-  if ((rc = finish(*e))) return rc;
-  std::memcpy(h_vxc_out, e->h_stage, nn * sizeof(double));
-  return 0;
+  return finish(*e);
 }
 
 int calchem_cuda_vxc_grad_force(uint64_t grid_id, const double* h_pa, const double* h_pb, int is_rks,
@@ -1378,22 +1403,21 @@ int calchem_xc_evaluate_rks(uint64_t grid_id, int xc_code, int precision, const 
   if (int rc0 = ensure_ws(*e)) return rc0;
   const size_t nn = (size_t)e->nn_total;
   const int M = e->n_mols;
-  std::memcpy(e->h_stage, h_d_total, nn * sizeof(double));
-  if (cudaMemcpyAsync(e->d_P, e->h_stage, nn * sizeof(double), cudaMemcpyHostToDevice, e->stream) != cudaSuccess)
+  if (cudaMemcpyAsync(e->d_P, h_d_total, nn * sizeof(double), cudaMemcpyHostToDevice, e->stream) != cudaSuccess)
     return -5;
   int rc = enqueue_eval(*e, kModeRks, xc_code, precision, e->d_P, nullptr, e->d_V, nullptr, nullptr, nullptr,
                         e->d_res, e->stream);
   if (rc) return rc;
-  double* h_res = e->h_stage + 2 * nn;
+  double* h_res = e->h_stage;
   int* h_status = reinterpret_cast<int*>(h_res + 3 * (size_t)M + 1);
-  if (cudaMemcpyAsync(e->h_stage, e->d_V, nn * sizeof(double), cudaMemcpyDeviceToHost, e->stream) != cudaSuccess ||
+  touch_pages(h_v_out, nn);
+  if (cudaMemcpyAsync(h_v_out, e->d_V, nn * sizeof(double), cudaMemcpyDeviceToHost, e->stream) != cudaSuccess ||
       cudaMemcpyAsync(h_res, e->d_res, 2 * (size_t)M * sizeof(double), cudaMemcpyDeviceToHost, e->stream) !=
           cudaSuccess ||
       cudaMemcpyAsync(h_status, e->d_counter + 2, sizeof(int), cudaMemcpyDeviceToHost, e->stream) != cudaSuccess ||
       cudaStreamSynchronize(e->stream) != cudaSuccess)
     return -5;
   if (*h_status != 0) return -7;
-  std::memcpy(h_v_out, e->h_stage, nn * sizeof(double));
   for (int i = 0; i < M; ++i) {
     exc_out[i] = h_res[2 * i];
     nelec_out[i] = h_res[2 * i + 1];
@@ -1418,14 +1442,13 @@ int calchem_xc_evaluate_rks_points(uint64_t grid_id, int xc_code, int precision,
   }
   const size_t nn = (size_t)e->nn_total;
   const int M = e->n_mols;
-  std::memcpy(e->h_stage, h_d_total, nn * sizeof(double));
   if (cudaMemsetAsync(e->d_pt_out, 0, np2 * sizeof(double), e->stream) != cudaSuccess ||
-      cudaMemcpyAsync(e->d_P, e->h_stage, nn * sizeof(double), cudaMemcpyHostToDevice, e->stream) != cudaSuccess)
+      cudaMemcpyAsync(e->d_P, h_d_total, nn * sizeof(double), cudaMemcpyHostToDevice, e->stream) != cudaSuccess)
     return -5;
   int rc = enqueue_eval(*e, kModeRks, xc_code, precision, e->d_P, nullptr, e->d_V, nullptr, nullptr, nullptr,
                         e->d_res, e->stream, e->d_pt_out);
   if (rc) return rc;
-  double* h_res = e->h_stage + 2 * nn;
+  double* h_res = e->h_stage;
   int* h_status = reinterpret_cast<int*>(h_res + 3 * (size_t)M + 1);
   if (cudaMemcpyAsync(h_res, e->d_res, 2 * (size_t)M * sizeof(double), cudaMemcpyDeviceToHost, e->stream) !=
           cudaSuccess ||
@@ -1463,28 +1486,24 @@ int calchem_xc_evaluate_uks(uint64_t grid_id, int xc_code, int precision, const 
   if (int rc0 = ensure_ws(*e)) return rc0;
   const size_t nn = (size_t)e->nn_total;
   const int M = e->n_mols;
-  std::memcpy(e->h_stage, h_pa, nn * sizeof(double));
-  std::memcpy(e->h_stage + nn, h_pb, nn * sizeof(double));
-  if (cudaMemcpyAsync(e->d_P, e->h_stage, nn * sizeof(double), cudaMemcpyHostToDevice, e->stream) != cudaSuccess ||
-      cudaMemcpyAsync(e->d_Pb, e->h_stage + nn, nn * sizeof(double), cudaMemcpyHostToDevice, e->stream) !=
-          cudaSuccess)
+  if (cudaMemcpyAsync(e->d_P, h_pa, nn * sizeof(double), cudaMemcpyHostToDevice, e->stream) != cudaSuccess ||
+      cudaMemcpyAsync(e->d_Pb, h_pb, nn * sizeof(double), cudaMemcpyHostToDevice, e->stream) != cudaSuccess)
     return -5;
   int rc = enqueue_eval(*e, kModeUks, xc_code, precision, e->d_P, e->d_Pb, e->d_V, e->d_Vb, nullptr, nullptr,
                         e->d_res, e->stream);
   if (rc) return rc;
-  double* h_res = e->h_stage + 2 * nn;
+  double* h_res = e->h_stage;
   int* h_status = reinterpret_cast<int*>(h_res + 3 * (size_t)M + 1);
-  if (cudaMemcpyAsync(e->h_stage, e->d_V, nn * sizeof(double), cudaMemcpyDeviceToHost, e->stream) != cudaSuccess ||
-      cudaMemcpyAsync(e->h_stage + nn, e->d_Vb, nn * sizeof(double), cudaMemcpyDeviceToHost, e->stream) !=
-          cudaSuccess ||
+  touch_pages(h_va_out, nn);
+  touch_pages(h_vb_out, nn);
+  if (cudaMemcpyAsync(h_va_out, e->d_V, nn * sizeof(double), cudaMemcpyDeviceToHost, e->stream) != cudaSuccess ||
+      cudaMemcpyAsync(h_vb_out, e->d_Vb, nn * sizeof(double), cudaMemcpyDeviceToHost, e->stream) != cudaSuccess ||
       cudaMemcpyAsync(h_res, e->d_res, 3 * (size_t)M * sizeof(double), cudaMemcpyDeviceToHost, e->stream) !=
           cudaSuccess ||
       cudaMemcpyAsync(h_status, e->d_counter + 2, sizeof(int), cudaMemcpyDeviceToHost, e->stream) != cudaSuccess ||
       cudaStreamSynchronize(e->stream) != cudaSuccess)
     return -5;
   if (*h_status != 0) return -7;
-  std::memcpy(h_va_out, e->h_stage, nn * sizeof(double));
-  std::memcpy(h_vb_out, e->h_stage + nn, nn * sizeof(double));
   for (int i = 0; i < M; ++i) {
     exc_out[i] = h_res[3 * i];
     nelec_out[2 * i] = h_res[3 * i + 1];
@@ -1601,15 +1620,15 @@ int calchem_xc_evaluate_rks_atoms(uint64_t grid_id, int xc_code, int precision, 
   if (!e->has_w) return -1;
   if (int rc0 = ensure_ws(*e)) return rc0;
   const size_t nn = (size_t)e->nn_total;
-  std::memcpy(e->h_stage, h_d_total, nn * sizeof(double));
-  if (cudaMemcpyAsync(e->d_P, e->h_stage, nn * sizeof(double), cudaMemcpyHostToDevice, e->stream) != cudaSuccess)
+  if (cudaMemcpyAsync(e->d_P, h_d_total, nn * sizeof(double), cudaMemcpyHostToDevice, e->stream) != cudaSuccess)
     return -5;
   int rc = enqueue_atom_shares(*e, xc_code, precision, e->d_P, e->d_res, h_v_out ? e->d_V : nullptr, e->d_atom_out,
                                e->stream);
   if (rc) return rc;
-  double* h_res = e->h_stage + 2 * nn;
+  double* h_res = e->h_stage;
   int* h_status = reinterpret_cast<int*>(h_res + 4);
-  if (h_v_out && cudaMemcpyAsync(e->h_stage, e->d_V, nn * sizeof(double), cudaMemcpyDeviceToHost, e->stream) !=
+  if (h_v_out) touch_pages(h_v_out, nn);
+  if (h_v_out && cudaMemcpyAsync(h_v_out, e->d_V, nn * sizeof(double), cudaMemcpyDeviceToHost, e->stream) !=
                      cudaSuccess)
     return -5;
   if (cudaMemcpyAsync(h_res, e->d_res, 2 * sizeof(double), cudaMemcpyDeviceToHost, e->stream) != cudaSuccess ||
@@ -1621,7 +1640,6 @@ int calchem_xc_evaluate_rks_atoms(uint64_t grid_id, int xc_code, int precision, 
   if (*h_status != 0) return -7;
   *exc_out = h_res[0];
   *nelec_out = h_res[1];
-  if (h_v_out) std::memcpy(h_v_out, e->h_stage, nn * sizeof(double));
   return 0;
 }
 
@@ -1648,8 +1666,7 @@ int calchem_xc_fxc_prepare(uint64_t grid_id, int xc_code, const double* h_d_tota
     return -4;
   }
   const size_t nn = (size_t)e->n_ao * e->n_ao;
-  std::memcpy(e->h_stage, h_d_total, nn * sizeof(double));
-  if (cudaMemcpyAsync(e->d_P, e->h_stage, nn * sizeof(double), cudaMemcpyHostToDevice, e->stream) != cudaSuccess)
+  if (cudaMemcpyAsync(e->d_P, h_d_total, nn * sizeof(double), cudaMemcpyHostToDevice, e->stream) != cudaSuccess)
     return -5;
   // The SIMT form's densities: once per ground state, so its speed matters little, while the kernel's finite
   // differences turn another form's roundings of rho (1e-16) into 5e-12 of dV, and into 4e-9 where the
@@ -1940,7 +1957,7 @@ int calchem_xc_graph_capture(uint64_t grid_id, int mode, int xc_code, int precis
   if (fp64_set_attributes() != cudaSuccess || mixed_set_attributes() != cudaSuccess ||
       f64tc_set_attributes() != cudaSuccess)
     return -5;
-  if (precision == CALCHEM_XC_MIXED || e->f64_ctas > 0) ao_cache_decide(*e, precision != CALCHEM_XC_MIXED);
+  if (precision == CALCHEM_XC_MIXED || f64tc_ready(*e, e->stream)) ao_cache_decide(*e, precision != CALCHEM_XC_MIXED);
   if (e->graph) {
     cudaGraphExecDestroy(e->graph);
     e->graph = nullptr;

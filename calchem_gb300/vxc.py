@@ -128,7 +128,7 @@ class GpuVxcGrid:
     def accumulate_vxc(self, wv) -> np.ndarray:
         lib = _native.load()
         w = np.ascontiguousarray(wv, dtype=np.float64).reshape(self.n_pts, 4)
-        out = np.zeros((self.n_ao, self.n_ao), dtype=np.float64)
+        out = np.empty((self.n_ao, self.n_ao), dtype=np.float64)
         _native.check("calchem_cuda_vxc_accum", lib.calchem_cuda_vxc_accum(
             self.grid_id, _native.ptr(w), _native.ptr(out), self.n_pts, self.n_ao))
         return out
@@ -371,7 +371,7 @@ class RksVxcEngine(_EngineBase):
     def evaluate(self, basis, grid, func, density_total, precision=None):
         lib = _native.load()
         P = _as_matrix(density_total, self.n_ao)
-        V = np.zeros((self.n_ao, self.n_ao), dtype=np.float64)
+        V = np.empty((self.n_ao, self.n_ao), dtype=np.float64)
         exc = np.zeros(1)
         ne = np.zeros(1)
         prec = self.precision if precision is None else _PRECISION[precision]
@@ -401,7 +401,7 @@ class RksVxcEngine(_EngineBase):
         if n_at <= 0:
             raise ValueError("set_point_atoms first")
         P = _as_matrix(density_total, self.n_ao)
-        V = np.zeros((self.n_ao, self.n_ao), dtype=np.float64)
+        V = np.empty((self.n_ao, self.n_ao), dtype=np.float64)
         out = np.zeros(2 * n_at)
         exc, ne = np.zeros(1), np.zeros(1)
         prec = self.precision if precision is None else _PRECISION[precision]
@@ -422,8 +422,8 @@ class UksVxcEngine(_EngineBase):
         lib = _native.load()
         Pa = _as_matrix(pa, self.n_ao)
         Pb = _as_matrix(pb, self.n_ao)
-        Va = np.zeros((self.n_ao, self.n_ao), dtype=np.float64)
-        Vb = np.zeros((self.n_ao, self.n_ao), dtype=np.float64)
+        Va = np.empty((self.n_ao, self.n_ao), dtype=np.float64)
+        Vb = np.empty((self.n_ao, self.n_ao), dtype=np.float64)
         exc = np.zeros(1)
         ne = np.zeros(2)
         prec = self.precision if precision is None else _PRECISION[precision]
@@ -577,7 +577,7 @@ class VxcGroup(_TileMixin):
         """-> (exc[n_mols], nelec[n_mols], [Vxc per member])."""
         lib = _native.load()
         P = self.pack(densities)
-        V = np.zeros(self.packed_size)
+        V = np.empty(self.packed_size)
         exc = np.zeros(self.n_mols)
         ne = np.zeros(self.n_mols)
         prec = self.precision if precision is None else _PRECISION[precision]
@@ -593,8 +593,8 @@ class VxcGroup(_TileMixin):
         lib = _native.load()
         Pa = self.pack(pas)
         Pb = self.pack(pbs)
-        Va = np.zeros(self.packed_size)
-        Vb = np.zeros(self.packed_size)
+        Va = np.empty(self.packed_size)
+        Vb = np.empty(self.packed_size)
         exc = np.zeros(self.n_mols)
         ne = np.zeros(2 * self.n_mols)
         prec = self.precision if precision is None else _PRECISION[precision]
