@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(kMT, MixCfg<kN>::kCtas) vxc_mixed_kernel(DevGr
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = warp_uniform(*tmem_slot);
   const uint32_t lane_base = (uint32_t)(32 * (warp & 3)) << 16;
   // TMEM: GEMM1 uses four kN-column accumulators (hh, hm+mh, hl+mm+lh, running sum); GEMM2, which
   // runs after GEMM1 is finished, uses 128 columns for its hh products and 128 for its corrections.
@@ -376,7 +376,8 @@ __global__ void __launch_bounds__(kMT, MixCfg<kN>::kCtas) vxc_mixed_kernel(DevGr
   const uint2* Dhl_b0 = Dhl_a0 + G.nn_total;
   const int* fexp_a0 = reinterpret_cast<const int*>(Dhl_a0 + 2 * G.nn_total);
   const int* fexp_b0 = fexp_a0 + G.n_total;
-  const uint32_t sb = smem_addr(stage);
+  const uint32_t sb = warp_uniform(smem_addr(stage));
+  const bool issuer = warp_uniform(warp) == 0 && elect_one();  // issues the MMAs (from uniform registers)
   // L2 policies: the packed A operand and the GEMM2 image tiles are read again (per N chunk, per
   // tile pair); the BF16 low planes are read for the last time by the GEMM1 epilogue
   const uint64_t pol_keep = l2_policy_evict_last(), pol_last_use = l2_policy_evict_first();
@@ -489,13 +490,11 @@ __global__ void __launch_bounds__(kMT, MixCfg<kN>::kCtas) vxc_mixed_kernel(DevGr
           gather_b<kN>(stage, Dhl, s_ao, n, m, kb, nc);
           fence_proxy_async_smem();
           if (!wait_tma()) { failed = true; break; }
-          if (tid == 0) {
+          if (issuer) {
             tc_fence_after();
-            const uint64_t ah = sdesc_sw128(sb), am = sdesc_sw128(sb + 16384), al = sdesc_sw128(sb + 32768);
-            const uint64_t aq = sdesc_sw128(sb + 49152);
-            // B pieces: kN rows of 128 bytes each, one after the other from +64 KB
-            const uint64_t bh = sdesc_sw128(sb + 65536), bm = sdesc_sw128(sb + 65536 + kN * 128);
-            const uint64_t bl = sdesc_sw128(sb + 65536 + 2 * kN * 128), bq = sdesc_sw128(sb + 65536 + 3 * kN * 128);
+            // A pieces of 16 KB, then the B pieces (kN rows of 128 bytes) one after the other from +64 KB
+            const uint64_t ah = sdesc_sw128(sb), am = ah + (16384 >> 4), al = ah + (32768 >> 4), aq = ah + (49152 >> 4);
+            const uint64_t bh = ah + (65536 >> 4), bm = bh + kN * 8, bl = bh + 2 * kN * 8, bq = bh + 3 * kN * 8;
             const bool group_start = (kb & 15) == 0;
 #pragma unroll
             for (int ks = 0; ks < 4; ++ks) {
@@ -782,7 +781,7 @@ __global__ void __launch_bounds__(kMT, MixCfg<kN>::kCtas) vxc_mixed_kernel(DevGr
     auto mma_half = [&](int da, int db, bool first) {
       uint64_t d[6];
 #pragma unroll
-      for (int t = 0; t < 6; ++t) d[t] = sdesc_sw128(sb + t * 16384);
+      for (int t = 0; t < 6; ++t) d[t] = sdesc_sw128(sb) + t * (16384 >> 4);
 #pragma unroll
       for (int ks = 0; ks < 4; ++ks) {
         const uint64_t o = (uint64_t)(ks * 2);
@@ -853,7 +852,7 @@ __global__ void __launch_bounds__(kMT, MixCfg<kN>::kCtas) vxc_mixed_kernel(DevGr
           }
           fence_proxy_async_smem();  // the tiles are read by the tensor core
           __syncthreads();
-          if (tid == 0) {
+          if (issuer) {
             tc_fence_after();
             mma_half(3, 0, kb2 == 0);  // A = Z, B = Phi
             mma_half(0, 3, false);     // A = Phi, B = Z
@@ -900,7 +899,7 @@ __global__ void __launch_bounds__(kMT, MixCfg<kN>::kCtas) vxc_mixed_kernel(DevGr
               tma_busy = true;
             }
             if (!wait_tma()) { failed = true; break; }
-            if (tid == 0) {
+            if (issuer) {
               tc_fence_after();
               mma_half(0, 3, rnd == 0);  // d[0..2] A (hi, mid, lo), d[3..5] B (hi, mid, lo)
               mma_commit(mbar);
