@@ -230,4 +230,11 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const float* v) {
   asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
+// *p += v where `on` (a predicated reduction: no branch)
+__device__ __forceinline__ void red_add_if(double* p, double v, bool on) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q red.global.add.f64 [%0], %1;\n\t}" ::"l"(p), "d"(v),
+               "r"((int)on)
+               : "memory");
+}
+
 }  // namespace cxc

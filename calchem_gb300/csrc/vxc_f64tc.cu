@@ -161,13 +161,6 @@ __device__ __forceinline__ void load4(const double* p, double (&x)[4]) {
   x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
 }
 
-// *p += v where `on` (a predicated reduction: no branch)
-__device__ __forceinline__ void red_add_if(double* p, double v, bool on) {
-  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %2, 0;\n\t@q red.global.add.f64 [%0], %1;\n\t}" ::"l"(p), "d"(v),
-               "r"((int)on)
-               : "memory");
-}
-
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])

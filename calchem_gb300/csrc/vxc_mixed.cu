@@ -807,8 +807,8 @@ __global__ void __launch_bounds__(kMT, MixCfg<kN>::kCtas) vxc_mixed_kernel(DevGr
         tmem_ld32(tWc + lane_base + (uint32_t)c0, wc);
 #pragma unroll
         for (int jj = 0; jj < 32; ++jj) wv[jj] += wc[jj];
-        if (i < m) {
-          const int ai = s_ao[i];
+        {
+          const int ai = s_ao[min(i, m - 1)];
 #pragma unroll
           for (int jj = 0; jj < 32; ++jj) {
             const int j = J + c0 + jj;
@@ -817,11 +817,12 @@ __global__ void __launch_bounds__(kMT, MixCfg<kN>::kCtas) vxc_mixed_kernel(DevGr
             // and skipping their updates changes an element of V by < 1e-11 per batch, far below
             // this form's ~1e-6 agreement with FP64 (max |dV| against FP64 on (H2O)61 and C8H18 the
             // same to three digits at 1e-13 and 1e-11), while it removes most of the FP64 atomics
-            if (j < m && (I != J || i >= j) && fabsf(wv[jj]) >= 1e-11f) {
-              const int aj = s_ao[j];
-              const int r = ai < aj ? ai : aj, c = ai < aj ? aj : ai;
-              atomicAdd(&V[(size_t)r * n + c], normal_f32_to_f64(wv[jj]));
-            }
+            // (a predicated reduction: a branch per element would keep the next one's address and value
+            // from being formed meanwhile; s_ao[j] beyond m is a stale row, in range and not used)
+            const int aj = s_ao[j];
+            const int r = ai < aj ? ai : aj, c = ai < aj ? aj : ai;
+            red_add_if(V + ((size_t)r * n + c), normal_f32_to_f64(wv[jj]),
+                       i < m && j < m && (I != J || i >= j) && fabsf(wv[jj]) >= 1e-11f);
           }
         }
       }
