@@ -100,7 +100,9 @@ static __device__ void becke_point(int n, const double* __restrict__ xyz, const 
     const double ax = xyz[3 * a], ay = xyz[3 * a + 1], az = xyz[3 * a + 2];
     const double ir = 1.0 / ra;
     const double dr0 = -(x - ax) * ir, dr1 = -(y - ay) * ir, dr2 = -(z - az) * ir;
-    double ph0 = 0, ph1 = 0, ph2 = 0, zz0 = 0, zz1 = 0, zz2 = 0;
+    // with k = slope / R_ab and m = mu_ab / R_ab: dZ/dR_a = sum_b d (dr - m (R_a - R_b)), d = (E_ab - E_ba) k,
+    // summed as dr sum d - sum d m (R_a - R_b)
+    double ph0 = 0, ph1 = 0, ph2 = 0, c = 0, zz0 = 0, zz1 = 0, zz2 = 0;
     const size_t row = (size_t)a * n;
     for (int b = 0; b < n; ++b) {
       if (b == a) continue;
@@ -110,17 +112,22 @@ static __device__ void becke_point(int n, const double* __restrict__ xyz, const 
       const double mu = clamp_unit((ra - W.dist[b]) * inv);
       const double v0 = ax - xyz[3 * b], v1 = ay - xyz[3 * b + 1], v2 = az - xyz[3 * b + 2];
       const double pa = W.e[row + b], pb = W.e[(size_t)b * n + a];
-      const double k = slope * inv;
-      const double ds0 = k * (dr0 - mu * v0 * inv), ds1 = k * (dr1 - mu * v1 * inv), ds2 = k * (dr2 - mu * v2 * inv);
-      zz0 += pa * ds0 - pb * ds0;
-      zz1 += pa * ds1 - pb * ds1;
-      zz2 += pa * ds2 - pb * ds2;
+      const double k = slope * inv, m = mu * inv;
+      const double d = (pa - pb) * k, dm = d * m;
+      c += d;
+      zz0 -= dm * v0;
+      zz1 -= dm * v1;
+      zz2 -= dm * v2;
       if (b == host) {
-        ph0 -= pb * ds0;
-        ph1 -= pb * ds1;
-        ph2 -= pb * ds2;
+        const double kb = pb * k;
+        ph0 = -kb * (dr0 - m * v0);
+        ph1 = -kb * (dr1 - m * v1);
+        ph2 = -kb * (dr2 - m * v2);
       }
     }
+    zz0 += c * dr0;
+    zz1 += c * dr1;
+    zz2 += c * dr2;
     const double w0 = pref * (ph0 - wn * zz0), w1 = pref * (ph1 - wn * zz1), w2 = pref * (ph2 - wn * zz2);
     W.wacc[3 * a] += w0;
     W.wacc[3 * a + 1] += w1;

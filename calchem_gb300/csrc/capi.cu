@@ -936,9 +936,9 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
   }
   const size_t nn = (size_t)n * n, na3 = 3 * (size_t)n_atoms;
   const size_t slab_stride = mixed ? grad_mixed_slab_doubles(e.max_m, n_atoms) : grad_slab_doubles(e.max_m, n_atoms);
-  // persistent CTAs (one per SM for FP64, two for the tensor-core form), fewer when the per-CTA
+  // persistent CTAs (two per SM), fewer when the per-CTA
   // scratch (AO planes and the warps' atom-pair tables) would take more than half of the free memory
-  int n_ctas = std::max(1, std::min(e.n_batches, g_sm_count * (mixed ? 2 : 1)));
+  int n_ctas = std::max(1, std::min(e.n_batches, 2 * g_sm_count));
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) {
     const size_t fit = free_b / 2 / (slab_stride * sizeof(double));
@@ -957,9 +957,9 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
                     : dalloc(&B.raw, e.n_pts) && dalloc(&B.xyz, na3) && dalloc(&B.inv, inv_r.size()) &&
                           dalloc(&B.aij, a_ij.size()) && dalloc(&B.pairs, pairs.size()) &&
                           dalloc(&B.pair_df, pair_df.size()));
-  // the tensor-core form runs the weight derivative as its own kernel when its tables fit
-  const bool becke_apart = mixed && xc >= 0 && becke_kernel_fits(n_atoms);
-  const int n_bk = becke_apart ? becke_kernel_ctas(e.n_pts) : 0;
+  // the weight derivative runs as its own kernel when its tables fit
+  const bool becke_apart = xc >= 0 && (mixed ? becke_kernel_fits(n_atoms) : becke_fp64_fits(n_atoms));
+  const int n_bk = !becke_apart ? 0 : mixed ? becke_kernel_ctas(e.n_pts) : becke_fp64_ctas(e.n_pts);
   if (ok && becke_apart) ok = dalloc(&B.fx, e.n_pts) && dalloc(&B.part2, (size_t)n_bk * na3);
   if (!ok) {
     cudaGetLastError();
@@ -1026,12 +1026,14 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
     A.Pa = reinterpret_cast<const double*>(e.d_mixed_ws);
     A.Pb = nullptr;
     if (launch_xc_grad_mixed(dev_grid(e), A, n_ctas, B.counter + 1, st) != cudaSuccess) return -5;
-    if (becke_apart) {
-      if (launch_becke_mixed(dev_grid(e), A, B.fx, B.part2, st) != cudaSuccess) return -5;
-      ++launches;
-    }
   } else if (launch_xc_grad(dev_grid(e), A, n_ctas, st) != cudaSuccess) {
     return -5;
+  }
+  if (becke_apart) {
+    if ((mixed ? launch_becke_mixed(dev_grid(e), A, B.fx, B.part2, st)
+               : launch_becke_fp64(dev_grid(e), A, B.fx, B.part2, st)) != cudaSuccess)
+      return -5;
+    ++launches;
   }
   if (launch_grad_reduce(B.part, e.n_batches, n_atoms, B.grad, st) != cudaSuccess) return -5;
   launches += 2;

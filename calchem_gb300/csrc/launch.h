@@ -63,6 +63,10 @@ cudaError_t launch_xc_grad_mixed(const DevGrid& G, const GradArgs& A, int n_ctas
 bool becke_kernel_fits(int n_atoms);
 int becke_kernel_ctas(int n_pts);
 cudaError_t launch_becke_mixed(const DevGrid& G, const GradArgs& A, const double* fx, double* part, cudaStream_t st);
+// The FP64 form's, likewise (becke.cu): rows part [becke_fp64_ctas(n_pts)][3 n_atoms].
+bool becke_fp64_fits(int n_atoms);
+int becke_fp64_ctas(int n_pts);
+cudaError_t launch_becke_fp64(const DevGrid& G, const GradArgs& A, const double* fx, double* part, cudaStream_t st);
 // grad[k] += sum over rows r (in order) of part[r][k]
 cudaError_t launch_grad_accumulate(const double* part, int n_rows, int n_atoms, double* grad, cudaStream_t st);
 // Dynamic shared-memory limits of the persistent kernels, set once per process (the launchers call

@@ -266,7 +266,7 @@ __device__ void density_from_t(const BatchDesc& bd, const double* __restrict__ s
   __syncthreads();
 }
 
-__global__ void __launch_bounds__(kGT, 1) xc_grad_kernel(DevGrid G, GradArgs A) {
+__global__ void __launch_bounds__(kGT, 2) xc_grad_kernel(DevGrid G, GradArgs A) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   GradSmem& S = *reinterpret_cast<GradSmem*>(smem_raw);
   double* acc = reinterpret_cast<double*>(smem_raw + sizeof(GradSmem));
@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(kGT, 1) xc_grad_kernel(DevGrid G, GradArgs A) 
   W.l = W.e + (size_t)n_at * n_at;
   const bool fused = A.xc >= 0;
   for (int k = tid; k < na3; k += kGT) acc[k] = 0.0;
-  if (fused)
+  if (fused && !A.fx_out)
     for (size_t k = tid; k < (size_t)kGWarps * per_warp; k += kGT) wscr[k] = 0.0;
   __syncthreads();
 
@@ -402,7 +402,8 @@ __global__ void __launch_bounds__(kGT, 1) xc_grad_kernel(DevGrid G, GradArgs A) 
       }
     }
     // (E) Becke weight derivative, one warp per point
-    if (fused && n_at > 1) {
+    if (A.fx_out && tid < kBlockPts && live) A.fx_out[pt] = S.fx[g];
+    if (fused && n_at > 1 && !A.fx_out) {
       for (int k = 0; k < kPtsPerWarp; ++k) {
         const int gg = warp * kPtsPerWarp + k;
         if (gg >= bd.n_pts) break;
@@ -420,7 +421,7 @@ __global__ void __launch_bounds__(kGT, 1) xc_grad_kernel(DevGrid G, GradArgs A) 
     for (int k = tid; k < na3; k += kGT) {
       double v = acc[k];
       acc[k] = 0.0;
-      if (fused) {
+      if (fused && !A.fx_out) {
         for (int w = 0; w < kGWarps; ++w) {
           double* wa = wscr + (size_t)w * per_warp + 2 * n_at;
           v += wa[k];
