@@ -110,6 +110,9 @@ struct Entry {
   double* d_atom_out = nullptr;     // 2 per atom (host-buffer calls)
   std::vector<int> h_host;          // host atom of every uploaded point (reference-layout uploads)
   std::vector<int> h_orig;          // caller's index of every uploaded point (empty: identity)
+  int* d_orig = nullptr;            // the same on the device (gradients)
+  void* d_grad = nullptr;           // gradient arena (grad_arena)
+  size_t grad_bytes = 0;
   int n_orig = 0;                   // points the caller passed (calchem_xc_upload_points*)
 
   void free_all() {
@@ -117,7 +120,7 @@ struct Entry {
                     d_P,      d_Pb,    d_V,     d_Vb,   d_rg,      d_red,   d_res,      d_counter, d_slab,
                     d_mixed_ws, d_mixed_slab, d_mol_n, d_mol_off, d_mol_ao_off, d_mol_boff, d_pt_out,
                     d_fxc, d_fxc_m, d_fxc_v, ao_cache.d, ao_cache.d_off, ao_cache.d_ok, f64_cache.d, f64_cache.d_off,
-                    f64_cache.d_ok, d_f64_slab, d_atom_pts, d_atom_off, d_atom_out};
+                    f64_cache.d_ok, d_f64_slab, d_orig, d_grad, d_atom_pts, d_atom_off, d_atom_out};
     for (void* p : ptrs)
       if (p) cudaFree(p);
     if (graph) cudaGraphExecDestroy(graph);
@@ -878,27 +881,60 @@ int grid_build_impl(int n_atoms, const int* z, const double* xyz_bohr, const std
   return 0;
 }
 
-// Device buffers of one gradient evaluation, freed on every return path.
+// Device buffers of one gradient evaluation, laid out in the grid's gradient arena (grad_arena).
 struct GradBufs {
   double *pa = nullptr, *pb = nullptr, *wxc = nullptr, *raw = nullptr, *xyz = nullptr, *inv = nullptr,
          *aij = nullptr, *part = nullptr, *slab = nullptr, *grad = nullptr;
   int *host = nullptr, *ao_atom = nullptr, *counter = nullptr;
   int2* pairs = nullptr;
   float2* pair_df = nullptr;
-  double *fx = nullptr, *part2 = nullptr;  // tensor-core form: per-point f, weight-derivative rows
-  ~GradBufs() {
-    void* ptrs[] = {pa, pb, wxc, raw, xyz, inv, aij, part, slab, grad, host, ao_atom, counter, pairs, pair_df,
-                    fx, part2};
-    for (void* p : ptrs)
-      if (p) cudaFree(p);
+  double *fx = nullptr, *part2 = nullptr;  // per-point f, weight-derivative rows (its own kernel)
+  double* raw_in = nullptr;                // the caller's raw weights and host atoms, in the caller's order
+  int* host_in = nullptr;
+};
+
+// Lays buffers out one after the other: with base = nullptr it only adds up their bytes.
+struct Arena {
+  unsigned char* base;
+  size_t off = 0;
+  explicit Arena(void* b) : base(static_cast<unsigned char*>(b)) {}
+  template <typename T>
+  void take(T** p, size_t n) {
+    if (base) *p = reinterpret_cast<T*>(base + off);
+    off += (std::max<size_t>(n, 1) * sizeof(T) + 1023) / 1024 * 1024;
   }
 };
 
+// The grid's gradient arena with at least `bytes`.  Allocating and freeing it on every call took 2 ms of an 11
+// ms gradient (0.7 GB of per-CTA scratch), so it is kept until the grid is released; grad_arena_trim gives
+// back one that holds more than a quarter of the free memory.
+bool grad_arena(Entry& e, size_t bytes) {
+  if (e.grad_bytes >= bytes) return true;
+  if (e.d_grad) cudaFree(e.d_grad);
+  e.d_grad = nullptr;
+  e.grad_bytes = 0;
+  if (cudaMalloc(&e.d_grad, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    e.d_grad = nullptr;
+    return false;
+  }
+  e.grad_bytes = bytes;
+  return true;
+}
+void grad_arena_trim(Entry& e) {
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && e.grad_bytes <= free_b / 4) return;
+  cudaGetLastError();
+  cudaFree(e.d_grad);
+  e.d_grad = nullptr;
+  e.grad_bytes = 0;
+}
+
 // Runs the gradient kernel on an uploaded single-molecule grid.  xc >= 0: fused form (h_raw and
-// the atoms' z / xyz used); xc < 0: drop-in form with h_wxc.  host_up: host atom per uploaded
-// point.  Returns 0, -1 (arguments), -3 (memory limit), -4 (allocation) or -5 (CUDA).
+// the atoms' z / xyz used); xc < 0: drop-in form with h_wxc.  host_atom: host atom per point (drop-in: per
+// uploaded point).  Returns 0, -1 (arguments), -3 (memory limit), -4 (allocation) or -5 (CUDA).
 int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_pa, const double* h_pb,
-                 const double* h_wxc, const double* h_raw, const int* host_up, int n_atoms, const int* z,
+                 const double* h_wxc, const double* h_raw, const int* host_atom, int n_atoms, const int* z,
                  const double* xyz, double* h_grad, size_t mem_limit) {
   const int n = e.n_ao;
   const bool mixed = precision == CALCHEM_XC_MIXED;
@@ -911,8 +947,29 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
     if (a.atom_index < 0 || a.atom_index >= n_atoms) return -1;
     for (int c = 0; c < a.n_funcs; ++c) ao_atom[a.ao_offset + c] = a.atom_index;
   }
-  for (int g = 0; g < e.n_pts; ++g)
-    if (host_up[g] < 0 || host_up[g] >= n_atoms) return -1;
+  // host_atom and h_raw are in the caller's order where the plan has one of its own (orig); points that the
+  // plan dropped may have any host
+  const bool planned = xc >= 0 && !e.h_orig.empty();
+  const int n_in = planned ? e.n_orig : e.n_pts;
+  unsigned worst = 0;
+  for (int g = 0; g < n_in; ++g) worst = std::max(worst, (unsigned)host_atom[g]);
+  if (worst >= (unsigned)n_atoms) {
+    if (!planned) return -1;
+    for (const int o : e.h_orig)
+      if ((unsigned)host_atom[o] >= (unsigned)n_atoms) return -1;
+  }
+  if (planned && !e.d_orig) {
+    if (!dalloc(&e.d_orig, e.n_pts)) {
+      cudaGetLastError();
+      return -4;
+    }
+    if (cudaMemcpy(e.d_orig, e.h_orig.data(), (size_t)e.n_pts * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess) {
+      cudaGetLastError();
+      cudaFree(e.d_orig);
+      e.d_orig = nullptr;
+      return -5;
+    }
+  }
   std::vector<double> inv_r, a_ij;
   std::vector<int2> pairs;
   std::vector<float2> pair_df;  // per ordered pair: 1 / R, a, (R_a - R_b) / R as float pairs
@@ -936,12 +993,12 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
   }
   const size_t nn = (size_t)n * n, na3 = 3 * (size_t)n_atoms;
   const size_t slab_stride = mixed ? grad_mixed_slab_doubles(e.max_m, n_atoms) : grad_slab_doubles(e.max_m, n_atoms);
-  // persistent CTAs (two per SM), fewer when the per-CTA
-  // scratch (AO planes and the warps' atom-pair tables) would take more than half of the free memory
+  // persistent CTAs (two per SM), fewer when the per-CTA scratch (AO planes and the warps' atom-pair tables)
+  // would take more than half of the free memory
   int n_ctas = std::max(1, std::min(e.n_batches, 2 * g_sm_count));
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) {
-    const size_t fit = free_b / 2 / (slab_stride * sizeof(double));
+    const size_t fit = (free_b + e.grad_bytes) / 2 / (slab_stride * sizeof(double));
     n_ctas = (int)std::max<size_t>(1, std::min<size_t>(n_ctas, fit));
   }
   size_t total = nn * sizeof(double) * (closed ? 1 : 2) + (size_t)e.n_pts * (xc < 0 ? 8 : 1) * sizeof(double) +
@@ -949,26 +1006,51 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
                  ((size_t)e.n_batches + 1) * na3 * sizeof(double) + slab_stride * n_ctas * sizeof(double) +
                  pairs.size() * sizeof(int2) + pair_df.size() * sizeof(float2) + 64;
   if (total > mem_limit) return -3;
-  GradBufs B;
-  bool ok = dalloc(&B.pa, nn) && (closed || dalloc(&B.pb, nn)) && dalloc(&B.host, e.n_pts) &&
-            dalloc(&B.ao_atom, n) && dalloc(&B.part, (size_t)e.n_batches * na3) && dalloc(&B.grad, na3) &&
-            dalloc(&B.slab, slab_stride * n_ctas) && dalloc(&B.counter, 2) &&
-            (xc < 0 ? dalloc(&B.wxc, (size_t)e.n_pts * 8)
-                    : dalloc(&B.raw, e.n_pts) && dalloc(&B.xyz, na3) && dalloc(&B.inv, inv_r.size()) &&
-                          dalloc(&B.aij, a_ij.size()) && dalloc(&B.pairs, pairs.size()) &&
-                          dalloc(&B.pair_df, pair_df.size()));
   // the weight derivative runs as its own kernel when its tables fit
   const bool becke_apart = xc >= 0 && (mixed ? becke_kernel_fits(n_atoms) : becke_fp64_fits(n_atoms));
   const int n_bk = !becke_apart ? 0 : mixed ? becke_kernel_ctas(e.n_pts) : becke_fp64_ctas(e.n_pts);
-  if (ok && becke_apart) ok = dalloc(&B.fx, e.n_pts) && dalloc(&B.part2, (size_t)n_bk * na3);
-  if (!ok) {
-    cudaGetLastError();
-    return -4;
-  }
+  GradBufs B;
+  auto lay_out = [&](void* base) {
+    Arena m(base);
+    m.take(&B.pa, nn);
+    if (!closed) m.take(&B.pb, nn);
+    m.take(&B.host, e.n_pts);
+    m.take(&B.ao_atom, n);
+    m.take(&B.part, (size_t)e.n_batches * na3);
+    m.take(&B.grad, na3);
+    m.take(&B.slab, slab_stride * n_ctas);
+    m.take(&B.counter, 2);
+    if (xc < 0) {
+      m.take(&B.wxc, (size_t)e.n_pts * 8);
+    } else {
+      m.take(&B.raw, e.n_pts);
+      m.take(&B.xyz, na3);
+      m.take(&B.inv, inv_r.size());
+      m.take(&B.aij, a_ij.size());
+      m.take(&B.pairs, pairs.size());
+      m.take(&B.pair_df, pair_df.size());
+    }
+    if (planned) {
+      m.take(&B.raw_in, n_in);
+      m.take(&B.host_in, n_in);
+    }
+    if (becke_apart) {
+      m.take(&B.fx, e.n_pts);
+      m.take(&B.part2, (size_t)n_bk * na3);
+    }
+    return m.off;
+  };
+  if (!grad_arena(e, lay_out(nullptr))) return -4;
+  lay_out(e.d_grad);
+  struct Trim {
+    Entry& e;
+    ~Trim() { grad_arena_trim(e); }
+  } trim{e};
   cudaStream_t st = e.stream;
-  ok = cudaMemcpyAsync(B.pa, h_pa, nn * sizeof(double), cudaMemcpyHostToDevice, st) == cudaSuccess &&
+  bool ok = cudaMemcpyAsync(B.pa, h_pa, nn * sizeof(double), cudaMemcpyHostToDevice, st) == cudaSuccess &&
        (closed || cudaMemcpyAsync(B.pb, h_pb, nn * sizeof(double), cudaMemcpyHostToDevice, st) == cudaSuccess) &&
-       cudaMemcpyAsync(B.host, host_up, (size_t)e.n_pts * sizeof(int), cudaMemcpyHostToDevice, st) == cudaSuccess &&
+       cudaMemcpyAsync(planned ? B.host_in : B.host, host_atom, (size_t)n_in * sizeof(int), cudaMemcpyHostToDevice,
+                       st) == cudaSuccess &&
        cudaMemcpyAsync(B.ao_atom, ao_atom.data(), (size_t)n * sizeof(int), cudaMemcpyHostToDevice, st) ==
            cudaSuccess &&
        cudaMemsetAsync(B.counter, 0, 2 * sizeof(int), st) == cudaSuccess &&
@@ -978,7 +1060,9 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
     ok = cudaMemcpyAsync(B.wxc, h_wxc, (size_t)e.n_pts * 8 * sizeof(double), cudaMemcpyHostToDevice, st) ==
          cudaSuccess;
   if (ok && xc >= 0)
-    ok = cudaMemcpyAsync(B.raw, h_raw, (size_t)e.n_pts * sizeof(double), cudaMemcpyHostToDevice, st) == cudaSuccess &&
+    ok = cudaMemcpyAsync(planned ? B.raw_in : B.raw, h_raw, (size_t)n_in * sizeof(double), cudaMemcpyHostToDevice,
+                         st) == cudaSuccess &&
+         (!planned || launch_grad_gather(B.raw_in, B.host_in, e.d_orig, e.n_pts, B.raw, B.host, st) == cudaSuccess) &&
          cudaMemcpyAsync(B.xyz, xyz, na3 * sizeof(double), cudaMemcpyHostToDevice, st) == cudaSuccess &&
          cudaMemcpyAsync(B.inv, inv_r.data(), inv_r.size() * sizeof(double), cudaMemcpyHostToDevice, st) ==
              cudaSuccess &&
@@ -1762,15 +1846,7 @@ int calchem_xc_nuclear_gradient(uint64_t grid_id, int xc_code, int precision, in
   std::fill(h_grad_out, h_grad_out + 3 * (size_t)n_atoms, 0.0);
   if (n_atoms == 1) return 0;  // translational invariance: no gradient for one atom (vxc.rs:1922-1924)
   if (int rc0 = ensure_ws(*e)) return rc0;
-  std::vector<double> raw(e->n_pts);
-  std::vector<int> host(e->n_pts);
-  for (int g = 0; g < e->n_pts; ++g) {
-    const int o = e->h_orig.empty() ? g : e->h_orig[g];
-    raw[g] = h_raw_w[o];
-    host[g] = h_host_atom[o];
-  }
-  return gradient_run(*e, xc_code, precision, h_pb == nullptr, h_pa, h_pb, nullptr, raw.data(), host.data(), n_atoms,
-                      z,
+  return gradient_run(*e, xc_code, precision, h_pb == nullptr, h_pa, h_pb, nullptr, h_raw_w, h_host_atom, n_atoms, z,
                       xyz_bohr, h_grad_out, SIZE_MAX);
 }
 

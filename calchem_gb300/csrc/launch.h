@@ -67,6 +67,9 @@ cudaError_t launch_becke_mixed(const DevGrid& G, const GradArgs& A, const double
 bool becke_fp64_fits(int n_atoms);
 int becke_fp64_ctas(int n_pts);
 cudaError_t launch_becke_fp64(const DevGrid& G, const GradArgs& A, const double* fx, double* part, cudaStream_t st);
+// raw[k] = raw_in[orig[k]], host[k] = host_in[orig[k]]: the caller's per-point arrays in planned order
+cudaError_t launch_grad_gather(const double* raw_in, const int* host_in, const int* orig, int n, double* raw, int* host,
+                               cudaStream_t st);
 // grad[k] += sum over rows r (in order) of part[r][k]
 cudaError_t launch_grad_accumulate(const double* part, int n_rows, int n_atoms, double* grad, cudaStream_t st);
 // Dynamic shared-memory limits of the persistent kernels, set once per process (the launchers call

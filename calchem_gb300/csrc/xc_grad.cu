@@ -451,6 +451,17 @@ __global__ void __launch_bounds__(256) grad_reduce_kernel(const double* __restri
   if (t == 0) grad[k] = accumulate ? grad[k] + s[0] : s[0];
 }
 
+// The caller's per-point arrays in planned order.
+__global__ void __launch_bounds__(256) grad_gather_kernel(const double* __restrict__ raw_in, const int* __restrict__ host_in,
+                                                          const int* __restrict__ orig, int n, double* __restrict__ raw,
+                                                          int* __restrict__ host) {
+  const int k = blockIdx.x * 256 + threadIdx.x;
+  if (k >= n) return;
+  const int o = orig[k];
+  raw[k] = raw_in[o];
+  host[k] = host_in[o];
+}
+
 }  // namespace
 
 size_t grad_smem_bytes(int n_atoms) { return sizeof(GradSmem) + (size_t)3 * n_atoms * sizeof(double); }
@@ -472,6 +483,12 @@ cudaError_t launch_xc_grad(const DevGrid& G, const GradArgs& A, int n_ctas, cuda
 
 cudaError_t launch_grad_reduce(const double* part, int n_batches, int n_atoms, double* grad, cudaStream_t st) {
   grad_reduce_kernel<<<3 * n_atoms, 256, 0, st>>>(part, n_batches, 3 * n_atoms, grad, 0);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_grad_gather(const double* raw_in, const int* host_in, const int* orig, int n, double* raw, int* host,
+                               cudaStream_t st) {
+  grad_gather_kernel<<<(n + 255) / 256, 256, 0, st>>>(raw_in, host_in, orig, n, raw, host);
   return cudaGetLastError();
 }
 
