@@ -30,6 +30,7 @@ CUDA_UNITS = {
     "fxc.cu": [],
     "xc_grad.cu": [],
     "xc_grad_mixed.cu": [],
+    "xc_grad_f64tc.cu": [],
     "becke.cu": [],
 }
 CXX_UNITS = {"host_prep.cpp": [], "integrals.cpp": []}

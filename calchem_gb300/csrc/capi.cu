@@ -992,23 +992,37 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
       }
   }
   const size_t nn = (size_t)n * n, na3 = 3 * (size_t)n_atoms;
-  const size_t slab_stride = mixed ? grad_mixed_slab_doubles(e.max_m, n_atoms) : grad_slab_doubles(e.max_m, n_atoms);
-  // persistent CTAs (two per SM), fewer when the per-CTA scratch (AO planes and the warps' atom-pair tables)
-  // would take more than half of the free memory
-  int n_ctas = std::max(1, std::min(e.n_batches, 2 * g_sm_count));
-  size_t free_b = 0, total_b = 0;
-  if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) {
-    const size_t fit = (free_b + e.grad_bytes) / 2 / (slab_stride * sizeof(double));
-    n_ctas = (int)std::max<size_t>(1, std::min<size_t>(n_ctas, fit));
-  }
-  size_t total = nn * sizeof(double) * (closed ? 1 : 2) + (size_t)e.n_pts * (xc < 0 ? 8 : 1) * sizeof(double) +
-                 (size_t)e.n_pts * sizeof(int) + (size_t)n * sizeof(int) + (inv_r.size() * 2 + na3) * sizeof(double) +
-                 ((size_t)e.n_batches + 1) * na3 * sizeof(double) + slab_stride * n_ctas * sizeof(double) +
-                 pairs.size() * sizeof(int2) + pair_df.size() * sizeof(float2) + 64;
-  if (total > mem_limit) return -3;
   // the weight derivative runs as its own kernel when its tables fit
   const bool becke_apart = xc >= 0 && (mixed ? becke_kernel_fits(n_atoms) : becke_fp64_fits(n_atoms));
   const int n_bk = !becke_apart ? 0 : mixed ? becke_kernel_ctas(e.n_pts) : becke_fp64_ctas(e.n_pts);
+  // the FP64 form's contractions run on the tensor cores where that kernel holds the batches and atoms and
+  // the weight derivative is not its own to do
+  bool f64tc = !mixed && grad_f64tc_fits(e.max_m, n_atoms) && (xc < 0 || becke_apart);
+  auto stride_of = [&](bool tc) {
+    return mixed ? grad_mixed_slab_doubles(e.max_m, n_atoms)
+                 : tc ? grad_f64tc_slab_doubles(e.max_m) : grad_slab_doubles(e.max_m, n_atoms);
+  };
+  const size_t fixed = nn * sizeof(double) * (closed ? 1 : 2) + (size_t)e.n_pts * (xc < 0 ? 8 : 1) * sizeof(double) +
+                       (size_t)e.n_pts * sizeof(int) + (size_t)n * sizeof(int) +
+                       (inv_r.size() * 2 + na3) * sizeof(double) + ((size_t)e.n_batches + 1) * na3 * sizeof(double) +
+                       pairs.size() * sizeof(int2) + pair_df.size() * sizeof(float2) + 64;
+  // persistent CTAs: up to two per SM, fewer when the per-CTA scratch (AO planes and the warps' atom-pair
+  // tables) would take more than half of the free memory
+  size_t free_b = 0, total_b = 0;
+  const bool know_free = cudaMemGetInfo(&free_b, &total_b) == cudaSuccess;
+  auto ctas_of = [&](int per_sm, size_t stride) {
+    const int c = std::max(1, std::min(e.n_batches, per_sm * g_sm_count));
+    const size_t fit = (free_b + e.grad_bytes) / 2 / (stride * sizeof(double));
+    return know_free ? (int)std::max<size_t>(1, std::min<size_t>(c, fit)) : c;
+  };
+  // the caller's limit: refused when the scratch of the SIMT form at one CTA per SM (or of the tensor-core
+  // form) does not fit, and kept to with fewer CTAs otherwise
+  const size_t least = stride_of(false) * ctas_of(mixed ? 2 : 1, stride_of(false)) * sizeof(double);
+  if (fixed + least > mem_limit) return -3;
+  if (f64tc && fixed + stride_of(true) * sizeof(double) > mem_limit) f64tc = false;
+  const size_t slab_stride = stride_of(f64tc);
+  const int n_ctas = (int)std::max<size_t>(
+      1, std::min<size_t>(ctas_of(2, slab_stride), (mem_limit - fixed) / (slab_stride * sizeof(double))));
   GradBufs B;
   auto lay_out = [&](void* base) {
     Arena m(base);
@@ -1110,6 +1124,11 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
     A.Pa = reinterpret_cast<const double*>(e.d_mixed_ws);
     A.Pb = nullptr;
     if (launch_xc_grad_mixed(dev_grid(e), A, n_ctas, B.counter + 1, st) != cudaSuccess) return -5;
+  } else if (f64tc) {
+    if (!f64tc_prepare(e, B.pa, closed ? nullptr : B.pb, st, &launches)) return -5;
+    A.Pa = reinterpret_cast<const double*>(e.d_mixed_ws);
+    A.Pb = nullptr;
+    if (launch_xc_grad_f64tc(dev_grid(e), A, n_ctas, B.counter + 1, st) != cudaSuccess) return -5;
   } else if (launch_xc_grad(dev_grid(e), A, n_ctas, st) != cudaSuccess) {
     return -5;
   }

@@ -53,6 +53,12 @@ size_t grad_smem_bytes(int n_atoms);
 int grad_max_atoms();
 cudaError_t launch_xc_grad(const DevGrid& G, const GradArgs& A, int n_ctas, cudaStream_t st);
 cudaError_t launch_grad_reduce(const double* part, int n_batches, int n_atoms, double* grad, cudaStream_t st);
+// The FP64 gradient's quadrature with its contractions on the tensor cores (xc_grad_f64tc.cu): A.Pa points at
+// the fixed-point densities of launch_f64tc_prepare; the weight derivative is left to A.fx_out's reader;
+// *status is set on a wait expiry.
+bool grad_f64tc_fits(int max_m, int n_atoms);
+size_t grad_f64tc_slab_doubles(int max_m);
+cudaError_t launch_xc_grad_f64tc(const DevGrid& G, const GradArgs& A, int n_ctas, int* status, cudaStream_t st);
 // Tensor-core form of the gradient (xc_grad_mixed.cu): GradArgs.Pa points at the split densities of
 // launch_mixed_prepare (alpha, then beta); part must be zeroed; *status is set on a wait expiry.
 size_t grad_mixed_slab_doubles(int max_m, int n_atoms);

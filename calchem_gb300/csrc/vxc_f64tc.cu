@@ -39,6 +39,7 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "f64_gemm.cuh"
 #include "f64_slices.cuh"
 #include "fp64_ao.cuh"
 #include "mixed_ops.cuh"
@@ -49,21 +50,7 @@ namespace cxc {
 
 namespace {
 
-using mix::st_shared_v4;
-using mix::sw128;
 using namespace f64s;
-
-constexpr int kT = 256;                       // threads per CTA, two CTAs per SM
-constexpr int kN = 48;                        // AO columns per accumulator
-constexpr int kCols = kN / 2;                 // columns per thread (two thread groups of 128)
-constexpr int kLevels = 5;
-constexpr uint32_t kTmem = 256;
-constexpr int kTiles = kSlices / 2;           // 128-byte rows hold two slices of 32 K values
-constexpr int kABytes = kTiles * 128 * 128;   // one K block (32) of a 128-row operand
-constexpr int kBTile = kN * 128;
-constexpr int kBBytes = kTiles * kBTile;
-constexpr int kMaxM = 2048;
-constexpr uint32_t kSpin = 1u << 26;
 
 constexpr int kOffCoef = kABytes + 2 * kBBytes;     // double [8][128]; two B buffers before it
 constexpr int kOffAo = kOffCoef + 8 * 128 * 8;      // uint16 [kMaxM]: AO (within the molecule) of each local row
@@ -77,10 +64,7 @@ constexpr int kSmem = kOffMisc + 96 + 1024;
 static_assert(2 * (kSmem + 1024) <= 233472, "two CTAs share one SM's shared memory");
 static_assert(kLevels * kN <= (int)kTmem, "the accumulators fit the CTA's TMEM columns");
 static_assert(8 * 128 * 8 <= kABytes, "the density sums live in the idle operand stage");
-constexpr int kENan = kScaleNan + 1023;  // biased exponents from here on give NaN
 constexpr int kENanMark = 4096;          // and are kept as this one where two of them are added up
-
-__host__ __device__ constexpr size_t up(size_t x, size_t k) { return (x + k - 1) / k * k; }
 
 // A batch's block: FP64 planes [4][m_k][128], the GEMM1 operand (m_k / 32 K blocks of 48 KB), the Phi
 // image (four 32-point K blocks of three tiles [m_r][128 B]), the Phi rows' exponents, the points'.
@@ -100,38 +84,6 @@ struct Block {
 };
 
 __host__ __device__ constexpr size_t z_bytes(int m) { return 12 * up(m, 128) * 128; }
-
-// Byte offset of slice s (even element pair words) for chunk c (8 K values) of row r in a K block's tiles.
-__device__ __forceinline__ uint32_t slice_off(int s, int r, int c) { return sw128(r, (s & 1) * 4 + c); }
-
-// Slices of 8 consecutive K values (Y[8]) stored as six 16-byte chunks: tile s >> 1 at base + (s >> 1) * tile.
-template <typename Store>
-__device__ __forceinline__ void store8(const unsigned long long (&Y)[8], int r, int c, Store&& store) {
-  uint32_t w[4][kSlices];
-#pragma unroll
-  for (int k = 0; k < 4; ++k) slice_pairs(Y[2 * k], Y[2 * k + 1], w[k]);
-#pragma unroll
-  for (int s = 0; s < kSlices; ++s) store(s >> 1, slice_off(s, r, c), make_uint4(w[0][s], w[1][s], w[2][s], w[3][s]));
-}
-
-// The GEMM1 A operand: Phi[g][mu] for 128 points, K = AOs, relative to each point's exponent.
-__device__ void pack_points(unsigned char* __restrict__ apack, const double* __restrict__ phi, const int* s_eg, int m,
-                            int m_k) {
-  for (int e = threadIdx.x; e < m_k / 8 * 128; e += kT) {
-    const int g = e & 127, c8 = e >> 7;
-    const int E = s_eg[g];
-    unsigned long long Y[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const int mu = 8 * c8 + k;
-      Y[k] = mu < m ? to_fixed(phi[(size_t)mu * 128 + g], E) : kBias;
-    }
-    unsigned char* t = apack + (size_t)(c8 >> 2) * kABytes;
-    store8(Y, g, c8 & 3, [&](int tile, uint32_t off, uint4 v) {
-      *reinterpret_cast<uint4*>(t + tile * 16384 + off) = v;
-    });
-  }
-}
 
 // One AO row over the batch's points into an image [4 K blocks][3 tiles][m_r rows][128 B], by one warp:
 // lane l holds points 4 l .. 4 l + 3.  Returns the row's exponent.
@@ -161,12 +113,6 @@ __device__ __forceinline__ void load4(const double* p, double (&x)[4]) {
   x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
 }
 
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-               : "r"(taddr));
-}
-
 __global__ void __launch_bounds__(kT, 2) vxc_f64tc_kernel(DevGrid G, EvalArgs A) {
   extern __shared__ unsigned char smem_raw[];
   unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -179,130 +125,20 @@ __global__ void __launch_bounds__(kT, 2) vxc_f64tc_kernel(DevGrid G, EvalArgs A)
   int* s_eg = reinterpret_cast<int*>(base + kOffEg);
   int* s_ef = reinterpret_cast<int*>(base + kOffEf);
   double(*red)[kT / 32] = reinterpret_cast<double(*)[kT / 32]>(base + kOffRed);
-  uint64_t* full = reinterpret_cast<uint64_t*>(base + kOffMisc);            // [3] A tile t has arrived
-  uint64_t* empty = reinterpret_cast<uint64_t*>(base + kOffMisc + 24);      // [3] the MMAs reading A tile t are done
-  uint64_t* full_b = reinterpret_cast<uint64_t*>(base + kOffMisc + 48);     // [2] B buffer (GEMM2) has arrived
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(base + kOffMisc + 64);
-  int* s_batch = reinterpret_cast<int*>(base + kOffMisc + 68);
+  int* s_batch = reinterpret_cast<int*>(base + kOffMisc + kGemmBytes);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = tid & 127, h = tid >> 7;
   const bool uks = A.mode == kModeUks;
 
-  if (tid == 0) {
-    for (int k = 0; k < 8; ++k) mbar_init(full + k, 1);  // full, empty, full_b
-    fence_mbar_init();
-  }
-  if (warp == 0) {
-    tmem_alloc(tmem_slot, kTmem);
-    tmem_relinquish();
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem = warp_uniform(*tmem_slot);
-  const uint32_t tl = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(h * kCols);  // this thread's columns
-  const uint32_t sb = warp_uniform(smem_addr(stage));
-  const bool issuer = warp_uniform(warp) == 0 && elect_one();  // copies the operands and issues the MMAs
-  const uint32_t idesc = idesc_bf16_f32(128, kN);
+  Gemm gemm;
+  gemm.begin(base, base + kOffMisc);
   bool failed = false;
 
   unsigned char* const slab = reinterpret_cast<unsigned char*>(A.slab + (size_t)blockIdx.x * A.slab_stride);
   unsigned char* const zimg = slab;  // the Z image, then the block of a batch without a cache block
   const unsigned long long* const Y0 = reinterpret_cast<const unsigned long long*>(A.Pa);
   const int* const f0 = reinterpret_cast<const int*>(Y0 + 2 * G.nn_total);
-  const uint64_t pol_keep = l2_policy_evict_last();
-
-  // One thread copies the operands and issues the MMAs.  An A tile (two slices) is copied again as soon as
-  // the MMAs reading it are done, so that the next K block's tiles arrive under the MMAs of the others.
-  // The state is that thread's: phases of the barriers, tiles whose release has not been waited for, copies
-  // not waited for (bits 0-2 A tiles, 3-4 B buffers).
-  uint32_t ph_full = 0, ph_empty = 0, pend = 0, inflight = 0;
-  auto wait_full = [&](int k) -> bool {  // k: 0-2 A tiles, 3-4 B buffers
-    uint64_t* bar = k < 3 ? full + k : full_b + (k - 3);
-    if (!mbar_wait_bounded(bar, (ph_full >> k) & 1u, kSpin)) return false;
-    ph_full ^= 1u << k;
-    inflight &= ~(1u << k);
-    return true;
-  };
-  auto wait_empty = [&](int t) -> bool {
-    if (!(pend >> t & 1u)) return true;
-    if (!mbar_wait_bounded(empty + t, (ph_empty >> t) & 1u, kSpin)) return false;
-    ph_empty ^= 1u << t;
-    pend &= ~(1u << t);
-    return true;
-  };
-  auto load_a = [&](const unsigned char* src, size_t tile_stride) -> bool {  // the three tiles of a K block
-#pragma unroll
-    for (int t = 0; t < kTiles; ++t) {
-      if (!wait_empty(t)) return false;
-      mbar_arrive_expect_tx(full + t, 16384);
-      bulk_g2s_hint(sb + t * 16384, src + t * tile_stride, 16384, full + t, pol_keep);
-      inflight |= 1u << t;
-    }
-    return true;
-  };
-  auto load_b = [&](int buf, const unsigned char* src, size_t tile_stride) {
-    mbar_arrive_expect_tx(full_b + buf, kBBytes);
-#pragma unroll
-    for (int t = 0; t < kTiles; ++t)
-      bulk_g2s_hint(sb + kABytes + buf * kBBytes + t * kBTile, src + t * tile_stride, kBTile, full_b + buf, pol_keep);
-    inflight |= 8u << buf;
-  };
-  // One K block of 32 against B buffer buf: slice products i + j <= 5, level min(i + j, 4) into
-  // accumulator columns 48 level; then the next K block's A copies (next != nullptr).  Returns with the
-  // MMAs done.
-  auto mma_round = [&](bool first, int buf, const unsigned char* next, size_t tile_stride) -> bool {
-    tc_fence_after();
-    const uint64_t db = sdesc_sw128(sb + kABytes) + (uint32_t)buf * (kBBytes >> 4);
-#pragma unroll
-    for (int t = 0; t < kTiles; ++t) {
-      if (!wait_full(t)) return false;
-      const uint64_t a = sdesc_sw128(sb) + t * 1024;
-#pragma unroll
-      for (int ks = 0; ks < 2; ++ks)
-#pragma unroll
-        for (int i = 2 * t; i < 2 * t + 2; ++i)
-#pragma unroll
-          for (int j = 0; i + j < kSlices; ++j) {
-            const int lev = i + j < kLevels ? i + j : kLevels - 1;
-            // each level's first product (i = 0, levels 0..4) overwrites at the start of a K group
-            const uint32_t acc = (first && ks == 0 && i == 0 && j < kLevels) ? 0u : 1u;
-            mma_bf16_ss(tmem + lev * kN, a + (i & 1) * 4 + ks * 2,
-                        db + (j >> 1) * (kBTile >> 4) + (j & 1) * 4 + ks * 2, idesc, acc);
-          }
-      mma_commit(empty + t);
-      pend |= 1u << t;
-    }
-    if (next) {
-      if (!load_a(next, tile_stride)) return false;
-    } else {
-#pragma unroll
-      for (int t = 0; t < kTiles; ++t)
-        if (!wait_empty(t)) return false;
-    }
-    tc_fence_before();
-    return true;
-  };
-  // the accumulators' K group into the thread's 64-bit sums
-  auto drain = [&](long long (&V)[kCols], int sh) {
-#pragma unroll
-    for (int c = 0; c < kCols; c += 8) {
-      uint32_t r[kLevels][8];
-#pragma unroll
-      for (int l = 0; l < kLevels; ++l) tmem_ld8(tl + l * kN + c, r[l]);
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-      for (int l = 0; l < kLevels; ++l)  // the loads' results are read after the wait
-#pragma unroll
-        for (int k = 0; k < 8; ++k) asm volatile("" : "+r"(r[l][k]));
-#pragma unroll
-      for (int k = 0; k < 8; ++k)
-        V[c + k] += level_sum(__uint_as_float(r[0][k]), __uint_as_float(r[1][k]), __uint_as_float(r[2][k]),
-                              __uint_as_float(r[3][k]), __uint_as_float(r[4][k])) >> sh;
-    }
-    tc_fence_before();
-  };
 
   while (!failed) {
     if (tid == 0) *s_batch = atomicAdd(A.counter, 1);
@@ -362,53 +198,12 @@ __global__ void __launch_bounds__(kT, 2) vxc_f64tc_kernel(DevGrid G, EvalArgs A)
       }
     }
 
-    const int sh = m > 1024 ? 1 : 0;
     double rho[2] = {0, 0}, gx[2] = {0, 0}, gy[2] = {0, 0}, gz[2] = {0, 0};
     for (int s = 0; s < (A.mode == kModeAccum ? 0 : uks ? 2 : 1) && !failed; ++s) {
       const unsigned long long* Yp = Y0 + (s ? G.nn_total : 0) + moff;
       const int* fp = f0 + (s ? G.n_total : 0) + roff;
       double sr = 0, sx = 0, sy = 0, sz = 0;
-      // B operand: kN density rows x 32 K, gathered through the batch's AO list (warps 2-7, under the MMAs
-      // of the K block before)
-      auto gather = [&](int nc, int kb, int buf) {
-        const int r = (tid - 64) >> 2, c = tid & 3;
-        const int k0 = kb * 32 + c * 8;
-        unsigned long long Y[8];
-        const unsigned long long* row = Yp + (nc + r < m ? (size_t)s_ao[nc + r] * n : 0);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) Y[k] = (nc + r < m && k0 + k < m) ? __ldg(row + s_ao[k0 + k]) : kBias;
-        const uint32_t o = sb + kABytes + buf * kBBytes;
-        store8(Y, r, c, [&](int tile, uint32_t off, uint4 v) { st_shared_v4(o + tile * kBTile + off, v); });
-        fence_proxy_async_smem();
-      };
-      int buf = 0;
-      bool bad = false;
-      if (issuer) bad = !load_a(blk + L.apack, 16384);
-      if (tid >= 64) gather(0, 0, 0);
-      __syncthreads();
-      for (int nc = 0; nc < m && !failed; nc += kN) {
-        // (double-buffered: slower threads may still read the previous chunk's)
-        int* const ef = s_ef + (nc / kN & 1) * 64;
-        if (tid < kN) ef[tid] = nc + tid < m ? fp[s_ao[nc + tid]] : 0;
-        long long V[kCols];
-#pragma unroll
-        for (int k = 0; k < kCols; ++k) V[k] = 0;
-        for (int kb = 0; kb < nkb; ++kb, buf ^= 1) {
-          const bool last_k = kb == nkb - 1;
-          const bool more = !last_k || nc + kN < m;
-          const int kb1 = last_k ? 0 : kb + 1;
-          if (issuer)
-            bad = bad || !mma_round((kb & 1) == 0, buf, more ? blk + L.apack + (size_t)kb1 * kABytes : nullptr, 16384);
-          else if (tid >= 64 && more)
-            gather(last_k ? nc + kN : nc, kb1, buf ^ 1);
-          if (__syncthreads_or(bad)) { failed = true; break; }
-          if ((kb & 1) || last_k) {
-            tc_fence_after();
-            drain(V, sh);
-            __syncthreads();
-          }
-        }
-        if (failed) break;
+      failed = !gemm.rows(blk + L.apack, Yp, fp, s_ao, s_ef, m, n, [&](int nc, const int* ef, long long (&V)[kCols]) {
         // rho = sum phi T, grad rho = 2 sum grad phi T; T = V 2^(E_f + E_g - 2096 + sh), the point's part
         // of the exponent applied to the sums
         // (columns beyond m have V = 0 and read the last row: no branches between the loads of a group)
@@ -424,18 +219,17 @@ __global__ void __launch_bounds__(kT, 2) vxc_f64tc_kernel(DevGrid G, EvalArgs A)
           }
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
-            const double t = scaled_or_nan(V[j0 + j], ef[h * kCols + j0 + j] - 1023 + sh);
+            const double t = scaled_or_nan(V[j0 + j], ef[h * kCols + j0 + j] - 1023 + sum_shift(m));
             sr = fma(p[j][0], t, sr);
             sx = fma(p[j][1], t, sx);
             sy = fma(p[j][2], t, sy);
             sz = fma(p[j][3], t, sz);
           }
         }
-      }
+      });
       if (failed) break;
       const int E = s_eg[g];
-      const double seg = E >= kENan ? __longlong_as_double(0x7FF8000000000000ll)
-                                    : (E > 51 ? __hiloint2double((E - 50) << 20, 0) : 0.0);
+      const double seg = point_scale(E);
       __syncthreads();
       dens[h][0][g] = sr * seg;
       dens[h][1][g] = sx * seg;
@@ -585,9 +379,9 @@ __global__ void __launch_bounds__(kT, 2) vxc_f64tc_kernel(DevGrid G, EvalArgs A)
       auto src_b = [&](int J, int kb) { return blk + L.img + ((size_t)kb * 3 * L.m_r + J) * 128; };
       const size_t st_a = (size_t)m_z * 128, st_b = (size_t)L.m_r * 128;
       bool bad = false;
-      if (issuer) {
-        bad = !load_a(src_a(0, 0), st_a);
-        load_b(0, src_b(0, 0), st_b);
+      if (gemm.issuer) {
+        bad = !gemm.load_a(src_a(0, 0), st_a);
+        gemm.load_b(0, src_b(0, 0), st_b);
       }
       for (int I = 0; I < m && !failed; I += 128) {
         for (int J = 0; J < m && !failed; J += kN) {
@@ -596,19 +390,19 @@ __global__ void __launch_bounds__(kT, 2) vxc_f64tc_kernel(DevGrid G, EvalArgs A)
           for (int k = 0; k < kCols; ++k) V[k] = 0;
           const int J1 = J + kN < m ? J + kN : 0, I1 = J1 ? I : I + 128;  // the next tile
           for (int kh = 0; kh < 2; ++kh) {
-            if (issuer)
+            if (gemm.issuer)
               for (int kb = 2 * kh; kb < 2 * kh + 2 && !bad; ++kb) {
                 const bool more = kb < 3 || I1 < m;
                 const unsigned char* next = nullptr;
                 if (more) {  // the other B buffer's MMAs (the K block before) are done
                   next = kb < 3 ? src_a(I, kb + 1) : src_a(I1, 0);
-                  load_b((kb + 1) & 1, kb < 3 ? src_b(J, kb + 1) : src_b(J1, 0), st_b);
+                  gemm.load_b((kb + 1) & 1, kb < 3 ? src_b(J, kb + 1) : src_b(J1, 0), st_b);
                 }
-                bad = !wait_full(3 + (kb & 1)) || !mma_round((kb & 1) == 0, kb & 1, next, st_a);
+                bad = !gemm.wait_full(3 + (kb & 1)) || !gemm.mma_round((kb & 1) == 0, kb & 1, next, st_a);
               }
             if (__syncthreads_or(bad)) { failed = true; break; }
             tc_fence_after();
-            drain(V, 0);
+            gemm.drain(V, 0);
             __syncthreads();
           }
           if (failed) break;
@@ -630,18 +424,8 @@ __global__ void __launch_bounds__(kT, 2) vxc_f64tc_kernel(DevGrid G, EvalArgs A)
     }
   }
 
-  if (failed) {
-    if (tid == 0) atomicExch(A.counter + 2, 1);
-    if (issuer) {
-      for (int k = 0; k < 5; ++k)
-        if (inflight >> k & 1u) wait_full(k);
-      for (int t = 0; t < kTiles; ++t) wait_empty(t);
-    }
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  if (warp == 0) tmem_dealloc(tmem, kTmem);
+  if (failed && tid == 0) atomicExch(A.counter + 2, 1);
+  gemm.end(failed);
 }
 
 // One CTA per packed density row: the row's exponent and the fixed-point Y of its elements.
