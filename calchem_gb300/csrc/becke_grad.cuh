@@ -1,5 +1,5 @@
 // becke_grad.cuh -- derivative of the Becke partition weight of one grid point with respect to the
-// nuclei (grid.rs:423-584), one warp per point; shared by the FP64 and tensor-core gradient kernels.
+// nuclei (grid.rs:423-584), one warp per point; shared by the gradient's kernels.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -9,28 +9,51 @@
 namespace cxc {
 namespace becke {
 
-// Becke step s(nu) and ds/dnu (grid.rs:129-140).
-__device__ __forceinline__ void step_d(double nu, double& s, double& ds) {
-  const double x = nu < -1.0 ? -1.0 : (nu > 1.0 ? 1.0 : nu);
-  const double f1 = 1.5 * x - 0.5 * x * x * x, d1 = 1.5 - 1.5 * x * x;
-  const double f2 = 1.5 * f1 - 0.5 * f1 * f1 * f1, d2 = 1.5 - 1.5 * f1 * f1;
-  const double f3 = 1.5 * f2 - 0.5 * f2 * f2 * f2, d3 = 1.5 - 1.5 * f2 * f2;
-  s = 0.5 * (1.0 - f3);
-  ds = -0.5 * d3 * d2 * d1;
+// v limited to [-1, 1], on the integer pipe (an FP64 comparison takes as long as an FP64 FMA)
+__device__ __forceinline__ double clamp_unit(double v) {
+  const int hi = __double2hiint(v);
+  const bool out = (hi & 0x7FFFFFFF) >= 0x3FF00000;
+  return out ? __hiloint2double((hi & (int)0x80000000) | 0x3FF00000, 0) : v;
 }
 
-__device__ __forceinline__ double clamp_unit(double v) { return v < -1.0 ? -1.0 : (v > 1.0 ? 1.0 : v); }
+// Becke step s(nu) and ds/dnu (grid.rs:129-140): three times f(x) = x (3 - x^2) / 2, f' = 3 (1 - x^2) / 2.
+__device__ __forceinline__ void step_d(double nu, double& s, double& ds) {
+  double x = clamp_unit(nu), d = -0.5;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const double x2 = x * x;
+    d *= fma(-1.5, x2, 1.5);
+    x *= fma(-0.5, x2, 1.5);
+  }
+  s = fma(-0.5, x, 0.5);
+  ds = d;
+}
 
-__host__ __device__ __forceinline__ size_t becke_scratch_doubles(int n) { return 5 * (size_t)n + 3 * (size_t)n * n; }
+// Row stride of the n x n tables: odd, so that lanes on consecutive rows of a table in shared memory fall into
+// different banks.
+__host__ __device__ __forceinline__ int becke_ld(int n) { return n | 1; }
 
-// Per-point pair tables of one warp (n x n, row-major), behind dist[n], cell[n] and wacc[3 n].
+__host__ __device__ __forceinline__ size_t becke_scratch_doubles(int n) {
+  return 5 * (size_t)n + 3 * (size_t)n * becke_ld(n);
+}
+
+// Per-point pair tables of one warp (n rows of becke_ld(n)), behind dist[n], cell[n] and wacc[3 n].
 struct BeckeScratch {
   double* dist;  // |r - R_c|
   double* cell;  // P_c = prod_{d != c} s_cd
   double* wacc;  // [3 n] the warp's weight-derivative sums
   double* s;     // s_cd (s_dc = 1 - s_cd, both stored; 1 for coincident atoms)
   double* e;     // prod_{d != c, k} s_cd at [c][k]
-  double* l;     // ds_cd/dmu_cd (the same for both orientations)
+  double* l;     // ds_cd/dmu_cd at [c][d], c < d
+  __device__ __forceinline__ void carve(double* base, int n) {
+    const size_t nn = (size_t)n * becke_ld(n);
+    dist = base;
+    cell = dist + n;
+    wacc = cell + n;
+    s = wacc + 3 * n;
+    e = s + nn;
+    l = e + nn;
+  }
 };
 
 // (E) raw_w f dW/dR for one point, one warp; wacc[3a + q] is owned by lane a % 32.
@@ -40,8 +63,11 @@ struct BeckeScratch {
 //      reference accumulates them) and every "product but one" prod_{d != c, k} s_cd as a prefix
 //      times a suffix product -- the reference's cell[c] / s_ck, or the explicit product when
 //      s_ck <= 1e-12 (grid.rs:500-515), without a division;
-//   3. lanes over atoms a != host: d(P_host / Z)/dR_a from the pairs (a, b) (grid.rs:517-583);
-//      the host atom gets minus their sum.
+//   3. lanes over the pairs: with k = ds/dmu / R_cd, m = mu_cd / R_cd and d = (E_cd - E_dc) k, the pair adds
+//      d to the sum that multiplies dr_c/dR_c in dZ/dR_c and d m (R_c - R_d) to the one subtracted from it,
+//      and the same with the other sign for atom d; they replace the pair's s and slope (grid.rs:517-583);
+//   4. lanes over atoms a != host: dZ/dR_a from the pairs' sums, dP_host/dR_a from the pair with the host;
+//      the host atom gets minus the others' sum.
 static __device__ void becke_point(int n, const double* __restrict__ xyz, const double* __restrict__ inv_r,
                             const double* __restrict__ a_ij, const int2* __restrict__ pairs, int n_pairs, int host,
                             double x, double y, double z, double pref_in, const BeckeScratch& W) {
@@ -51,28 +77,27 @@ static __device__ void becke_point(int n, const double* __restrict__ xyz, const 
     W.dist[c] = sqrt(dx * dx + dy * dy + dz * dz);
   }
   __syncwarp();
+  const int ld = becke_ld(n);
   for (int p = lane; p < n_pairs; p += 32) {
     const int c = pairs[p].x, d = pairs[p].y;
-    const size_t cd = (size_t)c * n + d, dc = (size_t)d * n + c;
-    const double inv = inv_r[cd];
-    double sv = 1.0, sl = 0.0;
+    const double inv = inv_r[(size_t)c * n + d];
+    double sv = 1.0, sc = 1.0, sl = 0.0;
     if (inv != 0.0) {
       const double mu = clamp_unit((W.dist[c] - W.dist[d]) * inv);
-      const double a = a_ij[cd];
-      double dsdnu;
-      step_d(mu + a * (1.0 - mu * mu), sv, dsdnu);
-      sl = dsdnu * (1.0 - 2.0 * a * mu);
+      const double a = a_ij[(size_t)c * n + d];
+      step_d(fma(a, fma(-mu, mu, 1.0), mu), sv, sl);
+      sl *= fma(-2.0 * a, mu, 1.0);
+      sc = 1.0 - sv;
     }
-    W.s[cd] = sv;
-    W.s[dc] = inv != 0.0 ? 1.0 - sv : 1.0;
-    W.l[cd] = sl;
-    W.l[dc] = sl;
+    W.s[c * ld + d] = sv;
+    W.s[d * ld + c] = sc;
+    W.l[c * ld + d] = sl;
   }
   __syncwarp();
   double zl = 0.0;
   for (int c = lane; c < n; c += 32) {
-    const double* __restrict__ sr = W.s + (size_t)c * n;
-    double* __restrict__ er = W.e + (size_t)c * n;
+    const double* __restrict__ sr = W.s + c * ld;
+    double* __restrict__ er = W.e + c * ld;
     double pre = 1.0;
     for (int k = 0; k < n; ++k) {
       er[k] = pre;
@@ -91,6 +116,31 @@ static __device__ void becke_point(int n, const double* __restrict__ xyz, const 
   __syncwarp();
   const double zs = zl;
   if (zs <= 1e-30) return;
+  for (int p = lane; p < n_pairs; p += 32) {
+    const int c = pairs[p].x, d = pairs[p].y;
+    const double slope = W.l[c * ld + d];
+    double q = 0.0, w0 = 0.0, w1 = 0.0, w2 = 0.0;
+    if ((__double2hiint(slope) & 0x7FFFFFFF) >= 0x39B40000) {  // |slope| above ~1e-30
+      const double inv = inv_r[(size_t)c * n + d];
+      const double mu = clamp_unit((W.dist[c] - W.dist[d]) * inv);
+      const double k = slope * inv, ec = W.e[c * ld + d], ed = W.e[d * ld + c];
+      q = (ec - ed) * k;
+      const double qm = q * (mu * inv);
+      w0 = qm * (xyz[3 * c] - xyz[3 * d]);
+      w1 = qm * (xyz[3 * c + 1] - xyz[3 * d + 1]);
+      w2 = qm * (xyz[3 * c + 2] - xyz[3 * d + 2]);
+      if (c == host) W.e[c * ld + d] = ec * k;  // E_{host a} k of the other atom a
+      if (d == host) W.e[d * ld + c] = ed * k;
+    } else {
+      if (c == host) W.e[c * ld + d] = 0.0;
+      if (d == host) W.e[d * ld + c] = 0.0;
+    }
+    W.l[c * ld + d] = q;
+    W.s[c * ld + d] = w0;
+    W.s[d * ld + c] = w1;
+    W.l[d * ld + c] = w2;
+  }
+  __syncwarp();
   const double wn = W.cell[host] / zs, pref = pref_in / zs;
   double h0 = 0, h1 = 0, h2 = 0;
   for (int a = lane; a < n; a += 32) {
@@ -98,33 +148,24 @@ static __device__ void becke_point(int n, const double* __restrict__ xyz, const 
     const double ra = W.dist[a];
     if (ra < 1e-14) continue;
     const double ax = xyz[3 * a], ay = xyz[3 * a + 1], az = xyz[3 * a + 2];
-    const double ir = 1.0 / ra;
-    const double dr0 = -(x - ax) * ir, dr1 = -(y - ay) * ir, dr2 = -(z - az) * ir;
-    // with k = slope / R_ab and m = mu_ab / R_ab: dZ/dR_a = sum_b d (dr - m (R_a - R_b)), d = (E_ab - E_ba) k,
-    // summed as dr sum d - sum d m (R_a - R_b)
-    double ph0 = 0, ph1 = 0, ph2 = 0, c = 0, zz0 = 0, zz1 = 0, zz2 = 0;
-    const size_t row = (size_t)a * n;
+    double c = 0, zz0 = 0, zz1 = 0, zz2 = 0;
     for (int b = 0; b < n; ++b) {
       if (b == a) continue;
-      const double inv = inv_r[row + b];
-      const double slope = W.l[row + b];
-      if (inv == 0.0 || fabs(slope) < 1e-30) continue;
-      const double mu = clamp_unit((ra - W.dist[b]) * inv);
-      const double v0 = ax - xyz[3 * b], v1 = ay - xyz[3 * b + 1], v2 = az - xyz[3 * b + 2];
-      const double pa = W.e[row + b], pb = W.e[(size_t)b * n + a];
-      const double k = slope * inv, m = mu * inv;
-      const double d = (pa - pb) * k, dm = d * m;
-      c += d;
-      zz0 -= dm * v0;
-      zz1 -= dm * v1;
-      zz2 -= dm * v2;
-      if (b == host) {
-        const double kb = pb * k;
-        ph0 = -kb * (dr0 - m * v0);
-        ph1 = -kb * (dr1 - m * v1);
-        ph2 = -kb * (dr2 - m * v2);
-      }
+      const int u = (b < a ? b : a) * ld + (b < a ? a : b), v = (b < a ? a : b) * ld + (b < a ? b : a);
+      const int sign = b < a ? (int)0x80000000 : 0;  // the pair (b, a) counts with the other sign
+      auto flip = [sign](double t) { return __hiloint2double(__double2hiint(t) ^ sign, __double2loint(t)); };
+      c += flip(W.l[u]);
+      zz0 -= flip(W.s[u]);
+      zz1 -= flip(W.s[v]);
+      zz2 -= flip(W.l[v]);
     }
+    const double ir = 1.0 / ra;
+    const double dr0 = -(x - ax) * ir, dr1 = -(y - ay) * ir, dr2 = -(z - az) * ir;
+    // dP_host/dR_a = -E_{host a} k (dr_a - mu_ah (R_a - R_h) / R_ah^2)
+    const double inv = inv_r[(size_t)a * n + host];
+    const double kb = W.e[host * ld + a], m = clamp_unit((ra - W.dist[host]) * inv) * inv;
+    const double ph0 = -kb * (dr0 - m * (ax - xyz[3 * host])), ph1 = -kb * (dr1 - m * (ay - xyz[3 * host + 1])),
+                 ph2 = -kb * (dr2 - m * (az - xyz[3 * host + 2]));
     zz0 += c * dr0;
     zz1 += c * dr1;
     zz2 += c * dr2;

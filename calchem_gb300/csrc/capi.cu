@@ -889,6 +889,7 @@ struct GradBufs {
   int2* pairs = nullptr;
   float2* pair_df = nullptr;
   double *fx = nullptr, *part2 = nullptr;  // per-point f, weight-derivative rows (its own kernel)
+  double* tables = nullptr;                // the FP64 weight derivative's pair tables (larger molecules)
   double* raw_in = nullptr;                // the caller's raw weights and host atoms, in the caller's order
   int* host_in = nullptr;
 };
@@ -993,14 +994,14 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
   }
   const size_t nn = (size_t)n * n, na3 = 3 * (size_t)n_atoms;
   // the weight derivative runs as its own kernel when its tables fit
-  const bool becke_apart = xc >= 0 && (mixed ? becke_kernel_fits(n_atoms) : becke_fp64_fits(n_atoms));
-  const int n_bk = !becke_apart ? 0 : mixed ? becke_kernel_ctas(e.n_pts) : becke_fp64_ctas(e.n_pts);
-  // the FP64 form's contractions run on the tensor cores where that kernel holds the batches and atoms and
-  // the weight derivative is not its own to do
-  bool f64tc = !mixed && grad_f64tc_fits(e.max_m, n_atoms) && (xc < 0 || becke_apart);
+  const bool becke_apart = xc >= 0 && n_atoms > 1 && (!mixed || becke_kernel_fits(n_atoms));
+  const int n_bk = !becke_apart ? 0 : mixed ? becke_kernel_ctas(e.n_pts) : becke_fp64_ctas(e.n_pts, n_atoms);
+  const size_t n_tables = becke_apart && !mixed ? becke_fp64_table_doubles(e.n_pts, n_atoms) : 0;
+  // the FP64 form's contractions run on the tensor cores where that kernel holds the batches and atoms
+  bool f64tc = !mixed && grad_f64tc_fits(e.max_m, n_atoms);
   auto stride_of = [&](bool tc) {
     return mixed ? grad_mixed_slab_doubles(e.max_m, n_atoms)
-                 : tc ? grad_f64tc_slab_doubles(e.max_m) : grad_slab_doubles(e.max_m, n_atoms);
+                 : tc ? grad_f64tc_slab_doubles(e.max_m) : grad_slab_doubles(e.max_m);
   };
   const size_t fixed = nn * sizeof(double) * (closed ? 1 : 2) + (size_t)e.n_pts * (xc < 0 ? 8 : 1) * sizeof(double) +
                        (size_t)e.n_pts * sizeof(int) + (size_t)n * sizeof(int) +
@@ -1015,9 +1016,11 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
     const size_t fit = (free_b + e.grad_bytes) / 2 / (stride * sizeof(double));
     return know_free ? (int)std::max<size_t>(1, std::min<size_t>(c, fit)) : c;
   };
-  // the caller's limit: refused when the scratch of the SIMT form at one CTA per SM (or of the tensor-core
-  // form) does not fit, and kept to with fewer CTAs otherwise
-  const size_t least = stride_of(false) * ctas_of(mixed ? 2 : 1, stride_of(false)) * sizeof(double);
+  // the caller's limit: refused when the scratch of the SIMT form at one CTA per SM (with eight warps' atom-pair
+  // tables each) does not fit, and kept to with fewer CTAs otherwise
+  const size_t pair_tables = 8 * (5 * (size_t)n_atoms + 3 * (size_t)n_atoms * n_atoms);
+  const size_t simt = stride_of(false) + (mixed ? 0 : pair_tables);
+  const size_t least = simt * ctas_of(mixed ? 2 : 1, simt) * sizeof(double);
   if (fixed + least > mem_limit) return -3;
   if (f64tc && fixed + stride_of(true) * sizeof(double) > mem_limit) f64tc = false;
   const size_t slab_stride = stride_of(f64tc);
@@ -1051,6 +1054,7 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
     if (becke_apart) {
       m.take(&B.fx, e.n_pts);
       m.take(&B.part2, (size_t)n_bk * na3);
+      m.take(&B.tables, n_tables);
     }
     return m.off;
   };
@@ -1134,7 +1138,7 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
   }
   if (becke_apart) {
     if ((mixed ? launch_becke_mixed(dev_grid(e), A, B.fx, B.part2, st)
-               : launch_becke_fp64(dev_grid(e), A, B.fx, B.part2, st)) != cudaSuccess)
+               : launch_becke_fp64(dev_grid(e), A, B.fx, B.part2, B.tables, st)) != cudaSuccess)
       return -5;
     ++launches;
   }

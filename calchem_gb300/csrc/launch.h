@@ -48,7 +48,7 @@ cudaError_t launch_fxc_coef(const double* rho_grad, const double* w, int n_pts, 
                             cudaStream_t st);
 // XC nuclear gradient (xc_grad.cu): per-CTA scratch, shared memory, the persistent kernel and the
 // batch-ordered sum of its [batch][atom][3] partials into grad.
-size_t grad_slab_doubles(int max_m, int n_atoms);
+size_t grad_slab_doubles(int max_m);
 size_t grad_smem_bytes(int n_atoms);
 int grad_max_atoms();
 cudaError_t launch_xc_grad(const DevGrid& G, const GradArgs& A, int n_ctas, cudaStream_t st);
@@ -69,10 +69,12 @@ cudaError_t launch_xc_grad_mixed(const DevGrid& G, const GradArgs& A, int n_ctas
 bool becke_kernel_fits(int n_atoms);
 int becke_kernel_ctas(int n_pts);
 cudaError_t launch_becke_mixed(const DevGrid& G, const GradArgs& A, const double* fx, double* part, cudaStream_t st);
-// The FP64 form's, likewise (becke.cu): rows part [becke_fp64_ctas(n_pts)][3 n_atoms].
-bool becke_fp64_fits(int n_atoms);
-int becke_fp64_ctas(int n_pts);
-cudaError_t launch_becke_fp64(const DevGrid& G, const GradArgs& A, const double* fx, double* part, cudaStream_t st);
+// The FP64 form's, likewise (becke.cu): rows part [becke_fp64_ctas][3 n_atoms], and for larger molecules
+// becke_fp64_table_doubles of scratch.
+int becke_fp64_ctas(int n_pts, int n_atoms);
+size_t becke_fp64_table_doubles(int n_pts, int n_atoms);
+cudaError_t launch_becke_fp64(const DevGrid& G, const GradArgs& A, const double* fx, double* part, double* tables,
+                              cudaStream_t st);
 // raw[k] = raw_in[orig[k]], host[k] = host_in[orig[k]]: the caller's per-point arrays in planned order
 cudaError_t launch_grad_gather(const double* raw_in, const int* host_in, const int* orig, int n, double* raw, int* host,
                                cudaStream_t st);

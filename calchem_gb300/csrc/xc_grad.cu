@@ -7,7 +7,7 @@
 //               + sum_g raw_w_g f_g d(Becke weight_g)/dR_A        (grid.rs:423-584)
 // with u_a = 2 v_gamma_aa grad rho_a + v_gamma_ab grad rho_b (and a <-> b).
 //
-// One persistent CTA of 256 threads takes 128-point batches from a device queue.  Per batch:
+// Persistent CTAs of 256 threads, two per SM, take 128-point batches from a device queue.  Per batch:
 //   (A) phi, grad phi and the six second derivatives of every candidate AO at the batch's points
 //       into ten planes of a per-CTA scratch slab (screening of ao_grid.rs for the Hessian form:
 //       shell cutoff r^2 > r2_cutoff; radial value, slope and curvature all below 1e-18);
@@ -17,16 +17,17 @@
 //       each AO row's force from T, Y, grad phi and the Hessian, reduces it over the points with
 //       warp shuffles and adds it, row by row in a fixed order, into the batch's per-atom sums;
 //       every point's total goes to its host atom with the opposite sign;
-//   (E) the Becke weight derivative, one warp per point, lanes over atoms (two passes of O(n^2)
-//       pair terms: cell functions, then the derivative of P_host / Z for every atom but the host,
-//       whose term is minus their sum);
-//   (F) the batch's per-atom sums go to its own row of a [batch][atom][3] array; a second kernel
+//   (E) the batch's per-atom sums go to its own row of a [batch][atom][3] array; a second kernel
 //       adds the rows in batch order.  Results are therefore deterministic.
-// The drop-in form (calchem_cuda_vxc_grad_force, cuda_kernels.cu:4351-4580) skips (B), (C) and
-// (E): the per-point coefficients come from the caller, and only the AO term is returned.
+// f goes to the weight derivative's own kernel (becke.cu).  The drop-in form (calchem_cuda_vxc_grad_force,
+// cuda_kernels.cu:4351-4580) skips (B) and (C): the per-point coefficients come from the caller, and only
+// the AO term is returned.
+//
+// xc_grad_f64tc.cu does the same with (B)'s and (D)'s contractions on the tensor cores, 2.6 times as fast; this
+// form runs for batches of more than 2048 AOs, more than 256 atoms, or a memory limit without room for one
+// CTA of the other.
 #include <cuda_runtime.h>
 
-#include "becke_grad.cuh"
 #include "common.cuh"
 #include "fp64_ao.cuh"
 #include "launch.h"
@@ -36,15 +37,10 @@ namespace cxc {
 
 namespace {
 
-using becke::BeckeScratch;
-using becke::becke_point;
-using becke::becke_scratch_doubles;
-
 constexpr int kGT = 256;        // threads
 constexpr int kGRows = 64;      // AO rows per tile (32 per half)
 constexpr int kGK = 32;         // depth per tile
 constexpr int kGWarps = kGT / 32;
-constexpr int kPtsPerWarp = kBlockPts / kGWarps;
 // slab planes
 constexpr int kPhi = 0, kGrad = 1, kHess = 4, kPsi = 10, kT = 12;
 constexpr int kGradPlanes = 14;
@@ -204,26 +200,12 @@ __global__ void __launch_bounds__(kGT, 2) xc_grad_kernel(DevGrid G, GradArgs A) 
   const int tid = threadIdx.x;
   const int g = tid & (kBlockPts - 1);
   const int h = tid >> 7;
-  const int warp = tid >> 5, lane = tid & 31;
   const int na3 = 3 * A.n_atoms;
   const int m_pad = (A.max_m + kGRows - 1) / kGRows * kGRows;
   const size_t plane = (size_t)m_pad * kBlockPts;
   double* slab = A.slab + (size_t)blockIdx.x * A.slab_stride;
-  // Becke scratch of each warp behind the planes: dist[n], cell[n], wacc[3n], s, e, l [n x n]
-  double* wscr = slab + (size_t)kGradPlanes * plane;
-  const int n_at = A.n_atoms;
-  const size_t per_warp = becke_scratch_doubles(n_at);
-  BeckeScratch W;
-  W.dist = wscr + (size_t)warp * per_warp;
-  W.cell = W.dist + n_at;
-  W.wacc = W.cell + n_at;
-  W.s = W.wacc + 3 * n_at;
-  W.e = W.s + (size_t)n_at * n_at;
-  W.l = W.e + (size_t)n_at * n_at;
   const bool fused = A.xc >= 0;
   for (int k = tid; k < na3; k += kGT) acc[k] = 0.0;
-  if (fused && !A.fx_out)
-    for (size_t k = tid; k < (size_t)kGWarps * per_warp; k += kGT) wscr[k] = 0.0;
   __syncthreads();
 
   while (true) {
@@ -332,38 +314,16 @@ __global__ void __launch_bounds__(kGT, 2) xc_grad_kernel(DevGrid G, GradArgs A) 
         acc[3 * S.host[gg] + tid] -= S.hsum[0][tid][gg] + S.hsum[1][tid][gg];
       }
     }
-    // (E) Becke weight derivative, one warp per point
-    if (A.fx_out && tid < kBlockPts && live) A.fx_out[pt] = S.fx[g];
-    if (fused && n_at > 1 && !A.fx_out) {
-      for (int k = 0; k < kPtsPerWarp; ++k) {
-        const int gg = warp * kPtsPerWarp + k;
-        if (gg >= bd.n_pts) break;
-        const double f = S.fx[gg];
-        const size_t p = (size_t)bd.pt_start + gg;
-        const double rw = A.raw_w[p];
-        if (fabs(f) < 1e-18 || rw == 0.0) continue;
-        becke_point(n_at, A.xyz, A.inv_r, A.a_ij, A.pairs, A.n_pairs, S.host[gg], G.px[p], G.py[p], G.pz[p], rw * f,
-                    W);
-      }
-    }
+    if (A.fx_out && tid < kBlockPts && live) A.fx_out[pt] = S.fx[g];  // (for the weight derivative)
     __syncthreads();
-    // (F) the batch's row of per-atom sums
+    // (E) the batch's row of per-atom sums
     double* out = A.part + (size_t)b * na3;
     for (int k = tid; k < na3; k += kGT) {
-      double v = acc[k];
+      out[k] = acc[k];
       acc[k] = 0.0;
-      if (fused && !A.fx_out) {
-        for (int w = 0; w < kGWarps; ++w) {
-          double* wa = wscr + (size_t)w * per_warp + 2 * n_at;
-          v += wa[k];
-          wa[k] = 0.0;
-        }
-      }
-      out[k] = v;
     }
     __syncthreads();
   }
-  (void)lane;
 }
 
 // grad[k] = sum over batches b (in order) of part[b][k]; one CTA per entry k.
@@ -397,9 +357,9 @@ __global__ void __launch_bounds__(256) grad_gather_kernel(const double* __restri
 
 size_t grad_smem_bytes(int n_atoms) { return sizeof(GradSmem) + (size_t)3 * n_atoms * sizeof(double); }
 
-size_t grad_slab_doubles(int max_m, int n_atoms) {
+size_t grad_slab_doubles(int max_m) {
   const size_t m_pad = (size_t)(max_m + kGRows - 1) / kGRows * kGRows;
-  return (size_t)kGradPlanes * m_pad * kBlockPts + (size_t)kGWarps * becke_scratch_doubles(n_atoms);
+  return (size_t)kGradPlanes * m_pad * kBlockPts;
 }
 
 int grad_max_atoms() { return kMaxGradAtoms; }
