@@ -75,7 +75,7 @@ struct Entry {
   double* d_rg = nullptr;
   double* d_red = nullptr;
   double* d_res = nullptr;
-  int* d_counter = nullptr;
+  int* d_counter = nullptr;   // queue heads [0], [1] and the status word [2], at d_res + 3 n_mols + 4
   double* d_slab = nullptr;
   size_t slab_stride = 0;
   int n_ctas = 0;
@@ -117,7 +117,7 @@ struct Entry {
 
   void free_all() {
     void* ptrs[] = {d_shells, d_prims, d_comps, d_prim_f, d_comp_f, d_shell_cf, d_pts,  d_batches, d_cand,  d_cand_loc, d_bao,   d_order,
-                    d_P,      d_Pb,    d_V,     d_Vb,   d_rg,      d_red,   d_res,      d_counter, d_slab,
+                    d_P,      d_Pb,    d_V,     d_Vb,   d_rg,      d_red,   d_res,      d_slab,
                     d_mixed_ws, d_mixed_slab, d_mol_n, d_mol_off, d_mol_ao_off, d_mol_boff, d_pt_out,
                     d_fxc, d_fxc_m, d_fxc_v, ao_cache.d, ao_cache.d_off, ao_cache.d_ok, f64_cache.d, f64_cache.d_off,
                     f64_cache.d_ok, d_f64_slab, d_orig, d_grad, d_atom_pts, d_atom_off, d_atom_out};
@@ -278,7 +278,7 @@ int ensure_ws(Entry& e) {
   const size_t nn = (size_t)e.nn_total;
   bool ok = dalloc(&e.d_P, nn) && dalloc(&e.d_Pb, nn) && dalloc(&e.d_V, nn) && dalloc(&e.d_Vb, nn) &&
             (e.n_mols != 1 || dalloc(&e.d_rg, (size_t)e.n_pts * 4)) && dalloc(&e.d_red, (size_t)e.n_batches * 3) &&
-            dalloc(&e.d_res, 3 * (size_t)e.n_mols + 8) && dalloc(&e.d_counter, 4) &&
+            dalloc(&e.d_res, 3 * (size_t)e.n_mols + 8) &&
             dalloc(&e.d_slab, e.slab_stride * e.n_ctas) &&
             cudaMalloc(&e.d_mixed_ws, nn * sizeof(uint2) * 2 + (size_t)e.n_ao * 2 * sizeof(int)) == cudaSuccess &&
             dalloc(&e.d_mixed_slab, e.mixed_slab_stride * e.mixed_ctas) &&
@@ -286,8 +286,7 @@ int ensure_ws(Entry& e) {
             cudaStreamCreateWithFlags(&e.stream, cudaStreamNonBlocking) == cudaSuccess;
   if (!ok) {
     cudaGetLastError();
-    void* ptrs[] = {e.d_P, e.d_Pb, e.d_V, e.d_Vb, e.d_rg, e.d_red, e.d_res, e.d_counter, e.d_slab, e.d_mixed_ws,
-                    e.d_mixed_slab};
+    void* ptrs[] = {e.d_P, e.d_Pb, e.d_V, e.d_Vb, e.d_rg, e.d_red, e.d_res, e.d_slab, e.d_mixed_ws, e.d_mixed_slab};
     for (void* p : ptrs)
       if (p) cudaFree(p);
     if (e.h_stage) cudaFreeHost(e.h_stage);
@@ -299,6 +298,7 @@ int ensure_ws(Entry& e) {
     e.stream = nullptr;
     return -4;
   }
+  e.d_counter = reinterpret_cast<int*>(e.d_res + 3 * (size_t)e.n_mols + 4);
   e.ws = true;
   return 0;
 }
@@ -561,19 +561,41 @@ bool f64tc_ready(Entry& e, cudaStream_t st) {
   return false;
 }
 
-// Fixed-point copies of the densities for the FP64 form: [alpha n^2][beta n^2] of 8 bytes, then the rows'
-// exponents [alpha n][beta n] (the layout of the tensor-core form's split densities).
-bool f64tc_prepare(Entry& e, const double* Pa, const double* Pb, cudaStream_t st, int* launches) {
-  const size_t nn = (size_t)e.nn_total;
-  unsigned long long* y = reinterpret_cast<unsigned long long*>(e.d_mixed_ws);
-  int* fx = reinterpret_cast<int*>(y + 2 * nn);
-  for (int s = 0; s < (Pb ? 2 : 1); ++s) {
-    if (launch_f64tc_prepare(s ? Pb : Pa, e.n_ao, e.d_mol_n, e.d_mol_off, e.d_mol_ao_off, e.n_mols, y + s * nn,
-                             fx + s * (size_t)e.n_ao, st) != cudaSuccess)
-      return false;
-    ++*launches;
-  }
-  return true;
+// The densities' operand copies of a tensor-core form (fp64: vxc_f64tc.cu's fixed point, else vxc_mixed.cu's
+// split): [alpha n^2][beta n^2] of 8 bytes, then the rows' exponents [alpha n][beta n].  The same launch
+// clears Va, Vb (nullptr: none) and the first n_counter words of the queues and the status.
+bool prepare(Entry& e, bool fp64, const double* Pa, const double* Pb, double* Va, double* Vb, int n_counter,
+             cudaStream_t st) {
+  PrepareArgs p{};
+  p.P[0] = Pa;
+  p.P[1] = Pb;
+  p.V[0] = Va;
+  p.V[1] = Vb;
+  p.n_spin = Pb ? 2 : 1;
+  p.n_total = e.n_ao;
+  p.mol_n = e.d_mol_n;
+  p.mol_off = e.d_mol_off;
+  p.mol_ao_off = e.d_mol_ao_off;
+  p.n_mols = e.n_mols;
+  p.out = e.d_mixed_ws;
+  p.nn = (size_t)e.nn_total;
+  p.fexp = reinterpret_cast<int*>(static_cast<unsigned char*>(e.d_mixed_ws) + 16 * p.nn);
+  p.counter = e.d_counter;
+  p.n_counter = n_counter;
+  return (fp64 ? launch_f64tc_prepare(p, st) : launch_mixed_prepare(p, st)) == cudaSuccess;
+}
+
+// The end of an evaluation of the grid's molecules into Va, Vb (nullptr: none).
+FinishArgs finish_args(const Entry& e, double* Va, double* Vb, int kind) {
+  FinishArgs f{};
+  f.n_mols = e.n_mols;
+  f.V[0] = Va;
+  f.V[1] = Vb;
+  f.n = e.max_n;
+  f.mol_n = e.d_mol_n;
+  f.mol_off = e.d_mol_off;
+  f.kind = kind;
+  return f;
 }
 
 void f64tc_args(Entry& e, cudaStream_t st, EvalArgs& A) {
@@ -590,11 +612,18 @@ int enqueue_eval(Entry& e, int mode, int xc, int precision, const double* Pa, co
                  double* point_out = nullptr, bool shares_only = false, bool simt = false) {
   const size_t nn = (size_t)e.nn_total;
   int launches = 0;
-  if (mode != kModeRho && !shares_only) {
-    if (cudaMemsetAsync(Va, 0, nn * sizeof(double), st) != cudaSuccess) return -5;
-    if (mode == kModeUks && cudaMemsetAsync(Vb, 0, nn * sizeof(double), st) != cudaSuccess) return -5;
+  const bool uks = mode == kModeUks;
+  const bool f64tc = precision == CALCHEM_XC_FP64 && !simt && f64tc_ready(e, st);
+  double* const clear_a = mode != kModeRho && !shares_only ? Va : nullptr;
+  double* const clear_b = clear_a && uks ? Vb : nullptr;
+  if (mode != kModeAccum && (f64tc || precision == CALCHEM_XC_MIXED)) {
+    if (!prepare(e, f64tc, Pa, uks ? Pb : nullptr, clear_a, clear_b, 4, st)) return -5;
+    ++launches;
+  } else {
+    if (clear_a && cudaMemsetAsync(clear_a, 0, nn * sizeof(double), st) != cudaSuccess) return -5;
+    if (clear_b && cudaMemsetAsync(clear_b, 0, nn * sizeof(double), st) != cudaSuccess) return -5;
+    if (cudaMemsetAsync(e.d_counter, 0, 4 * sizeof(int), st) != cudaSuccess) return -5;  // queues + status
   }
-  if (cudaMemsetAsync(e.d_counter, 0, 4 * sizeof(int), st) != cudaSuccess) return -5;  // queues + status
   EvalArgs A{};
   A.mode = mode;
   A.xc = xc;
@@ -612,21 +641,7 @@ int enqueue_eval(Entry& e, int mode, int xc, int precision, const double* Pa, co
   const DevGrid G = dev_grid(e);
   cudaError_t err;
   const bool prof = e.profiling && e.ev0 && e.ev1;
-  const bool f64tc = precision == CALCHEM_XC_FP64 && !simt && f64tc_ready(e, st);
   if (precision == CALCHEM_XC_MIXED) {
-    // packed fixed-point densities: [alpha n^2][beta n^2] uint2, then row exponents [alpha n][beta n]
-    uint2* pk = reinterpret_cast<uint2*>(e.d_mixed_ws);
-    int* fx = reinterpret_cast<int*>(pk + 2 * nn);
-    if (launch_mixed_prepare(Pa, e.n_ao, e.d_mol_n, e.d_mol_off, e.d_mol_ao_off, e.n_mols, pk, fx, st) !=
-        cudaSuccess)
-      return -5;
-    ++launches;
-    if (mode == kModeUks) {
-      if (launch_mixed_prepare(Pb, e.n_ao, e.d_mol_n, e.d_mol_off, e.d_mol_ao_off, e.n_mols, pk + nn, fx + e.n_ao,
-                               st) != cudaSuccess)
-        return -5;
-      ++launches;
-    }
     A.slab = e.d_mixed_slab;
     A.slab_stride = e.mixed_slab_stride;
     A.Pa = (const double*)e.d_mixed_ws;  // the tensor-core kernel reads the split copies
@@ -636,7 +651,6 @@ int enqueue_eval(Entry& e, int mode, int xc, int precision, const double* Pa, co
     err = launch_mixed(G, A, mixed_launch_ctas(e), st);
     if (prof) cudaEventRecord(e.ev1, st);
   } else if (f64tc) {
-    if (mode != kModeAccum && !f64tc_prepare(e, Pa, mode == kModeUks ? Pb : nullptr, st, &launches)) return -5;
     f64tc_args(e, st, A);
     if (prof) cudaEventRecord(e.ev0, st);
     err = launch_f64tc(G, A, e.f64_ctas, st);
@@ -650,21 +664,18 @@ int enqueue_eval(Entry& e, int mode, int xc, int precision, const double* Pa, co
   }
   if (err != cudaSuccess) return -5;
   ++launches;
-  if (mode == kModeRks || mode == kModeUks) {
-    if (launch_reduce(e.d_red, e.n_batches, e.d_mol_boff, e.n_mols, result, mode == kModeRks ? 2 : 3, st) !=
-        cudaSuccess)
-      return -5;
+  const int kind = f64tc ? kFinishSum : precision == CALCHEM_XC_MIXED ? kFinishFromUpper : kFinishFromLower;
+  if (mode == kModeRks || uks) {
+    FinishArgs f = finish_args(e, clear_a, clear_b, kind);
+    f.part = e.d_red;
+    f.n_batches = e.n_batches;
+    f.batch_off = e.d_mol_boff;
+    f.out = result;
+    f.n_out = uks ? 3 : 2;
+    if (launch_finish(f, st) != cudaSuccess) return -5;
     ++launches;
-    auto complete = [&](double* V) {
-      ++launches;
-      return f64tc ? launch_symmetrise(V, e.max_n, e.d_mol_n, e.d_mol_off, e.n_mols, 0, st)
-                   : launch_mirror(V, e.max_n, e.d_mol_n, e.d_mol_off, e.n_mols,
-                                   precision == CALCHEM_XC_MIXED ? 1 : 0, st);
-    };
-    if (!shares_only && complete(Va) != cudaSuccess) return -5;
-    if (mode == kModeUks && complete(Vb) != cudaSuccess) return -5;
   } else if (mode == kModeAccum && f64tc) {
-    if (launch_symmetrise(Va, e.max_n, e.d_mol_n, e.d_mol_off, e.n_mols, 1, st) != cudaSuccess) return -5;
+    if (launch_finish(finish_args(e, Va, nullptr, kFinishSumLower), st) != cudaSuccess) return -5;
     ++launches;
   }
   e.last_launches = launches;
@@ -674,14 +685,8 @@ int enqueue_eval(Entry& e, int mode, int xc, int precision, const double* Pa, co
 // TD-DFT kernel contraction of n_trials symmetric matrices d_m (each n x n) into d_v.
 int enqueue_fxc(Entry& e, int triplet, const double* d_m, int n_trials, double* d_v, cudaStream_t st) {
   const size_t nn = (size_t)e.n_ao * e.n_ao;
-  if (cudaMemsetAsync(d_v, 0, nn * n_trials * sizeof(double), st) != cudaSuccess ||
-      cudaMemsetAsync(e.d_counter, 0, 4 * sizeof(int), st) != cudaSuccess)
-    return -5;
   if (f64tc_ready(e, st)) {  // one launch per trial matrix; the AO cache, filled by the first, serves them all
-    int launches = 0;
     for (int t = 0; t < n_trials; ++t) {
-      // the queue head only: the status word keeps an earlier trial's failure
-      if (t > 0 && cudaMemsetAsync(e.d_counter, 0, sizeof(int), st) != cudaSuccess) return -5;
       EvalArgs A{};
       A.mode = kModeFxc;
       A.Va = d_v + t * nn;
@@ -690,16 +695,19 @@ int enqueue_fxc(Entry& e, int triplet, const double* d_m, int n_trials, double* 
       A.batch_red = e.d_red;
       A.counter = e.d_counter;
       A.max_m = e.max_m;
-      if (!f64tc_prepare(e, d_m + t * nn, nullptr, st, &launches)) return -5;
+      // (after the first trial the queue heads only: the status word keeps an earlier trial's failure)
+      if (!prepare(e, true, d_m + t * nn, nullptr, A.Va, nullptr, t ? 2 : 4, st)) return -5;
       f64tc_args(e, st, A);
       if (launch_f64tc(dev_grid(e), A, e.f64_ctas, st) != cudaSuccess ||
-          launch_symmetrise(A.Va, e.n_ao, nullptr, nullptr, 1, 0, st) != cudaSuccess)
+          launch_finish(finish_args(e, A.Va, nullptr, kFinishSum), st) != cudaSuccess)
         return -5;
-      launches += 2;
     }
-    e.last_launches = launches;
+    e.last_launches = 3 * n_trials;
     return 0;
   }
+  if (cudaMemsetAsync(d_v, 0, nn * n_trials * sizeof(double), st) != cudaSuccess ||
+      cudaMemsetAsync(e.d_counter, 0, 4 * sizeof(int), st) != cudaSuccess)
+    return -5;
   EvalArgs A{};
   A.mode = kModeFxc;
   A.xc = e.fxc_code;
@@ -715,7 +723,7 @@ int enqueue_fxc(Entry& e, int triplet, const double* d_m, int n_trials, double* 
   A.slab_stride = e.slab_stride;
   if (launch_fp64(dev_grid(e), A, e.n_ctas, st) != cudaSuccess) return -5;
   for (int t = 0; t < n_trials; ++t)
-    if (launch_mirror(d_v + t * nn, e.n_ao, 0, st) != cudaSuccess) return -5;
+    if (launch_finish(finish_args(e, d_v + t * nn, nullptr, kFinishFromLower), st) != cudaSuccess) return -5;
   e.last_launches = 1 + n_trials;
   return 0;
 }
@@ -726,16 +734,10 @@ int enqueue_fxc(Entry& e, int triplet, const double* d_m, int n_trials, double* 
 int enqueue_fxc_mixed(Entry& e, int triplet, const double* d_m, int n_trials, double* d_v, cudaStream_t st) {
   const size_t nn = (size_t)e.n_ao * e.n_ao;
   if (mixed_set_attributes() != cudaSuccess) return -5;
-  uint2* pk = reinterpret_cast<uint2*>(e.d_mixed_ws);
-  int* fx = reinterpret_cast<int*>(pk + 2 * nn);
   const DevGrid G = dev_grid(e);
   for (int t = 0; t < n_trials; ++t) {
     double* v = d_v + t * nn;
-    if (cudaMemsetAsync(v, 0, nn * sizeof(double), st) != cudaSuccess ||
-        cudaMemsetAsync(e.d_counter, 0, 4 * sizeof(int), st) != cudaSuccess)
-      return -5;
-    if (launch_mixed_prepare(d_m + t * nn, e.n_ao, nullptr, nullptr, nullptr, 1, pk, fx, st) != cudaSuccess)
-      return -5;
+    if (!prepare(e, false, d_m + t * nn, nullptr, v, nullptr, t ? 2 : 4, st)) return -5;
     EvalArgs A{};
     A.mode = kModeFxc;
     A.Pa = (const double*)e.d_mixed_ws;
@@ -751,7 +753,7 @@ int enqueue_fxc_mixed(Entry& e, int triplet, const double* d_m, int n_trials, do
     use_ao_cache(e, false, st, A);
     A.tile_n = e.tile_n;
     if (launch_mixed(G, A, mixed_launch_ctas(e), st) != cudaSuccess) return -5;
-    if (launch_mirror(v, e.n_ao, 1, st) != cudaSuccess) return -5;
+    if (launch_finish(finish_args(e, v, nullptr, kFinishFromUpper), st) != cudaSuccess) return -5;
   }
   e.last_launches = 3 * n_trials;
   return 0;
@@ -774,13 +776,13 @@ void touch_pages(double* p, size_t n) {
   }
 }
 
-// Waits for the grid's stream; -7 when a device-side wait of the last evaluation gave up.
+// Waits for the grid's stream, with the last host call's sums in h_stage; -7 when a device-side wait gave up.
 int finish(Entry& e) {
-  int* h_status = reinterpret_cast<int*>(e.h_stage + 3 * (size_t)e.n_mols + 1);
-  if (cudaMemcpyAsync(h_status, e.d_counter + 2, sizeof(int), cudaMemcpyDeviceToHost, e.stream) != cudaSuccess ||
+  const size_t at = 3 * (size_t)e.n_mols + 4;  // the queue heads and the status word follow the sums
+  if (cudaMemcpyAsync(e.h_stage, e.d_res, (at + 2) * sizeof(double), cudaMemcpyDeviceToHost, e.stream) != cudaSuccess ||
       cudaStreamSynchronize(e.stream) != cudaSuccess)
     return -5;
-  return *h_status != 0 ? -7 : 0;
+  return reinterpret_cast<const int*>(e.h_stage + at)[2] != 0 ? -7 : 0;
 }
 
 bool valid_xc(int xc) { return xc >= 0 && xc <= 8; }
@@ -1117,19 +1119,14 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
   if (e.profiling) cudaEventRecord(e.ev0, st);
   if (mixed) {
     // split copies of the spin densities for the tensor-core contractions (alpha, then beta)
-    uint2* pk = reinterpret_cast<uint2*>(e.d_mixed_ws);
-    int* fx = reinterpret_cast<int*>(pk + 2 * nn);
-    if (launch_mixed_prepare(B.pa, n, nullptr, nullptr, nullptr, 1, pk, fx, st) != cudaSuccess) return -5;
+    if (!prepare(e, false, B.pa, closed ? nullptr : B.pb, nullptr, nullptr, 0, st)) return -5;
     ++launches;
-    if (!closed) {
-      if (launch_mixed_prepare(B.pb, n, nullptr, nullptr, nullptr, 1, pk + nn, fx + n, st) != cudaSuccess) return -5;
-      ++launches;
-    }
     A.Pa = reinterpret_cast<const double*>(e.d_mixed_ws);
     A.Pb = nullptr;
     if (launch_xc_grad_mixed(dev_grid(e), A, n_ctas, B.counter + 1, st) != cudaSuccess) return -5;
   } else if (f64tc) {
-    if (!f64tc_prepare(e, B.pa, closed ? nullptr : B.pb, st, &launches)) return -5;
+    if (!prepare(e, true, B.pa, closed ? nullptr : B.pb, nullptr, nullptr, 0, st)) return -5;
+    ++launches;
     A.Pa = reinterpret_cast<const double*>(e.d_mixed_ws);
     A.Pb = nullptr;
     if (launch_xc_grad_f64tc(dev_grid(e), A, n_ctas, B.counter + 1, st) != cudaSuccess) return -5;
@@ -1517,16 +1514,11 @@ int calchem_xc_evaluate_rks(uint64_t grid_id, int xc_code, int precision, const 
   int rc = enqueue_eval(*e, kModeRks, xc_code, precision, e->d_P, nullptr, e->d_V, nullptr, nullptr, nullptr,
                         e->d_res, e->stream);
   if (rc) return rc;
-  double* h_res = e->h_stage;
-  int* h_status = reinterpret_cast<int*>(h_res + 3 * (size_t)M + 1);
+  const double* h_res = e->h_stage;
   touch_pages(h_v_out, nn);
-  if (cudaMemcpyAsync(h_v_out, e->d_V, nn * sizeof(double), cudaMemcpyDeviceToHost, e->stream) != cudaSuccess ||
-      cudaMemcpyAsync(h_res, e->d_res, 2 * (size_t)M * sizeof(double), cudaMemcpyDeviceToHost, e->stream) !=
-          cudaSuccess ||
-      cudaMemcpyAsync(h_status, e->d_counter + 2, sizeof(int), cudaMemcpyDeviceToHost, e->stream) != cudaSuccess ||
-      cudaStreamSynchronize(e->stream) != cudaSuccess)
+  if (cudaMemcpyAsync(h_v_out, e->d_V, nn * sizeof(double), cudaMemcpyDeviceToHost, e->stream) != cudaSuccess)
     return -5;
-  if (*h_status != 0) return -7;
+  if ((rc = finish(*e))) return rc;
   for (int i = 0; i < M; ++i) {
     exc_out[i] = h_res[2 * i];
     nelec_out[i] = h_res[2 * i + 1];
@@ -1557,14 +1549,8 @@ int calchem_xc_evaluate_rks_points(uint64_t grid_id, int xc_code, int precision,
   int rc = enqueue_eval(*e, kModeRks, xc_code, precision, e->d_P, nullptr, e->d_V, nullptr, nullptr, nullptr,
                         e->d_res, e->stream, e->d_pt_out);
   if (rc) return rc;
-  double* h_res = e->h_stage;
-  int* h_status = reinterpret_cast<int*>(h_res + 3 * (size_t)M + 1);
-  if (cudaMemcpyAsync(h_res, e->d_res, 2 * (size_t)M * sizeof(double), cudaMemcpyDeviceToHost, e->stream) !=
-          cudaSuccess ||
-      cudaMemcpyAsync(h_status, e->d_counter + 2, sizeof(int), cudaMemcpyDeviceToHost, e->stream) != cudaSuccess ||
-      cudaStreamSynchronize(e->stream) != cudaSuccess)
-    return -5;
-  if (*h_status != 0) return -7;
+  const double* h_res = e->h_stage;
+  if ((rc = finish(*e))) return rc;
   if (e->h_orig.empty()) {
     if (cudaMemcpy(h_point_out, e->d_pt_out, np2 * sizeof(double), cudaMemcpyDeviceToHost) != cudaSuccess) return -5;
   } else {  // back to the caller's point order; points the plan dropped (no AO reaches them) get 0
@@ -1601,18 +1587,13 @@ int calchem_xc_evaluate_uks(uint64_t grid_id, int xc_code, int precision, const 
   int rc = enqueue_eval(*e, kModeUks, xc_code, precision, e->d_P, e->d_Pb, e->d_V, e->d_Vb, nullptr, nullptr,
                         e->d_res, e->stream);
   if (rc) return rc;
-  double* h_res = e->h_stage;
-  int* h_status = reinterpret_cast<int*>(h_res + 3 * (size_t)M + 1);
+  const double* h_res = e->h_stage;
   touch_pages(h_va_out, nn);
   touch_pages(h_vb_out, nn);
   if (cudaMemcpyAsync(h_va_out, e->d_V, nn * sizeof(double), cudaMemcpyDeviceToHost, e->stream) != cudaSuccess ||
-      cudaMemcpyAsync(h_vb_out, e->d_Vb, nn * sizeof(double), cudaMemcpyDeviceToHost, e->stream) != cudaSuccess ||
-      cudaMemcpyAsync(h_res, e->d_res, 3 * (size_t)M * sizeof(double), cudaMemcpyDeviceToHost, e->stream) !=
-          cudaSuccess ||
-      cudaMemcpyAsync(h_status, e->d_counter + 2, sizeof(int), cudaMemcpyDeviceToHost, e->stream) != cudaSuccess ||
-      cudaStreamSynchronize(e->stream) != cudaSuccess)
+      cudaMemcpyAsync(h_vb_out, e->d_Vb, nn * sizeof(double), cudaMemcpyDeviceToHost, e->stream) != cudaSuccess)
     return -5;
-  if (*h_status != 0) return -7;
+  if ((rc = finish(*e))) return rc;
   for (int i = 0; i < M; ++i) {
     exc_out[i] = h_res[3 * i];
     nelec_out[2 * i] = h_res[3 * i + 1];
@@ -1734,19 +1715,15 @@ int calchem_xc_evaluate_rks_atoms(uint64_t grid_id, int xc_code, int precision, 
   int rc = enqueue_atom_shares(*e, xc_code, precision, e->d_P, e->d_res, h_v_out ? e->d_V : nullptr, e->d_atom_out,
                                e->stream);
   if (rc) return rc;
-  double* h_res = e->h_stage;
-  int* h_status = reinterpret_cast<int*>(h_res + 4);
+  const double* h_res = e->h_stage;
   if (h_v_out) touch_pages(h_v_out, nn);
   if (h_v_out && cudaMemcpyAsync(h_v_out, e->d_V, nn * sizeof(double), cudaMemcpyDeviceToHost, e->stream) !=
                      cudaSuccess)
     return -5;
-  if (cudaMemcpyAsync(h_res, e->d_res, 2 * sizeof(double), cudaMemcpyDeviceToHost, e->stream) != cudaSuccess ||
-      cudaMemcpyAsync(h_status, e->d_counter + 2, sizeof(int), cudaMemcpyDeviceToHost, e->stream) != cudaSuccess ||
-      cudaMemcpyAsync(h_atom_out, e->d_atom_out, 2 * (size_t)e->n_share_atoms * sizeof(double), cudaMemcpyDeviceToHost,
-                      e->stream) != cudaSuccess ||
-      cudaStreamSynchronize(e->stream) != cudaSuccess)
+  if (cudaMemcpyAsync(h_atom_out, e->d_atom_out, 2 * (size_t)e->n_share_atoms * sizeof(double), cudaMemcpyDeviceToHost,
+                      e->stream) != cudaSuccess)
     return -5;
-  if (*h_status != 0) return -7;
+  if ((rc = finish(*e))) return rc;
   *exc_out = h_res[0];
   *nelec_out = h_res[1];
   return 0;

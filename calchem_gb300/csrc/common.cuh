@@ -105,6 +105,50 @@ struct EvalArgs {
   int* ao_cache_ok;
 };
 
+// The first kernel of an evaluation of the tensor-core forms (one CTA per packed density row and spin): cuts the
+// rows of P[s] into the form's operands, and clears what the evaluation adds to, V[s] (unless nullptr) and the
+// first n_counter words at counter (unless nullptr).
+struct PrepareArgs {
+  const double* P[2];
+  double* V[2];
+  int n_spin;
+  int n_total;  // rows of the packed matrices (n for a single molecule)
+  const int* mol_n;
+  const long long* mol_off;
+  const int* mol_ao_off;
+  int n_mols;
+  void* out;    // 8 bytes per element, spin by spin (nn elements each)
+  size_t nn;
+  int* fexp;    // per row, spin by spin
+  int* counter;
+  int n_counter;
+};
+
+// The packed row blockIdx.x's molecule: its AO count and the row's first element.
+struct PreparedRow {
+  int n;
+  size_t off;
+};
+__device__ __forceinline__ PreparedRow prepared_row(const PrepareArgs& a) {
+  int mol = 0;
+  if (a.mol_ao_off) {  // the molecule whose row range [mol_ao_off[i], mol_ao_off[i + 1]) holds the row
+    int lo = 0, hi = a.n_mols - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (a.mol_ao_off[mid] <= (int)blockIdx.x) lo = mid; else hi = mid - 1;
+    }
+    mol = lo;
+  }
+  const int n = a.mol_n ? a.mol_n[mol] : a.n_total;
+  return {n, (size_t)(a.mol_off ? a.mol_off[mol] : 0ll) +
+                 (size_t)((int)blockIdx.x - (a.mol_ao_off ? a.mol_ao_off[mol] : 0)) * n};
+}
+__device__ __forceinline__ void prepared_clear(const PrepareArgs& a, PreparedRow r) {
+  if (double* V = a.V[blockIdx.y])
+    for (int j = threadIdx.x; j < r.n; j += blockDim.x) V[r.off + j] = 0.0;
+  if (a.counter && blockIdx.x == 0 && blockIdx.y == 0 && (int)threadIdx.x < a.n_counter) a.counter[threadIdx.x] = 0;
+}
+
 // Bytes of one batch's AO-cache block for m AOs: with m_k = m rounded up to 64, four FP32 planes
 // and four BF16 planes [m_k][128] (24 B per AO and point), the packed operand (m_k / 64 blocks of
 // 64 KB) and 128 row exponents, rounded up to 1 KB.

@@ -9,30 +9,41 @@ namespace cxc {
 // FP64 form (vxc_fp64.cu)
 cudaError_t launch_fp64(const DevGrid& G, const EvalArgs& A, int n_ctas, cudaStream_t st);
 size_t fp64_smem_bytes();
-// Per-molecule deterministic (Exc, N_a, N_b) sums: batches [batch_off[i], batch_off[i + 1]) go to
-// out[i * n_out ...]; batch_off = nullptr for one molecule.
-cudaError_t launch_reduce(const double* part, int n_batches, const int* batch_off, int n_mols, double* out, int n_out,
-                          cudaStream_t st);
-cudaError_t launch_reduce(const double* part, int n_batches, double* out, int n_out, cudaStream_t st);
-// Symmetric completion of each molecule's Vxc block (mol_n / mol_off = nullptr for one molecule).
-cudaError_t launch_mirror(double* V, int max_n, const int* mol_n, const long long* mol_off, int n_mols, int from_upper,
-                          cudaStream_t st);
-cudaError_t launch_mirror(double* V, int n, int from_upper, cudaStream_t st);
+// The end of an evaluation in one kernel: the per-molecule deterministic (Exc, N_a, N_b) sums (batches
+// [batch_off[i], batch_off[i + 1]) to out[i * n_out ...]; part = nullptr: none) and the completion of each
+// molecule's V blocks (V[0] = nullptr: none).  mol_n, mol_off, batch_off = nullptr for one molecule.
+enum FinishKind : int {
+  kFinishFromLower = 0,  // the lower triangle copied into the upper one (FP64 SIMT form)
+  kFinishFromUpper = 1,  // the upper into the lower (tensor-core form)
+  kFinishSum = 2,        // V + V^T (FP64 form on the tensor cores)
+  kFinishSumLower = 3    // the same in the lower triangle, zeros above it (the drop-in accumulation)
+};
+struct FinishArgs {
+  const double* part;
+  int n_batches;
+  const int* batch_off;
+  int n_mols;
+  double* out;
+  int n_out;
+  double* V[2];  // per spin (V[1] = nullptr: one)
+  int n;         // AOs (of the largest molecule)
+  const int* mol_n;
+  const long long* mol_off;
+  int kind;
+};
+cudaError_t launch_finish(const FinishArgs& F, cudaStream_t st);
 // Per-atom (Exc, tr(D Vxc)) shares: out[2 a ..] = sums of point_out over atom a's points.
 cudaError_t launch_atom_shares(const double* point_out, const int* atom_pts, const int* atom_off, int n_atoms,
                                double* out, cudaStream_t st);
 // FP64 form with its contractions on the tensor cores (vxc_f64tc.cu): A.Pa points at the fixed-point
 // densities of launch_f64tc_prepare (alpha, then beta, then the rows' exponents); V is accumulated as the
-// full square and completed by launch_symmetrise.
+// full square and completed by launch_finish (kFinishSum).
 int f64tc_max_m();
 size_t f64tc_slab_bytes(int max_m);
 size_t f64tc_cache_block_bytes(int m);
 cudaError_t f64tc_set_attributes();
 cudaError_t launch_f64tc(const DevGrid& G, const EvalArgs& A, int n_ctas, cudaStream_t st);
-cudaError_t launch_f64tc_prepare(const double* P, int n_total, const int* mol_n, const long long* mol_off,
-                                 const int* mol_ao_off, int n_mols, void* out, int* fexp, cudaStream_t st);
-cudaError_t launch_symmetrise(double* V, int max_n, const int* mol_n, const long long* mol_off, int n_mols,
-                              int lower_only, cudaStream_t st);
+cudaError_t launch_f64tc_prepare(const PrepareArgs& A, cudaStream_t st);
 // Tensor-core form (vxc_mixed.cu)
 int mixed_supported(int mode);
 size_t mixed_slab_doubles(int max_m);
@@ -41,8 +52,7 @@ int mixed_max_m();
 cudaError_t launch_closed_shell_points(int xc, int precision, int n, const double* rho, const double* gam,
                                        double* out, cudaStream_t st);
 cudaError_t launch_mixed(const DevGrid& G, const EvalArgs& A, int n_ctas, cudaStream_t st);
-cudaError_t launch_mixed_prepare(const double* P, int n_total, const int* mol_n, const long long* mol_off,
-                                 const int* mol_ao_off, int n_mols, void* out, int* fexp, cudaStream_t st);
+cudaError_t launch_mixed_prepare(const PrepareArgs& A, cudaStream_t st);
 // TD-DFT kernel coefficients per point (fxc.cu): rho_grad [n][4] of the total density -> out [n][11].
 cudaError_t launch_fxc_coef(const double* rho_grad, const double* w, int n_pts, int code, double* out,
                             cudaStream_t st);

@@ -25,12 +25,7 @@
 #include <mutex>
 
 #include "common.cuh"
-
-namespace cxc {
-cudaError_t launch_fp64(const DevGrid& G, const EvalArgs& A, int n_ctas, cudaStream_t st);
-cudaError_t launch_reduce(const double* part, int n_batches, double* out, int n_out, cudaStream_t st);
-cudaError_t launch_mirror(double* V, int n, int from_upper, cudaStream_t st);
-}  // namespace cxc
+#include "launch.h"
 
 namespace {
 
@@ -270,8 +265,11 @@ extern "C" int calchem_xc_evaluate_rks_static(const AoShellGpu* d_shells, int n_
   A.slab_stride = slab_stride;
   A.max_m = max_batch_ao;
   ok = cudaMemsetAsync(d_v, 0, nn * sizeof(double), st) == cudaSuccess &&
-       launch_fp64(G, A, n_ctas, st) == cudaSuccess && launch_reduce(red, n_batches, d_result, 2, st) == cudaSuccess &&
-       launch_mirror(d_v, n_ao, 0, st) == cudaSuccess && cudaStreamSynchronize(st) == cudaSuccess;
+       launch_fp64(G, A, n_ctas, st) == cudaSuccess &&
+       launch_finish(FinishArgs{red, n_batches, nullptr, 1, d_result, 2, {d_v, nullptr}, n_ao, nullptr, nullptr,
+                                kFinishFromLower},
+                     st) == cudaSuccess &&
+       cudaStreamSynchronize(st) == cudaSuccess;
   if (!ok) {
     cudaGetLastError();
     return -5;

@@ -31,7 +31,7 @@
 // as the tensor-core form of vxc_mixed.cu does.
 //
 // V is accumulated as the full square sum_b Z Phi^T (transposed, so that a warp's lanes add to
-// neighbouring elements) and symmetrised by a last kernel: half the MMAs of Z Phi^T + Phi Z^T on one
+// neighbouring elements) and symmetrised by launch_finish: half the MMAs of Z Phi^T + Phi Z^T on one
 // triangle.  Every mbarrier wait is bounded; one that expires sets the status word, waits (bounded) for
 // the CTA's own MMAs and copies, frees TMEM and returns.
 #include <cuda_runtime.h>
@@ -429,64 +429,22 @@ __global__ void __launch_bounds__(kT, 2) vxc_f64tc_kernel(DevGrid G, EvalArgs A)
 }
 
 // One CTA per packed density row: the row's exponent and the fixed-point Y of its elements.
-__global__ void __launch_bounds__(256) fixed_density_kernel(const double* __restrict__ D, int n_single,
-                                                           const int* __restrict__ mol_n,
-                                                           const long long* __restrict__ mol_off,
-                                                           const int* __restrict__ mol_ao_off, int n_mols,
-                                                           unsigned long long* __restrict__ out,
-                                                           int* __restrict__ fexp) {
+__global__ void __launch_bounds__(256) fixed_density_kernel(PrepareArgs A) {
   __shared__ uint32_t red[8];
-  int mol = 0;
-  if (mol_ao_off) {  // the molecule whose row range holds this row
-    int lo = 0, hi = n_mols - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (mol_ao_off[mid] <= (int)blockIdx.x) lo = mid; else hi = mid - 1;
-    }
-    mol = lo;
-  }
-  const int n = mol_n ? mol_n[mol] : n_single;
-  const size_t o = (size_t)(mol_off ? mol_off[mol] : 0ll) +
-                   (size_t)((int)blockIdx.x - (mol_ao_off ? mol_ao_off[mol] : 0)) * n;
+  const PreparedRow r = prepared_row(A);
+  const double* __restrict__ D = A.P[blockIdx.y] + r.off;
+  unsigned long long* __restrict__ out = static_cast<unsigned long long*>(A.out) + blockIdx.y * A.nn + r.off;
   uint32_t mx = 0;
-  for (int j = threadIdx.x; j < n; j += 256) mx = max(mx, (uint32_t)__double2hiint(D[o + j]) & 0x7FFFFFFFu);
+  for (int j = threadIdx.x; j < r.n; j += 256) mx = max(mx, (uint32_t)__double2hiint(D[j]) & 0x7FFFFFFFu);
   mx = __reduce_max_sync(0xFFFFFFFFu, mx);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = mx;
   __syncthreads();
 #pragma unroll
   for (int k = 0; k < 8; ++k) mx = max(mx, red[k]);
   const int E = max((int)(mx >> 20), 64);  // rows below 2^-959 count as zeros
-  if (threadIdx.x == 0) fexp[blockIdx.x] = E;
-  for (int j = threadIdx.x; j < n; j += 256) out[o + j] = to_fixed(D[o + j], E);
-}
-
-// V <- V + V^T of each molecule's block (blockIdx.y), 32 x 32 tile pairs; lower_only: the sums in the
-// lower triangle and zeros above it (the drop-in accumulation's result).
-__global__ void __launch_bounds__(256) symmetrise_kernel(double* __restrict__ V, int n_single,
-                                                        const int* __restrict__ mol_n,
-                                                        const long long* __restrict__ mol_off, int lower_only) {
-  __shared__ double ta[32][33], tb[32][33];
-  const int n = mol_n ? mol_n[blockIdx.y] : n_single;
-  double* Vm = V + (mol_off ? mol_off[blockIdx.y] : 0ll);
-  const int nt = (n + 31) / 32, tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  for (int p = blockIdx.x; p < nt * (nt + 1) / 2; p += gridDim.x) {
-    int I = (int)((sqrtf(8.f * p + 1.f) - 1.f) * 0.5f);
-    while (I * (I + 1) / 2 > p) --I;
-    while ((I + 1) * (I + 2) / 2 <= p) ++I;
-    const int J = p - I * (I + 1) / 2;  // tile (I, J), J <= I
-    for (int r = ty; r < 32; r += 8) {
-      const int ai = 32 * I + r, aj = 32 * J + tx, bi = 32 * J + r, bj = 32 * I + tx;
-      ta[r][tx] = ai < n && aj < n ? Vm[(size_t)ai * n + aj] : 0.0;
-      tb[r][tx] = bi < n && bj < n ? Vm[(size_t)bi * n + bj] : 0.0;
-    }
-    __syncthreads();
-    for (int r = ty; r < 32; r += 8) {
-      const int ai = 32 * I + r, aj = 32 * J + tx, bi = 32 * J + r, bj = 32 * I + tx;
-      if (ai < n && aj < n) Vm[(size_t)ai * n + aj] = lower_only && aj > ai ? 0.0 : ta[r][tx] + tb[tx][r];
-      if (I != J && bi < n && bj < n) Vm[(size_t)bi * n + bj] = lower_only ? 0.0 : ta[tx][r] + tb[r][tx];
-    }
-    __syncthreads();
-  }
+  if (threadIdx.x == 0) A.fexp[(size_t)blockIdx.y * A.n_total + blockIdx.x] = E;
+  for (int j = threadIdx.x; j < r.n; j += 256) out[j] = to_fixed(D[j], E);
+  prepared_clear(A, r);
 }
 
 }  // namespace
@@ -513,18 +471,8 @@ cudaError_t launch_f64tc(const DevGrid& G, const EvalArgs& A, int n_ctas, cudaSt
   return cudaGetLastError();
 }
 
-cudaError_t launch_f64tc_prepare(const double* P, int n_total, const int* mol_n, const long long* mol_off,
-                                 const int* mol_ao_off, int n_mols, void* out, int* fexp, cudaStream_t st) {
-  fixed_density_kernel<<<n_total, 256, 0, st>>>(P, n_total, mol_n, mol_off, mol_ao_off, n_mols,
-                                                reinterpret_cast<unsigned long long*>(out), fexp);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_symmetrise(double* V, int max_n, const int* mol_n, const long long* mol_off, int n_mols,
-                              int lower_only, cudaStream_t st) {
-  const int nt = (max_n + 31) / 32;
-  const unsigned bx = (unsigned)std::min(nt * (nt + 1) / 2, 4096);
-  symmetrise_kernel<<<dim3(bx, (unsigned)n_mols), 256, 0, st>>>(V, max_n, mol_n, mol_off, lower_only);
+cudaError_t launch_f64tc_prepare(const PrepareArgs& A, cudaStream_t st) {
+  fixed_density_kernel<<<dim3(A.n_total, A.n_spin), 256, 0, st>>>(A);
   return cudaGetLastError();
 }
 

@@ -27,6 +27,7 @@
 
 #include "common.cuh"
 #include "fp64_ao.cuh"
+#include "launch.h"
 #include "xc_device.cuh"
 
 namespace cxc {
@@ -353,38 +354,77 @@ __global__ void __launch_bounds__(kThreads, 1) vxc_fp64_kernel(DevGrid G, EvalAr
   }
 }
 
-// Deterministic final reduction of the per-batch (Exc, N_a, N_b) partials.
-__global__ void __launch_bounds__(256) reduce_batches_kernel(const double* __restrict__ part, int n_batches,
-                                                             const int* __restrict__ batch_off,
-                                                             double* __restrict__ out, int n_out) {
-  __shared__ double s[3][256];
+// The last kernel of an evaluation.  blockIdx.y: molecule, blockIdx.z: spin.
+//  * blockIdx.x == 0 of the first spin: the deterministic sum of the molecule's per-batch (Exc, N_a, N_b)
+//    partials, batches [batch_off[mol], batch_off[mol + 1]) (part == nullptr: none);
+//  * the others: the molecule's matrix completed in pairs of 32 x 32 tiles, by F.kind (launch.h).
+__global__ void __launch_bounds__(256) finish_kernel(FinishArgs F) {
+  __shared__ double ta[32][33], tb[32][33];
   const int t = threadIdx.x;
-  // one CTA per molecule: its batches are [batch_off[mol], batch_off[mol + 1])
-  const int b0 = batch_off ? batch_off[blockIdx.x] : 0;
-  const int b1 = batch_off ? batch_off[blockIdx.x + 1] : n_batches;
-  out += (size_t)blockIdx.x * n_out;
-  double a = 0, b = 0, c = 0;
-  for (int i = b0 + t; i < b1; i += 256) {
-    a += part[3 * (size_t)i];
-    b += part[3 * (size_t)i + 1];
-    c += part[3 * (size_t)i + 2];
+  if (blockIdx.x == 0) {
+    if (!F.part || blockIdx.z) return;
+    double(*s)[256] = reinterpret_cast<double(*)[256]>(&ta[0][0]);  // [3]: 768 of the 1056 elements
+    const int b0 = F.batch_off ? F.batch_off[blockIdx.y] : 0;
+    const int b1 = F.batch_off ? F.batch_off[blockIdx.y + 1] : F.n_batches;
+    double* out = F.out + (size_t)blockIdx.y * F.n_out;
+    double a = 0, b = 0, c = 0;
+    for (int i = b0 + t; i < b1; i += 256) {
+      a += F.part[3 * (size_t)i];
+      b += F.part[3 * (size_t)i + 1];
+      c += F.part[3 * (size_t)i + 2];
+    }
+    s[0][t] = a;
+    s[1][t] = b;
+    s[2][t] = c;
+    __syncthreads();
+    for (int o = 128; o > 0; o >>= 1) {
+      if (t < o) {
+        s[0][t] += s[0][t + o];
+        s[1][t] += s[1][t + o];
+        s[2][t] += s[2][t + o];
+      }
+      __syncthreads();
+    }
+    if (t == 0) {
+      out[0] = s[0][0];
+      if (F.n_out == 2) out[1] = s[1][0] + s[2][0];
+      else { out[1] = s[1][0]; out[2] = s[2][0]; }
+    }
+    return;
   }
-  s[0][t] = a;
-  s[1][t] = b;
-  s[2][t] = c;
-  __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
-    if (t < o) {
-      s[0][t] += s[0][t + o];
-      s[1][t] += s[1][t + o];
-      s[2][t] += s[2][t + o];
+  const int n = F.mol_n ? F.mol_n[blockIdx.y] : F.n;
+  double* V = F.V[blockIdx.z] + (F.mol_off ? F.mol_off[blockIdx.y] : 0ll);
+  const int nt = (n + 31) / 32, tx = t & 31, ty = t >> 5;
+  for (int p = (int)blockIdx.x - 1; p < nt * (nt + 1) / 2; p += (int)gridDim.x - 1) {
+    int I = (int)((sqrtf(8.f * p + 1.f) - 1.f) * 0.5f);
+    while (I * (I + 1) / 2 > p) --I;
+    while ((I + 1) * (I + 2) / 2 <= p) ++I;
+    const int J = p - I * (I + 1) / 2;  // tile (I, J) of the lower triangle and (J, I) of the upper
+    for (int r = ty; r < 32; r += 8) {
+      const int ai = 32 * I + r, aj = 32 * J + tx, bi = 32 * J + r, bj = 32 * I + tx;
+      ta[r][tx] = ai < n && aj < n ? V[(size_t)ai * n + aj] : 0.0;
+      tb[r][tx] = bi < n && bj < n ? V[(size_t)bi * n + bj] : 0.0;
     }
     __syncthreads();
-  }
-  if (t == 0) {
-    out[0] = s[0][0];
-    if (n_out == 2) out[1] = s[1][0] + s[2][0];
-    else { out[1] = s[1][0]; out[2] = s[2][0]; }
+    for (int r = ty; r < 32; r += 8) {
+      const int ai = 32 * I + r, aj = 32 * J + tx, bi = 32 * J + r, bj = 32 * I + tx;
+      if (ai < n && aj < n) {  // (in a diagonal tile this covers both triangles)
+        const bool above = aj > ai;
+        const double lo = ta[r][tx], up = tb[tx][r];  // V[ai][aj], V[aj][ai]
+        double v = lo;
+        if (F.kind == kFinishFromLower) v = above ? up : lo;
+        else if (F.kind == kFinishFromUpper) v = above ? lo : (ai == aj ? lo : up);
+        else v = F.kind == kFinishSumLower && above ? 0.0 : lo + up;
+        V[(size_t)ai * n + aj] = v;
+      }
+      if (I != J && bi < n && bj < n) {
+        const double up = tb[r][tx], lo = ta[tx][r];  // V[bi][bj] above the diagonal, V[bj][bi] below
+        V[(size_t)bi * n + bj] = F.kind == kFinishFromLower ? lo
+                                 : F.kind == kFinishFromUpper ? up
+                                 : F.kind == kFinishSumLower ? 0.0 : lo + up;
+      }
+    }
+    __syncthreads();
   }
 }
 
@@ -418,20 +458,6 @@ __global__ void __launch_bounds__(256) atom_shares_kernel(const double* __restri
   }
 }
 
-// Completes a symmetric matrix from one triangle: from_upper = 0 copies the lower triangle into
-// the upper one (FP64 path), from_upper = 1 the upper into the lower (tensor-core path).
-__global__ void mirror_kernel(double* __restrict__ V, int n_single, const int* __restrict__ mol_n,
-                              const long long* __restrict__ mol_off, int from_upper) {
-  // blockIdx.y = molecule; grid-stride over its n^2 elements
-  const int n = mol_n ? mol_n[blockIdx.y] : n_single;
-  double* Vm = V + (mol_off ? mol_off[blockIdx.y] : 0ll);
-  const size_t nn = (size_t)n * n;
-  for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < nn; idx += (size_t)gridDim.x * blockDim.x) {
-    const int i = (int)(idx / n), j = (int)(idx % n);
-    if (from_upper ? (j < i) : (j > i)) Vm[idx] = Vm[(size_t)j * n + i];
-  }
-}
-
 }  // namespace cxc
 
 // Launch helpers used by the C ABI layer.
@@ -453,26 +479,10 @@ cudaError_t launch_fp64(const DevGrid& G, const EvalArgs& A, int n_ctas, cudaStr
   return cudaGetLastError();
 }
 
-cudaError_t launch_reduce(const double* part, int n_batches, const int* batch_off, int n_mols, double* out, int n_out,
-                          cudaStream_t st) {
-  reduce_batches_kernel<<<n_mols, 256, 0, st>>>(part, n_batches, batch_off, out, n_out);
+cudaError_t launch_finish(const FinishArgs& F, cudaStream_t st) {
+  const int nt = (F.n + 31) / 32, tiles = F.V[0] ? std::min(nt * (nt + 1) / 2, 4096) : 0;
+  finish_kernel<<<dim3(1 + tiles, F.n_mols, F.V[1] ? 2 : 1), 256, 0, st>>>(F);
   return cudaGetLastError();
-}
-
-cudaError_t launch_reduce(const double* part, int n_batches, double* out, int n_out, cudaStream_t st) {
-  return launch_reduce(part, n_batches, nullptr, 1, out, n_out, st);
-}
-
-cudaError_t launch_mirror(double* V, int max_n, const int* mol_n, const long long* mol_off, int n_mols, int from_upper,
-                          cudaStream_t st) {
-  const size_t nn = (size_t)max_n * max_n;
-  const unsigned bx = (unsigned)std::min<size_t>((nn + 255) / 256, 4096);
-  mirror_kernel<<<dim3(bx, (unsigned)n_mols), 256, 0, st>>>(V, max_n, mol_n, mol_off, from_upper);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_mirror(double* V, int n, int from_upper, cudaStream_t st) {
-  return launch_mirror(V, n, nullptr, nullptr, 1, from_upper, st);
 }
 
 cudaError_t launch_atom_shares(const double* point_out, const int* atom_pts, const int* atom_off, int n_atoms,

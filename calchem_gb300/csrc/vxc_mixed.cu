@@ -931,27 +931,12 @@ __global__ void __launch_bounds__(kMT, MixCfg<kN>::kCtas) vxc_mixed_kernel(DevGr
 // D (FP64, n x n) -> per-row fixed-point split: row nu is scaled by 2^-f_nu (|x| < 1) and cut into
 // multiples of 2^-7, 2^-15, 2^-23, 2^-31 (computed in FP64, each exact in BF16); packed as
 // x = hi | mid << 16, y = lo | lo2 << 16.  One CTA per row.
-__global__ void __launch_bounds__(256) split_density_kernel(const double* __restrict__ D, int n_single,
-                                                           const int* __restrict__ mol_n,
-                                                           const long long* __restrict__ mol_off,
-                                                           const int* __restrict__ mol_ao_off, int n_mols,
-                                                           uint2* __restrict__ out, int* __restrict__ fexp) {
+__global__ void __launch_bounds__(256) split_density_kernel(PrepareArgs A) {
   __shared__ double red[256];
-  // packed row r belongs to the molecule whose row range [mol_ao_off[i], mol_ao_off[i + 1]) holds it
-  int mol = 0;
-  if (mol_ao_off) {
-    int lo = 0, hi = n_mols - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (mol_ao_off[mid] <= (int)blockIdx.x) lo = mid; else hi = mid - 1;
-    }
-    mol = lo;
-  }
-  const int n = mol_n ? mol_n[mol] : n_single;
-  const int row = (int)blockIdx.x - (mol_ao_off ? mol_ao_off[mol] : 0);
-  D += mol_off ? mol_off[mol] : 0ll;
-  out += mol_off ? mol_off[mol] : 0ll;
-  const double* d = D + (size_t)row * n;
+  const PreparedRow pr = prepared_row(A);
+  const int n = pr.n;
+  const double* __restrict__ d = A.P[blockIdx.y] + pr.off;
+  uint2* __restrict__ out = static_cast<uint2*>(A.out) + blockIdx.y * A.nn + pr.off;
   double mx = 0.0;
   for (int j = threadIdx.x; j < n; j += 256) mx = fmax(mx, fabs(d[j]));
   red[threadIdx.x] = mx;
@@ -962,7 +947,7 @@ __global__ void __launch_bounds__(256) split_density_kernel(const double* __rest
   }
   int f = 0;
   frexp(red[0], &f);
-  if (threadIdx.x == 0) fexp[blockIdx.x] = f;
+  if (threadIdx.x == 0) A.fexp[(size_t)blockIdx.y * A.n_total + blockIdx.x] = f;
   for (int j = threadIdx.x; j < n; j += 256) {
     const double x = ldexp(d[j], -f);
     const double h = rint(x * 128.0) / 128.0;
@@ -972,9 +957,10 @@ __global__ void __launch_bounds__(256) split_density_kernel(const double* __rest
     const double l = rint(r2 * 8388608.0) / 8388608.0;
     const double r3 = r2 - l;
     const double q = rint(r3 * 2147483648.0) / 2147483648.0;
-    out[(size_t)row * n + j] = make_uint2(pack_bf16x2(__float2bfloat16_rn((float)h), __float2bfloat16_rn((float)m)),
+    out[j] = make_uint2(pack_bf16x2(__float2bfloat16_rn((float)h), __float2bfloat16_rn((float)m)),
                                           pack_bf16x2(__float2bfloat16_rn((float)l), __float2bfloat16_rn((float)q)));
   }
+  prepared_clear(A, pr);
 }
 
 // The closed-shell point functional at n points (rho_a = rho_b = rho[i], all gammas = gam[i]):
@@ -1053,10 +1039,8 @@ cudaError_t launch_mixed(const DevGrid& G, const EvalArgs& A, int n_ctas, cudaSt
   return cudaGetLastError();
 }
 
-cudaError_t launch_mixed_prepare(const double* P, int n_total, const int* mol_n, const long long* mol_off,
-                                 const int* mol_ao_off, int n_mols, void* out, int* fexp, cudaStream_t st) {
-  split_density_kernel<<<n_total, 256, 0, st>>>(P, n_total, mol_n, mol_off, mol_ao_off, n_mols,
-                                                reinterpret_cast<uint2*>(out), fexp);
+cudaError_t launch_mixed_prepare(const PrepareArgs& A, cudaStream_t st) {
+  split_density_kernel<<<dim3(A.n_total, A.n_spin), 256, 0, st>>>(A);
   return cudaGetLastError();
 }
 
