@@ -32,6 +32,7 @@ CUDA_UNITS = {
     "xc_grad_mixed.cu": [],
     "xc_grad_f64tc.cu": [],
     "becke.cu": [],
+    "becke_mixed.cu": [],
 }
 CXX_UNITS = {"host_prep.cpp": [], "integrals.cpp": []}
 

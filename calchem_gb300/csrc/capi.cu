@@ -975,7 +975,7 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
   }
   std::vector<double> inv_r, a_ij;
   std::vector<int2> pairs;
-  std::vector<float2> pair_df;  // per ordered pair: 1 / R, a, (R_a - R_b) / R as float pairs
+  std::vector<float2> pair_df;  // rows over the pairs: 1 / R, a, (R_c - R_d) / R as float pairs
   if (xc >= 0) {
     becke_tables(n_atoms, z, xyz, inv_r, a_ij);
     for (int c = 0; c < n_atoms; ++c)
@@ -984,25 +984,25 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
       const float hi = (float)v;
       return make_float2(hi, (float)(v - (double)hi));
     };
-    pair_df.resize((size_t)n_atoms * n_atoms * 5);
-    for (int a = 0; a < n_atoms; ++a)
-      for (int b = 0; b < n_atoms; ++b) {
-        const size_t k = (size_t)a * n_atoms + b;
-        const double inv = inv_r[k];
-        pair_df[5 * k] = fpair(inv);
-        pair_df[5 * k + 1] = fpair(a_ij[k]);
-        for (int q = 0; q < 3; ++q) pair_df[5 * k + 2 + q] = fpair((xyz[3 * a + q] - xyz[3 * b + q]) * inv);
-      }
+    const size_t np = pairs.size();
+    if (mixed) pair_df.resize(np * 5);
+    for (size_t p = 0; p < pair_df.size() / 5; ++p) {
+      const int c = pairs[p].x, d = pairs[p].y;
+      const double inv = inv_r[(size_t)c * n_atoms + d];
+      pair_df[p] = fpair(inv);
+      pair_df[np + p] = fpair(a_ij[(size_t)c * n_atoms + d]);
+      for (int q = 0; q < 3; ++q) pair_df[(2 + q) * np + p] = fpair((xyz[3 * c + q] - xyz[3 * d + q]) * inv);
+    }
   }
   const size_t nn = (size_t)n * n, na3 = 3 * (size_t)n_atoms;
-  // the weight derivative runs as its own kernel when its tables fit
-  const bool becke_apart = xc >= 0 && n_atoms > 1 && (!mixed || becke_kernel_fits(n_atoms));
-  const int n_bk = !becke_apart ? 0 : mixed ? becke_kernel_ctas(e.n_pts) : becke_fp64_ctas(e.n_pts, n_atoms);
-  const size_t n_tables = becke_apart && !mixed ? becke_fp64_table_doubles(e.n_pts, n_atoms) : 0;
+  const bool becke_apart = xc >= 0 && n_atoms > 1;  // the weight derivative, a kernel of its own
+  const int n_bk = !becke_apart ? 0 : (mixed ? becke_mixed_ctas : becke_fp64_ctas)(e.n_pts, n_atoms);
+  const size_t n_tables =
+      !becke_apart ? 0 : (mixed ? becke_mixed_table_doubles : becke_fp64_table_doubles)(e.n_pts, n_atoms);
   // the FP64 form's contractions run on the tensor cores where that kernel holds the batches and atoms
   bool f64tc = !mixed && grad_f64tc_fits(e.max_m, n_atoms);
   auto stride_of = [&](bool tc) {
-    return mixed ? grad_mixed_slab_doubles(e.max_m, n_atoms)
+    return mixed ? grad_mixed_slab_doubles(e.max_m)
                  : tc ? grad_f64tc_slab_doubles(e.max_m) : grad_slab_doubles(e.max_m);
   };
   const size_t fixed = nn * sizeof(double) * (closed ? 1 : 2) + (size_t)e.n_pts * (xc < 0 ? 8 : 1) * sizeof(double) +
@@ -1090,8 +1090,8 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
              cudaSuccess &&
          (pairs.empty() || cudaMemcpyAsync(B.pairs, pairs.data(), pairs.size() * sizeof(int2), cudaMemcpyHostToDevice,
                                            st) == cudaSuccess) &&
-         cudaMemcpyAsync(B.pair_df, pair_df.data(), pair_df.size() * sizeof(float2), cudaMemcpyHostToDevice, st) ==
-             cudaSuccess;
+         (pair_df.empty() || cudaMemcpyAsync(B.pair_df, pair_df.data(), pair_df.size() * sizeof(float2),
+                                             cudaMemcpyHostToDevice, st) == cudaSuccess);
   if (!ok) return -5;
   GradArgs A{};
   A.xc = xc;
@@ -1134,8 +1134,7 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
     return -5;
   }
   if (becke_apart) {
-    if ((mixed ? launch_becke_mixed(dev_grid(e), A, B.fx, B.part2, st)
-               : launch_becke_fp64(dev_grid(e), A, B.fx, B.part2, B.tables, st)) != cudaSuccess)
+    if ((mixed ? launch_becke_mixed : launch_becke_fp64)(dev_grid(e), A, B.fx, B.part2, B.tables, st) != cudaSuccess)
       return -5;
     ++launches;
   }

@@ -176,8 +176,8 @@ struct GradArgs {
   const double* a_ij;      // n_atoms^2 Becke size adjustments
   const int2* pairs;       // the atom pairs (c, d), c < d
   int n_pairs;
-  // per ordered pair (a, b), 5 float pairs (hi, lo): 1 / R_ab, a_ab, (R_a - R_b) / R_ab (the
-  // double-float weight derivative of the tensor-core form)
+  // five rows of n_pairs float pairs (hi, lo): 1 / R_cd, a_cd, (R_c - R_d) / R_cd (the double-float weight
+  // derivative of the tensor-core form)
   const float2* pair_df;
   // when set, the quadrature kernel writes each point's energy density f here and leaves the weight
   // derivative to a separate kernel (becke_mixed_kernel, becke_fp64_kernel)

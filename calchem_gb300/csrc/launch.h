@@ -71,14 +71,15 @@ size_t grad_f64tc_slab_doubles(int max_m);
 cudaError_t launch_xc_grad_f64tc(const DevGrid& G, const GradArgs& A, int n_ctas, int* status, cudaStream_t st);
 // Tensor-core form of the gradient (xc_grad_mixed.cu): GradArgs.Pa points at the split densities of
 // launch_mixed_prepare (alpha, then beta); part must be zeroed; *status is set on a wait expiry.
-size_t grad_mixed_slab_doubles(int max_m, int n_atoms);
+size_t grad_mixed_slab_doubles(int max_m);
 int grad_mixed_max_m();
 cudaError_t launch_xc_grad_mixed(const DevGrid& G, const GradArgs& A, int n_ctas, int* status, cudaStream_t st);
-// The weight derivative of the tensor-core form as its own kernel (GradArgs.fx_out given to the
-// quadrature kernel): per-CTA rows of per-atom sums in part [becke_kernel_ctas(n_pts)][3 n_atoms].
-bool becke_kernel_fits(int n_atoms);
-int becke_kernel_ctas(int n_pts);
-cudaError_t launch_becke_mixed(const DevGrid& G, const GradArgs& A, const double* fx, double* part, cudaStream_t st);
+// The weight derivative of the tensor-core form (becke_mixed.cu) from the quadrature's GradArgs.fx_out: per-CTA
+// rows of per-atom sums in part [becke_mixed_ctas][3 n_atoms]; tables: becke_mixed_table_doubles of scratch.
+int becke_mixed_ctas(int n_pts, int n_atoms);
+size_t becke_mixed_table_doubles(int n_pts, int n_atoms);
+cudaError_t launch_becke_mixed(const DevGrid& G, const GradArgs& A, const double* fx, double* part, double* tables,
+                               cudaStream_t st);
 // The FP64 form's, likewise (becke.cu): rows part [becke_fp64_ctas][3 n_atoms], and for larger molecules
 // becke_fp64_table_doubles of scratch.
 int becke_fp64_ctas(int n_pts, int n_atoms);

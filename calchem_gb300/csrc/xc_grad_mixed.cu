@@ -3,7 +3,7 @@
 // The same quantity as xc_grad.cu (xc_nuclear_gradient, vxc.rs:1769-1912):
 //   dExc/dR_A = -2 sum_g sum_s sum_{i on A, A != host(g)} [ A_s,iq T_s,i + dphi_iq Y_s,i ] + ...
 // with A_s,iq = w v_rho_s dphi_iq + (w u_s) . Hphi_i,q, T_s = P_s Phi, Y_s = P_s Psi_s and
-// Psi_s = (w u_s) . grad Phi, plus the Becke weight derivative.  A row's term goes to its own atom
+// Psi_s = (w u_s) . grad Phi, plus the Becke weight derivative, becke_mixed.cu's part.  A row's term goes to its own atom
 // and, with the opposite sign, to the point's host atom (the reference adds both), so rows on the
 // host atom cancel exactly and are skipped here.
 //
@@ -22,10 +22,7 @@
 //       Hessian in double-float, sums consecutive rows of one atom per point, reduces those sums
 //       over the points with warp shuffles and adds them, in a fixed order, to the batch's row of
 //       per-atom sums; every point's total goes to its host atom with the opposite sign;
-//   (E) the Becke weight derivative in double-float (becke_grad.cuh): teams of 1-8 warps, one point
-//       per team, with the pair tables in the idle operand stage (up to 87 atoms), else one warp
-//       per point with the tables in the scratch slab;
-//   (F) a second kernel adds the batches' rows in batch order (deterministic).
+//   (E) a second kernel adds the batches' rows in batch order (deterministic).
 // Every mbarrier wait is bounded; on expiry the kernel sets the status word, waits (bounded) for its
 // own MMAs and bulk copies in flight, frees TMEM and returns.
 #include <cuda_bf16.h>
@@ -33,7 +30,6 @@
 
 #include <algorithm>
 
-#include "becke_grad.cuh"
 #include "common.cuh"
 #include "dfloat.cuh"
 #include "launch.h"
@@ -47,9 +43,6 @@ namespace cxc {
 namespace {
 
 using namespace mix;
-using becke::BeckeScratchDf;
-using becke::becke_point_df;
-using becke::becke_scratch_doubles;
 
 constexpr int kGM = kThreads;         // threads per CTA (two CTAs per SM)
 constexpr int kGWarpsM = kGM / 32;
@@ -276,16 +269,6 @@ __global__ void __launch_bounds__(kGM, 2) xc_grad_mixed_kernel(DevGrid G, GradAr
   float* p_lo = p_hi + P;
   unsigned char* apack = reinterpret_cast<unsigned char*>(p_lo + P);  // m_pad_all / 64 x 64 KB
   double* coef = reinterpret_cast<double*>(apack + (size_t)m_pad_all * 1024);  // [9][128]
-  double* bscr = coef + 9 * 128;
-  const size_t per_warp = becke_scratch_doubles(A.n_atoms);
-  BeckeScratchDf W;
-  W.dist = reinterpret_cast<df32*>(bscr + (size_t)warp * per_warp);
-  W.cell = reinterpret_cast<double*>(W.dist + A.n_atoms);
-  W.wacc = W.cell + A.n_atoms;
-  W.s = reinterpret_cast<df32*>(W.wacc + na3);
-  W.e = W.s + (size_t)A.n_atoms * A.n_atoms;
-  W.l = W.e + (size_t)A.n_atoms * A.n_atoms;
-  for (size_t k = tid; k < (size_t)kGWarpsM * per_warp; k += kGM) bscr[k] = 0.0;
 
   const uint2* Dhl_a0 = reinterpret_cast<const uint2*>(A.Pa);
   const uint2* Dhl_b0 = Dhl_a0 + G.nn_total;
@@ -647,67 +630,6 @@ __global__ void __launch_bounds__(kGM, 2) xc_grad_mixed_kernel(DevGrid G, GradAr
       }
       if (cur >= 0) out[3 * cur + tid] -= scale * run;
     }
-    // (E) Becke weight derivative: teams of 1-8 warps per point with the pair tables in the (idle)
-    // stage when one team's tables fit, else one warp per point with tables in the scratch slab
-    __syncthreads();
-    const size_t team_bytes = becke::becke_cta_bytes(A.n_atoms);
-    const bool cta_becke = team_bytes + (size_t)24 * A.n_atoms <= (size_t)kStageG;
-    if (A.fx_out) {
-      // the weight derivative runs as becke_mixed_kernel
-    } else if (A.n_atoms > 1 && cta_becke) {
-      int n_teams = 1;
-      while (n_teams < kGWarpsM && (size_t)(2 * n_teams) * team_bytes + (size_t)24 * A.n_atoms <= (size_t)kStageG)
-        n_teams *= 2;
-      const int nt = kGM / n_teams, team = tid / nt, tt = tid % nt;
-      df32* xyz_df = reinterpret_cast<df32*>(stage + (size_t)n_teams * team_bytes);
-      for (int k = tid; k < 3 * A.n_atoms; k += kGM) xyz_df[k] = df_from_double(A.xyz[k]);
-      becke::BeckeCta T;
-      T.carve(stage + (size_t)team * team_bytes, A.n_atoms);
-      for (int k = tt; k < na3; k += nt) T.wacc[k] = df32{0.f, 0.f};
-      __syncthreads();
-      for (int gg = team; gg < bd.n_pts; gg += n_teams) {
-        const double f = coef[8 * 128 + gg];
-        const size_t p = (size_t)bd.pt_start + gg;
-        const double rw = A.raw_w[p];
-        if (fabs(f) < 1e-18 || rw == 0.0) continue;
-        becke::becke_point_team(A.n_atoms, xyz_df, reinterpret_cast<const df32*>(A.pair_df), s_host[gg],
-                                df_from_double(G.px[p]), df_from_double(G.py[p]), df_from_double(G.pz[p]),
-                                df_from_double(rw * f), T, tt, nt, team);
-      }
-      __syncthreads();
-      for (int k = tid; k < na3; k += kGM) {
-        double v = 0.0;
-        for (int t = 0; t < n_teams; ++t) {
-          becke::BeckeCta Tt;
-          Tt.carve(stage + (size_t)t * team_bytes, A.n_atoms);
-          v += df_to_double(Tt.wacc[k]);
-        }
-        out[k] += v;
-      }
-    } else if (A.n_atoms > 1) {
-      for (int k = 0; k < 128 / kGWarpsM; ++k) {
-        const int gg = warp * (128 / kGWarpsM) + k;
-        if (gg >= bd.n_pts) break;
-        const double f = coef[8 * 128 + gg];
-        const size_t p = (size_t)bd.pt_start + gg;
-        const double rw = A.raw_w[p];
-        if (fabs(f) < 1e-18 || rw == 0.0) continue;
-        becke_point_df(A.n_atoms, A.xyz, reinterpret_cast<const df32*>(A.pair_df), A.pairs, A.n_pairs, s_host[gg], G.px[p], G.py[p], G.pz[p],
-                       rw * f, W);
-      }
-    }
-    __syncthreads();
-    if (!A.fx_out && A.n_atoms > 1 && !cta_becke) {
-      for (int k = tid; k < na3; k += kGM) {
-        double v = 0.0;
-        for (int w = 0; w < kGWarpsM; ++w) {
-          double* wa = bscr + (size_t)w * per_warp + 2 * A.n_atoms;
-          v += wa[k];
-          wa[k] = 0.0;
-        }
-        out[k] += v;
-      }
-    }
     __syncthreads();
   }
 
@@ -722,61 +644,10 @@ __global__ void __launch_bounds__(kGM, 2) xc_grad_mixed_kernel(DevGrid G, GradAr
   if (warp == 0) tmem_dealloc(tmem, kTmemColsG);
 }
 
-// The Becke weight derivative as its own kernel (atoms whose pair tables fit in shared memory):
-// one team of nt threads per CTA (a warp for up to 40 atoms, else the whole 256-thread CTA), the
-// team's tables in dynamic shared memory, kBeckePts consecutive points per CTA, and one row of
-// per-atom sums per CTA (part[cta][3 n_atoms]).  Separate from the quadrature kernel so that many
-// more teams are resident per SM than its two CTAs of eight warps allow.
-constexpr int kBeckePts = 16;
-
-__global__ void becke_mixed_kernel(DevGrid G, GradArgs A, const double* __restrict__ fx, double* __restrict__ part) {
-  extern __shared__ __align__(16) unsigned char bsm[];
-  const int na = A.n_atoms, na3 = 3 * na;
-  const int tid = threadIdx.x, nt = blockDim.x;
-  becke::BeckeCta T;
-  T.carve(bsm, na);
-  // the nuclei as double-floats behind the team's tables
-  df32* xyz_df = reinterpret_cast<df32*>(bsm + becke::becke_cta_bytes(na));
-  for (int k = tid; k < 3 * na; k += nt) xyz_df[k] = df_from_double(A.xyz[k]);
-  for (int k = tid; k < na3; k += nt) T.wacc[k] = df32{0.f, 0.f};
-  becke::team_sync(nt, 0);
-  const int p0 = blockIdx.x * kBeckePts;
-  for (int k = 0; k < kBeckePts; ++k) {
-    const int p = p0 + k;
-    if (p >= G.n_pts) break;
-    const double f = fx[p], rw = A.raw_w[p];
-    if (fabs(f) < 1e-18 || rw == 0.0) continue;
-    becke::becke_point_team(na, xyz_df, reinterpret_cast<const df32*>(A.pair_df), A.host[p], df_from_double(G.px[p]),
-                            df_from_double(G.py[p]), df_from_double(G.pz[p]), df_from_double(rw * f), T, tid, nt, 0);
-  }
-  becke::team_sync(nt, 0);
-  double* out = part + (size_t)blockIdx.x * na3;
-  for (int k = tid; k < na3; k += nt) out[k] = df_to_double(T.wacc[k]);
-}
-
-// Whether the separate weight-derivative kernel applies (its team's tables fit in shared memory),
-// its launch shape, and the number of CTAs (rows of its partial sums).
-int becke_kernel_threads(int n_atoms) { return n_atoms <= 40 ? 32 : 256; }
-size_t becke_kernel_smem(int n_atoms) { return becke::becke_cta_bytes(n_atoms) + (size_t)24 * n_atoms; }
-bool becke_kernel_fits(int n_atoms) {
-  return n_atoms > 1 && becke::becke_cta_bytes(n_atoms) + (size_t)24 * n_atoms <= (size_t)kStageG;
-}
-int becke_kernel_ctas(int n_pts) { return (n_pts + kBeckePts - 1) / kBeckePts; }
-
-cudaError_t launch_becke_mixed(const DevGrid& G, const GradArgs& A, const double* fx, double* part, cudaStream_t st) {
-  const int nt = becke_kernel_threads(A.n_atoms);
-  const size_t smem = becke_kernel_smem(A.n_atoms);
-  const cudaError_t e = cudaFuncSetAttribute(becke_mixed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  becke_mixed_kernel<<<becke_kernel_ctas(G.n_pts), nt, smem, st>>>(G, A, fx, part);
-  return cudaGetLastError();
-}
-
-size_t grad_mixed_slab_doubles(int max_m, int n_atoms) {
+size_t grad_mixed_slab_doubles(int max_m) {
   const size_t m_pad = (size_t)(max_m + 127) / 128 * 128, P = m_pad * 128;
   // planes: 10 FP32 + 10 BF16; T planes: 2 spins x (FP32 hi + FP32 lo); Psi (FP32 hi + lo); packed A
-  const size_t bytes = P * (kPlanesG * 4 + kPlanesG * 2 + 16 + 8 + 8) + 9 * 128 * sizeof(double) +
-                       (size_t)kGWarpsM * becke_scratch_doubles(n_atoms) * sizeof(double);
+  const size_t bytes = P * (kPlanesG * 4 + kPlanesG * 2 + 16 + 8 + 8) + 9 * 128 * sizeof(double);
   return (bytes / sizeof(double) + 127) / 128 * 128;  // 1 KB multiples keep every CTA's slab aligned
 }
 

@@ -60,6 +60,13 @@ def test_tensor_core_form_on_both_team_shapes(native_lib, waters):
     assert np.max(np.abs(g["mixed"] - g["fp64"])) < 5e-9
 
 
+@pytest.mark.parametrize("waters", [1, 3, 5, 6, 13, 24, 25])
+def test_tensor_core_form_at_its_edges(native_lib, waters):
+    """Teams of one, two and eight warps, one to three ranges of a row per atom, the last count with its pair
+    tables in shared memory (72 atoms) and the first without."""
+    test_tensor_core_form_on_both_team_shapes(native_lib, waters)
+
+
 def check(oracle, mol, name, half, grid):
     basis = BasisSet.from_name(name, mol)
     eng = RksVxcEngine(basis, grid)
