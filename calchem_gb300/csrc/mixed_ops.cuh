@@ -129,6 +129,14 @@ __device__ __forceinline__ void acc_prod(CompSum& A, df32 x, df32 t) {
   A.c = __fadd_rn(A.c, __fadd_rn(q.lo, e));
 }
 
+// the sum's first product
+__device__ __forceinline__ CompSum first_prod(df32 x, df32 t) {
+  CompSum A;
+  A.s = __fmul_rn(x.hi, t.hi);
+  A.c = __fmaf_rn(x.hi, t.lo, __fmaf_rn(x.lo, t.hi, __fmaf_rn(x.hi, t.hi, -A.s)));
+  return A;
+}
+
 // The same product summed by FP32 FMAs: s collects x.hi t.hi, c the cross terms x.hi t.lo +
 // x.lo t.hi; the rounding of each FMA into s is not recovered.  The double-float value's low part
 // still enters (its error is the same at every point of a radial shell and would not average out);

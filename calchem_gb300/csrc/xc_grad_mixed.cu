@@ -252,7 +252,7 @@ __global__ void __launch_bounds__(kGM, 2) xc_grad_mixed_kernel(DevGrid G, GradAr
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
+  const uint32_t tmem = warp_uniform(*tmem_slot);
   const uint32_t lane_base = (uint32_t)(32 * (warp & 3)) << 16;
   const uint32_t tH = tmem, tC1 = tmem + 64, tC2 = tmem + 128, tS = tmem + 192;
   uint32_t phase = 0, tphase = 0;
@@ -274,7 +274,8 @@ __global__ void __launch_bounds__(kGM, 2) xc_grad_mixed_kernel(DevGrid G, GradAr
   const uint2* Dhl_b0 = Dhl_a0 + G.nn_total;
   const int* fexp_a0 = reinterpret_cast<const int*>(Dhl_a0 + 2 * G.nn_total);
   const int* fexp_b0 = fexp_a0 + G.n_total;
-  const uint32_t sb = smem_addr(stage);
+  const uint32_t sb = warp_uniform(smem_addr(stage));
+  const bool issuer = warp_uniform(warp) == 0 && elect_one();  // issues the MMAs (from uniform registers)
   const uint32_t idesc = idesc_bf16_f32(128, kNc);
   const double scale = A.closed ? -4.0 : -2.0;
 
@@ -306,12 +307,11 @@ __global__ void __launch_bounds__(kGM, 2) xc_grad_mixed_kernel(DevGrid G, GradAr
       gather_b(stage, Dhl, s_ao, n, m, kb, nc);
       fence_proxy_async_smem();
       if (!wait_tma()) { failed = true; return; }
-      if (tid == 0) {
+      if (issuer) {
         tc_fence_after();
-        const uint64_t ah = sdesc_sw128(sb), am = sdesc_sw128(sb + 16384), al = sdesc_sw128(sb + 32768);
-        const uint64_t aq = sdesc_sw128(sb + 49152);
-        const uint64_t bh = sdesc_sw128(sb + 65536), bm = sdesc_sw128(sb + 73728), bl = sdesc_sw128(sb + 81920);
-        const uint64_t bq = sdesc_sw128(sb + 90112);
+        // A pieces of 16 KB, then the B pieces of 8 KB
+        const uint64_t ah = sdesc_sw128(sb), am = ah + (16384 >> 4), al = ah + (32768 >> 4), aq = ah + (49152 >> 4);
+        const uint64_t bh = ah + (65536 >> 4), bm = bh + (8192 >> 4), bl = bh + (16384 >> 4), bq = bh + (24576 >> 4);
         const bool group_start = (kb & 15) == 0;
 #pragma unroll
         for (int ks = 0; ks < 4; ++ks) {
@@ -539,9 +539,13 @@ __global__ void __launch_bounds__(kGM, 2) xc_grad_mixed_kernel(DevGrid G, GradAr
         chunk(nc, m, nkb, n, Dhl, [&](bool first_group) {
           // the group's 32 columns in runs of one atom: each thread sums its point's terms per run,
           // and a finished run's sum over the warp's 32 points goes to the warp's run list
-          df32 r0 = {0.f, 0.f}, r1 = r0, r2 = r0;
+          CompSum q0, q1, q2;
           int cur = -1, nrun = 0;
           auto flush = [&]() {
+            df32 r0 = two_sum(q0.s, q0.c), r1 = two_sum(q1.s, q1.c), r2 = two_sum(q2.s, q2.c);
+            hs0 = df_add(hs0, r0);
+            hs1 = df_add(hs1, r1);
+            hs2 = df_add(hs2, r2);
 #pragma unroll
             for (int off = 16; off > 0; off >>= 1) {
               r0 = df_add(r0, df32{__shfl_xor_sync(0xffffffffu, r0.hi, off), __shfl_xor_sync(0xffffffffu, r0.lo, off)});
@@ -567,7 +571,7 @@ __global__ void __launch_bounds__(kGM, 2) xc_grad_mixed_kernel(DevGrid G, GradAr
               if (at != cur) {
                 if (cur >= 0) flush();
                 cur = at;
-                r0 = r1 = r2 = df32{0.f, 0.f};
+                q0 = q1 = q2 = CompSum{};
               }
               if (i < m && live && at != hg) {
                 const df32 yv = df_ldexp(y[j], ep + s_fx[col]);
@@ -578,18 +582,19 @@ __global__ void __launch_bounds__(kGM, 2) xc_grad_mixed_kernel(DevGrid G, GradAr
                 const df32 hxx = ld_df(hi + 4 * P, lo + 4 * P, o), hxy = ld_df(hi + 5 * P, lo + 5 * P, o),
                            hxz = ld_df(hi + 6 * P, lo + 6 * P, o), hyy = ld_df(hi + 7 * P, lo + 7 * P, o),
                            hyz = ld_df(hi + 8 * P, lo + 8 * P, o), hzz = ld_df(hi + 9 * P, lo + 9 * P, o);
-                const df32 a0 = df_add(df_add(df_mul(c0, d0), df_mul(ux, hxx)), df_add(df_mul(uy, hxy), df_mul(uz, hxz)));
-                const df32 a1 = df_add(df_add(df_mul(c0, d1), df_mul(ux, hxy)), df_add(df_mul(uy, hyy), df_mul(uz, hyz)));
-                const df32 a2 = df_add(df_add(df_mul(c0, d2), df_mul(ux, hxz)), df_add(df_mul(uy, hyz), df_mul(uz, hzz)));
-                const df32 v0 = df_add(df_mul(a0, t), df_mul(d0, yv));
-                const df32 v1 = df_add(df_mul(a1, t), df_mul(d1, yv));
-                const df32 v2 = df_add(df_mul(a2, t), df_mul(d2, yv));
-                r0 = df_add(r0, v0);
-                r1 = df_add(r1, v1);
-                r2 = df_add(r2, v2);
-                hs0 = df_add(hs0, v0);
-                hs1 = df_add(hs1, v1);
-                hs2 = df_add(hs2, v2);
+                auto dot = [&](df32 d, df32 x, df32 y, df32 z) {
+                  CompSum a = first_prod(c0, d);
+                  acc_prod(a, ux, x);
+                  acc_prod(a, uy, y);
+                  acc_prod(a, uz, z);
+                  return two_sum(a.s, a.c);
+                };
+                acc_prod(q0, dot(d0, hxx, hxy, hxz), t);
+                acc_prod(q1, dot(d1, hxy, hyy, hyz), t);
+                acc_prod(q2, dot(d2, hxz, hyz, hzz), t);
+                acc_prod(q0, d0, yv);
+                acc_prod(q1, d1, yv);
+                acc_prod(q2, d2, yv);
               }
             }
           }
