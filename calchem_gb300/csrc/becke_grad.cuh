@@ -14,17 +14,17 @@ __device__ __forceinline__ double clamp_unit(double v) {
   return out ? __hiloint2double((hi & (int)0x80000000) | 0x3FF00000, 0) : v;
 }
 
-// Becke step s(nu) and ds/dnu (grid.rs:129-140): three times f(x) = x (3 - x^2) / 2, f' = 3 (1 - x^2) / 2.
-__device__ __forceinline__ void step_d(double nu, double& s, double& ds) {
-  double x = clamp_unit(nu), d = -0.5;
+// Becke step s(nu) (grid.rs:129-140): three times f(x) = x (3 - x^2) / 2 = x (1 + y / 2) with y = 1 - x^2.  d is the
+// product of the three y: ds/dnu = -(3/2)^3 d / 2.
+__device__ __forceinline__ void step_d(double nu, double& s, double& d) {
+  double x = clamp_unit(nu);
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    const double x2 = x * x;
-    d *= fma(-1.5, x2, 1.5);
-    x *= fma(-0.5, x2, 1.5);
+    const double y = fma(-x, x, 1.0);
+    d = k ? d * y : y;
+    x *= fma(0.5, y, 1.0);
   }
   s = fma(-0.5, x, 0.5);
-  ds = d;
 }
 
 // Row stride of the n x n tables: odd, so that lanes on consecutive rows of a table in shared memory fall into
@@ -54,7 +54,8 @@ struct BeckeScratch {
   }
 };
 
-// (E) raw_w f dW/dR for one point, one warp; wacc[3a + q] is owned by lane a % 32.
+// (E) raw_w f dW/dR for one point, one warp; wacc[3a + q] is owned by lane a % 32.  tab, rows over the pairs (c < d):
+// 1 / R_cd (0 for coincident atoms), the size adjustment a_cd, 27/8 a_cd, and (R_c - R_d) / R_cd.
 //   1. lanes over the unordered pairs (c < d): s_cd from mu_cd = (r_c - r_d) / R_cd and the size
 //      adjustment, and its slope (grid.rs:447-476);
 //   2. lanes over atoms c: the cell function P_c (factors multiplied in increasing d, as the
@@ -67,7 +68,7 @@ struct BeckeScratch {
 //   4. lanes over atoms a != host: dZ/dR_a from the pairs' sums, dP_host/dR_a from the pair with the host;
 //      the host atom gets minus the others' sum.
 static __device__ void becke_point(int n, const double* __restrict__ xyz, const double* __restrict__ inv_r,
-                            const double* __restrict__ a_ij, const int2* __restrict__ pairs, int n_pairs, int host,
+                            const double* __restrict__ tab, const int2* __restrict__ pairs, int n_pairs, int host,
                             double x, double y, double z, double pref_in, const BeckeScratch& W) {
   const int lane = threadIdx.x & 31;
   for (int c = lane; c < n; c += 32) {
@@ -78,13 +79,12 @@ static __device__ void becke_point(int n, const double* __restrict__ xyz, const 
   const int ld = becke_ld(n);
   for (int p = lane; p < n_pairs; p += 32) {
     const int c = pairs[p].x, d = pairs[p].y;
-    const double inv = inv_r[(size_t)c * n + d];
+    const double inv = tab[p];
     double sv = 1.0, sc = 1.0, sl = 0.0;
     if (inv != 0.0) {
       const double mu = clamp_unit((W.dist[c] - W.dist[d]) * inv);
-      const double a = a_ij[(size_t)c * n + d];
-      step_d(fma(a, fma(-mu, mu, 1.0), mu), sv, sl);
-      sl *= fma(-2.0 * a, mu, 1.0);
+      step_d(fma(tab[n_pairs + p], fma(-mu, mu, 1.0), mu), sv, sl);
+      sl *= fma(tab[2 * n_pairs + p], mu, -1.6875);
       sc = 1.0 - sv;
     }
     W.s[c * ld + d] = sv;
@@ -119,14 +119,14 @@ static __device__ void becke_point(int n, const double* __restrict__ xyz, const 
     const double slope = W.l[c * ld + d];
     double q = 0.0, w0 = 0.0, w1 = 0.0, w2 = 0.0;
     if ((__double2hiint(slope) & 0x7FFFFFFF) >= 0x39B40000) {  // |slope| above ~1e-30
-      const double inv = inv_r[(size_t)c * n + d];
+      const double inv = tab[p];
       const double mu = clamp_unit((W.dist[c] - W.dist[d]) * inv);
       const double k = slope * inv, ec = W.e[c * ld + d], ed = W.e[d * ld + c];
       q = (ec - ed) * k;
-      const double qm = q * (mu * inv);
-      w0 = qm * (xyz[3 * c] - xyz[3 * d]);
-      w1 = qm * (xyz[3 * c + 1] - xyz[3 * d + 1]);
-      w2 = qm * (xyz[3 * c + 2] - xyz[3 * d + 2]);
+      const double qm = q * mu;
+      w0 = qm * tab[3 * n_pairs + p];
+      w1 = qm * tab[4 * n_pairs + p];
+      w2 = qm * tab[5 * n_pairs + p];
       if (c == host) W.e[c * ld + d] = ec * k;  // E_{host a} k of the other atom a
       if (d == host) W.e[d * ld + c] = ed * k;
     } else {

@@ -886,7 +886,7 @@ int grid_build_impl(int n_atoms, const int* z, const double* xyz_bohr, const std
 // Device buffers of one gradient evaluation, laid out in the grid's gradient arena (grad_arena).
 struct GradBufs {
   double *pa = nullptr, *pb = nullptr, *wxc = nullptr, *raw = nullptr, *xyz = nullptr, *inv = nullptr,
-         *aij = nullptr, *part = nullptr, *slab = nullptr, *grad = nullptr;
+         *pair_tab = nullptr, *part = nullptr, *slab = nullptr, *grad = nullptr;
   int *host = nullptr, *ao_atom = nullptr, *counter = nullptr;
   int2* pairs = nullptr;
   float2* pair_df = nullptr;
@@ -976,6 +976,7 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
   std::vector<double> inv_r, a_ij;
   std::vector<int2> pairs;
   std::vector<float2> pair_df;  // rows over the pairs: 1 / R, a, (R_c - R_d) / R as float pairs
+  std::vector<double> pair_tab;  // and for the FP64 form: 1 / R, a, 27/8 a, (R_c - R_d) / R
   if (xc >= 0) {
     becke_tables(n_atoms, z, xyz, inv_r, a_ij);
     for (int c = 0; c < n_atoms; ++c)
@@ -986,12 +987,23 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
     };
     const size_t np = pairs.size();
     if (mixed) pair_df.resize(np * 5);
-    for (size_t p = 0; p < pair_df.size() / 5; ++p) {
+    else pair_tab.resize(np * 6);
+    for (size_t p = 0; p < np; ++p) {
       const int c = pairs[p].x, d = pairs[p].y;
-      const double inv = inv_r[(size_t)c * n_atoms + d];
-      pair_df[p] = fpair(inv);
-      pair_df[np + p] = fpair(a_ij[(size_t)c * n_atoms + d]);
-      for (int q = 0; q < 3; ++q) pair_df[(2 + q) * np + p] = fpair((xyz[3 * c + q] - xyz[3 * d + q]) * inv);
+      const double inv = inv_r[(size_t)c * n_atoms + d], a = a_ij[(size_t)c * n_atoms + d];
+      if (mixed) {
+        pair_df[p] = fpair(inv);
+        pair_df[np + p] = fpair(a);
+      } else {
+        pair_tab[p] = inv;
+        pair_tab[np + p] = a;
+        pair_tab[2 * np + p] = 3.375 * a;
+      }
+      for (int q = 0; q < 3; ++q) {
+        const double e = (xyz[3 * c + q] - xyz[3 * d + q]) * inv;
+        if (mixed) pair_df[(2 + q) * np + p] = fpair(e);
+        else pair_tab[(3 + q) * np + p] = e;
+      }
     }
   }
   const size_t nn = (size_t)n * n, na3 = 3 * (size_t)n_atoms;
@@ -1008,7 +1020,7 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
   const size_t fixed = nn * sizeof(double) * (closed ? 1 : 2) + (size_t)e.n_pts * (xc < 0 ? 8 : 1) * sizeof(double) +
                        (size_t)e.n_pts * sizeof(int) + (size_t)n * sizeof(int) +
                        (inv_r.size() * 2 + na3) * sizeof(double) + ((size_t)e.n_batches + 1) * na3 * sizeof(double) +
-                       pairs.size() * sizeof(int2) + pair_df.size() * sizeof(float2) + 64;
+                       pairs.size() * sizeof(int2) + (pair_df.size() + pair_tab.size()) * sizeof(double) + 64;
   // persistent CTAs: up to two per SM, fewer when the per-CTA scratch (AO planes and the warps' atom-pair
   // tables) would take more than half of the free memory
   size_t free_b = 0, total_b = 0;
@@ -1045,7 +1057,7 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
       m.take(&B.raw, e.n_pts);
       m.take(&B.xyz, na3);
       m.take(&B.inv, inv_r.size());
-      m.take(&B.aij, a_ij.size());
+      m.take(&B.pair_tab, pair_tab.size());
       m.take(&B.pairs, pairs.size());
       m.take(&B.pair_df, pair_df.size());
     }
@@ -1086,8 +1098,8 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
          cudaMemcpyAsync(B.xyz, xyz, na3 * sizeof(double), cudaMemcpyHostToDevice, st) == cudaSuccess &&
          cudaMemcpyAsync(B.inv, inv_r.data(), inv_r.size() * sizeof(double), cudaMemcpyHostToDevice, st) ==
              cudaSuccess &&
-         cudaMemcpyAsync(B.aij, a_ij.data(), a_ij.size() * sizeof(double), cudaMemcpyHostToDevice, st) ==
-             cudaSuccess &&
+         (pair_tab.empty() || cudaMemcpyAsync(B.pair_tab, pair_tab.data(), pair_tab.size() * sizeof(double),
+                                              cudaMemcpyHostToDevice, st) == cudaSuccess) &&
          (pairs.empty() || cudaMemcpyAsync(B.pairs, pairs.data(), pairs.size() * sizeof(int2), cudaMemcpyHostToDevice,
                                            st) == cudaSuccess) &&
          (pair_df.empty() || cudaMemcpyAsync(B.pair_df, pair_df.data(), pair_df.size() * sizeof(float2),
@@ -1104,7 +1116,7 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
   A.ao_atom = B.ao_atom;
   A.xyz = B.xyz;
   A.inv_r = B.inv;
-  A.a_ij = B.aij;
+  A.pair_tab = B.pair_tab;
   A.pairs = B.pairs;
   A.n_pairs = (int)pairs.size();
   A.pair_df = B.pair_df;

@@ -173,9 +173,10 @@ struct GradArgs {
   const int* ao_atom;      // per AO: atom of its shell
   const double* xyz;       // atoms, Bohr (3 n_atoms)
   const double* inv_r;     // n_atoms^2 inverse distances (0: coincident)
-  const double* a_ij;      // n_atoms^2 Becke size adjustments
   const int2* pairs;       // the atom pairs (c, d), c < d
   int n_pairs;
+  // FP64 form: six rows of n_pairs (becke_point)
+  const double* pair_tab;
   // five rows of n_pairs float pairs (hi, lo): 1 / R_cd, a_cd, (R_c - R_d) / R_cd (the double-float weight
   // derivative of the tensor-core form)
   const float2* pair_df;
