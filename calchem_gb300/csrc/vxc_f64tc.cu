@@ -9,15 +9,15 @@
 // operands' rounding are below 2^-54 of the row maxima's product per term, as the roundings of an FP64
 // FMA chain are; rho, the functional, Z and all sums stay in FP64.
 //
-// What bounds it: GB300 has 2 FP64 FMA lanes per SM and clock, so the SIMT form spends 4 m^2 FP64 FMAs a
+// What bounds it: GB300 has 2 FP64 FMA lanes per SM and clock, so the SIMT form spends 2 m^2 FP64 FMAs a
 // point there; here the tensor cores take them and the FP64 pipe is left with ~m (4 for rho and
 // grad rho, 4 for Z, 2 for the conversion of T) FMAs a point and the functional.  Two CTAs of 256
 // threads share an SM (240 TMEM columns and ~109 KB of shared memory each), so that one CTA's FP64
 // phases run under the other's copies and MMAs.  N = 48 columns is what five accumulators leave of
 // 256 TMEM columns.
 //
-// Measured against the SIMT form (whole host calls, FP64): C8H18 B3LYP Fine 32.9 -> 2.42 ms, 24 waters
-// B3LYP Medium 30.9 -> 2.20 ms, C6H14 PBE open shell 7.33 -> 0.79 ms, one water 0.63 -> 0.16 ms; the
+// Measured against the SIMT form (whole host calls, FP64): C8H18 B3LYP Fine 32.9 -> 2.38 ms, 24 waters
+// B3LYP Medium 30.9 -> 2.02 ms, C6H14 PBE open shell 7.33 -> 0.77 ms, one water 0.63 -> 0.16 ms; the
 // relative error of V against a plain FP64 evaluation is the same (2.6e-15 on C8H18, 2.7e-15 before).
 // On C8H18 a batch takes a CTA 280 us (210 alone on its SM): 36 % in MMA rounds, whose 128 x 32-byte A
 // reads bind them to shared memory (44 cycles per MMA of N = 48, 43 at N = 16), 46 % in rho, functional
@@ -25,7 +25,7 @@
 // ms: A tiles reloaded one by one under the others' MMAs and B gathered under them (-4 %), MMAs issued
 // from uniform registers (-3 %), rho's loads and V's reductions free of branches (-5 %).  Measured without
 // effect: L2 prefetches of the operands and planes, the next Z row's loads in registers.
-
+//
 // AO values, their packed slices and exponents depend on the grid and basis only: batches with a block
 // in the grid's AO cache compute them in the first launch that reaches them and read them afterwards,
 // as the tensor-core form of vxc_mixed.cu does.

@@ -8,6 +8,10 @@
 // A row's force on its atom is summed per point over runs of columns of one atom, a run's sum is reduced
 // over the warp's 32 points, and the runs are added to the batch's per-atom sums in a fixed order, so that
 // results are deterministic.
+//
+// The SIMT form is bound by its 2 m^2 FMAs a point and spin on the FP64 pipe; here that pipe keeps the Hessians
+// and the force terms, which run under the other CTA's copies and MMAs.  Eight waters
+// B3LYP Medium: 5.50 -> 2.11 ms.
 #include <cuda_runtime.h>
 
 #include "common.cuh"
