@@ -21,7 +21,7 @@ namespace {
 constexpr int kWarps = 4;
 constexpr int kPtsPerWarp = 4;             // with tables in shared memory
 constexpr int kGlobalCtas = 304;           // with tables in device memory,
-constexpr size_t kGlobalBytes = (size_t)4 << 30;  // which take this much at most
+constexpr size_t kGlobalBytes = (size_t)4 << 30;  // which take this much at most (and what the caller can spare)
 constexpr size_t kBeckeSmem = 200 << 10;
 
 __global__ void __launch_bounds__(32 * kWarps) becke_fp64_kernel(DevGrid G, GradArgs A, const double* __restrict__ fx,
@@ -56,22 +56,21 @@ bool in_smem(int n_atoms) { return smem_bytes(n_atoms) <= kBeckeSmem; }
 
 }  // namespace
 
-int becke_fp64_ctas(int n_pts, int n_atoms) {
+int becke_fp64_ctas(int n_pts, int n_atoms, size_t budget) {
   const int c = (n_pts + kWarps * kPtsPerWarp - 1) / (kWarps * kPtsPerWarp);
   if (in_smem(n_atoms)) return c;
-  return std::max<size_t>(1, std::min<size_t>({(size_t)c, (size_t)kGlobalCtas, kGlobalBytes / smem_bytes(n_atoms)}));
+  return std::max<size_t>(1, std::min<size_t>({(size_t)c, (size_t)kGlobalCtas,
+                                                    std::min(kGlobalBytes, budget) / smem_bytes(n_atoms)}));
 }
 
-size_t becke_fp64_table_doubles(int n_pts, int n_atoms) {
-  return in_smem(n_atoms) ? 0
-                          : (size_t)becke_fp64_ctas(n_pts, n_atoms) * kWarps * becke::becke_scratch_doubles(n_atoms);
+size_t becke_fp64_table_doubles(int n_ctas, int n_atoms) {
+  return in_smem(n_atoms) ? 0 : (size_t)n_ctas * kWarps * becke::becke_scratch_doubles(n_atoms);
 }
 
 cudaError_t launch_becke_fp64(const DevGrid& G, const GradArgs& A, const double* fx, double* part, double* tables,
-                              cudaStream_t st) {
+                              int n_ctas, cudaStream_t st) {
   const bool shared = in_smem(A.n_atoms);
   const size_t smem = shared ? smem_bytes(A.n_atoms) : 0;
-  const int n_ctas = becke_fp64_ctas(G.n_pts, A.n_atoms);
   if (shared) {
     const cudaError_t e = cudaFuncSetAttribute(becke_fp64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;

@@ -37,7 +37,7 @@ constexpr int kPts = 16;              // points of a CTA with its tables in shar
 constexpr size_t kTableSmem = 98304;  // shared memory of a CTA: two of them per SM at the least
 constexpr int kTeam = 256;            // threads per point at most
 constexpr int kGlobalCtas = 608;      // CTAs with their tables in device memory,
-constexpr size_t kGlobalBytes = (size_t)4 << 30;  // which take this much at most
+constexpr size_t kGlobalBytes = (size_t)4 << 30;  // which take this much at most (and what the caller can spare)
 
 // ---- two FP32 values in one register pair; every operation rounds each value to nearest ----------------
 struct f2 {
@@ -409,19 +409,19 @@ bool in_smem(int n) { return atom_bytes(n, team_threads(n)) + table_bytes(n) <= 
 
 }  // namespace
 
-int becke_mixed_ctas(int n_pts, int n_atoms) {
+int becke_mixed_ctas(int n_pts, int n_atoms, size_t budget) {
   if (in_smem(n_atoms)) return (n_pts + kPts - 1) / kPts;
   return (int)std::max<size_t>(
-      1, std::min<size_t>({(size_t)n_pts, (size_t)kGlobalCtas, kGlobalBytes / table_bytes(n_atoms)}));
+      1, std::min<size_t>({(size_t)n_pts, (size_t)kGlobalCtas, std::min(kGlobalBytes, budget) / table_bytes(n_atoms)}));
 }
 
-size_t becke_mixed_table_doubles(int n_pts, int n_atoms) {
-  return in_smem(n_atoms) ? 0 : (size_t)becke_mixed_ctas(n_pts, n_atoms) * table_bytes(n_atoms) / sizeof(double);
+size_t becke_mixed_table_doubles(int n_ctas, int n_atoms) {
+  return in_smem(n_atoms) ? 0 : (size_t)n_ctas * table_bytes(n_atoms) / sizeof(double);
 }
 
 cudaError_t launch_becke_mixed(const DevGrid& G, const GradArgs& A, const double* fx, double* part, double* tables,
-                               cudaStream_t st) {
-  const int n = A.n_atoms, nt = team_threads(n), n_ctas = becke_mixed_ctas(G.n_pts, n);
+                               int n_ctas, cudaStream_t st) {
+  const int n = A.n_atoms, nt = team_threads(n);
   const bool shared = in_smem(n);
   const size_t smem = atom_bytes(n, nt) + (shared ? table_bytes(n) : 0);
   auto* kernel = nt == 32 ? becke_mixed_kernel<true> : becke_mixed_kernel<false>;

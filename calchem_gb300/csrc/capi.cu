@@ -1007,10 +1007,6 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
     }
   }
   const size_t nn = (size_t)n * n, na3 = 3 * (size_t)n_atoms;
-  const bool becke_apart = xc >= 0 && n_atoms > 1;  // the weight derivative, a kernel of its own
-  const int n_bk = !becke_apart ? 0 : (mixed ? becke_mixed_ctas : becke_fp64_ctas)(e.n_pts, n_atoms);
-  const size_t n_tables =
-      !becke_apart ? 0 : (mixed ? becke_mixed_table_doubles : becke_fp64_table_doubles)(e.n_pts, n_atoms);
   // the FP64 form's contractions run on the tensor cores where that kernel holds the batches and atoms
   bool f64tc = !mixed && grad_f64tc_fits(e.max_m, n_atoms);
   auto stride_of = [&](bool tc) {
@@ -1025,6 +1021,12 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
   // tables) would take more than half of the free memory
   size_t free_b = 0, total_b = 0;
   const bool know_free = cudaMemGetInfo(&free_b, &total_b) == cudaSuccess;
+  // the weight derivative, a kernel of its own, whose tables take a quarter of it at most
+  const bool becke_apart = xc >= 0 && n_atoms > 1;
+  const size_t spare = know_free ? (free_b + e.grad_bytes) / 4 : SIZE_MAX;
+  const int n_bk = !becke_apart ? 0 : (mixed ? becke_mixed_ctas : becke_fp64_ctas)(e.n_pts, n_atoms, spare);
+  const size_t n_tables =
+      !becke_apart ? 0 : (mixed ? becke_mixed_table_doubles : becke_fp64_table_doubles)(n_bk, n_atoms);
   auto ctas_of = [&](int per_sm, size_t stride) {
     const int c = std::max(1, std::min(e.n_batches, per_sm * g_sm_count));
     const size_t fit = (free_b + e.grad_bytes) / 2 / (stride * sizeof(double));
@@ -1127,7 +1129,7 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
   A.counter = B.counter;
   A.slab = B.slab;
   A.slab_stride = slab_stride;
-  int launches = 0;
+  int launches = planned ? 1 : 0;  // the gather
   if (e.profiling) cudaEventRecord(e.ev0, st);
   if (mixed) {
     // split copies of the spin densities for the tensor-core contractions (alpha, then beta)
@@ -1146,7 +1148,8 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
     return -5;
   }
   if (becke_apart) {
-    if ((mixed ? launch_becke_mixed : launch_becke_fp64)(dev_grid(e), A, B.fx, B.part2, B.tables, st) != cudaSuccess)
+    if ((mixed ? launch_becke_mixed : launch_becke_fp64)(dev_grid(e), A, B.fx, B.part2, B.tables, n_bk, st) !=
+        cudaSuccess)
       return -5;
     ++launches;
   }

@@ -74,18 +74,17 @@ cudaError_t launch_xc_grad_f64tc(const DevGrid& G, const GradArgs& A, int n_ctas
 size_t grad_mixed_slab_doubles(int max_m);
 int grad_mixed_max_m();
 cudaError_t launch_xc_grad_mixed(const DevGrid& G, const GradArgs& A, int n_ctas, int* status, cudaStream_t st);
-// The weight derivative of the tensor-core form (becke_mixed.cu) from the quadrature's GradArgs.fx_out: per-CTA
-// rows of per-atom sums in part [becke_mixed_ctas][3 n_atoms]; tables: becke_mixed_table_doubles of scratch.
-int becke_mixed_ctas(int n_pts, int n_atoms);
-size_t becke_mixed_table_doubles(int n_pts, int n_atoms);
+// The weight derivative from the quadrature's GradArgs.fx_out (becke_mixed.cu, becke.cu): per-CTA rows of per-atom
+// sums in part [n_ctas][3 n_atoms], n_ctas = becke_*_ctas; for larger molecules becke_*_table_doubles of scratch,
+// which n_ctas keeps within budget bytes (one CTA at the least).
+int becke_mixed_ctas(int n_pts, int n_atoms, size_t budget);
+size_t becke_mixed_table_doubles(int n_ctas, int n_atoms);
 cudaError_t launch_becke_mixed(const DevGrid& G, const GradArgs& A, const double* fx, double* part, double* tables,
-                               cudaStream_t st);
-// The FP64 form's, likewise (becke.cu): rows part [becke_fp64_ctas][3 n_atoms], and for larger molecules
-// becke_fp64_table_doubles of scratch.
-int becke_fp64_ctas(int n_pts, int n_atoms);
-size_t becke_fp64_table_doubles(int n_pts, int n_atoms);
+                               int n_ctas, cudaStream_t st);
+int becke_fp64_ctas(int n_pts, int n_atoms, size_t budget);
+size_t becke_fp64_table_doubles(int n_ctas, int n_atoms);
 cudaError_t launch_becke_fp64(const DevGrid& G, const GradArgs& A, const double* fx, double* part, double* tables,
-                              cudaStream_t st);
+                              int n_ctas, cudaStream_t st);
 // raw[k] = raw_in[orig[k]], host[k] = host_in[orig[k]]: the caller's per-point arrays in planned order
 cudaError_t launch_grad_gather(const double* raw_in, const int* host_in, const int* orig, int n, double* raw, int* host,
                                cudaStream_t st);
