@@ -1,5 +1,5 @@
 // becke_grad.cuh -- derivative of the Becke partition weight of one grid point with respect to the
-// nuclei (grid.rs:423-584), one warp per point.
+// nuclei (grid.rs:423-584), one team of threads per point.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -35,11 +35,11 @@ __host__ __device__ __forceinline__ size_t becke_scratch_doubles(int n) {
   return 5 * (size_t)n + 3 * (size_t)n * becke_ld(n);
 }
 
-// Per-point pair tables of one warp (n rows of becke_ld(n)), behind dist[n], cell[n] and wacc[3 n].
+// Per-point pair tables of one team (n rows of becke_ld(n)), behind dist[n], cell[n] and wacc[3 n].
 struct BeckeScratch {
   double* dist;  // |r - R_c|
   double* cell;  // P_c = prod_{d != c} s_cd
-  double* wacc;  // [3 n] the warp's weight-derivative sums
+  double* wacc;  // [3 n] the team's weight-derivative sums
   double* s;     // s_cd (s_dc = 1 - s_cd, both stored; 1 for coincident atoms)
   double* e;     // prod_{d != c, k} s_cd at [c][k]
   double* l;     // ds_cd/dmu_cd at [c][d], c < d
@@ -54,7 +54,8 @@ struct BeckeScratch {
   }
 };
 
-// (E) raw_w f dW/dR for one point, one warp; wacc[3a + q] is owned by lane a % 32.  tab, rows over the pairs (c < d):
+// raw_w f dW/dR for one point by a team of kTeam threads (a warp or more; tid within it; red: 3 doubles per warp of
+// scratch for more); wacc[3a + q] is owned by thread a % kTeam.  tab, rows over the pairs (c < d):
 // 1 / R_cd (0 for coincident atoms), the size adjustment a_cd, 27/8 a_cd, and (R_c - R_d) / R_cd.
 //   1. lanes over the unordered pairs (c < d): s_cd from mu_cd = (r_c - r_d) / R_cd and the size
 //      adjustment, and its slope (grid.rs:447-476);
@@ -67,17 +68,22 @@ struct BeckeScratch {
 //      and the same with the other sign for atom d; they replace the pair's s and slope (grid.rs:517-583);
 //   4. lanes over atoms a != host: dZ/dR_a from the pairs' sums, dP_host/dR_a from the pair with the host;
 //      the host atom gets minus the others' sum.
-static __device__ void becke_point(int n, const double* __restrict__ xyz, const double* __restrict__ inv_r,
+template <int kTeam>
+__device__ void becke_point(int n, const double* __restrict__ xyz, const double* __restrict__ inv_r,
                             const double* __restrict__ tab, const int2* __restrict__ pairs, int n_pairs, int host,
-                            double x, double y, double z, double pref_in, const BeckeScratch& W) {
-  const int lane = threadIdx.x & 31;
-  for (int c = lane; c < n; c += 32) {
+                            double x, double y, double z, double pref_in, const BeckeScratch& W, int tid, double* red) {
+  const int lane = tid & 31;
+  auto team_sync = [] {
+    if (kTeam == 32) __syncwarp();
+    else __syncthreads();
+  };
+  for (int c = tid; c < n; c += kTeam) {
     const double dx = x - xyz[3 * c], dy = y - xyz[3 * c + 1], dz = z - xyz[3 * c + 2];
     W.dist[c] = sqrt(dx * dx + dy * dy + dz * dz);
   }
-  __syncwarp();
+  team_sync();
   const int ld = becke_ld(n);
-  for (int p = lane; p < n_pairs; p += 32) {
+  for (int p = tid; p < n_pairs; p += kTeam) {
     const int c = pairs[p].x, d = pairs[p].y;
     const double inv = tab[p];
     double sv = 1.0, sc = 1.0, sl = 0.0;
@@ -91,9 +97,9 @@ static __device__ void becke_point(int n, const double* __restrict__ xyz, const 
     W.s[d * ld + c] = sc;
     W.l[c * ld + d] = sl;
   }
-  __syncwarp();
+  team_sync();
   double zl = 0.0;
-  for (int c = lane; c < n; c += 32) {
+  for (int c = tid; c < n; c += kTeam) {
     const double* __restrict__ sr = W.s + c * ld;
     double* __restrict__ er = W.e + c * ld;
     double pre = 1.0;
@@ -102,19 +108,23 @@ static __device__ void becke_point(int n, const double* __restrict__ xyz, const 
       if (k != c) pre *= sr[k];
     }
     W.cell[c] = pre;
-    zl += pre;
+    if (kTeam == 32) zl += pre;
     double suf = 1.0;
     for (int k = n - 1; k >= 0; --k) {
       er[k] *= suf;
       if (k != c) suf *= sr[k];
     }
   }
+  if (kTeam > 32) {
+    team_sync();
+    for (int c = lane; c < n; c += 32) zl += W.cell[c];
+  }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) zl += __shfl_xor_sync(0xffffffffu, zl, o);
-  __syncwarp();
-  const double zs = zl;
+  if (kTeam == 32) team_sync();
+  const double zs = zl;  // the same in every thread
   if (zs <= 1e-30) return;
-  for (int p = lane; p < n_pairs; p += 32) {
+  for (int p = tid; p < n_pairs; p += kTeam) {
     const int c = pairs[p].x, d = pairs[p].y;
     const double slope = W.l[c * ld + d];
     double q = 0.0, w0 = 0.0, w1 = 0.0, w2 = 0.0;
@@ -138,10 +148,10 @@ static __device__ void becke_point(int n, const double* __restrict__ xyz, const 
     W.s[d * ld + c] = w1;
     W.l[d * ld + c] = w2;
   }
-  __syncwarp();
+  team_sync();
   const double wn = W.cell[host] / zs, pref = pref_in / zs;
   double h0 = 0, h1 = 0, h2 = 0;
-  for (int a = lane; a < n; a += 32) {
+  for (int a = tid; a < n; a += kTeam) {
     if (a == host) continue;
     const double ra = W.dist[a];
     if (ra < 1e-14) continue;
@@ -181,13 +191,27 @@ static __device__ void becke_point(int n, const double* __restrict__ xyz, const 
     h1 += __shfl_xor_sync(0xffffffffu, h1, o);
     h2 += __shfl_xor_sync(0xffffffffu, h2, o);
   }
-  __syncwarp();
-  if (lane == 0) {
-    W.wacc[3 * host] += h0;
-    W.wacc[3 * host + 1] += h1;
-    W.wacc[3 * host + 2] += h2;
+  if (kTeam == 32) {
+    __syncwarp();
+    if (lane == 0) {
+      W.wacc[3 * host] += h0;
+      W.wacc[3 * host + 1] += h1;
+      W.wacc[3 * host + 2] += h2;
+    }
+    __syncwarp();
+  } else {
+    if (lane == 0) {
+      red[3 * (tid >> 5)] = h0;
+      red[3 * (tid >> 5) + 1] = h1;
+      red[3 * (tid >> 5) + 2] = h2;
+    }
+    __syncthreads();
+    if (tid < 3) {
+      double h = 0.0;
+      for (int w = 0; w < kTeam / 32; ++w) h += red[3 * w + tid];
+      W.wacc[3 * host + tid] += h;
+    }
   }
-  __syncwarp();
 }
 
 }  // namespace becke

@@ -39,6 +39,12 @@ def test_weight_derivative_at_team_sizes(native_lib, oracle, n):
     check(oracle, mol, "sto-3g", density(n, n + 5), scattered(mol, 400, n))
 
 
+@pytest.mark.parametrize("n", [95, 96])
+def test_weight_derivative_where_tables_leave_shared_memory(native_lib, oracle, n):
+    mol = hydrogens(n)
+    check(oracle, mol, "sto-3g", density(n, n + 5), scattered(mol, 200, n))
+
+
 def test_weight_derivative_with_size_adjustments(native_lib, oracle):
     mol = workloads.water_cluster(5, 5)
     P = workloads.seeded_density_rks(BasisSet.from_name("sto-3g", mol).overlap(), 25, 3)
