@@ -1,5 +1,5 @@
 """The Becke weight derivative of the FP64 gradient at the atom counts where its path changes: two atoms, rows
-longer than a warp, the largest count with its pair tables in shared memory (becke.cu, 45 atoms) and the first
+longer than a warp, the largest count with its pair tables in shared memory (becke.cu, 95 atoms) and the first
 with them in device memory.  The points are near the atoms, between them and far outside (where
 every cell function is small or many are alike); hydrogens, so that the size adjustments vanish, and a
 mixed molecule, where they do not.
