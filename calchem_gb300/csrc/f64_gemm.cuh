@@ -220,6 +220,7 @@ struct Gemm {
   template <typename Epi>
   __device__ __forceinline__ bool rows(const unsigned char* apack, const unsigned long long* __restrict__ Yp,
                                        const int* __restrict__ fp, const uint16_t* s_ao, int* s_ef, int m, int n, Epi&& epi) {
+    if (m == 0) return true;  // no chunk would wait for the first copies
     const int tid = threadIdx.x, nkb = (m + 31) / 32, sh = sum_shift(m);
     auto gather = [&](int nc, int kb, int buf) {
       const int r = (tid - 64) >> 2, c = tid & 3;
