@@ -109,6 +109,7 @@ struct Entry {
   int* d_atom_off = nullptr;
   double* d_atom_out = nullptr;     // 2 per atom (host-buffer calls)
   std::vector<int> h_host;          // host atom of every uploaded point (reference-layout uploads)
+  std::vector<int> h_m;             // AOs of every batch
   std::vector<int> h_orig;          // caller's index of every uploaded point (empty: identity)
   int* d_orig = nullptr;            // the same on the device (gradients)
   void* d_grad = nullptr;           // gradient arena (grad_arena)
@@ -167,6 +168,10 @@ bool dalloc(T** p, size_t count) {
   if (count == 0) count = 1;
   return cudaMalloc((void**)p, count * sizeof(T)) == cudaSuccess;
 }
+
+// Waits for what the legacy stream was given: a device memset, and the last part of a copy from pageable memory, may
+// still be under way when their calls return, and nothing orders them before kernels on non-blocking streams.
+bool settle() { return cudaStreamSynchronize(cudaStreamLegacy) == cudaSuccess; }
 
 // Host-side tables derived from a reference-layout upload.
 struct HostPlan {
@@ -384,6 +389,7 @@ int upload_impl(const AoShellGpu* h_shells, int n_shells, const AoPrimGpu* h_pri
     soa[3 * (size_t)n_pts + g] = h_w ? h_w[g] : 0.0;
   }
   e->has_w = h_w != nullptr;
+  for (const BatchDesc& d : hp.batches) e->h_m.push_back(d.m);
   e->h_host.resize(n_pts);
   for (int g = 0; g < n_pts; ++g) e->h_host[g] = h_pts[g].host_atom;
   // float-pair copies of the basis constants: hi = float(x), lo = float(x - hi)
@@ -416,7 +422,8 @@ int upload_impl(const AoShellGpu* h_shells, int n_shells, const AoPrimGpu* h_pri
        cudaMemcpy(e->d_cand_loc, hp.cand_loc.data(), hp.cand_loc.size() * sizeof(int), cudaMemcpyHostToDevice) ==
            cudaSuccess &&
        cudaMemcpy(e->d_bao, hp.bao.data(), hp.bao.size() * sizeof(int), cudaMemcpyHostToDevice) == cudaSuccess &&
-       cudaMemcpy(e->d_order, hp.order.data(), hp.order.size() * sizeof(int), cudaMemcpyHostToDevice) == cudaSuccess;
+       cudaMemcpy(e->d_order, hp.order.data(), hp.order.size() * sizeof(int), cudaMemcpyHostToDevice) == cudaSuccess &&
+       settle();
   if (!ok) {
     cudaGetLastError();
     e->free_all();
@@ -477,22 +484,17 @@ void ao_cache_free(AoCache& c) {
   c = AoCache();
 }
 
-// Decides and allocates a form's AO cache on its first evaluation (not inside a stream
+// Decides and allocates a form's AO cache on its first evaluation, whose stream is st (not inside a stream
 // capture: callers that capture decide first).  The per-batch AO values and gradients depend only on
 // the grid and basis, so CalChem's engine computes them once per geometry and reuses them every
 // SCF iteration (vxc.rs:386-394, 600-716); here the cache also holds the packed GEMM1 operand and
 // the row exponents.  Off when the blocks exceed the cap or the free device memory (minus 1 GiB).  The
 // FP64 form's cache (`fp64`) also stays within a quarter of the free memory: its blocks are 56 B per AO and
 // point, and a program may hold many FP64 engines.
-void ao_cache_decide(Entry& e, bool fp64) {
+void ao_cache_decide(Entry& e, bool fp64, cudaStream_t st) {
   AoCache& c = fp64 ? e.f64_cache : e.ao_cache;
   if (c.state != 0) return;
   c.state = 1;
-  std::vector<BatchDesc> hb(e.n_batches);
-  if (cudaMemcpy(hb.data(), e.d_batches, hb.size() * sizeof(BatchDesc), cudaMemcpyDeviceToHost) != cudaSuccess) {
-    cudaGetLastError();
-    return;
-  }
   size_t free_b = 0, tot_b = 0;
   if (cudaMemGetInfo(&free_b, &tot_b) != cudaSuccess) {
     cudaGetLastError();
@@ -508,7 +510,7 @@ void ao_cache_decide(Entry& e, bool fp64) {
   std::vector<long long> off(e.n_batches, -1);
   size_t total = 0;
   for (int b = 0; b < e.n_batches; ++b) {
-    const size_t bb = fp64 ? f64tc_cache_block_bytes(hb[b].m) : ao_cache_block_bytes(hb[b].m);
+    const size_t bb = fp64 ? f64tc_cache_block_bytes(e.h_m[b]) : ao_cache_block_bytes(e.h_m[b]);
     if (total + bb > limit) continue;
     off[b] = (long long)total;
     total += bb;
@@ -517,10 +519,11 @@ void ao_cache_decide(Entry& e, bool fp64) {
   const bool ok = cudaMalloc(&c.d, total) == cudaSuccess &&
                   cudaMalloc(&c.d_off, off.size() * sizeof(long long)) == cudaSuccess &&
                   cudaMalloc(&c.d_ok, (size_t)e.n_batches * sizeof(int)) == cudaSuccess &&
-                  cudaMemcpy(c.d_off, off.data(), off.size() * sizeof(long long), cudaMemcpyHostToDevice) ==
+                  cudaMemcpyAsync(c.d_off, off.data(), off.size() * sizeof(long long), cudaMemcpyHostToDevice, st) ==
                       cudaSuccess &&
-                  cudaMemset(c.d_ok, 0, (size_t)e.n_batches * sizeof(int)) == cudaSuccess;
-  if (!ok) {
+                  cudaMemsetAsync(c.d_ok, 0, (size_t)e.n_batches * sizeof(int), st) == cudaSuccess;
+  // waited for: `off` goes out of scope, and later evaluations may use other streams
+  if (cudaStreamSynchronize(st) != cudaSuccess || !ok) {
     cudaGetLastError();
     ao_cache_free(c);
     c.state = 1;
@@ -533,7 +536,8 @@ void ao_cache_decide(Entry& e, bool fp64) {
 // A form's AO cache for a launch on st: decided now unless st is being captured.
 void use_ao_cache(Entry& e, bool fp64, cudaStream_t st, EvalArgs& A) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) ao_cache_decide(e, fp64);
+  if (cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone)
+    ao_cache_decide(e, fp64, st);
   const AoCache& c = fp64 ? e.f64_cache : e.ao_cache;
   if (c.state != 2) return;
   A.ao_cache = c.d;
@@ -966,7 +970,8 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
       cudaGetLastError();
       return -4;
     }
-    if (cudaMemcpy(e.d_orig, e.h_orig.data(), (size_t)e.n_pts * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess) {
+    if (cudaMemcpy(e.d_orig, e.h_orig.data(), (size_t)e.n_pts * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess ||
+        !settle()) {
       cudaGetLastError();
       cudaFree(e.d_orig);
       e.d_orig = nullptr;
@@ -1445,7 +1450,8 @@ int calchem_xc_set_weights(uint64_t grid_id, const double* h_weights, int n_pts)
   Entry* e = find(grid_id);
   if (!e || e->n_mols != 1 || e->n_pts != n_pts) return -2;
   if (cudaMemcpy(e->d_pts + 3 * (size_t)n_pts, h_weights, n_pts * sizeof(double), cudaMemcpyHostToDevice) !=
-      cudaSuccess)
+          cudaSuccess ||
+      !settle())
     return -5;
   e->has_w = true;
   return 0;
@@ -1685,7 +1691,8 @@ int calchem_xc_set_point_atoms(uint64_t grid_id, const int* h_host_atom, int n_p
     return -4;
   }
   if (cudaMemcpy(e->d_atom_pts, pts.data(), pts.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess ||
-      cudaMemcpy(e->d_atom_off, off.data(), off.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess)
+      cudaMemcpy(e->d_atom_off, off.data(), off.size() * sizeof(int), cudaMemcpyHostToDevice) != cudaSuccess ||
+      !settle())
     return -5;
   e->n_share_atoms = n_atoms;
   return 0;
@@ -2013,7 +2020,9 @@ int calchem_xc_group_create(const uint64_t* member_ids, int n_members, uint64_t 
        cudaMemcpy(g->d_mol_ao_off, g->h_mol_ao_off.data(), (n_members + 1) * sizeof(int), cudaMemcpyHostToDevice) ==
            cudaSuccess &&
        cudaMemcpy(g->d_mol_boff, g->h_mol_boff.data(), (n_members + 1) * sizeof(int), cudaMemcpyHostToDevice) ==
-           cudaSuccess;
+           cudaSuccess &&
+       settle();
+  for (const BatchDesc& d : batches) g->h_m.push_back(d.m);
   if (!ok) return fail(-5);
   g_grids[group_id] = g;
   return 0;
@@ -2049,7 +2058,8 @@ int calchem_xc_graph_capture(uint64_t grid_id, int mode, int xc_code, int precis
   if (fp64_set_attributes() != cudaSuccess || mixed_set_attributes() != cudaSuccess ||
       f64tc_set_attributes() != cudaSuccess)
     return -5;
-  if (precision == CALCHEM_XC_MIXED || f64tc_ready(*e, e->stream)) ao_cache_decide(*e, precision != CALCHEM_XC_MIXED);
+  if (precision == CALCHEM_XC_MIXED || f64tc_ready(*e, e->stream))
+    ao_cache_decide(*e, precision != CALCHEM_XC_MIXED, e->stream);
   if (e->graph) {
     cudaGraphExecDestroy(e->graph);
     e->graph = nullptr;
