@@ -344,7 +344,10 @@ __global__ void __launch_bounds__(kT, 2) vxc_f64tc_kernel(DevGrid G, EvalArgs A)
       for (int k = 0; k < kT / 32; ++k) t += red[tid][k];
       A.batch_red[3 * (size_t)b + tid] = t;
     }
-    if (A.mode == kModeRho || A.shares_only || m == 0) continue;  // (m == 0: a batch that no AO reaches)
+    if (A.mode == kModeRho || A.shares_only || m == 0) {  // (m == 0: a batch that no AO reaches)
+      fence_proxy_async_smem();  // the functional's halves met in the stage; the next batch's copies write it
+      continue;
+    }
 
     for (int s = 0; s < (uks ? 2 : 1) && !failed; ++s) {
       double* Vm = (s ? A.Vb : A.Va) + moff;

@@ -882,7 +882,8 @@ __global__ void __launch_bounds__(kMT, MixCfg<kN>::kCtas) vxc_mixed_kernel(DevGr
           *reinterpret_cast<uint4*>(img + img_tile(3 + t, ib, kb2, n_ib) + sw) = z3[t];
         }
       }
-      fence_proxy_async_global();  // the tiles are read by bulk copies
+      fence_proxy_async_global();  // the tiles are read by bulk copies, into the stage, where the functional's
+      fence_proxy_async_smem();    // halves met
       __syncthreads();
       for (int I = 0; I < m && !failed; I += 128) {
         for (int J = 0; J <= I && !failed; J += 128) {

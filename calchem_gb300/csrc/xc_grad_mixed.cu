@@ -612,6 +612,7 @@ __global__ void __launch_bounds__(kGM, 2) xc_grad_mixed_kernel(DevGrid G, GradAr
             }
           }
         }
+        fence_proxy_async_smem();  // the run lists lie where the next bulk copies write
         __syncthreads();
       }
     }
@@ -635,6 +636,7 @@ __global__ void __launch_bounds__(kGM, 2) xc_grad_mixed_kernel(DevGrid G, GradAr
       }
       if (cur >= 0) out[3 * cur + tid] -= scale * run;
     }
+    fence_proxy_async_smem();  // (as the host sums)
     __syncthreads();
   }
 
