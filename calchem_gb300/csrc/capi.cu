@@ -780,13 +780,22 @@ void touch_pages(double* p, size_t n) {
   }
 }
 
-// Waits for the grid's stream, with the last host call's sums in h_stage; -7 when a device-side wait gave up.
+// Waits for the grid's stream, with the last host call's sums in h_stage; -7 when a device-side wait gave up.  The
+// caller's outputs are copied after it, so that they stay as they were then.
 int finish(Entry& e) {
   const size_t at = 3 * (size_t)e.n_mols + 4;  // the queue heads and the status word follow the sums
   if (cudaMemcpyAsync(e.h_stage, e.d_res, (at + 2) * sizeof(double), cudaMemcpyDeviceToHost, e.stream) != cudaSuccess ||
       cudaStreamSynchronize(e.stream) != cudaSuccess)
     return -5;
   return reinterpret_cast<const int*>(e.h_stage + at)[2] != 0 ? -7 : 0;
+}
+
+// n doubles from the device to the caller's output.
+int fetch(Entry& e, double* out, const double* d, size_t n) {
+  return cudaMemcpyAsync(out, d, n * sizeof(double), cudaMemcpyDeviceToHost, e.stream) == cudaSuccess &&
+                 cudaStreamSynchronize(e.stream) == cudaSuccess
+             ? 0
+             : -5;
 }
 
 bool valid_xc(int xc) { return xc >= 0 && xc <= 8; }
@@ -1167,11 +1176,10 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
   if (e.profiling) cudaEventRecord(e.ev1, st);
   e.last_launches = launches;
   int status = 0;
-  if (cudaMemcpyAsync(h_grad, B.grad, na3 * sizeof(double), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-      cudaMemcpyAsync(&status, B.counter + 1, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+  if (cudaMemcpyAsync(&status, B.counter + 1, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
       cudaStreamSynchronize(st) != cudaSuccess)
     return -5;
-  return status ? -7 : 0;
+  return status ? -7 : fetch(e, h_grad, B.grad, na3);
 }
 
 }  // namespace
@@ -1207,10 +1215,8 @@ int calchem_cuda_vxc_eval_rho(uint64_t grid_id, const double* h_p_mat, double* h
   int rc = enqueue_eval(*e, kModeRho, 0, CALCHEM_XC_FP64, e->d_P, nullptr, nullptr, nullptr, nullptr, e->d_rg,
                         nullptr, e->stream);
   if (rc) return rc;
-  if (cudaMemcpyAsync(h_rho_grad_out, e->d_rg, (size_t)n_pts * 4 * sizeof(double), cudaMemcpyDeviceToHost,
-                      e->stream) != cudaSuccess)
-    return -5;
-  return finish(*e);
+  if ((rc = finish(*e))) return rc;
+  return fetch(*e, h_rho_grad_out, e->d_rg, (size_t)n_pts * 4);
 }
 
 int calchem_cuda_vxc_accum(uint64_t grid_id, const double* h_wv_in, double* h_vxc_out, int n_pts, int n_ao) {
@@ -1228,9 +1234,8 @@ int calchem_cuda_vxc_accum(uint64_t grid_id, const double* h_wv_in, double* h_vx
                         nullptr, e->stream);
   if (rc) return rc;
   touch_pages(h_vxc_out, nn);
-  if (cudaMemcpyAsync(h_vxc_out, e->d_V, nn * sizeof(double), cudaMemcpyDeviceToHost, e->stream) != cudaSuccess)
-    return -5;
-  return finish(*e);
+  if ((rc = finish(*e))) return rc;
+  return fetch(*e, h_vxc_out, e->d_V, nn);
 }
 
 int calchem_cuda_vxc_grad_force(uint64_t grid_id, const double* h_pa, const double* h_pb, int is_rks,
@@ -1536,9 +1541,7 @@ int calchem_xc_evaluate_rks(uint64_t grid_id, int xc_code, int precision, const 
   if (rc) return rc;
   const double* h_res = e->h_stage;
   touch_pages(h_v_out, nn);
-  if (cudaMemcpyAsync(h_v_out, e->d_V, nn * sizeof(double), cudaMemcpyDeviceToHost, e->stream) != cudaSuccess)
-    return -5;
-  if ((rc = finish(*e))) return rc;
+  if ((rc = finish(*e)) || (rc = fetch(*e, h_v_out, e->d_V, nn))) return rc;
   for (int i = 0; i < M; ++i) {
     exc_out[i] = h_res[2 * i];
     nelec_out[i] = h_res[2 * i + 1];
@@ -1610,10 +1613,10 @@ int calchem_xc_evaluate_uks(uint64_t grid_id, int xc_code, int precision, const 
   const double* h_res = e->h_stage;
   touch_pages(h_va_out, nn);
   touch_pages(h_vb_out, nn);
-  if (cudaMemcpyAsync(h_va_out, e->d_V, nn * sizeof(double), cudaMemcpyDeviceToHost, e->stream) != cudaSuccess ||
-      cudaMemcpyAsync(h_vb_out, e->d_Vb, nn * sizeof(double), cudaMemcpyDeviceToHost, e->stream) != cudaSuccess)
-    return -5;
   if ((rc = finish(*e))) return rc;
+  if (cudaMemcpyAsync(h_va_out, e->d_V, nn * sizeof(double), cudaMemcpyDeviceToHost, e->stream) != cudaSuccess)
+    return -5;
+  if ((rc = fetch(*e, h_vb_out, e->d_Vb, nn))) return rc;
   for (int i = 0; i < M; ++i) {
     exc_out[i] = h_res[3 * i];
     nelec_out[2 * i] = h_res[3 * i + 1];
@@ -1738,13 +1741,11 @@ int calchem_xc_evaluate_rks_atoms(uint64_t grid_id, int xc_code, int precision, 
   if (rc) return rc;
   const double* h_res = e->h_stage;
   if (h_v_out) touch_pages(h_v_out, nn);
+  if ((rc = finish(*e))) return rc;
   if (h_v_out && cudaMemcpyAsync(h_v_out, e->d_V, nn * sizeof(double), cudaMemcpyDeviceToHost, e->stream) !=
                      cudaSuccess)
     return -5;
-  if (cudaMemcpyAsync(h_atom_out, e->d_atom_out, 2 * (size_t)e->n_share_atoms * sizeof(double), cudaMemcpyDeviceToHost,
-                      e->stream) != cudaSuccess)
-    return -5;
-  if ((rc = finish(*e))) return rc;
+  if ((rc = fetch(*e, h_atom_out, e->d_atom_out, 2 * (size_t)e->n_share_atoms))) return rc;
   *exc_out = h_res[0];
   *nelec_out = h_res[1];
   return 0;
@@ -1834,7 +1835,6 @@ int calchem_xc_fxc_contract_ex(uint64_t grid_id, int triplet, int precision, con
     }
     e->fxc_cap = n_trials;
   }
-  int st = 0;
   if (cudaMemcpyAsync(e->d_fxc_m, h_m, nn * n_trials * sizeof(double), cudaMemcpyHostToDevice, e->stream) !=
       cudaSuccess)
     return -5;
@@ -1843,12 +1843,8 @@ int calchem_xc_fxc_contract_ex(uint64_t grid_id, int triplet, int precision, con
                    ? enqueue_fxc_mixed(*e, triplet, e->d_fxc_m, n_trials, e->d_fxc_v, e->stream)
                    : enqueue_fxc(*e, triplet, e->d_fxc_m, n_trials, e->d_fxc_v, e->stream))
     return rc;
-  if (cudaMemcpyAsync(h_v_out, e->d_fxc_v, nn * n_trials * sizeof(double), cudaMemcpyDeviceToHost, e->stream) !=
-          cudaSuccess ||
-      cudaMemcpyAsync(&st, e->d_counter + 2, sizeof(int), cudaMemcpyDeviceToHost, e->stream) != cudaSuccess ||
-      cudaStreamSynchronize(e->stream) != cudaSuccess)
-    return -5;
-  return st != 0 ? -7 : 0;
+  if (int rc = finish(*e)) return rc;
+  return fetch(*e, h_v_out, e->d_fxc_v, nn * n_trials);
 }
 
 int calchem_xc_nuclear_gradient(uint64_t grid_id, int xc_code, int precision, int n_atoms, const int* z,

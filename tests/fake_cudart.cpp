@@ -29,6 +29,7 @@ std::map<std::string, int> g_calls, g_fail;
 size_t g_total = (size_t)280 << 30, g_used = 0;
 int g_status = 0, g_unsettled = 0;
 bool g_capturing = false;
+cudaError_t g_last = cudaSuccess;
 uintptr_t g_next = 16;
 
 uintptr_t id(cudaStream_t s) { return (uintptr_t)s <= 2 ? 0 : (uintptr_t)s; }
@@ -46,7 +47,7 @@ cudaError_t called(const char* name) {
   auto it = g_fail.find(name);
   if (it == g_fail.end() || --it->second > 0) return cudaSuccess;
   g_fail.erase(it);
-  return cudaErrorUnknown;
+  return g_last = cudaErrorUnknown;
 }
 
 void drain(uintptr_t s) {
@@ -59,7 +60,7 @@ void drain_all() {
 }
 
 cudaError_t take(void** p, size_t n, bool device) {
-  if (device && g_used + n > g_total) return cudaErrorMemoryAllocation;
+  if (device && g_used + n > g_total) return g_last = cudaErrorMemoryAllocation;
   void* q = mmap(nullptr, n ? n : 1, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS | MAP_NORESERVE, -1, 0);
   if (q == MAP_FAILED) return cudaErrorMemoryAllocation;
   (device ? g_device : g_pinned)[q] = n;
@@ -96,7 +97,10 @@ extern "C" {
 void fake_set_memory(size_t total) { g_total = total; }
 size_t fake_used() { return g_used; }
 void fake_status(int s) { g_status = s; }
-void fake_fail(const char* name, int nth) { g_fail[name] = nth; }  // the nth call from now on fails
+void fake_fail(const char* name, int nth) {  // the nth call from now on fails (0: none does)
+  if (nth > 0) g_fail[name] = nth;
+  else g_fail.erase(name);
+}
 int fake_calls(const char* name) { return g_calls[name]; }
 int fake_unsettled() { return g_unsettled; }  // launches that found writes of the legacy stream not ordered before
 int fake_host_copies() {                      // copies from or into pageable memory still to be done
@@ -129,7 +133,7 @@ cudaError_t cudaMemGetInfo(size_t* f, size_t* t) {
 }
 cudaError_t cudaMalloc(void** p, size_t n) {
   const cudaError_t e = called("cudaMalloc");
-  return e != cudaSuccess ? cudaErrorMemoryAllocation : take(p, n, true);
+  return e != cudaSuccess ? g_last = cudaErrorMemoryAllocation : take(p, n, true);
 }
 cudaError_t cudaMallocHost(void** p, size_t n) { return take(p, n, false); }
 cudaError_t cudaFree(void* p) { called("cudaFree"); return give(p, true); }
@@ -203,7 +207,11 @@ cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventElapsedTime(float* t, cudaEvent_t, cudaEvent_t) { *t = 0.f; return cudaSuccess; }
-cudaError_t cudaGetLastError() { return called("cudaGetLastError"); }
+cudaError_t cudaGetLastError() {
+  const cudaError_t e = g_last;
+  g_last = cudaSuccess;
+  return e;
+}
 
 // ---- what nvcc's host stubs call ----
 void** __cudaRegisterFatBinary(void*) { static void* h; return &h; }

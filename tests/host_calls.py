@@ -22,7 +22,7 @@ def molecule():
     host = rng.integers(0, 3, 3000).astype(np.int32)
     x = mol.coords_bohr[host] + rng.normal(size=(3000, 3))
     xyzw = np.concatenate([x, rng.uniform(0.1, 1.0, (3000, 1))], axis=1)
-    return mol, basis, MolecularGrid(xyzw, xyzw[:, 3], host, GridLevel.COARSE), np.eye(basis.n_ao)
+    return mol, basis, MolecularGrid(xyzw, xyzw[:, 3].copy(), host, GridLevel.COARSE), np.eye(basis.n_ao)
 
 
 def dropin(basis, grid):
@@ -58,6 +58,55 @@ def check_uploads_come_before_kernels(fake):
     _native.check("set_weights", _native.load().calchem_xc_set_weights(g.grid_id, _native.ptr(w), len(w)))
     g.accumulate_vxc(np.zeros((g.n_pts, 4)))
     assert fake.fake_unsettled() == 0
+
+
+def host_calls():
+    """(name, call -> status, the call's outputs) of every evaluation on host buffers, both precisions."""
+    lib = _native.load()
+    mol, basis, grid, P = molecule()
+    n = basis.n_ao
+    z, xyz = np.array(mol.z, dtype=np.int32), np.ascontiguousarray(mol.coords_bohr)
+    p = _native.ptr
+    out = lambda *shape: np.full(shape, 7.0)  # noqa: E731
+    for prec, name in ((0, "fp64"), (1, "mixed")):
+        eng = RksVxcEngine(basis, grid, precision=name, tile=64)
+        eng.set_point_atoms(grid.host_atom, 3)
+        e, ne, v, vb, sh, pt, g = out(1), out(2), out(n, n), out(n, n), out(6), out(len(grid), 2), np.zeros((3, 3))
+        gid = eng.grid_id
+        yield name + " rks", lambda: lib.calchem_xc_evaluate_rks(gid, 2, prec, p(P), p(e), p(ne), p(v)), (e, ne, v)
+        yield name + " uks", lambda: lib.calchem_xc_evaluate_uks(
+            gid, 2, prec, p(P), p(P), p(e), p(ne), p(v), p(vb)), (e, ne, v, vb)
+        yield name + " points", lambda: lib.calchem_xc_evaluate_rks_points(
+            gid, 2, prec, p(P), p(e), p(ne), p(pt)), (e, ne, pt)
+        yield name + " atoms", lambda: lib.calchem_xc_evaluate_rks_atoms(
+            gid, 2, prec, p(P), p(e), p(ne), p(sh), p(v)), (e, ne, sh, v)
+        yield name + " shares", lambda: lib.calchem_xc_evaluate_rks_atoms(
+            gid, 2, prec, p(P), p(e), p(ne), p(sh), None), (e, ne, sh)
+        yield name + " gradient", lambda: lib.calchem_xc_nuclear_gradient(  # (fills its output with zeros first)
+            gid, 2, prec, 3, p(z), p(xyz), p(grid.raw_weight), p(grid.host_atom), len(grid), p(P), None, p(g)), (g,)
+        eng.close()
+        fxc = FxcKernel(basis, grid, "pbe", P, name)
+        yield name + " fxc", lambda: lib.calchem_xc_fxc_contract_ex(fxc.grid_id, 0, prec, p(P), 1, p(v)), (v,)
+        fxc.close()
+    d, _ = dropin(basis, grid)
+    rg, wv, wxc, f = out(d.n_pts, 4), np.zeros((d.n_pts, 4)), np.zeros((d.n_pts, 8)), out(3, 3)
+    yield "rho", lambda: lib.calchem_cuda_vxc_eval_rho(d.grid_id, p(P), p(rg), d.n_pts, n), (rg,)
+    yield "accum", lambda: lib.calchem_cuda_vxc_accum(d.grid_id, p(wv), p(v), d.n_pts, n), (v,)
+    yield "force", lambda: lib.calchem_cuda_vxc_grad_force(d.grid_id, p(P), p(P), 1, p(wxc), p(f), d.n_pts, n, 3, 0), (f,)
+
+
+def check_outputs_stay_as_they_were_when_a_wait_expired(fake):
+    """-7: the status word is read before anything is copied to the caller."""
+    for name, call, outputs in host_calls():
+        before = [o.copy() for o in outputs]
+        assert call() == 0, name
+        for o, b in zip(outputs, before):
+            o[...] = b
+        fake.fake_status(1)
+        assert call() == -7, name
+        fake.fake_status(0)
+        for o, b in zip(outputs, before):
+            assert np.array_equal(o, b), name
 
 
 CHECKS = {k[len("check_"):]: v for k, v in list(globals().items()) if k.startswith("check_")}
