@@ -780,6 +780,26 @@ void touch_pages(double* p, size_t n) {
   }
 }
 
+// Declared before a call's first copy from or into memory that it does not own: on a return path that has not
+// waited for the stream (ok() not called), the copies under way are waited for.
+class CopiesDone {
+ public:
+  explicit CopiesDone(cudaStream_t s) : st(s) {}
+  ~CopiesDone() {
+    if (waited) return;
+    cudaStreamSynchronize(st);
+    cudaGetLastError();
+  }
+  int ok() {
+    waited = true;
+    return 0;
+  }
+
+ private:
+  cudaStream_t st;
+  bool waited = false;
+};
+
 // Waits for the grid's stream, with the last host call's sums in h_stage; -7 when a device-side wait gave up.  The
 // caller's outputs are copied after it, so that they stay as they were then.
 int finish(Entry& e) {
@@ -1095,6 +1115,7 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
     ~Trim() { grad_arena_trim(e); }
   } trim{e};
   cudaStream_t st = e.stream;
+  CopiesDone copies(st);
   bool ok = cudaMemcpyAsync(B.pa, h_pa, nn * sizeof(double), cudaMemcpyHostToDevice, st) == cudaSuccess &&
        (closed || cudaMemcpyAsync(B.pb, h_pb, nn * sizeof(double), cudaMemcpyHostToDevice, st) == cudaSuccess) &&
        cudaMemcpyAsync(planned ? B.host_in : B.host, host_atom, (size_t)n_in * sizeof(int), cudaMemcpyHostToDevice,
@@ -1179,7 +1200,9 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
   if (cudaMemcpyAsync(&status, B.counter + 1, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
       cudaStreamSynchronize(st) != cudaSuccess)
     return -5;
-  return status ? -7 : fetch(e, h_grad, B.grad, na3);
+  if (status) return -7;
+  const int rc = fetch(e, h_grad, B.grad, na3);
+  return rc ? rc : copies.ok();
 }
 
 }  // namespace
@@ -1210,13 +1233,15 @@ int calchem_cuda_vxc_eval_rho(uint64_t grid_id, const double* h_p_mat, double* h
   if (!e || e->n_mols != 1 || e->n_pts != n_pts || e->n_ao != n_ao) return -2;
   if (int rc0 = ensure_ws(*e)) return rc0;
   const size_t nn = (size_t)n_ao * n_ao;
+  CopiesDone copies(e->stream);
   if (cudaMemcpyAsync(e->d_P, h_p_mat, nn * sizeof(double), cudaMemcpyHostToDevice, e->stream) != cudaSuccess)
     return -5;
   int rc = enqueue_eval(*e, kModeRho, 0, CALCHEM_XC_FP64, e->d_P, nullptr, nullptr, nullptr, nullptr, e->d_rg,
                         nullptr, e->stream);
   if (rc) return rc;
   if ((rc = finish(*e))) return rc;
-  return fetch(*e, h_rho_grad_out, e->d_rg, (size_t)n_pts * 4);
+  if ((rc = fetch(*e, h_rho_grad_out, e->d_rg, (size_t)n_pts * 4))) return rc;
+  return copies.ok();
 }
 
 int calchem_cuda_vxc_accum(uint64_t grid_id, const double* h_wv_in, double* h_vxc_out, int n_pts, int n_ao) {
@@ -1227,6 +1252,7 @@ int calchem_cuda_vxc_accum(uint64_t grid_id, const double* h_wv_in, double* h_vx
   if (!e || e->n_mols != 1 || e->n_pts != n_pts || e->n_ao != n_ao) return -2;
   if (int rc0 = ensure_ws(*e)) return rc0;
   const size_t nn = (size_t)n_ao * n_ao;
+  CopiesDone copies(e->stream);
   if (cudaMemcpyAsync(e->d_rg, h_wv_in, (size_t)n_pts * 4 * sizeof(double), cudaMemcpyHostToDevice, e->stream) !=
       cudaSuccess)
     return -5;
@@ -1235,7 +1261,8 @@ int calchem_cuda_vxc_accum(uint64_t grid_id, const double* h_wv_in, double* h_vx
   if (rc) return rc;
   touch_pages(h_vxc_out, nn);
   if ((rc = finish(*e))) return rc;
-  return fetch(*e, h_vxc_out, e->d_V, nn);
+  if ((rc = fetch(*e, h_vxc_out, e->d_V, nn))) return rc;
+  return copies.ok();
 }
 
 int calchem_cuda_vxc_grad_force(uint64_t grid_id, const double* h_pa, const double* h_pb, int is_rks,
@@ -1534,6 +1561,7 @@ int calchem_xc_evaluate_rks(uint64_t grid_id, int xc_code, int precision, const 
   if (int rc0 = ensure_ws(*e)) return rc0;
   const size_t nn = (size_t)e->nn_total;
   const int M = e->n_mols;
+  CopiesDone copies(e->stream);
   if (cudaMemcpyAsync(e->d_P, h_d_total, nn * sizeof(double), cudaMemcpyHostToDevice, e->stream) != cudaSuccess)
     return -5;
   int rc = enqueue_eval(*e, kModeRks, xc_code, precision, e->d_P, nullptr, e->d_V, nullptr, nullptr, nullptr,
@@ -1546,7 +1574,7 @@ int calchem_xc_evaluate_rks(uint64_t grid_id, int xc_code, int precision, const 
     exc_out[i] = h_res[2 * i];
     nelec_out[i] = h_res[2 * i + 1];
   }
-  return 0;
+  return copies.ok();
 }
 
 int calchem_xc_evaluate_rks_points(uint64_t grid_id, int xc_code, int precision, const double* h_d_total,
@@ -1566,6 +1594,7 @@ int calchem_xc_evaluate_rks_points(uint64_t grid_id, int xc_code, int precision,
   }
   const size_t nn = (size_t)e->nn_total;
   const int M = e->n_mols;
+  CopiesDone copies(e->stream);
   if (cudaMemsetAsync(e->d_pt_out, 0, np2 * sizeof(double), e->stream) != cudaSuccess ||
       cudaMemcpyAsync(e->d_P, h_d_total, nn * sizeof(double), cudaMemcpyHostToDevice, e->stream) != cudaSuccess)
     return -5;
@@ -1589,7 +1618,7 @@ int calchem_xc_evaluate_rks_points(uint64_t grid_id, int xc_code, int precision,
     exc_out[i] = h_res[2 * i];
     nelec_out[i] = h_res[2 * i + 1];
   }
-  return 0;
+  return copies.ok();
 }
 
 int calchem_xc_evaluate_uks(uint64_t grid_id, int xc_code, int precision, const double* h_pa, const double* h_pb,
@@ -1604,6 +1633,7 @@ int calchem_xc_evaluate_uks(uint64_t grid_id, int xc_code, int precision, const 
   if (int rc0 = ensure_ws(*e)) return rc0;
   const size_t nn = (size_t)e->nn_total;
   const int M = e->n_mols;
+  CopiesDone copies(e->stream);
   if (cudaMemcpyAsync(e->d_P, h_pa, nn * sizeof(double), cudaMemcpyHostToDevice, e->stream) != cudaSuccess ||
       cudaMemcpyAsync(e->d_Pb, h_pb, nn * sizeof(double), cudaMemcpyHostToDevice, e->stream) != cudaSuccess)
     return -5;
@@ -1622,7 +1652,7 @@ int calchem_xc_evaluate_uks(uint64_t grid_id, int xc_code, int precision, const 
     nelec_out[2 * i] = h_res[3 * i + 1];
     nelec_out[2 * i + 1] = h_res[3 * i + 2];
   }
-  return 0;
+  return copies.ok();
 }
 
 int calchem_xc_evaluate_rks_device(uint64_t grid_id, int xc_code, int precision, const double* d_total,
@@ -1734,6 +1764,7 @@ int calchem_xc_evaluate_rks_atoms(uint64_t grid_id, int xc_code, int precision, 
   if (!e->has_w) return -1;
   if (int rc0 = ensure_ws(*e)) return rc0;
   const size_t nn = (size_t)e->nn_total;
+  CopiesDone copies(e->stream);
   if (cudaMemcpyAsync(e->d_P, h_d_total, nn * sizeof(double), cudaMemcpyHostToDevice, e->stream) != cudaSuccess)
     return -5;
   int rc = enqueue_atom_shares(*e, xc_code, precision, e->d_P, e->d_res, h_v_out ? e->d_V : nullptr, e->d_atom_out,
@@ -1748,7 +1779,7 @@ int calchem_xc_evaluate_rks_atoms(uint64_t grid_id, int xc_code, int precision, 
   if ((rc = fetch(*e, h_atom_out, e->d_atom_out, 2 * (size_t)e->n_share_atoms))) return rc;
   *exc_out = h_res[0];
   *nelec_out = h_res[1];
-  return 0;
+  return copies.ok();
 }
 
 int calchem_xc_evaluate_rks_atoms_device(uint64_t grid_id, int xc_code, int precision, const double* d_total,
@@ -1774,6 +1805,7 @@ int calchem_xc_fxc_prepare(uint64_t grid_id, int xc_code, const double* h_d_tota
     return -4;
   }
   const size_t nn = (size_t)e->n_ao * e->n_ao;
+  CopiesDone copies(e->stream);
   if (cudaMemcpyAsync(e->d_P, h_d_total, nn * sizeof(double), cudaMemcpyHostToDevice, e->stream) != cudaSuccess)
     return -5;
   // The SIMT form's densities: once per ground state, so its speed matters little, while the kernel's finite
@@ -1787,7 +1819,7 @@ int calchem_xc_fxc_prepare(uint64_t grid_id, int xc_code, const double* h_d_tota
     return -5;
   if ((rc = finish(*e))) return rc;
   e->fxc_code = xc_code;
-  return 0;
+  return copies.ok();
 }
 
 int calchem_xc_fxc_contract_device(uint64_t grid_id, int triplet, const double* d_m, int n_trials, double* d_v_out,
@@ -1835,6 +1867,7 @@ int calchem_xc_fxc_contract_ex(uint64_t grid_id, int triplet, int precision, con
     }
     e->fxc_cap = n_trials;
   }
+  CopiesDone copies(e->stream);
   if (cudaMemcpyAsync(e->d_fxc_m, h_m, nn * n_trials * sizeof(double), cudaMemcpyHostToDevice, e->stream) !=
       cudaSuccess)
     return -5;
@@ -1843,8 +1876,9 @@ int calchem_xc_fxc_contract_ex(uint64_t grid_id, int triplet, int precision, con
                    ? enqueue_fxc_mixed(*e, triplet, e->d_fxc_m, n_trials, e->d_fxc_v, e->stream)
                    : enqueue_fxc(*e, triplet, e->d_fxc_m, n_trials, e->d_fxc_v, e->stream))
     return rc;
-  if (int rc = finish(*e)) return rc;
-  return fetch(*e, h_v_out, e->d_fxc_v, nn * n_trials);
+  int rc = finish(*e);
+  if (rc || (rc = fetch(*e, h_v_out, e->d_fxc_v, nn * n_trials))) return rc;
+  return copies.ok();
 }
 
 int calchem_xc_nuclear_gradient(uint64_t grid_id, int xc_code, int precision, int n_atoms, const int* z,

@@ -109,6 +109,21 @@ def check_outputs_stay_as_they_were_when_a_wait_expired(fake):
             assert np.array_equal(o, b), name
 
 
+def check_errors_leave_no_copy_under_way(fake):
+    """-5 from any copy, clear, launch or wait: nothing still reads or writes the caller's memory afterwards."""
+    for name, call, _ in host_calls():
+        assert call() == 0, name  # (scratch and caches are there)
+        for f in (b"cudaMemcpyAsync", b"cudaMemsetAsync", b"cudaLaunchKernel", b"cudaStreamSynchronize"):
+            for nth in range(1, 40):
+                fake.fake_fail(f, nth)
+                rc = call()
+                assert fake.fake_host_copies() == 0, (name, f, nth)
+                if rc == 0:
+                    break
+                assert rc == -5, (name, f, nth, rc)
+            fake.fake_fail(f, 0)
+
+
 CHECKS = {k[len("check_"):]: v for k, v in list(globals().items()) if k.startswith("check_")}
 
 if __name__ == "__main__":
