@@ -1497,12 +1497,13 @@ int calchem_xc_set_ao_cache(uint64_t grid_id, int enable, size_t* bytes_out) {
     if (bytes_out) *bytes_out = e->ao_cache.bytes;
     return 0;
   }
-  if (bytes_out) *bytes_out = 0;
-  const int want = enable ? 0 : 1;  // 0: allowed (decided at the next evaluation), 1: off
-  if (enable && e->ao_cache.state != 1 && e->f64_cache.state != 1) {  // already allowed
+  if (enable) {  // a cache that is off is decided again at its form's next evaluation; one that is there stays
+    for (AoCache* c : {&e->ao_cache, &e->f64_cache})
+      if (c->state == 1) c->state = 0;
     if (bytes_out) *bytes_out = e->ao_cache.bytes;
     return 0;
   }
+  if (bytes_out) *bytes_out = 0;
   // evaluations in flight on any stream may still read the cache
   if (cudaDeviceSynchronize() != cudaSuccess) return -5;
   if (e->graph) {  // a captured graph holds the cache pointers
@@ -1511,7 +1512,7 @@ int calchem_xc_set_ao_cache(uint64_t grid_id, int enable, size_t* bytes_out) {
   }
   for (AoCache* c : {&e->ao_cache, &e->f64_cache}) {
     ao_cache_free(*c);
-    c->state = want;
+    c->state = 1;
   }
   return 0;
 }

@@ -229,8 +229,8 @@ int calchem_xc_set_weights(uint64_t grid_id, const double* h_weights, int n_pts)
  * memory budget (memory_limit_bytes of its upload or group) and by the free device memory less
  * 1 GiB: the batches whose blocks fit within that limit, taken in batch order, are cached and the
  * others evaluate their AOs every time (the reference caches all or nothing).  enable = 0 waits for the device,
- * frees the cache, disables it and drops a captured graph; enable = 1 allows it again (a no-op when
- * allowed, the default); -1 only reports its size in *bytes_out (0 when none).  Results are the
+ * frees the cache, disables it and drops a captured graph; enable = 1 allows it again (a cache that is off is
+ * decided anew at the next evaluation; one that is there, and a captured graph, stay); -1 only reports its size in *bytes_out (0 when none).  Results are the
  * same with and without the cache.  The FP64 form keeps a cache of its own under the same switch, cap and
  * budget (FP64 planes and packed slices, 56 B per AO and point, within a quarter of the free device
  * memory); its size is not part of *bytes_out. */

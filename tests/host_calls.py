@@ -124,6 +124,35 @@ def check_errors_leave_no_copy_under_way(fake):
             fake.fake_fail(f, 0)
 
 
+def check_allowing_the_ao_cache_again_changes_nothing(fake):
+    """set_ao_cache(1) where the caller did not switch it off: what is cached or captured stays, also after the FP64
+    form found no room for a cache of its own; and that form asks again at its next evaluation."""
+    lib = _native.load()
+    _, basis, grid, P = molecule()
+    eng = RksVxcEngine(basis, grid, precision="mixed", tile=64)
+    eng.evaluate(basis, grid, "pbe", P)
+    size = eng.ao_cache_bytes()
+    assert size > 0
+    d = np.zeros(basis.n_ao ** 2 + 2)
+    _native.check("capture", lib.calchem_xc_graph_capture(eng.grid_id, 0, 2, 1, _native.ptr(d), None, _native.ptr(d),
+                                                          _native.ptr(d), None))
+    os.environ["CALCHEM_MAX_AO_GRID_BYTES"] = "0"
+    eng.evaluate(basis, grid, "pbe", P, precision="fp64")  # no cache
+    del os.environ["CALCHEM_MAX_AO_GRID_BYTES"]
+    used = fake.fake_used()
+    eng.set_ao_cache(True)
+    assert eng.ao_cache_bytes() == size and lib.calchem_xc_graph_launch(eng.grid_id, None) == 0
+    eng.evaluate(basis, grid, "pbe", P, precision="fp64")
+    assert fake.fake_used() > used and eng.ao_cache_bytes() == size
+    eng.set_ao_cache(False)
+    assert eng.ao_cache_bytes() == 0 and lib.calchem_xc_graph_launch(eng.grid_id, None) == -1
+    eng.evaluate(basis, grid, "pbe", P)
+    assert eng.ao_cache_bytes() == 0
+    eng.set_ao_cache(True)
+    eng.evaluate(basis, grid, "pbe", P)
+    assert eng.ao_cache_bytes() == size
+
+
 CHECKS = {k[len("check_"):]: v for k, v in list(globals().items()) if k.startswith("check_")}
 
 if __name__ == "__main__":
