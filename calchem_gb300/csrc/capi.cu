@@ -96,8 +96,8 @@ struct Entry {
   double* d_fxc_m = nullptr;        // trial matrices / results of host-buffer contractions
   double* d_fxc_v = nullptr;
   int fxc_cap = 0;                  // trial matrices d_fxc_m and d_fxc_v hold
-  // FP64 form on the tensor cores: scratch per CTA (0 CTAs: the budget or the batches' size leaves the
-  // SIMT form, launch_fp64)
+  // FP64 form on the tensor cores: scratch of its CTAs (nullptr: not used yet, or no room and the SIMT form,
+  // launch_fp64, runs)
   unsigned char* d_f64_slab = nullptr;
   size_t f64_slab_stride = 0;
   int f64_ctas = 0;
@@ -262,20 +262,6 @@ size_t workspace_bytes(const Entry& e) {
   return t;
 }
 
-// CTAs of the FP64 form on the tensor cores (two per SM) that fit the grid's budget beside `total` bytes.
-// The SIMT form (one CTA per SM, the scratch already counted) is kept instead where a batch has more AOs
-// than the kernel holds or where so few CTAs fit that it would be no slower: one CTA of this form works
-// ~5 times as fast as one of the SIMT form (C8H18, m ~ 150), and a factor 4 is asked for.
-void plan_f64tc(Entry& e, size_t& total, size_t mem_limit) {
-  e.f64_ctas = 0;
-  if (e.max_m > f64tc_max_m() || total > mem_limit) return;
-  e.f64_slab_stride = f64tc_slab_bytes(e.max_m);
-  const int n = (int)std::min<size_t>(std::min(e.n_batches, 2 * g_sm_count), (mem_limit - total) / e.f64_slab_stride);
-  if (n < 1 || 4 * n < e.n_ctas) return;
-  e.f64_ctas = n;
-  total += e.f64_slab_stride * n;
-}
-
 // Allocates the evaluation workspace on first use.  Uploads through calchem_xc_upload_points and
 // groups defer it, so that grids uploaded only to be grouped hold no workspace.
 int ensure_ws(Entry& e) {
@@ -357,7 +343,6 @@ int upload_impl(const AoShellGpu* h_shells, int n_shells, const AoPrimGpu* h_pri
   e->slab_stride = slab_stride;
   e->mixed_ctas = mixed_ctas;
   e->mixed_slab_stride = mixed_stride;
-  plan_f64tc(*e, total, mem_limit);
   e->bytes = total;
   e->n_prims = n_prims;
   e->n_comps = n_comps;
@@ -477,6 +462,12 @@ size_t ao_cache_cap() {
   return (size_t)32 << 30;
 }
 
+// What the grid's memory budget leaves beside its uploads and workspace (bytes) and what was allocated since.
+size_t budget_left(const Entry& e) {
+  const size_t used = e.bytes + e.ao_cache.bytes + e.f64_cache.bytes + e.f64_slab_stride * e.f64_ctas;
+  return e.mem_limit > used ? e.mem_limit - used : 0;
+}
+
 void ao_cache_free(AoCache& c) {
   if (c.d) cudaFree(c.d);
   if (c.d_off) cudaFree(c.d_off);
@@ -503,9 +494,7 @@ void ao_cache_decide(Entry& e, bool fp64, cudaStream_t st) {
   // the cache's limit: the cap, the grid's budget and the free device memory less 1 GiB; batches (in
   // batch order) whose blocks fit within it get one (offset -1: evaluated every time)
   const size_t reserve = (size_t)1 << 30;
-  const size_t used = e.bytes + e.ao_cache.bytes + e.f64_cache.bytes;
-  const size_t budget = e.mem_limit > used ? e.mem_limit - used : 0;  // within the grid's budget
-  size_t limit = std::min({ao_cache_cap(), budget, free_b > reserve ? free_b - reserve : (size_t)0});
+  size_t limit = std::min({ao_cache_cap(), budget_left(e), free_b > reserve ? free_b - reserve : (size_t)0});
   if (fp64) limit = std::min(limit, free_b / 4);
   std::vector<long long> off(e.n_batches, -1);
   size_t total = 0;
@@ -552,17 +541,31 @@ int mixed_launch_ctas(const Entry& e) {
 
 // Whether the FP64 form on the tensor cores runs for an evaluation on st: its scratch is allocated on first
 // use, but not inside a stream capture (calchem_xc_graph_capture asks before it begins), where the SIMT
-// form's scratch, there since the workspace was allocated, serves.
+// form's scratch, there since the workspace was allocated, serves.  Two CTAs per SM, as far as the grid's budget
+// and half of the free memory hold their scratch.  The SIMT form (one CTA per SM) runs instead where a batch has more
+// AOs than the kernel holds, or while so few CTAs fit that it would be no slower: one CTA of this form works ~5 times
+// as fast as one of the SIMT form (C8H18, m ~ 150), and a factor 4 is asked for.
 bool f64tc_ready(Entry& e, cudaStream_t st) {
-  if (e.f64_ctas <= 0) return false;
   if (e.d_f64_slab) return true;
+  if (e.max_m > f64tc_max_m()) return false;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return false;
-  if (cudaMalloc(&e.d_f64_slab, e.f64_slab_stride * e.f64_ctas) == cudaSuccess) return true;
-  cudaGetLastError();  // no room
-  e.d_f64_slab = nullptr;
-  e.f64_ctas = 0;
-  return false;
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  e.f64_slab_stride = f64tc_slab_bytes(e.max_m);
+  const int n = (int)std::min<size_t>(std::min(e.n_batches, 2 * g_sm_count),
+                                      std::min(budget_left(e), free_b / 2) / e.f64_slab_stride);
+  if (n < 1 || 4 * n < e.n_ctas) return false;
+  if (cudaMalloc(&e.d_f64_slab, e.f64_slab_stride * n) != cudaSuccess) {
+    cudaGetLastError();
+    e.d_f64_slab = nullptr;
+    return false;
+  }
+  e.f64_ctas = n;
+  return true;
 }
 
 // The densities' operand copies of a tensor-core form (fp64: vxc_f64tc.cu's fixed point, else vxc_mixed.cu's
@@ -1975,7 +1978,6 @@ int calchem_xc_group_create(const uint64_t* member_ids, int n_members, uint64_t 
     delete g;
     return -3;
   }
-  plan_f64tc(*g, total, memory_limit_bytes);
   g->bytes = total;
   auto fail = [&](int code) {
     cudaGetLastError();

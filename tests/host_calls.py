@@ -153,7 +153,81 @@ def check_allowing_the_ao_cache_again_changes_nothing(fake):
     assert eng.ao_cache_bytes() == size
 
 
+class Budgeted:
+    """The molecule uploaded with a memory budget; least() is the smallest that its upload accepts."""
+
+    ids = 10 ** 6
+
+    def __init__(self, limit):
+        self.lib = _native.load()
+        _, basis, grid, self.P = molecule()
+        sh, pr, co = basis.gpu_arrays()
+        Budgeted.ids += 1
+        self.id = Budgeted.ids
+        p = _native.ptr
+        self.rc = self.lib.calchem_xc_upload_points_spatial(p(sh), len(sh), p(pr), len(pr), p(co), len(co), p(grid.xyzw),
+                                                           len(grid), basis.n_ao, 128, self.id, int(limit))
+
+    @staticmethod
+    def least():
+        lo, hi = 0, 1 << 34
+        while hi - lo > 1:
+            mid = (lo + hi) // 2
+            b = Budgeted(mid)
+            lo, hi = (lo, mid) if b.rc == 0 else (mid, hi)
+            b.release()
+        return hi
+
+    def launches(self, precision):
+        """One evaluation: 3 launches on the tensor cores (prepare, quadrature, finish), 2 in the FP64 SIMT form."""
+        e, ne, v = np.zeros(1), np.zeros(2), np.zeros_like(self.P)
+        p = _native.ptr
+        _native.check("rks", self.lib.calchem_xc_evaluate_rks(self.id, 2, precision, p(self.P), p(e), p(ne), p(v)))
+        return self.lib.calchem_xc_last_launch_count(self.id)
+
+    def cache(self):
+        out = (ctypes.c_size_t * 1)()
+        _native.check("set_ao_cache", self.lib.calchem_xc_set_ao_cache(self.id, -1, out))
+        return int(out[0])
+
+    def release(self):
+        self.lib.calchem_cuda_vxc_release(self.id)
+
+
+def check_a_budget_is_charged_with_what_is_allocated(fake):
+    """A grid's memory budget: the tensor-core form's cache gets all that the workspace leaves as long as the FP64 form
+    has not been used, and that form takes its scratch from what is left then."""
+    least = Budgeted.least()
+    b = Budgeted(1 << 40)
+    assert b.launches(1) == 3
+    whole = b.cache()
+    assert whole > 0 and b.launches(0) == 3  # (no limit that matters: both forms on the tensor cores)
+    b.release()
+    b = Budgeted(least + whole)
+    assert b.launches(1) == 3 and b.cache() == whole
+    assert b.launches(0) == 2  # nothing left
+    b.release()
+    b = Budgeted(least + whole)
+    assert b.launches(0) == 3 and b.launches(1) == 3 and b.cache() < whole
+    b.release()
+    b = Budgeted(least)
+    assert b.launches(0) == 2 and b.launches(1) == 3 and b.cache() == 0
+    b.release()
+
+
+def check_the_fp64_form_asks_again_for_scratch(fake):
+    """Device memory too short for the tensor-core form's scratch is no decision for the grid's life."""
+    b = Budgeted(1 << 40)
+    b.launches(1)
+    fake.fake_set_memory(ctypes.c_size_t(fake.fake_used() + 4096))
+    assert b.launches(0) == 2
+    fake.fake_set_memory(ctypes.c_size_t(280 << 30))
+    assert b.launches(0) == 3
+
+
 CHECKS = {k[len("check_"):]: v for k, v in list(globals().items()) if k.startswith("check_")}
 
 if __name__ == "__main__":
-    CHECKS[sys.argv[2]](ctypes.CDLL(sys.argv[1]))
+    runtime = ctypes.CDLL(sys.argv[1])
+    runtime.fake_used.restype = ctypes.c_size_t
+    CHECKS[sys.argv[2]](runtime)
