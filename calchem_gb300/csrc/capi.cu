@@ -462,10 +462,25 @@ size_t ao_cache_cap() {
   return (size_t)32 << 30;
 }
 
-// What the grid's memory budget leaves beside its uploads and workspace (bytes) and what was allocated since.
+// What the grid holds of its memory budget: its uploads and workspace (bytes) and what was allocated since.
+size_t budget_used(const Entry& e) {
+  return e.bytes + e.ao_cache.bytes + e.f64_cache.bytes + e.f64_slab_stride * e.f64_ctas + e.grad_bytes;
+}
+
+void grad_arena_free(Entry& e) {
+  if (e.d_grad) cudaFree(e.d_grad);
+  e.d_grad = nullptr;
+  e.grad_bytes = 0;
+}
+
+// What the budget leaves to another buffer; the gradient's, which nothing reads between gradients, make room for it
+// (make_room, before it is allocated).
 size_t budget_left(const Entry& e) {
-  const size_t used = e.bytes + e.ao_cache.bytes + e.f64_cache.bytes + e.f64_slab_stride * e.f64_ctas;
+  const size_t used = budget_used(e) - e.grad_bytes;
   return e.mem_limit > used ? e.mem_limit - used : 0;
+}
+void make_room(Entry& e, size_t bytes) {
+  if (budget_used(e) + bytes > e.mem_limit) grad_arena_free(e);
 }
 
 void ao_cache_free(AoCache& c) {
@@ -505,6 +520,7 @@ void ao_cache_decide(Entry& e, bool fp64, cudaStream_t st) {
     total += bb;
   }
   if (total == 0) return;
+  make_room(e, total);
   const bool ok = cudaMalloc(&c.d, total) == cudaSuccess &&
                   cudaMalloc(&c.d_off, off.size() * sizeof(long long)) == cudaSuccess &&
                   cudaMalloc(&c.d_ok, (size_t)e.n_batches * sizeof(int)) == cudaSuccess &&
@@ -550,15 +566,16 @@ bool f64tc_ready(Entry& e, cudaStream_t st) {
   if (e.max_m > f64tc_max_m()) return false;
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return false;
+  e.f64_slab_stride = f64tc_slab_bytes(e.max_m);
+  const int most = std::min(e.n_batches, 2 * g_sm_count);
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
-  e.f64_slab_stride = f64tc_slab_bytes(e.max_m);
-  const int n = (int)std::min<size_t>(std::min(e.n_batches, 2 * g_sm_count),
-                                      std::min(budget_left(e), free_b / 2) / e.f64_slab_stride);
+  const int n = (int)std::min<size_t>(most, std::min(budget_left(e), free_b / 2) / e.f64_slab_stride);
   if (n < 1 || 4 * n < e.n_ctas) return false;
+  make_room(e, e.f64_slab_stride * n);
   if (cudaMalloc(&e.d_f64_slab, e.f64_slab_stride * n) != cudaSuccess) {
     cudaGetLastError();
     e.d_f64_slab = nullptr;
@@ -946,12 +963,10 @@ struct Arena {
 
 // The grid's gradient arena with at least `bytes`.  Allocating and freeing it on every call took 2 ms of an 11
 // ms gradient (0.7 GB of per-CTA scratch), so it is kept until the grid is released; grad_arena_trim gives
-// back one that holds more than a quarter of the free memory.
+// back one that the grid's budget does not hold or that takes more than a quarter of the free memory.
 bool grad_arena(Entry& e, size_t bytes) {
   if (e.grad_bytes >= bytes) return true;
-  if (e.d_grad) cudaFree(e.d_grad);
-  e.d_grad = nullptr;
-  e.grad_bytes = 0;
+  grad_arena_free(e);
   if (cudaMalloc(&e.d_grad, bytes) != cudaSuccess) {
     cudaGetLastError();
     e.d_grad = nullptr;
@@ -962,11 +977,10 @@ bool grad_arena(Entry& e, size_t bytes) {
 }
 void grad_arena_trim(Entry& e) {
   size_t free_b = 0, total_b = 0;
-  if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && e.grad_bytes <= free_b / 4) return;
+  if (cudaMemGetInfo(&free_b, &total_b) == cudaSuccess && e.grad_bytes <= free_b / 4 && budget_used(e) <= e.mem_limit)
+    return;
   cudaGetLastError();
-  cudaFree(e.d_grad);
-  e.d_grad = nullptr;
-  e.grad_bytes = 0;
+  grad_arena_free(e);
 }
 
 // Runs the gradient kernel on an uploaded single-molecule grid.  xc >= 0: fused form (h_raw and
@@ -1044,6 +1058,7 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
     }
   }
   const size_t nn = (size_t)n * n, na3 = 3 * (size_t)n_atoms;
+  if (e.grad_bytes > mem_limit) grad_arena_free(e);
   // the FP64 form's contractions run on the tensor cores where that kernel holds the batches and atoms
   bool f64tc = !mixed && grad_f64tc_fits(e.max_m, n_atoms);
   auto stride_of = [&](bool tc) {
@@ -1077,7 +1092,7 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
   if (fixed + least > mem_limit) return -3;
   if (f64tc && fixed + stride_of(true) * sizeof(double) > mem_limit) f64tc = false;
   const size_t slab_stride = stride_of(f64tc);
-  const int n_ctas = (int)std::max<size_t>(
+  int n_ctas = (int)std::max<size_t>(
       1, std::min<size_t>(ctas_of(2, slab_stride), (mem_limit - fixed) / (slab_stride * sizeof(double))));
   GradBufs B;
   auto lay_out = [&](void* base) {
@@ -1111,7 +1126,13 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
     }
     return m.off;
   };
-  if (!grad_arena(e, lay_out(nullptr))) return -4;
+  size_t need = lay_out(nullptr);
+  if (know_free && need > free_b + e.grad_bytes) {  // the rest of the buffers leaves the scratch less than half
+    const size_t cta = slab_stride * sizeof(double);
+    n_ctas = (int)std::max<long long>(1, n_ctas - (long long)((need - free_b - e.grad_bytes + cta - 1) / cta));
+    need = lay_out(nullptr);
+  }
+  if (!grad_arena(e, need)) return -4;
   lay_out(e.d_grad);
   struct Trim {
     Entry& e;

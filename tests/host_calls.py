@@ -190,6 +190,13 @@ class Budgeted:
         _native.check("set_ao_cache", self.lib.calchem_xc_set_ao_cache(self.id, -1, out))
         return int(out[0])
 
+    def gradient(self, precision):
+        mol, _, grid, P = molecule()
+        z, xyz, g = np.array(mol.z, dtype=np.int32), np.ascontiguousarray(mol.coords_bohr), np.zeros((3, 3))
+        p = _native.ptr
+        return self.lib.calchem_xc_nuclear_gradient(self.id, 2, precision, 3, p(z), p(xyz), p(grid.raw_weight),
+                                                    p(grid.host_atom), len(grid), p(P), None, p(g))
+
     def release(self):
         self.lib.calchem_cuda_vxc_release(self.id)
 
@@ -223,6 +230,70 @@ def check_the_fp64_form_asks_again_for_scratch(fake):
     assert b.launches(0) == 2
     fake.fake_set_memory(ctypes.c_size_t(280 << 30))
     assert b.launches(0) == 3
+
+
+def check_a_gradients_buffers_stay_within_the_budget(fake):
+    """They are kept for the next gradient where the grid's budget holds them, given back where it does not, and never
+    keep a cache or another form's scratch from what it would get without them."""
+    least = Budgeted.least()
+    for precision in (0, 1):
+        b = Budgeted(1 << 40)
+        b.launches(1)
+        whole = b.cache()
+        before = fake.fake_used()
+        assert b.gradient(precision) == 0
+        kept = fake.fake_used() - before
+        assert kept > 0
+        n = fake.fake_calls(b"cudaMalloc")
+        assert b.gradient(precision) == 0 and fake.fake_calls(b"cudaMalloc") == n
+        b.release()
+
+        b = Budgeted(least + whole)  # (the buffers are kept only where the limit allows it)
+        b.launches(1)
+        assert b.cache() == whole
+        before = fake.fake_used()
+        assert b.gradient(precision) == 0
+        assert fake.fake_used() - before < 20000  # (the order of the points stays: 4 B each)
+        b.release()
+
+        b = Budgeted(least + max(whole, kept))
+        assert b.gradient(precision) == 0  # first, into the budget that the cache asks for next
+        assert b.launches(1) == 3 and b.cache() == whole
+        b.release()
+
+
+def check_a_force_call_keeps_no_more_than_its_limit(fake):
+    """calchem_cuda_vxc_grad_force: neither its own buffers nor those of a gradient before it take more device memory
+    than the limit it is given, and the limit it refuses does not depend on them."""
+    lib = _native.load()
+    mol, basis, grid, P = molecule()
+    d, wq = dropin(basis, grid)
+    w, f = np.zeros((d.n_pts, 8)), np.zeros((3, 3))
+    p = _native.ptr
+
+    def force(limit):
+        return lib.calchem_cuda_vxc_grad_force(d.grid_id, p(P), p(P), 1, p(w), p(f), d.n_pts, basis.n_ao, 3,
+                                               ctypes.c_size_t(limit))
+
+    def least():
+        lo, hi = 1, 1 << 34
+        while hi - lo > 1:
+            mid = (lo + hi) // 2
+            rc = force(mid)
+            assert rc in (0, -3)
+            lo, hi = (lo, mid) if rc == 0 else (mid, hi)
+        return hi
+    empty = fake.fake_used()
+    limit = least()
+    assert fake.fake_used() - empty <= limit + 20 * 1024  # (each of some twenty buffers starts on a multiple of 1 KB)
+    _native.check("weights", lib.calchem_xc_set_weights(d.grid_id, p(wq), len(wq)))
+    z, xyz = np.array(mol.z, dtype=np.int32), np.ascontiguousarray(mol.coords_bohr)
+    host = np.zeros(d.n_pts, np.int32)
+    assert lib.calchem_xc_nuclear_gradient(d.grid_id, 2, 1, 3, p(z), p(xyz), p(wq), p(host), d.n_pts, p(P), None,
+                                           p(f)) == 0
+    assert fake.fake_used() - empty > limit + 20 * 1024
+    assert least() == limit
+    assert fake.fake_used() - empty <= limit + 20 * 1024
 
 
 CHECKS = {k[len("check_"):]: v for k, v in list(globals().items()) if k.startswith("check_")}
