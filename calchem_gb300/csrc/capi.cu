@@ -103,6 +103,7 @@ struct Entry {
   int f64_ctas = 0;
   AoCache ao_cache;   // of the tensor-core form (vxc_mixed.cu)
   AoCache f64_cache;  // of the FP64 form (vxc_f64tc.cu)
+  bool captured = false;  // a graph holds the FP64 form's scratch and cache
   // per-atom share sums (calchem_xc_set_point_atoms): planned point indices grouped by host atom
   int n_share_atoms = 0;
   int* d_atom_pts = nullptr;
@@ -163,10 +164,19 @@ bool mul_ok(size_t a, size_t b, size_t* out) {
   return true;
 }
 
+// Device memory that a call cannot do without.  Where there is none left, the grids give back what they hold
+// beyond their uploads and workspaces.
+bool yield_memory();
+bool device_alloc(void** p, size_t bytes) {
+  if (cudaMalloc(p, bytes) == cudaSuccess) return true;
+  cudaGetLastError();
+  return yield_memory() && cudaMalloc(p, bytes) == cudaSuccess;
+}
+
 template <typename T>
 bool dalloc(T** p, size_t count) {
   if (count == 0) count = 1;
-  return cudaMalloc((void**)p, count * sizeof(T)) == cudaSuccess;
+  return device_alloc((void**)p, count * sizeof(T));
 }
 
 // Waits for what the legacy stream was given: a device memset, and the last part of a copy from pageable memory, may
@@ -271,7 +281,7 @@ int ensure_ws(Entry& e) {
             (e.n_mols != 1 || dalloc(&e.d_rg, (size_t)e.n_pts * 4)) && dalloc(&e.d_red, (size_t)e.n_batches * 3) &&
             dalloc(&e.d_res, 3 * (size_t)e.n_mols + 8) &&
             dalloc(&e.d_slab, e.slab_stride * e.n_ctas) &&
-            cudaMalloc(&e.d_mixed_ws, nn * sizeof(uint2) * 2 + (size_t)e.n_ao * 2 * sizeof(int)) == cudaSuccess &&
+            device_alloc(&e.d_mixed_ws, nn * sizeof(uint2) * 2 + (size_t)e.n_ao * 2 * sizeof(int)) &&
             dalloc(&e.d_mixed_slab, e.mixed_slab_stride * e.mixed_ctas) &&
             cudaMallocHost((void**)&e.h_stage, (3 * (size_t)e.n_mols + 8) * sizeof(double)) == cudaSuccess &&
             cudaStreamCreateWithFlags(&e.stream, cudaStreamNonBlocking) == cudaSuccess;
@@ -490,13 +500,36 @@ void ao_cache_free(AoCache& c) {
   c = AoCache();
 }
 
+// The FP64 form's scratch and cache (unless a graph holds them) and the gradient's buffers of every grid.  False:
+// there were none, or work in flight could not be waited for.
+bool yield_memory() {
+  auto holds = [](const Entry& e) {
+    return e.grad_bytes || (!e.captured && (e.d_f64_slab || e.f64_cache.state == 2));
+  };
+  if (std::none_of(g_grids.begin(), g_grids.end(), [&](const auto& g) { return holds(*g.second); })) return false;
+  if (cudaDeviceSynchronize() != cudaSuccess) {  // evaluations on any stream may use them
+    cudaGetLastError();
+    return false;
+  }
+  for (auto& g : g_grids) {
+    Entry& e = *g.second;
+    grad_arena_free(e);
+    if (e.captured) continue;
+    if (e.d_f64_slab) cudaFree(e.d_f64_slab);
+    e.d_f64_slab = nullptr;
+    e.f64_ctas = 0;
+    if (e.f64_cache.state == 2) ao_cache_free(e.f64_cache);
+  }
+  return true;
+}
+
 // Decides and allocates a form's AO cache on its first evaluation, whose stream is st (not inside a stream
 // capture: callers that capture decide first).  The per-batch AO values and gradients depend only on
 // the grid and basis, so CalChem's engine computes them once per geometry and reuses them every
 // SCF iteration (vxc.rs:386-394, 600-716); here the cache also holds the packed GEMM1 operand and
 // the row exponents.  Off when the blocks exceed the cap or the free device memory (minus 1 GiB).  The
-// FP64 form's cache (`fp64`) also stays within a quarter of the free memory: its blocks are 56 B per AO and
-// point, and a program may hold many FP64 engines.
+// FP64 form's cache (`fp64`) also stays within a quarter of the free memory and, with those of other grids, within
+// half of the device's: its blocks are 56 B per AO and point, and a program may hold many FP64 engines.
 void ao_cache_decide(Entry& e, bool fp64, cudaStream_t st) {
   AoCache& c = fp64 ? e.f64_cache : e.ao_cache;
   if (c.state != 0) return;
@@ -510,7 +543,11 @@ void ao_cache_decide(Entry& e, bool fp64, cudaStream_t st) {
   // batch order) whose blocks fit within it get one (offset -1: evaluated every time)
   const size_t reserve = (size_t)1 << 30;
   size_t limit = std::min({ao_cache_cap(), budget_left(e), free_b > reserve ? free_b - reserve : (size_t)0});
-  if (fp64) limit = std::min(limit, free_b / 4);
+  if (fp64) {
+    size_t held = 0;
+    for (const auto& g : g_grids) held += g.second->f64_cache.bytes;
+    limit = std::min({limit, free_b / 4, tot_b / 2 > held ? tot_b / 2 - held : (size_t)0});
+  }
   std::vector<long long> off(e.n_batches, -1);
   size_t total = 0;
   for (int b = 0; b < e.n_batches; ++b) {
@@ -543,6 +580,8 @@ void use_ao_cache(Entry& e, bool fp64, cudaStream_t st, EvalArgs& A) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone)
     ao_cache_decide(e, fp64, st);
+  else if (fp64)
+    e.captured = true;  // (with the scratch of the same launch)
   const AoCache& c = fp64 ? e.f64_cache : e.ao_cache;
   if (c.state != 2) return;
   A.ao_cache = c.d;
@@ -967,7 +1006,7 @@ struct Arena {
 bool grad_arena(Entry& e, size_t bytes) {
   if (e.grad_bytes >= bytes) return true;
   grad_arena_free(e);
-  if (cudaMalloc(&e.d_grad, bytes) != cudaSuccess) {
+  if (!device_alloc(&e.d_grad, bytes)) {
     cudaGetLastError();
     e.d_grad = nullptr;
     return false;
@@ -1560,7 +1599,10 @@ int calchem_xc_eval_closed_shell(int xc_code, int precision, int n, const double
     return -1;
   if (!device_ok()) return -3;
   double* d = nullptr;
-  if (cudaMalloc(&d, (size_t)n * 5 * sizeof(double)) != cudaSuccess) return -4;
+  if (!dalloc(&d, (size_t)n * 5)) {
+    cudaGetLastError();
+    return -4;
+  }
   double* d_rho = d;
   double* d_gam = d + n;
   double* d_out = d + 2 * (size_t)n;

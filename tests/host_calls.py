@@ -296,6 +296,42 @@ def check_a_force_call_keeps_no_more_than_its_limit(fake):
     assert fake.fake_used() - empty <= limit + 20 * 1024
 
 
+def check_kept_memory_makes_way_for_what_a_call_needs(fake):
+    """As many grids fit the device as their uploads and workspaces allow: caches, scratch and gradient buffers that
+    were allocated where there was room are given back when there is none, except those that a graph holds."""
+    lib = _native.load()
+    os.environ["CALCHEM_MAX_AO_GRID_BYTES"] = "0"
+    b = Budgeted(1 << 40)
+    before = fake.fake_used()
+    b.release()
+    empty = fake.fake_used()
+    b = Budgeted(1 << 40)
+    b.launches(1)  # (uses the workspace, and nothing else without a cache)
+    each = fake.fake_used() - empty
+    assert before - empty < each
+    b.release()
+    del os.environ["CALCHEM_MAX_AO_GRID_BYTES"]
+    many = 30
+    fake.fake_set_memory(ctypes.c_size_t(empty + many * each + (32 << 20)))
+    first = Budgeted(1 << 40)
+    assert first.launches(0) == 3
+    d = np.zeros_like(first.P)
+    p = _native.ptr
+    _native.check("capture", lib.calchem_xc_graph_capture(first.id, 0, 2, 0, p(d), None, p(d), p(d), None))
+    held = fake.fake_used() - empty
+    assert each < held < each + (32 << 20)
+    rest = []
+    for _ in range(many - 1):
+        rest.append(Budgeted(1 << 40))
+        assert rest[-1].rc == 0
+        assert rest[-1].launches(0) in (2, 3) and rest[-1].launches(1) == 3
+        assert rest[-1].gradient(0) == 0
+    assert all(r.launches(0) in (2, 3) for r in rest)
+    n = fake.fake_calls(b"cudaMalloc")
+    assert first.launches(0) == 3 and lib.calchem_xc_graph_launch(first.id, None) == 0
+    assert fake.fake_calls(b"cudaMalloc") == n  # the graph's grid kept its own
+
+
 CHECKS = {k[len("check_"):]: v for k, v in list(globals().items()) if k.startswith("check_")}
 
 if __name__ == "__main__":
