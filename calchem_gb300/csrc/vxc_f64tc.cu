@@ -255,6 +255,7 @@ __global__ void __launch_bounds__(kT, 2) vxc_f64tc_kernel(DevGrid G, EvalArgs A)
       const bool on = live && !(rho[0] < 1e-18);
       const double gam = gx[0] * gx[0] + gy[0] * gy[0] + gz[0] * gz[0];
       if (on) part = xc_eval_cs(A.xc, 0.5 * rho[0], 0.25 * gam, h ? 2 : 1);
+      part.f += rho[0] - rho[0];  // (NaN where a density row holds infinities or NaN, which the functional drops)
       if (h == 1) {
         dens[1][0][g] = part.f;
         dens[1][1][g] = part.vr;
@@ -308,14 +309,14 @@ __global__ void __launch_bounds__(kT, 2) vxc_f64tc_kernel(DevGrid G, EvalArgs A)
           coef[3][g] = w * (kc[3] * gz[0] + gc * c[2]);
         }
       } else {
-        const double ra = fmax(rho[0], 0.0), rb = fmax(rho[1], 0.0);
+        const double ra = rho[0] < 0.0 ? 0.0 : rho[0], rb = rho[1] < 0.0 ? 0.0 : rho[1];  // (NaN stays)
         if (live && !(ra + rb < 1e-18)) {
           const double w = G.pw[pt];
           const double gaa = gx[0] * gx[0] + gy[0] * gy[0] + gz[0] * gz[0];
           const double gab = gx[0] * gx[1] + gy[0] * gy[1] + gz[0] * gz[1];
           const double gbb = gx[1] * gx[1] + gy[1] * gy[1] + gz[1] * gz[1];
           const XcVal o = xc_eval(A.xc, ra, rb, gaa, gab, gbb);
-          e_loc = w * o.f;
+          e_loc = w * (o.f + (ra - ra) + (rb - rb));
           na_loc = w * ra;
           nb_loc = w * rb;
           coef[0][g] = 0.5 * w * o.vra;

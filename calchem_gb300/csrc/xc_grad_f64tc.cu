@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(kT, 2) xc_grad_f64tc_kernel(DevGrid G, GradArg
       double fx = 0.0;
       if (fused) {
         const int o = A.closed ? 0 : 1;
-        const double ra = fmax(rho[0], 0.0), rb = fmax(rho[o], 0.0);
+        const double ra = rho[0] < 0.0 ? 0.0 : rho[0], rb = rho[o] < 0.0 ? 0.0 : rho[o];  // (NaN stays)
         if (live && !(ra + rb < 1e-18)) {
           const double gaa = gx[0] * gx[0] + gy[0] * gy[0] + gz[0] * gz[0];
           const double gab = gx[0] * gx[o] + gy[0] * gy[o] + gz[0] * gz[o];
@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(kT, 2) xc_grad_f64tc_kernel(DevGrid G, GradArg
             coef[6][g] = w * (2.0 * v.vgbb * gy[o] + v.vgab * gy[0]);
             coef[7][g] = w * (2.0 * v.vgbb * gz[o] + v.vgab * gz[0]);
           }
-          fx = v.f;
+          fx = v.f + (ra - ra) + (rb - rb);
         }
         if (live && A.fx_out) A.fx_out[pt] = fx;
       }

@@ -1,6 +1,6 @@
 """The FP64 forms on either side of the rules that choose between the tensor cores (vxc_f64tc.cu, xc_grad_f64tc.cu) and
 the SIMT kernels (vxc_fp64.cu, xc_grad.cu): atom and AO counts where the gradient changes over, memory budgets that
-leave no room for the tensor-core form's scratch, and rows of widely differing entries.
+leave no room for the tensor-core form's scratch, numbers that are not finite, and rows of widely differing entries.
 
 Error of an integer-slice product (f64_slices.cuh), per term and relative to the product of the two operand rows'
 largest entries: 2 x 2^-53 from rounding the operands to 53 bits at their row's largest entry; 20 x 2^-54 at most from
@@ -129,6 +129,44 @@ def test_budget_without_room_for_the_scratch(water):
         a, b = simt.fxc(P, trials, triplet), tc.fxc(P, trials, triplet)
         assert (simt.launches(), tc.launches()) == (1 + len(trials), 3 * len(trials))
         assert close(a, b) and np.array_equal(b, b.transpose(0, 2, 1))
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+def test_numbers_that_are_not_finite(water, bad):
+    """They show in the results wherever the SIMT form's show them, and the next call's results are clean."""
+    basis, _, simt, tc = water
+    n = basis.n_ao
+    P = make_positive_density(n, 7)
+    B = P.copy()
+    B[3, 5] = B[5, 3] = bad
+    wv = np.random.default_rng(4).normal(size=(tc.grid.n_pts, 4))
+    wb = wv.copy()
+    wb[200] = bad
+    calls = {"rks": lambda g, p, w: g.evaluate(p), "uks": lambda g, p, w: g.evaluate(P, p),
+             "uks alpha": lambda g, p, w: g.evaluate(p, P), "rho": lambda g, p, w: (g.grid.eval_rho_grad(p),),
+             "accum": lambda g, p, w: (g.grid.accumulate_vxc(w),)}
+    for name, call in calls.items():
+        bad_simt, bad_tc = call(simt, B, wb), call(tc, B, wb)
+        assert not all(np.all(np.isfinite(x)) for x in bad_tc), name
+        for a, b in zip(bad_simt, bad_tc):
+            assert np.all(np.isfinite(a) | ~np.isfinite(b)), name
+        assert all(np.all(np.isfinite(x)) for x in call(tc, P, wv)), name
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
+@pytest.mark.parametrize("closed", [True, False])
+def test_gradient_of_a_density_that_is_not_finite(native_lib, bad, closed):
+    """Every component: each atom's weight derivative takes in every point."""
+    mol = distorted_water()
+    basis = BasisSet.from_name("6-31g(d)", mol)
+    grid = scattered(mol, 500, 3)
+    P = make_positive_density(basis.n_ao, 7)
+    B = P.copy()
+    B[3, 5] = B[5, 3] = bad
+    eng = RksVxcEngine(basis, grid)
+    assert not np.any(np.isfinite(eng.nuclear_gradient(mol, grid, "b3lyp", B, None if closed else P)))
+    assert np.all(np.isfinite(eng.nuclear_gradient(mol, grid, "b3lyp", P, None if closed else P)))
+    eng.close()
 
 
 def aos(ob, layout):
