@@ -1130,7 +1130,7 @@ int gradient_run(Entry& e, int xc, int precision, bool closed, const double* h_p
   const size_t least = simt * ctas_of(mixed ? 2 : 1, simt) * sizeof(double);
   if (fixed + least > mem_limit) return -3;
   if (f64tc && fixed + stride_of(true) * sizeof(double) > mem_limit) f64tc = false;
-  const size_t slab_stride = stride_of(f64tc);
+  const size_t slab_stride = std::max<size_t>(stride_of(f64tc), 1);  // (0 AOs in every batch: no scratch)
   int n_ctas = (int)std::max<size_t>(
       1, std::min<size_t>(ctas_of(2, slab_stride), (mem_limit - fixed) / (slab_stride * sizeof(double))));
   GradBufs B;

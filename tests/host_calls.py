@@ -332,6 +332,34 @@ def check_kept_memory_makes_way_for_what_a_call_needs(fake):
     assert fake.fake_calls(b"cudaMalloc") == n  # the graph's grid kept its own
 
 
+def nothing_reached(basis):
+    """A reference-layout upload whose points all are in batches without candidate shells."""
+    pts = np.zeros(300, dtype=_native.GRID_PT)
+    pts["x"] = 300.0
+    pts["batch_id"] = np.arange(300) // 100
+    off = np.array([0, 0, 0, 0, 1], np.int32)
+    return GpuVxcGrid.upload(*basis.gpu_arrays(), pts, off, np.zeros(1, np.int32), basis.n_ao)
+
+
+def check_a_grid_that_no_shell_reaches(fake):
+    """Every call on it succeeds (each in a process that a division by zero would end)."""
+    lib = _native.load()
+    mol, basis, _, P = molecule()
+    g = nothing_reached(basis)
+    n, p = basis.n_ao, _native.ptr
+    g.eval_rho_grad(P)
+    g.accumulate_vxc(np.ones((300, 4)))
+    g.eval_grad_force(P, P, True, np.ones((300, 8)), 3)
+    w, host, f = np.ones(300), np.zeros(300, np.int32), np.zeros((3, 3))
+    _native.check("weights", lib.calchem_xc_set_weights(g.grid_id, p(w), 300))
+    z, xyz = np.array(mol.z, dtype=np.int32), np.ascontiguousarray(mol.coords_bohr)
+    e, ne, v = np.zeros(1), np.zeros(2), np.zeros((n, n))
+    for precision in (0, 1):
+        assert lib.calchem_xc_evaluate_rks(g.grid_id, 2, precision, p(P), p(e), p(ne), p(v)) == 0
+        assert lib.calchem_xc_nuclear_gradient(g.grid_id, 2, precision, 3, p(z), p(xyz), p(w), p(host), 300, p(P), None,
+                                               p(f)) == 0
+
+
 CHECKS = {k[len("check_"):]: v for k, v in list(globals().items()) if k.startswith("check_")}
 
 if __name__ == "__main__":

@@ -129,3 +129,25 @@ def test_shares_alone_over_cached_batches(native_lib):
                 eng.grid_id, 3, code, _native.ptr(P), _native.ptr(e), _native.ptr(ne), _native.ptr(out), None))
             assert e[0] == exc and np.array_equal(out[0::2], ea) and np.array_equal(out[1::2], ta)
         eng.close()
+
+
+def test_grid_that_no_shell_reaches(native_lib):
+    """Every batch's candidate list empty: zeros throughout."""
+    from tests.host_calls import nothing_reached
+    mol = distorted_water()
+    basis = BasisSet.from_name("6-31g(d)", mol)
+    P = make_positive_density(basis.n_ao, 7)
+    g = nothing_reached(basis)
+    assert not np.any(g.eval_rho_grad(P)) and not np.any(g.accumulate_vxc(np.ones((300, 4))))
+    assert not np.any(g.eval_grad_force(P, P, True, np.ones((300, 8)), 3))
+    w, host, f = np.ones(300), np.zeros(300, np.int32), np.ones((3, 3))
+    p = _native.ptr
+    _native.check("weights", native_lib.calchem_xc_set_weights(g.grid_id, p(w), 300))
+    for Pb in (None, P):
+        assert not any(np.any(x) for x in evaluate(g, P, Pb))
+    z, xyz = np.array(mol.z, dtype=np.int32), np.ascontiguousarray(mol.coords_bohr)
+    for precision in (0, 1):
+        _native.check("gradient", native_lib.calchem_xc_nuclear_gradient(
+            g.grid_id, 2, precision, 3, p(z), p(xyz), p(w), p(host), 300, p(P), None, p(f)))
+        assert not np.any(f)
+    g.release()
