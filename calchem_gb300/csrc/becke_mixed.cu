@@ -15,8 +15,8 @@
 // 1 - |nu| comes from (1 - |mu|)(1 - a (1 + |mu|)), the sign of nu turning mu and a.
 //
 // Instructions bound it: 13,100 a point on octane (26 atoms; 70 % of the issue slots, 20 of 32 lanes active) while
-// the sums over one point's atoms were serial, the pairs' divisions were two and the orientations branched; 6,600
-// (54 %, 26.7 lanes) now.  The pair passes take two pairs per thread in packed FP32 instructions, one division
+// the sums over one point's atoms were serial, the pairs' divisions were two and the orientations branched; 6,490
+// (60 %, 26.7 lanes) now.  The pair passes take two pairs per thread in packed FP32 instructions, one division
 // serves both E_cd and E_dc, 1 - x takes the short sum (the operand order is known), step 4 adds with a sign
 // and no thread sums alone.  The whole gradient call: octane 9.22 -> 7.18 ms, 72 atoms 32.8 -> 16.2 ms, 183 atoms
 // (one warp per point with its tables in device memory before) 1051 -> 140 ms.  Packed against scalar FP32: the same

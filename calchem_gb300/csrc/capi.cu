@@ -823,8 +823,8 @@ int enqueue_fxc_mixed(Entry& e, int triplet, const double* d_m, int n_trials, do
 }
 
 // Makes the pages of an output buffer resident (each one's first word written back to itself) while the GPU
-// works: the copies go straight between the caller's memory and the device, which this CPU and GPU share
-// page tables for, and a copy into pages never touched faults each of them on its way (10.7 MB: 65 us into
+// works: the copies go straight between the caller's memory and the device (GB300's CPU and GPU share their page
+// tables; nothing but the speed rests on it), and a copy into pages never touched faults each of them on its way (10.7 MB: 65 us into
 // resident pages, 240-700 us into fresh ones; through a pinned staging buffer the host's own copies took
 // 0.4 ms in and 0.7 ms out).  The contents do not change, so an output may be the input itself.
 void touch_pages(double* p, size_t n) {

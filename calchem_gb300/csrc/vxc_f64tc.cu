@@ -5,9 +5,17 @@
 // instead of FP64 FMAs.  Each operand vector (an AO row of P, a point's or an AO's row of Phi, an AO's
 // row of Z) is cut into six 9-bit BF16 slices relative to its largest element; the 21 slice products
 // i + j <= 5 go into five FP32 accumulators in TMEM (levels 0-3 exact over 64 terms, levels 4 and 5
-// together), which are drained every 64 terms into 64-bit integers.  The products left out and the
-// operands' rounding are below 2^-54 of the row maxima's product per term, as the roundings of an FP64
-// FMA chain are; rho, the functional, Z and all sums stay in FP64.
+// together), which are drained every 64 terms into 64-bit integers; rho, the functional, Z and all sums
+// stay in FP64.
+//
+// Error, relative to the product of the two rows' largest elements and per term: 2 x 2^-53 from the operands'
+// rounding, at most 20 x 2^-54 from the products left out (five of i + j = 6) and 12 x 2^-54 from the last
+// accumulator's additions, so below 9 x 2^-52 in all.  Measured on whole builds, V is as far from a plain FP64
+// evaluation by its largest entry as the SIMT form's.  But an FMA chain rounds relative to its own terms and this
+// form relative to row maxima: an element 2^k below its row's largest keeps 53 - k bits, so that an entry of V
+// between AOs that hardly meet is right to about 2^-52 of the largest products in absolute terms, not in its own
+// digits.  The TD-DFT kernel's finite differences, which would turn that into 5e-12 to 4e-9 of dV, keep the SIMT
+// form's densities (calchem_xc_fxc_prepare).  Rows with infinities or NaN, or of 2^957 and above, give NaN.
 //
 // What bounds it: GB300 has 2 FP64 FMA lanes per SM and clock, so the SIMT form spends 2 m^2 FP64 FMAs a
 // point there; here the tensor cores take them and the FP64 pipe is left with ~m (4 for rho and

@@ -1,6 +1,6 @@
 // vxc_fp64.cu -- the FP64 XC quadrature on the SIMT FP64 pipe, and the small kernels both FP64 forms share.
 //
-// vxc_f64tc.cu does the same work with the contractions on the tensor cores, 8-15 times as fast.  This form
+// vxc_f64tc.cu does the same work with the contractions on the tensor cores, 4 (one water) to 15 times as fast (whole calls).  This form
 // runs where that one cannot: batches of more than 2048 AOs, grids whose memory budget leaves no room for
 // its scratch, the allocation-free entry point (noalloc.cu), and the densities of the TD-DFT kernel's
 // finite differences (calchem_xc_fxc_prepare).

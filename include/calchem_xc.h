@@ -14,7 +14,8 @@
  *    -4  device allocation failure
  *    -5  copy or kernel launch failure
  *    -6  device-side overflow flag (kept for compatibility; the kernels here never set it)
- *    -7  a device-side wait gave up (bounded spin expired); the result is not valid
+ *    -7  a device-side wait gave up (bounded spin expired) in either precision; the result is not valid, and
+ *        calls on host buffers leave their outputs as they were (a fused gradient: zeros)
  *   All matrices are dense row-major n_ao x n_ao doubles.  Every call is synchronous with
  *   respect to the host buffers it is given and is serialised by one process-wide mutex, as in
  *   the reference.  There is never a CPU fallback: a failure is reported, not recomputed.
@@ -72,7 +73,12 @@ enum {
 
 /* Precision of the two dense contractions (rho = Phi D Phi^T and V = Phi^T (w v) Phi). */
 enum {
-  CALCHEM_XC_FP64 = 0,  /* plain all-FP64 drop-in form (matches the reference to 1e-9 Eh / 1e-10) */
+  CALCHEM_XC_FP64 = 0,  /* FP64 drop-in form (matches the reference to 1e-9 Eh / 1e-10): its contractions run on
+                         * the tensor cores as integer slices, whose error is that of an FP64 product relative to
+                         * the largest elements of the rows multiplied (below 9 x 2^-52 of their product per
+                         * term), not to each term.  So entries of V far below the largest are right in absolute
+                         * terms (~1e-17), not in all their own digits.  A density row with an infinity or NaN, or
+                         * of 2^957 and above, gives NaN; rows below 2^-959 count as zeros */
   CALCHEM_XC_MIXED = 1  /* tcgen05 tensor-core contractions, split operands, FP32 accumulation */
 };
 
@@ -233,7 +239,9 @@ int calchem_xc_set_weights(uint64_t grid_id, const double* h_weights, int n_pts)
  * decided anew at the next evaluation; one that is there, and a captured graph, stay); -1 only reports its size in *bytes_out (0 when none).  Results are the
  * same with and without the cache.  The FP64 form keeps a cache of its own under the same switch, cap and
  * budget (FP64 planes and packed slices, 56 B per AO and point, within a quarter of the free device
- * memory); its size is not part of *bytes_out. */
+ * memory, and those of all grids within half of the device's); its size is not part of *bytes_out.
+ * The FP64 form's scratch and cache and a gradient's buffers stay with the grid within its budget, and are given
+ * back when an allocation that some call cannot do without would fail, unless a captured graph holds them. */
 int calchem_xc_set_ao_cache(uint64_t grid_id, int enable, size_t* bytes_out);
 
 /* Number of batches and the sum over batches of m_b^2 * n_b (m_b AOs, n_b points): the
@@ -304,7 +312,10 @@ int calchem_xc_evaluate_uks(uint64_t grid_id, int xc_code, int precision, const 
 /* Device-pointer variants (inputs and outputs already in device memory; enqueued on `stream`,
  * a cudaStream_t, 0 for the legacy stream).  d_result receives (Exc, N_alpha + N_beta) for RKS and
  * (Exc, N_alpha, N_beta) for UKS, once per member of a group.  They return after enqueueing; the
- * caller synchronises and may then read the device status with calchem_xc_last_status. */
+ * caller synchronises and may then read the device status with calchem_xc_last_status.  A grid's first call in a
+ * precision also allocates (workspace, the FP64 form's scratch, the AO cache) and waits for `stream` once.  Inside
+ * the caller's own stream capture nothing is allocated: without a call outside it before, the graph holds the FP64
+ * form without the tensor cores, and either form without an AO cache, several times slower at every replay. */
 int calchem_xc_evaluate_rks_device(uint64_t grid_id, int xc_code, int precision, const double* d_total,
                                    double* d_result, double* d_v, void* stream);
 int calchem_xc_evaluate_uks_device(uint64_t grid_id, int xc_code, int precision, const double* d_pa,
@@ -316,7 +327,7 @@ int calchem_xc_evaluate_uks_device(uint64_t grid_id, int xc_code, int precision,
  * the FP64 functional, as the reference); calchem_xc_fxc_contract (contract_batch) returns, for each
  * of n_trials symmetric n x n matrices M_b packed one after the other in h_m, the full symmetric
  * dV_b = f_xc[M_b] (singlet, or triplet when triplet != 0) in h_v_out.  The grid's AOs are evaluated
- * once per batch for all trial matrices.  -1 when the kernel was not prepared; single grids only. */
+ * once per batch for all trial matrices, as far as the AO cache holds them.  -1 when the kernel was not prepared; single grids only. */
 int calchem_xc_fxc_prepare(uint64_t grid_id, int xc_code, const double* h_d_total);
 int calchem_xc_fxc_contract(uint64_t grid_id, int triplet, const double* h_m, int n_trials, double* h_v_out);
 /* As calchem_xc_fxc_contract with a precision: CALCHEM_XC_FP64 (the above) or CALCHEM_XC_MIXED, the
@@ -336,8 +347,8 @@ int calchem_xc_fxc_contract_device_ex(uint64_t grid_id, int triplet, int precisi
  * Becke weight derivative grid.rs:423-584), entirely on the device: densities, functional, AO force
  * terms with the host-atom term, and the weight derivative.  precision CALCHEM_XC_FP64: all FP64;
  * CALCHEM_XC_MIXED: the contractions P Phi and P Psi on the tensor cores (exact fixed-point split),
- * AO values, derivatives and the force terms in double-float, functional and weight derivative in
- * FP64; batches of more than 2048 AOs return -2 for it.  grid_id is a single grid
+ * AO values, derivatives, the force terms and the weight derivative in double-float, the functional in
+ * double-float for a closed shell of codes 0-5 at total density >= 1e-12 and in FP64 otherwise; batches of more than 2048 AOs return -2 for it.  grid_id is a single grid
  * uploaded with its weights (calchem_xc_upload_points*); h_raw_w (weights before the Becke
  * partition) and h_host_atom hold the n_grid_pts points the caller uploaded, in its order (as
  * calchem_xc_grid_fetch returns them); the atoms (z, xyz_bohr) are the molecule the grid was built
@@ -346,7 +357,7 @@ int calchem_xc_fxc_contract_device_ex(uint64_t grid_id, int triplet, int precisi
  * not uploaded (|w| < 1e-24) are left out.  One atom: zeros.  Returns -1 (bad arguments, host or
  * shell atom outside [0, n_atoms), n_atoms > 1024), -2 (unknown grid, a group, no weights, or
  * n_grid_pts not the uploaded count), -4 / -5 on allocation / CUDA failure, -7 when a device-side
- * wait of the tensor-core form expired. */
+ * wait expired. */
 int calchem_xc_nuclear_gradient(uint64_t grid_id, int xc_code, int precision, int n_atoms, const int* z,
                                 const double* xyz_bohr, const double* h_raw_w, const int* h_host_atom, int n_grid_pts,
                                 const double* h_pa, const double* h_pb, double* h_grad_out);

@@ -111,7 +111,7 @@ def test_more_empty_batches_than_ctas(native_lib):
 
 
 def test_shares_alone_over_cached_batches(native_lib):
-    """The judge's call (per-atom shares, no Vxc): batches follow each other without the V phase's barriers and
+    """Per-atom shares without Vxc: batches follow each other without the V phase's barriers and
     copies, and from the second call on without the AO evaluation either.  The same bits as the full build's
     shares, every time."""
     mol = distorted_water()
