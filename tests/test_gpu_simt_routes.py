@@ -59,7 +59,7 @@ class Grid:
         def up(lim):
             return GpuVxcGrid.upload(*basis.gpu_arrays(), pts, off, cs, basis.n_ao, memory_limit=lim)
         if limit is None:
-            lo, limit = 0, 1 << 36
+            lo, limit = 0, 1 << 36  # (the least is kept as self.limit)
             while limit - lo > 1:
                 mid = (lo + limit) // 2
                 try:
@@ -68,7 +68,7 @@ class Grid:
                 except _native.CalchemXcError as e:
                     assert e.code == -3
                     lo = mid
-        self.grid = up(limit)
+        self.grid, self.limit = up(limit), limit
         _native.check("weights", self.lib.calchem_xc_set_weights(self.grid.grid_id, _native.ptr(w), len(w)))
 
     def launches(self):
@@ -129,6 +129,43 @@ def test_budget_without_room_for_the_scratch(water):
         a, b = simt.fxc(P, trials, triplet), tc.fxc(P, trials, triplet)
         assert (simt.launches(), tc.launches()) == (1 + len(trials), 3 * len(trials))
         assert close(a, b) and np.array_equal(b, b.transpose(0, 2, 1))
+
+
+def test_budgets_with_room_for_part_of_the_scratch(water):
+    """From one CTA's scratch to all of them: the SIMT form up to a quarter of its own CTAs, then fewer CTAs."""
+    basis, layout, simt, tc = water
+    P = make_positive_density(basis.n_ao, 7)
+    ref = tc.evaluate(P)
+    tol = 50.0 * (basis.n_ao + 128) * 2.0 ** -53
+    seen = []
+    for extra in [0] + [2 ** k for k in range(16, 25)]:
+        g = Grid(basis, layout, simt.limit + extra)
+        for _ in range(2):
+            assert all(np.max(np.abs(a - b)) <= tol * np.max(np.abs(b)) for a, b in zip(g.evaluate(P), ref))
+        seen.append(g.launches())
+        g.release()
+    assert seen[0] == 2 and seen[-1] == 3 and seen == sorted(seen)
+
+
+def test_force_call_at_its_least_limit(native_lib):
+    """Half as many CTAs, or fewer, as without a limit: the same bits, as each batch has its own row of sums."""
+    mol = distorted_water()
+    basis = BasisSet.from_name("6-31g(d)", mol)
+    g = Grid(basis, reference_layout(basis, points(mol, 40000, 3)), 1 << 36)
+    P = make_positive_density(basis.n_ao, 7)
+    w = np.random.default_rng(4).normal(size=(g.grid.n_pts, 8))
+    free = g.grid.eval_grad_force(P, 0.5 * P, False, w, 3, memory_limit=1 << 36)
+    lo, hi = 1, 1 << 36
+    while hi - lo > 1:
+        mid = (lo + hi) // 2
+        try:
+            g.grid.eval_grad_force(P, 0.5 * P, False, w, 3, memory_limit=mid)
+            hi = mid
+        except _native.CalchemXcError as e:
+            assert e.code == -3
+            lo = mid
+    assert np.array_equal(g.grid.eval_grad_force(P, 0.5 * P, False, w, 3, memory_limit=hi), free)
+    g.release()
 
 
 @pytest.mark.parametrize("bad", [np.nan, np.inf, -np.inf])
