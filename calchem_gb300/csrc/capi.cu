@@ -168,7 +168,8 @@ bool mul_ok(size_t a, size_t b, size_t* out) {
 // beyond their uploads and workspaces.
 bool yield_memory();
 bool device_alloc(void** p, size_t bytes) {
-  if (cudaMalloc(p, bytes) == cudaSuccess) return true;
+  const cudaError_t err = cudaMalloc(p, bytes);
+  if (err != cudaErrorMemoryAllocation) return err == cudaSuccess;
   cudaGetLastError();
   return yield_memory() && cudaMalloc(p, bytes) == cudaSuccess;
 }
@@ -606,14 +607,18 @@ bool f64tc_ready(Entry& e, cudaStream_t st) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) return false;
   e.f64_slab_stride = f64tc_slab_bytes(e.max_m);
-  const int most = std::min(e.n_batches, 2 * g_sm_count);
+  int n = std::min(e.n_batches, 2 * g_sm_count);
+  auto enough = [&](size_t bytes) {
+    n = (int)std::min<size_t>(n, bytes / e.f64_slab_stride);
+    return n >= 1 && 4 * n >= e.n_ctas;
+  };
+  if (!enough(budget_left(e))) return false;
   size_t free_b = 0, total_b = 0;
   if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
-  const int n = (int)std::min<size_t>(most, std::min(budget_left(e), free_b / 2) / e.f64_slab_stride);
-  if (n < 1 || 4 * n < e.n_ctas) return false;
+  if (!enough(free_b / 2)) return false;
   make_room(e, e.f64_slab_stride * n);
   if (cudaMalloc(&e.d_f64_slab, e.f64_slab_stride * n) != cudaSuccess) {
     cudaGetLastError();
